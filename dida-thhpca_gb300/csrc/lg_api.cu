@@ -428,6 +428,7 @@ int upload(lg_ctx* c, const T* h, size_t n, const T** out) {
 int ensure_hx(lg_ctx* c, size_t entries) {
   if (entries <= c->hx_entries_cap && c->hx.yb) return LG_OK;
   dfree(c->hx.yb); dfree(c->hx.yb32); dfree(c->hx.dis); dfree(c->hx.lnp); dfree(c->hx.rdiag);
+  dfree(c->hx.yexp);
   c->hx_entries_cap = 0;  // until every buffer of the new size exists
   const size_t cap = entries + 1;
   const size_t k = (size_t)c->cfg.ens;
@@ -437,6 +438,8 @@ int ensure_hx(lg_ctx* c, size_t entries) {
   r |= dalloc(&c->hx.dis, cap);
   r |= dalloc(&c->hx.lnp, cap);
   r |= dalloc(&c->hx.rdiag, cap);
+  if (c->cfg.precision == LG_PREC_FP64 && lg::gram64_tc_supported(c->cfg.ens))
+    r |= dalloc(&c->hx.yexp, cap);
   if (r != LG_OK) return LG_ERR_NOMEM;
   c->hx_entries_cap = cap;
   return LG_OK;
@@ -1400,6 +1403,10 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
   CK(record_event(c->ev[5], st));
   CK(cudaStreamWaitEvent(st, c->ev_hx, 0));
   const bool mixed_tc = lg::mixed_precision(g.precision) && lg::gram_tc_supported(k);
+  if (c->hx.yexp) {
+    lg::launch_row_exponents(k, c->obs.n_entries, c->hx.yb, c->hx.yexp, st);
+    launches += 1;
+  }
   lg::RecDev rec{};
   if (mixed_tc) {
     const int nb = c->tune.lnp_buckets;
@@ -1455,7 +1462,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
       else if (mixed_tc)
         lg::launch_gram_tc_stream(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, rec, st);
       else
-        lg::launch_gram64(geo, c->hx, c->lists, b, axb, L.C, L.t, st);
+        lg::launch_gram64(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, st);
       CK(record_event(kv[1], st));
       CK(record_event(kv[2], st));
       if (cube_trans_fp32(c)) {
@@ -1570,7 +1577,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
     else if (mixed_tc)
       lg::launch_gram_tc(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, s_g, &rec);
     else
-      lg::launch_gram64(geo, c->hx, c->lists, b, axb, L.C, L.t, s_g);
+      lg::launch_gram64(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, s_g);
     CK(cudaMemsetAsync(L.ovf_n, 0, sizeof(int), s_g));
     CK(record_event(kv[1], s_g));
     if (nl >= 3) {
@@ -2262,6 +2269,7 @@ void lg_destroy(lg_ctx* c) {
   dfree(c->d_glat); dfree(c->d_glon); dfree(c->d_ca); dfree(c->d_cb); dfree(c->d_blk);
   dfree(c->d_lat_block); dfree(c->d_lon_block); dfree(c->d_nb_off); dfree(c->d_nb_blk);
   dfree(c->hx.yb); dfree(c->hx.yb32); dfree(c->hx.dis); dfree(c->hx.lnp); dfree(c->hx.rdiag);
+  dfree(c->hx.yexp);
   dfree(c->lists.cnt); dfree(c->lists.off); dfree(c->lists.ent); dfree(c->lists.rloc);
   dfree(c->lists.capped);
   if (c->d_scan_tmp) cudaFree(c->d_scan_tmp);
@@ -2326,7 +2334,7 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   else if (precision == LG_PREC_MIXED && lg::gram_tc_supported(ens))
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
   else
-    lg::launch_gram64(geo, hx, l, b, nullptr, C, t, st);
+    lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
   lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail, st);
   int h_fail = 0;
   if (cudaGetLastError() != cudaSuccess ||

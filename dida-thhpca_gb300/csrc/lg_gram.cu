@@ -18,18 +18,6 @@ namespace lg {
 constexpr int kTE = 32;        // entries per tile
 constexpr int kGramThreads = 256;
 
-__device__ inline double alnp_level(const Geometry& g, int kk, double aps) {
-  // ps2alnp (obs_make.F90:418-437), with ph_lev(nz+1) evaluated
-  auto lev = [&](int k1) {
-    if (g.vcoord == LG_VCOORD_SIGMA)
-      return __dadd_rn(__dmul_rn(g.ca[k1 - 1], __dsub_rn(aps, g.ptop)), g.ptop);
-    const double t1 = __dmul_rn(g.ca[k1 - 1], __dsub_rn(g.p0, g.ptop));
-    const double t2 = __dmul_rn(g.cb[k1 - 1], __dsub_rn(aps, g.ptop));
-    return __dadd_rn(__dadd_rn(t1, t2), g.ptop);
-  };
-  return log(__dmul_rn(0.5, __dadd_rn(lev(kk), lev(kk + 1))));
-}
-
 // Thread roles.  The lower triangle of C is cut into 4 x 4 register blocks
 // (NB = nb (nb + 1) / 2 of them, nb = ceil(k / 4)).  With NB <= 256 the
 // threads form G = floor(256 / NB) groups, each owning every block, and group
@@ -42,9 +30,8 @@ __device__ inline double alnp_level(const Geometry& g, int kk, double aps) {
 template <int kMaxBlk>
 __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
     gram64_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, const double* axb,
-                  double* Cout, double* tout) {
+                  double* Cout, double* tout, int marked) {
   constexpr int kQueueCap = kTE + kGramThreads;
-  const int s = blockIdx.x;
   const int k = g.ens;
   const int kp = (k + 3) & ~3;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -58,6 +45,17 @@ __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
   __shared__ int q_n;
   __shared__ double s_al;
 
+  // marked = 0: block s does solve s.  marked = 1 (after gram64_tc_kernel):
+  // block i looks at solves 256 i .. 256 i + 255 and does those that kernel
+  // left to this one.
+  int s = marked ? (int)blockIdx.x * kGramThreads : (int)blockIdx.x;
+  const int s_end = marked ? min(b.nsolves, s + kGramThreads) : s + 1;
+  const auto is_marked = [&](int i) {
+    return (unsigned long long)__double_as_longlong(Cout[(size_t)i * k * k]) == kGramMark;
+  };
+  if (marked && !__syncthreads_or(s + tid < s_end && is_marked(s + tid))) return;
+  for (; s < s_end; ++s) {
+  if (marked && !is_marked(s)) continue;  // the same word for every thread
   int64_t base = 0;
   int p = 0;
   int col = 0, kk = 1;
@@ -239,11 +237,18 @@ __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
   }
   if (tid < k) tout[(size_t)s * k + tid] = tacc;
   if (b.work && tid == 0) atomicAdd(b.work, (unsigned long long)nproc);
+  __syncthreads();
+  }  // solves of this block
 }
 
 void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
-                   const double* axb, double* C, double* t, cudaStream_t stream) {
+                   const double* axb, double* C, double* t, int* err, cudaStream_t stream) {
   if (b.nsolves == 0) return;
+  // up to 64 members: exact slices on the tensor cores, then the solves they
+  // cannot hold (non-finite or extreme values) here
+  const int marked = gram64_tc_supported(g.ens) && (b.mode == 1 || hx.yexp) ? 1 : 0;
+  if (marked) launch_gram64_tc(g, hx, l, b, axb, C, t, err, stream);
+  const int grid = marked ? (b.nsolves + kGramThreads - 1) / kGramThreads : b.nsolves;
   const int kp = (g.ens + 3) & ~3;
   const int nb = kp / 4;
   const int NB = nb * (nb + 1) / 2;
@@ -253,9 +258,9 @@ void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const S
     const size_t red = sizeof(double) * (size_t)(G - 1) * NB * 16;
     const size_t smem = std::max(tile, red);
     cudaFuncSetAttribute(gram64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gram64_kernel<1><<<b.nsolves, kGramThreads, smem, stream>>>(g, hx, l, b, axb, C, t);
+    gram64_kernel<1><<<grid, kGramThreads, smem, stream>>>(g, hx, l, b, axb, C, t, marked);
   } else {
-    gram64_kernel<3><<<b.nsolves, kGramThreads, tile, stream>>>(g, hx, l, b, axb, C, t);
+    gram64_kernel<3><<<grid, kGramThreads, tile, stream>>>(g, hx, l, b, axb, C, t, marked);
   }
 }
 

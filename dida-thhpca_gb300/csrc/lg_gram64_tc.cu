@@ -1,0 +1,815 @@
+// lg_gram64_tc.cu -- FP64 weighted Gram matrices of up to 64 members on the
+// 5th-generation tensor cores, by exact integer slices.
+//
+// Same quantities as lg_gram.cu (letkf_core.F90:58-75,146-195):
+//   z_e = y_e rr_e,  rr_e = sqrt(rdiaginv(e) rloc_k(e)),  d~_e = rr_e d_e
+//   C = sum_e z_e z_e^T,   t = sum_e z_e d~_e
+//
+// Why: the FP64 pipe of this GPU multiplies 2 lanes per cycle per SM, so the
+// k(k+1)/2 products of one 64-member entry take about 1040 cycles of an SM, and
+// the plain FP64 Gram (gram64_kernel) was 80 to 95 % of a plain-FP64 analysis.
+// Here each z_ei is rounded once to a 53-bit integer Z relative to the largest
+// |z| of the chunk (below a power of two 2^S), and Z is cut into six signed
+// 9-bit digits,
+//   z = 2^(S-53) Z,   Z = sum_a d_a 2^(45-9a),   -256 <= d_a <= 256,
+// which are exact in FP16.  A product of digits has at most 16 bits and a
+// tcgen05.mma accumulator holds 24 exactly, so the FP32 sums of up to 256
+// entries are exact integers; they are combined in 64-bit integers.  Pairs of
+// slices (a, b) with a + b >= 7 (below 2^-63 of the largest product) are left
+// out, and of the rest only one of (a, b) and (b, a) is formed (C is symmetric).
+// Slices lie in shared memory as [zero 5 0 1 3 2 4], 64 rows each, so that two
+// neighbours make one M = 128 operand (rows "first | second"):
+//   block 0   A = [5;0] x B = [0]              50 | 00
+//   1..4      A = [0;1] x B = [1 3 2 4]        01 03 02 04 | 11 13 12 14
+//   5         A = [3;2] x B = [3]              33 | 23
+//   6         A = [2;4] x B = [2], + [zero;5] x [1]   22 | 42 + 51
+//   d~        A = [5;0], [1;3], [2;4] x B = the six slices of d~ (N = 16)
+// 448 + 48 of the 512 tensor-memory columns.  An element's error is about
+// 2^-54 of the chunk's largest |z| times |z| per entry, adding up as a random
+// walk; a chain of FP64 additions loses 2^-53 of the partial sum at each.
+//
+// One persistent CTA per SM (the accumulators fill tensor memory), 20 warps in
+// three roles that work on neighbouring chunks of up to 1536 entries.  Seven
+// warps drop the candidates whose vertical weight cannot be non-zero by an
+// integer compare of |ln p - ln p_e|, queue the others in list order, and weigh
+// the queue densely (the only FP64 work, some 35 instructions per kept entry).
+// Twelve warps convert 64 entries at a time by integer arithmetic into one of
+// two operand buffers, take finished sums out of tensor memory and write C and
+// t.  One warp issues the MMAs (a converting warp that issued them was late for
+// its next stage by the MMAs' own time, 2500 cycles).  The rows' largest values
+// and the levels' ln p come from small kernels before this one.
+//
+// Measured alone (one stream), against gram64_kernel: 921 600 solves of 40
+// members with 379 kept entries each (of 1562 candidates) 727 -> 128 ms;
+// 129 600 solves of 64 members with 954 kept entries 595 -> 58 ms; 82 944
+// solves of 40 members with 24 entries 5.6 -> 4.1 ms; 2592 of 16 members with
+// 51 entries 0.18 -> 0.10 ms.  It wins at every size measured, so up to 64
+// members (the tensor-memory columns' limit) every solve comes here.  Bound by
+// the converting warps: some 50 instructions per element at three warps per
+// scheduler, then taking the sums out (once per 256 entries).
+//
+// A solve with a non-finite weight, row or innovation, or with magnitudes
+// outside 2^+-400, is marked by a bit pattern in its first Gram element that no
+// other solve can produce, and redone by gram64_kernel.
+#include "lg_device.cuh"
+#include "lg_internal.h"
+#include "lg_tc.cuh"
+
+namespace lg {
+namespace g64 {
+
+constexpr int kPWarps = 7, kXWarps = 12;              // weighing; converting and adding up
+constexpr int kMmaWarp = kPWarps;                     // issues the MMAs
+constexpr int kX0 = kMmaWarp + 1;                     // first converting warp (a multiple of 4)
+constexpr int kPThreads = 32 * kPWarps, kXThreads = 32 * kXWarps;
+constexpr int kThreads = 32 * (kX0 + kXWarps);
+constexpr int kStage = 64;                            // entries per stage (4 K = 16 chunks)
+constexpr int kSlice = 64 * 16 * 2;                   // 2048 B: 64 rows x K = 16 FP16
+constexpr int kTileD = 7 * kSlice;                    // the d~ tile after zero and six slices
+constexpr int kChunkBytes = kTileD + 16 * 16 * 2;
+constexpr int kStageBytes = 4 * kChunkBytes;          // 59392 B
+constexpr int kQueue = 1536;                          // entries of a chunk (one scale)
+constexpr int kPer = 4;                               // candidates per thread and refill
+constexpr int kRefill = kPer * kPThreads;
+constexpr int kGroup = 4;                             // stages per exact FP32 sum (256 entries)
+constexpr int kQueueBytes = kQueue * (16 + 8);
+constexpr int kSmem = 2 * kStageBytes + 2 * kQueueBytes + 64 * 65 * 8;
+// C's exact sums are kept in units of 2^-51 of the largest product times 2^-1:
+// twice the sum of 1536 products stays below 2^63
+constexpr int kDrop = 10;
+// named barriers: the converting and the weighing warps' own; queue full and
+// queue empty, operand buffer converted (two each); tensor memory drained
+constexpr int kBarX = 1, kBarP = 2, kBarFull = 3, kBarEmpty = 5, kBarStage = 7, kBarDrain = 9;
+constexpr int kXMma = kXThreads + 32;
+constexpr int kTmemCols = 512;
+constexpr int kColD = 448;                            // first column of the d~ products
+constexpr int kExLimit = 400;
+
+constexpr long long bias() {  // 256 in every digit
+  long long b = 0;
+  for (int j = 0; j < 6; ++j) b += 256ll << (9 * j);
+  return b;
+}
+
+// kind::f16, FP16 A/B, FP32 D, K-major, M = 128, N
+__host__ __device__ constexpr uint32_t idesc(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+
+__device__ inline void mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t id, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(da), "l"(db), "r"(id), "r"(acc));
+}
+
+// eight consecutive accumulator columns of this thread's lane (no wait)
+__device__ inline void tmem_ld8(uint32_t taddr, float* v) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ inline void tmem_ld4(uint32_t taddr, float* v) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ inline void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ inline void bar_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ inline void bar_arrive(int id, int count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+// v 2^ex rounded to nearest-even
+__device__ inline double fixed_to_double(long long v, int ex) {
+  if (v == 0) return 0.0;
+  const bool neg = v < 0;
+  const unsigned long long m = neg ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int z = __clzll((long long)m);
+  unsigned long long mant;
+  if (z >= 11) {
+    mant = m << (z - 11);
+  } else {
+    const int drop = 11 - z;
+    mant = m >> drop;
+    const unsigned long long rest = m << (64 - drop);
+    mant += (rest > 0x8000000000000000ull || (rest == 0x8000000000000000ull && (mant & 1))) ? 1 : 0;
+  }
+  const unsigned long long bits = ((unsigned long long)(63 - z + ex + 1023 - 1) << 52) + mant;
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
+// (hi 2^27 + lo) 2^ex rounded to nearest-even
+__device__ inline double wide_to_double(long long hi, long long lo, int ex) {
+  __int128 v = ((__int128)hi << 27) + lo;
+  if (v == 0) return 0.0;
+  const bool neg = v < 0;
+  unsigned __int128 m = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
+  const unsigned long long mh = (unsigned long long)(m >> 64), ml = (unsigned long long)m;
+  const int p = mh ? 127 - __clzll((long long)mh) : 63 - __clzll((long long)ml);
+  unsigned long long mant;
+  if (p <= 52) {
+    mant = ml << (52 - p);
+  } else {
+    const int drop = p - 52;
+    mant = (unsigned long long)(m >> drop);
+    const unsigned __int128 rest = m & (((unsigned __int128)1 << drop) - 1);
+    const unsigned __int128 half = (unsigned __int128)1 << (drop - 1);
+    if (rest > half || (rest == half && (mant & 1))) ++mant;  // may carry into the exponent
+  }
+  const unsigned long long bits = ((unsigned long long)(p + ex + 1023 - 1) << 52) + mant;
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
+// 32 (Z + bias) and the sign of one element: y (bit pattern) times the entry's
+// weight mantissa.  par: (R >> 29, R & (2^29 - 1), shift base, entry) with rr =
+// R 2^(er - 1080), R < 2^58.  Y = |y| 2^(58 + ...) at the chunk's scale: the
+// shift base is the row's largest biased exponent plus how far the row's bound
+// lies below the chunk's, so Y R / 2^58 = 32 |Z| + at most two units.  The
+// digits are those of |Z| (9 bits each from bit 5 on: three in each 32-bit
+// word); the sign is applied to them in FP16.
+__device__ inline unsigned long long digits_of(unsigned hi, unsigned lo, const int4& par) {
+  const int e = (int)((hi << 1) >> 21);
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  const int sh = min(par.z - e, 63);
+  const unsigned long long Y = ((((unsigned long long)mh << 32) | lo) << 6) >> sh;
+  const unsigned yh = (unsigned)(Y >> 29), yl = (unsigned)Y & 0x1fffffffu;
+  const unsigned rh = (unsigned)par.x, rl = (unsigned)par.y;
+  unsigned long long mid = (unsigned long long)yl * rh + (1ull << 28);
+  mid += (unsigned long long)yh * rl;
+  return (unsigned long long)yh * rh + (16ull + ((unsigned long long)bias() << 5)) +
+         (unsigned)(mid >> 29);
+}
+
+// the digit pairs of two neighbouring entries as packed FP16, slice a = 0..5;
+// hi0, hi1: words whose top bits are the two signs
+__device__ inline void digit_pairs(unsigned long long z0, unsigned long long z1, unsigned hi0,
+                                   unsigned hi1, uint32_t* out) {
+  const unsigned a0 = (unsigned)z0, b0 = (unsigned)z1;
+  const unsigned a1 = (unsigned)(z0 >> 32), b1 = (unsigned)(z1 >> 32);
+  // u + 1024 in FP16 is 0x6400 | u for u < 1024; minus 1280 leaves the signed
+  // digit: +-1 (u + 1024) -+ 1280, both exact
+  const unsigned sg = ((hi0 >> 16) & 0x8000u) | (hi1 & 0x80000000u);
+  const uint32_t one = sg | 0x3c003c00u, off = sg ^ 0xe500e500u;
+  auto pack = [&](unsigned x, unsigned y, unsigned mask) -> uint32_t {
+    const unsigned t = (x & (mask & 0xffffu)) | 0x64006400u;
+    const unsigned h = (y & (mask & 0xffff0000u)) | t;
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(h), "r"(one), "r"(off));
+    return r;
+  };
+  out[5] = pack(a0 >> 5, b0 << 11, 0x01ff01ffu);
+  out[4] = pack(a0 >> 14, b0 << 2, 0x01ff01ffu);
+  out[3] = pack(a0 >> 23, b0 >> 7, 0x01ff01ffu);
+  out[2] = pack(a1, b1 << 16, 0x01ff01ffu);
+  out[1] = pack(a1 >> 9, b1 << 7, 0x01ff01ffu);
+  out[0] = pack(a1 >> 18, b1 >> 2, 0x03ff03ffu);
+}
+// memory position of slice a in [zero 5 0 1 3 2 4]
+__host__ __device__ constexpr int slice_pos(int a) {
+  return a == 5 ? 1 : a == 0 ? 2 : a == 1 ? 3 : a == 3 ? 4 : a == 2 ? 5 : 6;
+}
+
+// Gaspari-Cohn as schr2 (lg_device.cuh) without its divisions: the same
+// polynomial with fused multiply-adds, 1/12 rounded once and 1/ri by two
+// Newton steps from the hardware approximation; agrees to a few ulp of 1.
+__device__ inline double taper_fast(double ri) {
+  if (ri > 2.0) return 0.0;
+  if (ri > 1.0) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ri));
+    r = fma(r, fma(-ri, r, 1.0), r);
+    r = fma(r, fma(-ri, r, 1.0), r);
+    double t = fma(ri, 1.0 / 12.0, -0.5);
+    t = fma(t, ri, 0.625);
+    t = fma(t, ri, (double)1.666667f);
+    t = fma(t, ri, -5.0);
+    t = fma(t, ri, 4.0);
+    return fma(-(double)0.6666667f, r, t);
+  }
+  if (ri > 0.0) {
+    const double t = fma(fma(-0.25, ri, 0.5), ri, 0.625);
+    return fma(fma(t, ri, -(double)1.666667f), ri * ri, 1.0);
+  }
+  return 1.0;
+}
+
+}  // namespace g64
+
+// High word of the largest |y| of each H(x) row: its biased exponent from bit 20
+// on (0: all zero; 2047: a non-finite value), the leading mantissa bits below.
+__global__ void row_exponent_kernel(int ens, int64_t rows, const double* yb, int* yexp) {
+  const int64_t r = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const int lane = threadIdx.x & 31;
+  unsigned e = 0;
+  for (int i = lane; i < ens; i += 32)
+    e = max(e, (unsigned)__double2hiint(yb[(size_t)r * ens + i]) & 0x7fffffffu);
+  e = __reduce_max_sync(0xffffffffu, e);
+  if (lane == 0) yexp[r] = (int)e;
+}
+
+void launch_row_exponents(int ens, int64_t rows, const double* yb, int* yexp,
+                          cudaStream_t stream) {
+  if (rows == 0) return;
+  row_exponent_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(ens, rows, yb, yexp);
+}
+
+// ln p of each solve's level into the first element of its t (which
+// gram64_tc_kernel reads before it writes t)
+__global__ void level_lnp_kernel(Geometry g, SolveBatch b, const double* axb, double* t) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= b.nsolves) return;
+  int col, kk;
+  solve_col_level(b, s, col, kk);
+  const int glat = col % g.num_lat + 1, glon = col / g.num_lat + 1;
+  const size_t ci = (size_t)(glat - 1 + g.halo) +
+                    (size_t)(g.num_lat + 2 * g.halo) * (size_t)(glon - 1 + g.halo);
+  t[(size_t)s * g.ens] = alnp_level(g, kk, axb[g.ps_row + (size_t)g.n * ci]);
+}
+
+// what the weighing warps tell the converting ones about a queue
+struct QueueHead {
+  int s;         // solve, < 0: no more
+  int stages;    // stages of kStage entries (0: nothing with weight)
+  int S, Sd;     // |z| < 2^S, |d~| < 2^Sd
+  int first;     // the solve's first chunk: C and t are written, else added to
+  int bad;       // leave the solve to gram64_kernel
+};
+
+// kR: units (member, 4 entries) of a stage per converting thread -- 2 up to 48
+// members, 3 above -- and with it the columns of a warp quadruple (8 kR)
+template <int kR>
+__global__ void __launch_bounds__(g64::kThreads, 1)
+    gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, double* Cout, double* tout,
+                     int* err) {
+  using namespace g64;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ uint64_t mbar[2];
+  __shared__ uint32_t tmem_base_sh;
+  __shared__ int s_wcnt[2][kPWarps];
+  __shared__ longlong2 s_t[2][64];
+  __shared__ int s_kmax, s_dmax, s_nf;
+  __shared__ QueueHead s_head[2];
+
+  const int k = g.ens;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool batch = b.mode == 1;
+  // the zero slices of the two operand buffers
+  auto zero_blocks = [&](int t, int nt) {
+    for (int i = t; i < 8 * kSlice / 16; i += nt)
+      *reinterpret_cast<uint4*>(smem_raw + (i / (kSlice / 16)) * kChunkBytes +
+                                i % (kSlice / 16) * 16) = make_uint4(0, 0, 0, 0);
+  };
+  if (tid == 0) {
+    tc::mbar_init(&mbar[0], 1);
+    tc::mbar_init(&mbar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  zero_blocks(tid, kThreads);
+  tc::fence_proxy_async();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc::smem_u32(&tmem_base_sh)),
+                 "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_base_sh;
+  auto q_par = [&](int qb) {
+    return reinterpret_cast<int4*>(smem_raw + 2 * kStageBytes + qb * kQueueBytes);
+  };
+  auto q_d = [&](int qb) { return reinterpret_cast<long long*>(q_par(qb) + kQueue); };
+
+  if (warp < kX0) {
+  // registers: 256 x 48 + 384 x 128 within the launch's 640 x 96
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+  if (warp < kPWarps) {
+    // ================= weighing warps
+    const bool vertical = !batch && g.vert_dist > 0.0;
+    // |al - ln p| beyond this (one part in 2^50 above 2 vert_dist) has z > 2, so
+    // weight zero; compared on the bit pattern, a NaN stays a candidate
+    const long long lim_bits =
+        __double_as_longlong(2.0 * g.vert_dist * (1.0 + 8.8817841970012523e-16));
+    const double inv_vd = 1.0 / g.vert_dist;
+    int work = 0;
+    unsigned nq = 0;  // queues filled so far
+    auto fill = [&](int s, int64_t base, int p, double al, int& scan, bool& first) -> bool {
+      const int qb = nq & 1;
+      int4* const par = q_par(qb);
+      long long* const qd = q_d(qb);
+      if (nq >= 2) bar_sync(kBarEmpty + qb, kThreads);
+      if (tid == 0) {
+        s_kmax = 0;
+        s_dmax = 0;
+        s_nf = 0;
+      }
+      int qn = 0;
+      while (qn <= kQueue - kRefill && scan < p) {
+        int ent[kPer];
+        double dz[kPer];
+        unsigned m[kPer];
+        bool keep[kPer];
+        const int i0 = scan + warp * (32 * kPer) + lane;
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+          keep[r] = i0 + 32 * r < p;
+          ent[r] = i0 + 32 * r;
+          dz[r] = 0.0;
+          if (keep[r] && !batch) ent[r] = l.ent[base + i0 + 32 * r];
+        }
+        if (vertical) {
+#pragma unroll
+          for (int r = 0; r < kPer; ++r)
+            if (keep[r]) dz[r] = hx.lnp[ent[r]];
+#pragma unroll
+          for (int r = 0; r < kPer; ++r) {
+            dz[r] = al - dz[r];
+            const long long a = __double_as_longlong(dz[r]) & 0x7fffffffffffffffll;
+            keep[r] = keep[r] && !(a > lim_bits && a <= 0x7ff0000000000000ll);
+          }
+        }
+        int c = 0;
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+          m[r] = __ballot_sync(0xffffffffu, keep[r]);
+          c += __popc(m[r]);
+        }
+        const int pb = (scan / kRefill) & 1;  // double-buffered counts: one barrier per refill
+        if (lane == 0) s_wcnt[pb][warp] = c;
+        bar_sync(kBarP, kPThreads);
+        int off = qn;
+#pragma unroll
+        for (int w = 0; w < kPWarps; ++w) {
+          off += w < warp ? s_wcnt[pb][w] : 0;
+          qn += s_wcnt[pb][w];
+        }
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+          if (keep[r]) {
+            const int pos = off + __popc(m[r] & ((1u << lane) - 1u));
+            par[pos] = make_int4(__double2loint(dz[r]), __double2hiint(dz[r]), i0 + 32 * r, ent[r]);
+          }
+          off += __popc(m[r]);
+        }
+        scan += kRefill;
+      }
+      bar_sync(kBarP, kPThreads);
+      // weights, densely (FP64): rr into par, d~ into qd
+      int kmax = 0, dmax = 0, cnt = 0;
+      bool nf = false;
+      for (int q = tid; q < qn; q += kPThreads) {
+        const int4 c = par[q];
+        const int ent = c.w;
+        const int64_t i = base + c.z;
+        double rl, rdg, dep;
+        int e;
+        if (batch) {
+          rl = b.b_rloc[i];
+          rdg = (double)b.b_rdiag[i];
+          dep = b.b_dep[i];
+          const double* y = b.b_hx + (size_t)i * k;
+          unsigned em = 0;
+          for (int j = 0; j < k; ++j) em = max(em, (unsigned)__double2hiint(y[j]) & 0x7fffffffu);
+          e = (int)em;
+        } else {
+          rl = l.rloc[i];
+          rdg = (double)hx.rdiag[ent];
+          dep = hx.dis[ent];
+          e = hx.yexp[ent];
+          if (vertical) {
+            const double z = fabs(__hiloint2double(c.y, c.x)) * inv_vd;
+            rl = rl * (g.gc_filter_vertical ? taper_fast(z) : schr(z));
+          }
+        }
+        double w = sqrt(rdg * rl), d = 0.0;
+        if (w != 0.0) {
+          d = w * dep;
+          const int ew = (__double2hiint(w) >> 20) & 0x7ff;
+          const int ed = (__double2hiint(d) >> 20) & 0x7ff;
+          ++cnt;
+          nf |= (e >> 20) == 2047 || ew == 2047 || ed == 2047;
+          if (e >> 20) {
+            // the bound |z| < 2^(kz - 1022): the product of the mantissas (each
+            // rounded up, so at most 4) decides whether it carries
+            const double fy = __hiloint2double((e & 0xfffff) | 0x3ff00000, -1);
+            const double fw = __hiloint2double((__double2hiint(w) & 0xfffff) | 0x3ff00000, -1);
+            kmax = max(kmax, (e >> 20) + ew + ((__double2hiint(fy * fw) >> 20) - 1023));
+            dmax = max(dmax, ed);
+          } else {
+            w = 0.0;  // a row of zeros
+          }
+        }
+        *reinterpret_cast<double*>(&par[q]) = w;
+        qd[q] = __double_as_longlong(d);
+      }
+      kmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)kmax);
+      dmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)dmax);
+      work += cnt;
+      nf = __any_sync(0xffffffffu, nf);
+      if (lane == 0) {
+        atomicMax(&s_kmax, kmax);
+        atomicMax(&s_dmax, dmax);
+        if (nf) s_nf = 1;
+      }
+      bar_sync(kBarP, kPThreads);
+      kmax = s_kmax;
+      dmax = s_dmax;
+      const int S = kmax - 2045, Sd = dmax - 1022;  // |z| < 2^S
+      const bool bad = s_nf != 0 || (kmax && (S > kExLimit || S < -kExLimit)) ||
+                       (dmax && (Sd > kExLimit || Sd < -kExLimit));
+      const int qr = kmax && !bad ? (qn + kStage - 1) / kStage * kStage : 0;
+      for (int q = tid; q < qr; q += kPThreads) {
+        int4 pr = make_int4(0, 0, 0, 0);
+        long long dq = 0;
+        unsigned long long u = 0;
+        if (q < qn) {
+          u = *reinterpret_cast<unsigned long long*>(&par[q]);
+          pr.w = par[q].w;
+        } else {
+          pr.w = par[0].w;  // padding: weight zero, a valid row
+        }
+        if (u << 1) {
+          const int ew = (int)(u >> 52) & 0x7ff;
+          const unsigned long long R = ((u & 0xfffffffffffffull) | 0x10000000000000ull) << 5;
+          pr = make_int4((int)(R >> 29), (int)(R & 0x1fffffffull), kmax - ew, pr.w);
+          const unsigned long long dv = (unsigned long long)qd[q];
+          const int ed = (int)(dv >> 52) & 0x7ff;
+          if (ed > 0) {
+            const int sh = min(dmax - ed, 62);
+            const unsigned long long mnt = (dv & 0xfffffffffffffull) | 0x10000000000000ull;
+            dq = (long long)((mnt + (sh ? 1ull << (sh - 1) : 0ull)) >> sh);
+            dq = (long long)((unsigned long long)dq | (dv & 0x8000000000000000ull));
+          }
+        }
+        par[q] = pr;
+        // 32 (|D| + bias) and the sign in the top bit, as digits_of leaves Z
+        qd[q] = ((dq & 0x7fffffffffffffffll) + bias()) * 32 | (dq & (1ll << 63));
+      }
+      if (tid == 0) s_head[qb] = QueueHead{s, qr / kStage, S, Sd, first ? 1 : 0, bad ? 1 : 0};
+      bar_arrive(kBarFull + qb, kThreads);
+      ++nq;
+      first = false;
+      return !bad;
+    };
+    for (int s = blockIdx.x; s < b.nsolves; s += gridDim.x) {
+      int64_t base;
+      int p, col = 0, kk = 1;
+      if (batch) {
+        base = b.b_off[s];
+        p = b.b_nobsl[s];
+      } else {
+        solve_col_level(b, s, col, kk);
+        base = l.off[col];
+        p = l.cnt[col];
+      }
+      const double al = vertical ? tout[(size_t)s * k] : 0.0;
+      int scan = 0;
+      bool first = true;
+      while (fill(s, base, p, al, scan, first) && scan < p) {
+      }
+    }
+    const int qb = nq & 1;
+    if (nq >= 2) bar_sync(kBarEmpty + qb, kThreads);
+    if (tid == 0) s_head[qb] = QueueHead{-1, 0, 0, 0, 0, 0};
+    bar_arrive(kBarFull + qb, kThreads);
+    work = (int)__reduce_add_sync(0xffffffffu, (unsigned)work);
+    if (b.work && lane == 0 && work) atomicAdd(b.work, (unsigned long long)work);
+  } else if (warp == kMmaWarp) {
+    // ================= the issuing warp
+    unsigned n = 0;  // stages issued (buffer n & 1)
+    bool started = false;
+    for (unsigned nq = 0;; ++nq) {
+      const int qb = nq & 1;
+      bar_sync(kBarFull + qb, kThreads);
+      const int stages = s_head[qb].s < 0 ? -1 : s_head[qb].stages;
+      if (stages < 0) break;
+      bar_arrive(kBarEmpty + qb, kThreads);
+      for (int st = 0; st < stages; ++st, ++n) {
+        bar_sync(kBarStage + (n & 1), kXMma);
+        if (st % kGroup == 0) {
+          // a new exact sum: the finished one is out of tensor memory
+          if (started) bar_sync(kBarDrain, kXMma);
+          started = true;
+        }
+        if (lane == 0) {
+          tc::fence_after();
+          const uint32_t sb = tc::smem_u32(smem_raw) + (n & 1) * kStageBytes;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            auto at = [&](int pos) {
+              return tc::make_desc(sb + c * kChunkBytes + pos * kSlice, 128, 256);
+            };
+            const uint64_t dt = tc::make_desc(sb + c * kChunkBytes + kTileD, 128, 256);
+            const uint32_t more = (st % kGroup > 0 || c > 0) ? 1u : 0u;
+            mma(tmem, at(1), at(2), idesc(64), more);         // [5;0] x 0
+            mma(tmem + 64, at(2), at(3), idesc(256), more);   // [0;1] x 1 3 2 4
+            mma(tmem + 320, at(4), at(4), idesc(64), more);   // [3;2] x 3
+            mma(tmem + 384, at(5), at(5), idesc(64), more);   // [2;4] x 2
+            mma(tmem + 384, at(0), at(3), idesc(64), 1u);     // [zero;5] x 1
+            mma(tmem + kColD, at(1), dt, idesc(16), more);
+            mma(tmem + kColD + 16, at(3), dt, idesc(16), more);
+            mma(tmem + kColD + 32, at(5), dt, idesc(16), more);
+          }
+          tc::mma_commit(&mbar[n & 1]);
+        }
+        __syncwarp();
+      }
+    }
+    if (started) bar_sync(kBarDrain, kXMma);
+  }
+  } else {
+    // ================= converting warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+    const int xt = tid - 32 * kX0;
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool low = (warp & 3) < 2;         // accumulator rows 0..63: the first slice of A
+    const int row = (warp & 1) * 32 + lane;  // member of this thread's accumulator row
+    constexpr int kW = kR == 2 ? 8 : 4;      // accumulator columns taken out at a time
+    constexpr int cw = kR;                   // octets of columns of each warp quadruple
+    const int j0 = (warp - kX0) / 4 * 8 * cw;
+    const int noct = max(0, min(cw, (k - j0 + 7) / 8));  // uniform in a warp
+    // unit u of a stage: entries 4 (u & 1) .. + 3 of the 8-entry group u / 2k, member
+    // (u / 2) % k -- two lanes fill the 16 bytes of an operand row.  This thread's
+    // units: member, first entry (< 0: none), place in the operand buffer
+    int um[kR], uq[kR], ud[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const int u = xt + r * kXThreads, ug = (u >> 1) / k;
+      um[r] = (u >> 1) - ug * k;
+      uq[r] = u < 16 * k ? ug * 8 + (u & 1) * 4 : -1;
+      ud[r] = (ug >> 1) * kChunkBytes + (um[r] >> 3) * 256 + (ug & 1) * 128 + (um[r] & 7) * 16 +
+              (u & 1) * 8;
+    }
+    // the chunk's sums, 64 x 65
+    long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + 2 * kQueueBytes);
+    bool ok = true;
+    unsigned n = 0, nq = 0;  // stages issued (buffer n & 1), queues taken
+    for (;; ++nq) {
+      const int qb = nq & 1;
+      bar_sync(kBarFull + qb, kThreads);
+      const QueueHead h = s_head[qb];
+      if (h.s < 0) break;
+      const int4* const par = q_par(qb);
+      const long long* const qd = q_d(qb);
+      double* const C = Cout + (size_t)h.s * k * k;
+      double* const tv = tout + (size_t)h.s * k;
+      long long acc[8 * cw], thi = 0, tlo = 0;
+#pragma unroll
+      for (int j = 0; j < 8 * cw; ++j) acc[j] = 0;
+      auto drain = [&](unsigned last) {
+        // the exact FP32 sums of the stages up to `last`, added as integers
+        if (ok && !tc::mbar_wait(&mbar[last & 1], (last >> 1) & 1)) ok = false;
+        tc::fence_after();
+#pragma unroll
+        for (int o = 0; o < cw * (8 / kW); ++o) {
+          if (o >= noct * (8 / kW)) continue;
+          float v[7][kW];
+#pragma unroll
+          for (int m = 0; m < 7; ++m) {
+            const uint32_t at = lane_addr + 64u * m + (uint32_t)(j0 + kW * o);
+            if constexpr (kW == 8)
+              tmem_ld8(at, v[m]);
+            else
+              tmem_ld4(at, v[m]);
+          }
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < kW; ++j) {
+            int x[7];
+#pragma unroll
+            for (int m = 0; m < 7; ++m) x[m] = __float2int_rn(v[m][j]);
+            // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
+            // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
+            long long& A = acc[kW * o + j];
+            if (low) {  // 50 01 03 02 04 33 22
+              A += (long long)x[1] * (1 << 27);
+              A += (long long)x[3] * (1 << 18);
+              A += (long long)x[2] * (1 << 9);
+              const int y = 2 * x[4] + x[6] + ((x[0] + (x[5] >> 10) + 128) >> 8);
+              A += (y + 1) >> 1;
+            } else {    // 00 11 13 12 14 23 42+51
+              A += (long long)((unsigned long long)(unsigned)(x[0] * 8) << 32);
+              A += (long long)x[1] * (1 << 17);
+              A += (long long)x[3] * (1 << 9);
+              A += x[2] + ((x[4] + x[5] + ((x[6] + 256) >> 9) + 256) >> 9);
+            }
+          }
+        }
+        if (j0 == 0) {
+          float v[3][8];
+#pragma unroll
+          for (int m = 0; m < 3; ++m) tmem_ld8(lane_addr + kColD + 16u * m, v[m]);
+          tmem_wait_ld();
+          long long x[3][6];
+#pragma unroll
+          for (int m = 0; m < 3; ++m)
+#pragma unroll
+            for (int j = 0; j < 6; ++j) x[m][j] = __float2int_rn(v[m][j]);
+          // rows 5|0, 1|3, 2|4 of z against d~ slices 0..5, a + b <= 6; thi in
+          // units of weight 2, tlo of weight 5
+          long long w6;
+          if (low) {
+            thi += (x[1][0] << 9) + x[1][1] + x[2][0];
+            tlo += (x[1][2] << 18) + (x[1][3] << 9) + x[1][4] + (x[2][1] << 18) + (x[2][2] << 9) +
+                   x[2][3] + x[0][0];
+            w6 = x[0][1] + x[1][5] + x[2][4];
+          } else {
+            thi += (x[0][0] << 18) + (x[0][1] << 9) + x[0][2];
+            tlo += (x[0][3] << 18) + (x[0][4] << 9) + x[0][5] + (x[1][0] << 18) + (x[1][1] << 9) +
+                   x[1][2] + (x[2][0] << 9) + x[2][1];
+            w6 = x[1][3] + x[2][2];
+          }
+          tlo += (w6 + 256) >> 9;
+        }
+        tc::fence_before();
+        bar_arrive(kBarDrain, kXMma);
+      };
+      const double* const ysrc = batch ? b.b_hx + (size_t)b.b_off[h.s] * k : hx.yb;
+      uint2 y[kR][4];
+      auto load = [&](int st, int r) {
+        if (uq[r] < 0) return;
+        const int q0 = st * kStage + uq[r];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          y[r][e] = __ldg(reinterpret_cast<const uint2*>(ysrc + (size_t)par[q0 + e].w * k + um[r]));
+      };
+      if (h.stages > 0) {
+#pragma unroll
+        for (int r = 0; r < kR; ++r) load(0, r);
+      }
+      for (int st = 0; st < h.stages; ++st, ++n) {
+        unsigned char* const buf = smem_raw + (n & 1) * kStageBytes;
+        if (n >= 2 && ok && !tc::mbar_wait(&mbar[n & 1], ((n - 2) >> 1) & 1)) ok = false;
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+          if (uq[r] < 0) continue;
+          const int q0 = st * kStage + uq[r];
+          uint32_t o[2][6];
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            digit_pairs(digits_of(y[r][2 * e].y, y[r][2 * e].x, par[q0 + 2 * e]),
+                        digits_of(y[r][2 * e + 1].y, y[r][2 * e + 1].x, par[q0 + 2 * e + 1]),
+                        y[r][2 * e].y, y[r][2 * e + 1].y, o[e]);
+          if (st + 1 < h.stages) load(st + 1, r);  // in flight beside the rest of this stage
+          unsigned char* const dst = buf + ud[r];
+#pragma unroll
+          for (int a = 0; a < 6; ++a)
+            *reinterpret_cast<uint2*>(dst + slice_pos(a) * kSlice) = make_uint2(o[0][a], o[1][a]);
+        }
+        if (warp == kX0 + kXWarps - 1) {
+          // d~ slices: row b of the 16-row tile, two entries per lane
+          const int q0 = st * kStage + 2 * lane;
+          uint32_t o[6];
+          const unsigned long long d0 = (unsigned long long)qd[q0], d1 = (unsigned long long)qd[q0 + 1];
+          digit_pairs(d0 & ~(1ull << 63), d1 & ~(1ull << 63), (unsigned)(d0 >> 32),
+                      (unsigned)(d1 >> 32), o);
+          unsigned char* const dst = buf + (lane >> 3) * kChunkBytes + kTileD +
+                                     ((lane >> 2) & 1) * 128 + (lane & 3) * 4;
+#pragma unroll
+          for (int a = 0; a < 6; ++a) *reinterpret_cast<uint32_t*>(dst + a * 16) = o[a];
+        }
+        tc::fence_proxy_async();
+        bar_arrive(kBarStage + (n & 1), kXMma);
+        // a new exact sum starts with this stage: take the finished one out
+        if (st > 0 && st % kGroup == 0) drain(n - 1);
+      }
+      bar_arrive(kBarEmpty + qb, kThreads);  // this thread is done with the queue
+      if (h.bad) {
+        bar_sync(kBarX, kXThreads);  // an earlier chunk's C is written
+        if (xt == 0) C[0] = __longlong_as_double((long long)kGramMark);
+        continue;
+      }
+      if (h.stages == 0 && !h.first) continue;
+      if (h.stages > 0) {
+        drain(n - 1);
+        // the two row halves meet in shared memory
+        if (!low) {
+#pragma unroll
+          for (int j = 0; j < 8 * cw; ++j)
+            if (j < 8 * noct) U[row * 65 + j0 + j] = acc[j];
+        }
+        if (j0 == 0) s_t[low ? 0 : 1][row] = make_longlong2(thi, tlo);
+        bar_sync(kBarX, kXThreads);
+        if (low) {
+#pragma unroll
+          for (int j = 0; j < 8 * cw; ++j)
+            if (j < 8 * noct) U[row * 65 + j0 + j] += acc[j];
+        }
+        bar_sync(kBarX, kXThreads);
+      }
+      const int ex2 = 2 * h.S - 62 + kDrop, ext = h.S + h.Sd - 61;
+      // C = (U + U^T) / 2 in place (rows i and k - 1 - i of the triangle share one
+      // row of k + 1 elements), then out in rows
+      if (h.stages > 0) {
+        for (int r = xt; r < (k + 1) / 2 * (k + 1); r += kXThreads) {
+          const int a = r / (k + 1), c = r - a * (k + 1);
+          if (2 * a == k - 1 && c > a) continue;  // odd k: the middle row meets itself
+          const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
+          const long long v =
+              __double_as_longlong(fixed_to_double(U[i * 65 + j] + U[j * 65 + i], ex2));
+          U[i * 65 + j] = v;
+          U[j * 65 + i] = v;
+        }
+        bar_sync(kBarX, kXThreads);
+      }
+      for (int r = xt, j = xt / k, i = xt - j * k; r < k * k; r += kXThreads) {
+        double v = h.stages > 0 ? __longlong_as_double(U[j * 65 + i]) : 0.0;
+        if (!h.first) v += C[r];
+        C[r] = v;
+        i += kXThreads;
+        while (i >= k) {
+          i -= k;
+          ++j;
+        }
+      }
+      if (xt < k) {
+        double v = 0.0;
+        if (h.stages > 0)
+          v = wide_to_double(s_t[0][xt].x + s_t[1][xt].x, s_t[0][xt].y + s_t[1][xt].y, ext);
+        tv[xt] = h.first ? v : tv[xt] + v;
+      }
+      if (h.stages > 0) bar_sync(kBarX, kXThreads);  // U and s_t are free again
+    }
+    if (n > 0 && !tc::mbar_wait(&mbar[(n - 1) & 1], ((n - 1) >> 1) & 1)) ok = false;
+    if (!ok) atomicExch(err, LG_ERR_TIMEOUT);
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kTmemCols));
+}
+
+bool gram64_tc_supported(int ens) { return ens <= 64; }
+
+void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
+                      const double* axb, double* C, double* t, int* err, cudaStream_t stream) {
+  if (b.nsolves == 0) return;
+  const int grid = b.nsolves < 152 ? b.nsolves : 152;
+  if (b.mode == 0 && g.vert_dist > 0.0)
+    level_lnp_kernel<<<(b.nsolves + 127) / 128, 128, 0, stream>>>(g, b, axb, t);
+  auto run = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g64::kSmem);
+    kernel<<<grid, g64::kThreads, g64::kSmem, stream>>>(g, hx, l, b, C, t, err);
+  };
+  if (g.ens <= 48)
+    run(gram64_tc_kernel<2>);
+  else
+    run(gram64_tc_kernel<3>);
+}
+
+}  // namespace lg

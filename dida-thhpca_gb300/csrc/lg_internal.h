@@ -46,6 +46,21 @@ struct Geometry {
   const int* nb_blk;     // neighbour blocks in traversal order
 };
 
+#ifdef __CUDACC__
+// ln p of model level kk (1-based) for surface pressure aps
+__device__ inline double alnp_level(const Geometry& g, int kk, double aps) {
+  // ps2alnp (obs_make.F90:418-437), with ph_lev(nz+1) evaluated
+  auto lev = [&](int k1) {
+    if (g.vcoord == LG_VCOORD_SIGMA)
+      return __dadd_rn(__dmul_rn(g.ca[k1 - 1], __dsub_rn(aps, g.ptop)), g.ptop);
+    const double t1 = __dmul_rn(g.ca[k1 - 1], __dsub_rn(g.p0, g.ptop));
+    const double t2 = __dmul_rn(g.cb[k1 - 1], __dsub_rn(aps, g.ptop));
+    return __dadd_rn(__dadd_rn(t1, t2), g.ptop);
+  };
+  return log(__dmul_rn(0.5, __dadd_rn(lev(kk), lev(kk + 1))));
+}
+#endif
+
 // Observations and their block copies on the device.
 struct ObsDev {
   int n_obs;
@@ -94,6 +109,7 @@ struct HxDev {
   double* dis;    // n_entries
   double* lnp;    // n_entries, log(ph)
   float* rdiag;   // n_entries, REAL(4) R^-1
+  int* yexp;      // n_entries, FP64 path up to 64 members: largest biased exponent of the row
 };
 
 // Per-column neighbour lists.
@@ -193,8 +209,17 @@ void launch_clear_selection(const int* fresh, int* cnt, int n, int* col_stats,
 void launch_scan_counts(const int* cnt, int64_t* off, int n, void* tmp, size_t tmp_bytes,
                         cudaStream_t stream);
 size_t scan_tmp_bytes(int n);
+// FP64 Gram matrices and projections: exact slices on the tensor cores up to 64
+// members (lg_gram64_tc.cu; mode 0 needs hx.yexp), the FP64 pipe otherwise
 void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
-                   const double* axb, double* C, double* t, cudaStream_t stream);
+                   const double* axb, double* C, double* t, int* err, cudaStream_t stream);
+bool gram64_tc_supported(int ens);
+void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
+                      const double* axb, double* C, double* t, int* err, cudaStream_t stream);
+void launch_row_exponents(int ens, int64_t rows, const double* yb, int* yexp, cudaStream_t stream);
+// first Gram element of a solve that gram64_tc_kernel leaves to gram64_kernel:
+// a NaN with a payload no arithmetic here produces
+constexpr unsigned long long kGramMark = 0x7ff9676d61726b21ull;
 bool gram_tc_supported(int ens);
 void launch_gram_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
                     const double* axb, double* C, double* t, int* err, cudaStream_t stream,

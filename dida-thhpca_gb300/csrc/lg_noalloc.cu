@@ -100,7 +100,7 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
   if (precision == LG_PREC_MIXED && lg::gram_tc_supported(ens))
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
   else
-    lg::launch_gram64(geo, hx, l, b, nullptr, C, t, st);
+    lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
   lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
                        st);
   int h_fail = 0;

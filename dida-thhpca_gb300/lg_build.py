@@ -23,6 +23,7 @@ UNITS = {
     "lg_hx.cu": ["-fmad=false"],
     "lg_search.cu": ["-fmad=false"],
     "lg_gram.cu": [],
+    "lg_gram64_tc.cu": [],
     "lg_eig.cu": [],
     "lg_gram_tc.cu": [],
     "lg_gram_tc128.cu": [],
