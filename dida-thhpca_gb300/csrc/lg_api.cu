@@ -132,6 +132,7 @@ struct lg_ctx {
   double* d_trans = nullptr;
   size_t trans_cap = 0;
   bool use_eig2 = false;
+  bool use_ft = false;  // plain FP64: tridiagonal form in the Gram matrices' place, no QL
   // mixed precision: the vector transform (Xb.W, w-bar) in FP64 from FP64
   // reflectors and rotations instead of FP32 (LETKF_GB300_VEC64=1 at
   // lg_create; a diagnostic that isolates the FP32 transform's share of the
@@ -518,6 +519,10 @@ int lg_create(lg_ctx** out, const lg_config* cfg) {
   if (g.overlap > 0) c->cfg.vert_dist = 0.0;
   c->cubes = g.cube_n > 1 || g.overlap > 0 || (g.cube_nz > 1 && c->cfg.vert_dist > 0.0);
   c->vec64 = getenv("LETKF_GB300_VEC64") != nullptr;
+  if (lg::prepare_ft_nodes() != LG_OK) {
+    delete c;
+    return LG_ERR_CUDA;
+  }
   cudaGetDevice(&c->dev);
   // Scheduling priorities of the solve streams (Gram, vector update, QL): a
   // level 0 (lowest, the default stream's), 1 or 2 (highest) each.  Pending
@@ -1130,6 +1135,7 @@ int prepare_capacity(lg_ctx* c) {
   const int nsel = col_end(c) - col_begin(c);
   c->chunk = (int)std::min<size_t>((size_t)nsel, std::max<size_t>(1, budget / per_col));
   c->use_eig2 = lg::eig2_supported(geo);
+  c->use_ft = c->use_eig2 && !lg::mixed_precision(g.precision) && lg::ft_supported(geo);
   c->rot_cap = 3 * k * k;
   // test hook: a small log forces the overflow fallback path
   if (const char* env = getenv("LETKF_GB300_ROT_CAP")) c->rot_cap = std::max(1, atoi(env));
@@ -1202,7 +1208,7 @@ int prepare_capacity(lg_ctx* c) {
     r |= dalloc(&L.C, cap * k * k);
     r |= dalloc(&L.t, cap * k);
     r |= dalloc(&L.ovf_n, 1);
-    if (c->use_eig2) {
+    if (c->use_eig2 && !c->use_ft) {
       r |= dalloc(&L.tri, cap * lg::eig2_tri_doubles(k));
       r |= dalloc(&L.lam, cap * k);
       r |= dalloc(&L.rot_cs, (cap * (size_t)c->rot_cap + rot_pairs_per_slot - 1) /
@@ -1482,6 +1488,14 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
                              c->d_status + 1, st);
         CK(record_event(kv[6], st));
         launches += 5;
+      } else if (lg::ft_supported(geo)) {
+        lg::launch_tridiag_in_place(k, b.nsolves, L.C, st);
+        CK(record_event(kv[3], st));
+        for (int e = 4; e < 6; ++e) CK(record_event(kv[e], st));
+        lg::launch_ft(geo, b, true, L.t, L.C, (size_t)k * k, xb, axb, xa, axa, c->d_trans, nullptr,
+                      c->d_status + 1, st);
+        CK(record_event(kv[6], st));
+        launches += 3;
       } else {
         lg::launch_eig_apply(geo, b, L.C, L.t, xb, axb, xa, axa, c->d_trans, nullptr,
                              c->d_status + 1, st);
@@ -1585,7 +1599,19 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
       CK(cudaStreamWaitEvent(s_e, c->ev_phase[0][set], 0));
     }
     CK(record_event(kv[2], s_e));
-    if (c->use_eig2) {
+    if (c->use_ft) {
+      lg::launch_tridiag_in_place(k, b.nsolves, L.C, s_e);
+      CK(record_event(kv[3], s_e));
+      CK(record_event(kv[4], s_e));
+      if (nl >= 3) {
+        CK(cudaEventRecord(c->ev_phase[2][set], s_e));
+        CK(cudaStreamWaitEvent(s_v, c->ev_phase[2][set], 0));
+      }
+      CK(record_event(kv[5], s_v));
+      lg::launch_ft(geo, b, false, L.t, L.C, (size_t)k * k, xb, axb, xa, axa, nullptr, nullptr,
+                    c->d_status + 1, s_v);
+      launches += 2;
+    } else if (c->use_eig2) {
       if (s_q == s_e) {
         lg::launch_eig2(geo, b, L.C, L.t, xb, axb, xa, axa, L.tri, L.lam, L.rot_cs, L.rot_i,
                         L.rot_n, c->rot_cap, L.ovf_list, L.ovf_n, c->d_status + 1, fp32_vec,
@@ -2302,6 +2328,7 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   if (precision == LG_PREC_MIXED_TF32 && !lg::gram_tf32_supported(ens)) return LG_ERR_UNSUPPORTED;
   if (nbatch == 0) return LG_OK;
   if (!d_nobsl || !d_off || !d_trans || !d_wbar) return LG_ERR_ARG;
+  if (lg::prepare_ft_nodes() != LG_OK) return LG_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream_v;
   Geometry geo{};
   geo.ens = ens;
@@ -2335,7 +2362,14 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
   else
     lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
-  lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail, st);
+  if (lg::ft_supported(geo)) {
+    lg::launch_tridiag_in_place(ens, nbatch, C, st);
+    lg::launch_ft(geo, b, true, t, C, (size_t)ens * ens, nullptr, nullptr, nullptr, nullptr,
+                  d_trans, d_wbar, fail, st);
+  } else {
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
+                         st);
+  }
   int h_fail = 0;
   if (cudaGetLastError() != cudaSuccess ||
       cudaMemcpyAsync(&h_fail, fail, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -73,7 +73,8 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
   const size_t need = (size_t)nbatch * ((size_t)ens * ens + ens) + 8;
   if (need > kScratchDoubles) return LG_ERR_SHAPE;
   double* scratch = nullptr;
-  const int r = scratch_address(&scratch);
+  int r = scratch_address(&scratch);
+  if (r == LG_OK) r = lg::prepare_ft_nodes();
   if (r != LG_OK) return r;
   double* C = scratch;
   double* t = C + (size_t)nbatch * ens * ens;
@@ -101,8 +102,14 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
   else
     lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
-  lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
-                       st);
+  if (lg::ft_supported(geo)) {
+    lg::launch_tridiag_in_place(ens, nbatch, C, st);
+    lg::launch_ft(geo, b, true, t, C, (size_t)ens * ens, nullptr, nullptr, nullptr, nullptr,
+                  d_trans, d_wbar, fail, st);
+  } else {
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
+                         st);
+  }
   int h_fail = 0;
   if (cudaGetLastError() != cudaSuccess ||
       cudaMemcpyAsync(&h_fail, fail, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

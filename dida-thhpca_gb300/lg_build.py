@@ -30,6 +30,7 @@ UNITS = {
     "lg_gram_tf32.cu": [],
     "lg_gram_col.cu": [],
     "lg_eig2.cu": [],
+    "lg_ft.cu": [],
     "lg_noalloc.cu": [],
     "lg_prepost.cu": [],
     "lg_cube.cu": [],

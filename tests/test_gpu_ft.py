@@ -1,0 +1,75 @@
+"""FP64 transform without eigenvalues (lg_ft.cu): W = sqrt(k-1) A^(-1/2) and
+overline_w = A^-1 t from shifted tridiagonal solves.
+
+Member counts around a warp's 32 lanes and the ends of the range (7, 64),
+spectra from C = 0 to a condition number of 10^9, and analyses with one and four
+variables (16 and 6 solves per warp).
+
+Yardstick: numpy's eigh in FP64.  Both it and the kernel are backward stable:
+each returns the function of a matrix within about k 2^-53 |A| of A, and a
+change E of A moves A^(-1/2) by at most |E| lambda_min^(-3/2) / 2 and A^-1 t by
+|E| |t| / lambda_min^2.  The tolerances are those bounds with 8 k 2^-53 |A| for
+the two evaluations' |E| together.
+"""
+import numpy as np
+import pytest
+
+from test_gpu_gram64 import _batch, _case
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(case, rho, trans, wbar):
+    hx, rd, dep, rloc = case
+    k = hx.shape[1]
+    rr = np.sqrt(rd.astype(np.float64) * rloc)
+    z = hx * rr[:, None]
+    t = z.T @ (rr * dep)
+    lam, v = np.linalg.eigh(z.T @ z)
+    lam = np.maximum(lam, 0.0) + (k - 1) / rho
+    w = (v * np.sqrt((k - 1) / lam)) @ v.T
+    wb = v @ ((v.T @ t) / lam)
+    err = 8 * k * 2.0 ** -53 * lam.max()
+    tol_w = err * 0.5 * np.sqrt(k - 1) * lam.min() ** -1.5 + 1e-14
+    tol_b = err * np.linalg.norm(t) / lam.min() ** 2 + 1e-14 * np.abs(wb).max()
+    assert np.abs(wbar - wb).max() <= tol_b
+    assert np.abs(trans.T - wbar[:, None] - w).max() <= tol_w + 4 * 2.0 ** -53 * np.abs(wbar).max()
+
+
+@pytest.mark.parametrize("k", [7, 8, 31, 32, 33, 40, 63, 64])
+def test_member_counts_and_condition_numbers(k):
+    rng = np.random.default_rng(k)
+    cases = []
+    for scale in (0.0, 1e-9, 1e-3, 1.0, 1e2, 1e4, 1e6):
+        for p in (3, 5 * k):  # rank-deficient and full
+            hx, rd, dep, rloc = _case(rng, k, p)
+            cases.append((hx, (rd * np.float32(scale)).astype(np.float32), dep, rloc))
+    st, tr, wb = _batch(cases, 1.05)
+    assert st == 0
+    for c, t, w in zip(cases, tr, wb):
+        _check(c, 1.05, t, w)
+
+
+@pytest.mark.parametrize("name,ens", [("tiny2d", 7), ("tiny2d", 33), ("tiny3d", 9), ("tiny3d", 64)])
+def test_analysis_against_the_ql_route(name, ens, monkeypatch):
+    """The same analysis with the QL route (a sweep limit below the default
+    selects it; 59 sweeps still converge) agrees to rounding: the increments
+    within 1e-10 of their largest, the repository's tolerance for the path."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset(name).replace(ens=ens)
+    w = synth.make_workload(cfg)
+    out = []
+    for limit in (None, "59"):
+        if limit:
+            monkeypatch.setenv("LETKF_GB300_QL_ITERS", limit)
+        ctx = lg.Letkf(cfg)
+        ctx.set_obs(w.obs)
+        xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+        ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+        ctx.letkf_final()
+        out.append(xa + axa[..., None])
+    h = cfg.halo
+    i = slice(h, -h)
+    inc = np.abs(out[1] - (w.xb + w.axb[..., None]))[i, i].max()
+    assert np.abs(out[0] - out[1])[i, i].max() <= 1e-10 * inc
