@@ -208,10 +208,6 @@ __device__ inline double group_sum_exact(double v, int f) { return sum_exact<fal
 // step: 1 where the step has a reflector, 0 where it has none.  A matrix with
 // an h outside [2^-200, 2^200] is marked by H[0] = 1 (the QL kernel passes it
 // to the FP64 fallback solver); the double H is kept for reference.
-//
-// u32 = 2 (FP64 transform without eigenvalues, lg_ft.cu): FP64 reflectors with
-// H[i] = 1/h (0: no reflector); tri may be Cin itself with a stride of n n
-// (from 7 members on: 3n + n(n-1)/2 <= n n), the matrix is read first.
 __device__ inline float rsqrt_f32_of(double h) {
   // 1/sqrt(h) for a normal h in [2^-200, 2^200]: h = m 2^e2 with e2 even and m
   // in [1, 4) (exponent bits only), then rsqrtf(m) 2^(-e2/2)
@@ -222,7 +218,7 @@ __device__ inline float rsqrt_f32_of(double h) {
 }
 
 __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const double* Cin,
-                                                     double* tri, size_t tri_stride, int u32) {
+                                                     double* tri, int u32) {
   const int s = blockIdx.x;
   if (s >= nsolves) return;
   const int lane = threadIdx.x;
@@ -247,7 +243,7 @@ __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const d
       }
     }
   }
-  double* out = tri + (size_t)s * tri_stride;
+  double* out = tri + (size_t)s * e2::tri_stride(n);
   double* D = out;
   double* E = out + n;
   double* H = out + 2 * n;
@@ -260,7 +256,7 @@ __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const d
   for (int i = n - 1; i >= 1; --i) {
     const int l = i - 1;
     double* row = P + tri_idx(i);  // u: row i, columns 0..l
-    double h = 0.0, inv_h = 0.0, ei;
+    double h = 0.0, ei;
     if (l > 0) {
       double ss = 0.0;
       for (int c = lane; c <= l; c += 32) ss = fma(row[c], row[c], ss);
@@ -305,7 +301,7 @@ __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const d
         // the group sums meet in exact fixed-point sums on the integer pipe:
         // the FP64 pipe then issues about R + ceil(R / f) instructions instead
         // of R per 32 rows.
-        inv_h = rcp_nr(h);
+        const double inv_h = rcp_nr(h);
         double fs = 0.0;
         const int R = l + 1;
         const int nfull = R > 32 ? ((R - 1) / 32) * 32 : 0;
@@ -377,7 +373,7 @@ __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const d
       ei = row[l];
     }
     // reflector of step i: u = row i (scaled), h
-    if (u32 == 1) {
+    if (u32) {
       const int eh = dexp(h);
       const bool in_range = eh >= 1023 - 200 && eh <= 1023 + 200;
       extreme |= !is_zero_bits(h) && !in_range;
@@ -388,7 +384,7 @@ __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const d
       for (int c = lane; c < i; c += 32) U[e2::uoff(i) + c] = row[c];
     }
     if (lane == 0) {
-      H[i] = u32 == 2 ? inv_h : h;
+      H[i] = h;
       E[i] = ei;
     }
     __syncwarp();
@@ -397,7 +393,7 @@ __global__ void __launch_bounds__(32) tridiag_kernel(int n, int nsolves, const d
   if (lane == 0) {
     H[0] = extreme ? 1.0 : 0.0;
     E[0] = 0.0;
-    if (u32 == 1) Act32[0] = 0.0f;
+    if (u32) Act32[0] = 0.0f;
   }
 }
 
@@ -1142,13 +1138,6 @@ void launch_trans(const Geometry& g, const SolveBatch& b, const double* t, const
 // ------------------------------------------------------------ host launchers
 size_t eig2_tri_doubles(int n) { return (size_t)n * (n + 3); }
 
-void launch_tridiag_in_place(int n, int nsolves, double* C, cudaStream_t stream) {
-  if (nsolves == 0) return;
-  const size_t smem = sizeof(double) * ((size_t)n * (n + 1) / 2 + n);
-  cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  tridiag_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, C, C, (size_t)n * n, 2);
-}
-
 bool eig2_supported(const Geometry& g) {
   const bool vertical = g.vert_dist > 0.0;
   const int per = 1 + (vertical ? g.n_var : g.n);
@@ -1180,7 +1169,7 @@ void launch_eig2_t(const Geometry& g, const SolveBatch& b, const double* C, cons
     } else {
       cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem_t);
-      tridiag_kernel<<<ns, 32, smem_t, stream>>>(n, ns, C, tri, eig2_tri_doubles(n), u32);
+      tridiag_kernel<<<ns, 32, smem_t, stream>>>(n, ns, C, tri, u32);
     }
     if (ev_tri) record_event(ev_tri, stream);
   }

@@ -4,7 +4,7 @@
 // letkf_core.F90:98-225 diagonalises A; only W x (the state rows, or every unit
 // vector for an explicit trans) and overline_w = A^-1 t are used.  Both are
 // functions of T applied to vectors, so after the Householder reduction
-// (tridiag_kernel) this kernel computes, per vector, y = Q^T x, f(T) y and
+// (lg_tri.cu) this kernel computes, per vector, y = Q^T x, f(T) y and
 // Q f(T) y, with
 //   T^(-1/2) = sum_j w_j (T + s_j I)^-1,
 // the N-point midpoint rule of (2/pi) int_0^inf (T + s^2)^-1 ds in the variable
@@ -139,7 +139,8 @@ __device__ inline void cp_async8(void* dst, const void* src) {
 // vector), F (the forward solve), A (the sum over nodes); per block: the
 // factors R of 32 (slot, node) pairs -- in the reductions' phases the same
 // space holds two rows of reflectors per slot -- and T's two diagonals.
-// tri: per solve D[n] | E[n] | 1/h[n] (0: no reflector) | U, stride tri_stride.
+// tri: per solve D[n] | E[n] | H[n] (0: no reflector, else P = I - H u u^T) | U,
+// stride tri_stride.
 template <bool kCore>
 __global__ void ft_kernel(Geometry g, SolveBatch b, const double* tin, const double* tri,
                           size_t tri_stride, const double* xb, const double* axb, double* xa,
@@ -226,7 +227,7 @@ __global__ void ft_kernel(Geometry g, SolveBatch b, const double* tin, const dou
         const double* u = T + 3 * n + (size_t)i * (i - 1) / 2;
         double* d = ub + (size_t)(buf * slots + sl) * n;
         for (int c = lane; c < i; c += 32) ft::cp_async8(d + c, u + c);
-        if (lane == 0) ft::cp_async8(d + n - 1, T + 2 * n + i);  // 1/h (i <= n - 1: free)
+        if (lane == 0) ft::cp_async8(d + n - 1, T + 2 * n + i);  // H (i <= n - 1: free)
       }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };

@@ -282,7 +282,7 @@ void launch_eig_apply(const Geometry& g, const SolveBatch& b, const double* C, c
                       double* trans, double* wbar, int* eig_fail, cudaStream_t stream);
 size_t eig2_tri_doubles(int n);
 // FP64 transform without eigenvalues (lg_ft.cu), 7 to 64 members: tridiagonal
-// form in the Gram matrices' place (D | E | 1/h | reflectors), then the state
+// form in the Gram matrices' place (lg_tri.cu: D | E | H | reflectors), then the state
 // rows' update (core false, as launch_eig2's vectors) or explicit trans and
 // overline_w (core true, as launch_eig_apply's modes 1 and cubes).
 // prepare_ft_nodes: the node table, once per device, outside stream captures.

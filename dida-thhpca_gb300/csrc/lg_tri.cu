@@ -1,0 +1,356 @@
+// lg_tri.cu -- Householder reduction C = Q T Q^T of up to 64 members in fixed
+// point on the integer pipe (the FP64 path's tridiagonalisation).
+//
+// The FP64 pipe retires one warp instruction per 17 cycles per SM, the integer
+// pipe up to four a cycle, so a multiply-add of 59-bit fixed-point numbers
+// (three 32 x 32 -> 64-bit multiply-adds) costs less than a tenth of an FP64
+// one.  Everything in the reduction is bounded by |C| once C is scaled, so fixed
+// point loses nothing: C is scaled by a power of two 2^E just above its
+// Frobenius norm and held as integers of 2^(E-59), where FP64 would round each
+// result to 2^-53 of itself.
+//
+//   A   X = a 2^(59-E), |X| <= 2^59, held as Xh 2^30 + Xl, -2^29 <= Xl < 2^29
+//   w   the reflector P = I - w w^T, |w|^2 = 2, as w 2^58, split the same way
+//   p = A w, K = w^T p / 2, q = p - K w: integers of 2^(E-59);  A -= w q^T + q w^T
+// A product of an A-type and a w-type number is 4 Xh Wh + (Xh Wl + Xl Wh) / 2^28
+// (Xl Wl, below one unit, is dropped).  The row norms bound the sums (Cauchy):
+// sum Xh Wh < 2^58, sum Xh Wl < 2^61, sum Xl Wh < 2^61: no 64-bit sum overflows.
+// The two square roots of a step (the row's norm, and |u| of the reflector)
+// start from the FP32 reciprocal square root and take one third-order step in
+// integers, to about 2^-60.  No FP64 instruction is issued.
+//
+// One warp per matrix, the packed lower triangle in shared memory; lanes take
+// rows (split over lanes where fewer than 32 are left) in A w and elements in
+// the update, as in tridiag_kernel (lg_eig2.cu).  Output in the Gram matrix's
+// place: D[n] | E[n] | H[n] (1: reflector w, 0: none) | w rows (FP64).
+// A non-finite C gives a NaN diagonal, which the transform reports.
+//
+// Measured alone against tridiag_kernel: 921 600 matrices of 40 members 116 ->
+// 65 ms, 129 600 of 64 members 54 -> 34 ms, 2592 of 16 members 81 -> 66 us.  Bound
+// by instruction issue (0.68 of the slots at 40 members; 0.47 at 64, where the
+// triangles leave twelve warps per SM).
+#include "lg_device.cuh"
+#include "lg_internal.h"
+
+namespace lg {
+namespace tri {
+
+__device__ inline int idx(int j) { return j * (j + 1) / 2; }
+
+__device__ inline long long join(int2 v) { return (long long)v.y * (1 << 30) + v.x; }
+// x = y 2^30 + x', -2^29 <= x' < 2^29
+__device__ inline int2 split(long long v) {
+  const int h = (int)((v + (1 << 29)) >> 30);
+  return make_int2((int)v - (int)((unsigned)h << 30), h);
+}
+
+__device__ inline long long warp_add(long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// v 2^ex (ex from an exponent as 2^(ex)), rounded to nearest-even; results below
+// the normal range become 0
+__device__ inline double to_double(long long v, int ex) {
+  if (v == 0) return 0.0;
+  const bool neg = v < 0;
+  const unsigned long long m = neg ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int z = __clzll((long long)m);
+  const unsigned long long t = m << z;  // leading one at bit 63
+  unsigned long long mant = t >> 11;
+  const unsigned rest = (unsigned)t & 0x7ffu;
+  mant += (rest > 0x400u || (rest == 0x400u && (mant & 1))) ? 1 : 0;
+  const int e = 63 - z + ex + 1023 - 1;  // the leading one adds 1
+  if (e < 0) return 0.0;
+  const unsigned long long bits = ((unsigned long long)e << 52) + mant;
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
+// For v > 0: v = x 2^(2 r) with x in [1/4, 1); y = 1/sqrt(x) in units of 2^-60
+// (to about 2^-59), r returned.  y0 from FP32 (error below 2^-22), then
+// y = y0 (1 + e/2 + 3 e^2 / 8), e = 1 - x y0^2; the next term is below 2^-66.
+__device__ inline unsigned long long rsqrt_fixed(unsigned __int128 v, int& r) {
+  const unsigned long long vh = (unsigned long long)(v >> 64);
+  const int z = vh ? __clzll((long long)vh) : 64 + __clzll((long long)(unsigned long long)v);
+  const int p = 128 - z;       // v in [2^(p-1), 2^p)
+  r = (p + 1) >> 1;            // 2^(2r - 2) <= v < 2^(2r)
+  const int up = 128 - 2 * r;  // x = v 2^(-2r): 64-bit fraction = top 64 bits of v << up
+  const unsigned long long x = (unsigned long long)((v << up) >> 64);
+  const float y0f = rsqrtf((float)(unsigned)(x >> 32) * 2.3283064365386963e-10f);
+  const unsigned y0 = (unsigned)(y0f * 1073741824.0f);  // 2^30 y0, at most 2^31
+  const unsigned long long y2 = (unsigned long long)y0 * y0;  // 2^60 y0^2
+  const long long e = (1ll << 60) - (long long)__umul64hi(x, y2);
+  const long long e8 = e >> 8;
+  const long long c = (e >> 1) + ((3 * ((e8 * e8) >> 44)) >> 3);
+  return ((unsigned long long)y0 << 30) + (unsigned long long)(long long)(((__int128)c * y0) >> 30);
+}
+
+}  // namespace tri
+
+__global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, double* C) {
+  using namespace tri;
+  const int s = blockIdx.x;
+  if (s >= nsolves) return;
+  const int lane = threadIdx.x;
+  extern __shared__ int4 sm4[];
+  int4* const WQ = sm4;                                // n: (wl, wh, ql, qh)
+  int2* const A = reinterpret_cast<int2*>(sm4 + n);    // packed lower triangle
+  double* const M = C + (size_t)s * n * n;
+  const int np = idx(n);
+  // ---- scale: 2^E just above the Frobenius norm (FP32 sum relative to the
+  // largest exponent, rounded up)
+  unsigned emax = 0;
+  for (int t = lane; t < n * n; t += 32)
+    emax = max(emax, ((unsigned)__double2hiint(M[t]) >> 20) & 0x7ffu);
+  emax = __reduce_max_sync(0xffffffffu, emax);
+  double* const D = M;
+  double* const E = M + n;
+  double* const H = M + 2 * n;
+  double* const U = M + 3 * n;
+  if (emax == 0 || emax >= 2047u - 8u) {  // all zero, or not representable: NaN
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+      D[i] = emax ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+      E[i] = 0.0;
+      H[i] = 0.0;
+    }
+    return;
+  }
+  float fro = 0.0f;
+  for (int t = lane; t < n * n; t += 32) {
+    const int hi = __double2hiint(M[t]) & 0x7fffffff;
+    const int d = (int)emax - (hi >> 20);
+    // mantissa to 20 bits, rounded up, at 2^-d
+    const float f = d > 60 ? 0.0f
+                           : __int_as_float(((127 - d) << 23) | ((hi & 0xfffff) << 3)) * 1.00001f;
+    fro = fmaf(f, f, fro);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
+  // |C|_F < 2^(emax - 1023) sqrt(fro) 1.001; E = the exponent above
+  const int ef = (int)((__float_as_uint(sqrtf(fro) * 1.001f) >> 23) & 0xffu) - 127 + 1;
+  const int Eb = (int)emax + ef;  // E + 1023
+  {
+    int j = 0, c = lane;
+    while (c > j) {
+      c -= j + 1;
+      ++j;
+    }
+    for (int t = lane; t < np; t += 32) {
+      const double a = M[(size_t)j * n + c];
+      const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+      const int e = (int)(u >> 52) & 0x7ff;
+      long long x = 0;
+      if (e) {
+        const int sh = min(Eb - e, 62);  // >= 1
+        x = (long long)((((u & 0xfffffffffffffull) | 0x10000000000000ull) << 7) +
+                        (1ull << (sh - 1))) >> sh;
+        if (u >> 63) x = -x;
+      }
+      A[t] = split(x);
+      c += 32;
+      while (c > j) {
+        c -= j + 1;
+        ++j;
+      }
+    }
+  }
+  __syncwarp();
+  const int ex = Eb - 1023 - 59;  // a = X 2^ex
+  for (int i = n - 1; i >= 1; --i) {
+    const int l = i - 1;
+    int2* const row = A + idx(i);
+    // the row's integers, brought up to [2^56, 2^57) at the largest
+    long long x0 = lane <= l ? join(row[lane]) : 0, x1 = lane + 32 <= l ? join(row[lane + 32]) : 0;
+    const unsigned long long m0 = (unsigned long long)llabs(x0), m1 = (unsigned long long)llabs(x1);
+    const unsigned long long mm = m0 | m1;  // the leading bit is what counts
+    const unsigned mh = __reduce_or_sync(0xffffffffu, (unsigned)(mm >> 32));
+    const unsigned ml = __reduce_or_sync(0xffffffffu, (unsigned)mm);
+    double* const u_out = U + (size_t)i * (i - 1) / 2;
+    if (l == 0 || (mh | ml) == 0) {
+      // nothing to reduce: e is the element beside the diagonal
+      const long long e = __shfl_sync(0xffffffffu, l < 32 ? x0 : x1, l & 31);
+      for (int c = lane; c < i; c += 32) u_out[c] = 0.0;
+      if (lane == 0) {
+        E[i] = to_double(e, ex);
+        H[i] = 0.0;
+      }
+      __syncwarp();
+      continue;
+    }
+    const int lead = mh ? 63 - __clz((int)mh) : 31 - __clz((int)ml);
+    const int up = 56 - lead;  // may be negative (down to -3)
+    x0 = up >= 0 ? x0 << up : x0 >> -up;
+    x1 = up >= 0 ? x1 << up : x1 >> -up;
+    // squared norm in units of 2^30
+    const int2 s0 = split(x0), s1 = split(x1);
+    long long S1 = (long long)s0.y * s0.y + (long long)s1.y * s1.y;
+    long long S2 = 2 * ((long long)s0.y * s0.x + (long long)s1.y * s1.x) +
+                   (((long long)s0.x * s0.x + (long long)s1.x * s1.x) >> 30);
+    S1 = warp_add(S1);
+    S2 = warp_add(S2);
+    const unsigned __int128 N = ((unsigned __int128)(unsigned long long)S1 << 30) + (__int128)S2;
+    int r;
+    const unsigned long long yn = rsqrt_fixed(N, r);
+    // norm = sqrt(N 2^30) = N 2^30 / (2^(r + 15) x^(-1/2)...) = x y 2^(r + 15), x = N 2^(-2r)
+    const unsigned long long xn = (unsigned long long)((N << (128 - 2 * r)) >> 64);
+    // x y < 1: a fraction of 2^-60; norm' = (x y) 2^(r + 15), r + 15 in 57 .. 60
+    const unsigned long long rt = __umul64hi(xn, yn);
+    const int ds = 60 - (r + 15);  // 0 .. 3
+    const long long alpha = (long long)((rt + (ds ? 1ull << (ds - 1) : 0ull)) >> ds);
+    const long long f = __shfl_sync(0xffffffffu, l < 32 ? x0 : x1, l & 31);
+    const long long af = llabs(f);
+    // u_l = f + sign(f) alpha; h = N + |f| alpha (units of 2^30)
+    const unsigned __int128 hh = N + (((unsigned __int128)(unsigned long long)af *
+                                       (unsigned long long)alpha) >> 30);
+    int rh;
+    const unsigned long long yh = rsqrt_fixed(hh, rh);  // 1/sqrt(h) = yh 2^-60 2^-(rh + 15)
+    const long long ul = f >= 0 ? f + alpha : f - alpha;
+    if (lane == (l & 31)) {
+      if (l < 32)
+        x0 = ul;
+      else
+        x1 = ul;
+    }
+    // w 2^58 = u yh 2^(58 - 60 - rh - 15): (u 2^3)(yh) / 2^64 is u yh 2^-61, so a
+    // further shift by rh + 15 + 2 - 61 = rh - 44 (13 to 17: rh + 15 in 57 .. 61)
+    auto to_w = [&](long long x) -> long long {
+      const __int128 t = (__int128)x * (long long)yh;
+      const int sh = rh + 17;
+      return (long long)((t + ((__int128)1 << (sh - 1))) >> sh);
+    };
+    const long long w0 = to_w(x0), w1 = to_w(x1);
+    if (lane <= l) {
+      const int2 w = split(w0);
+      row[lane] = w;
+      WQ[lane].x = w.x;
+      WQ[lane].y = w.y;
+      u_out[lane] = to_double(w0, -58);
+    }
+    if (lane + 32 <= l) {
+      const int2 w = split(w1);
+      row[lane + 32] = w;
+      WQ[lane + 32].x = w.x;
+      WQ[lane + 32].y = w.y;
+      u_out[lane + 32] = to_double(w1, -58);
+    }
+    if (lane == 0) {
+      E[i] = to_double(f >= 0 ? -alpha : alpha, ex - up);
+      H[i] = 1.0;
+    }
+    __syncwarp();
+    // ---- p = A w: rows 0 .. nfull - 1 a lane each, the rest split over f lanes
+    const int R = l + 1;
+    const int nfull = R > 32 ? 32 : 0;
+    long long pf = 0, ps = 0;  // p of this lane's full row, of its split row
+    if (nfull) {
+      const int j = lane, tj = idx(j);
+      long long hs = 0, ms = 1 << 27;
+      int tc = 0;
+#pragma unroll 4
+      for (int c = 0; c < R; ++c) {
+        const int2 a = A[(c <= j) ? tj + c : tc + j];
+        const int2 w = row[c];
+        hs += (long long)a.y * w.y;
+        ms += (long long)a.y * w.x;
+        ms += (long long)a.x * w.y;
+        tc += c + 1;
+      }
+      pf = 4 * hs + (ms >> 28);
+    }
+    const int rr = R - nfull;                 // 1..32
+    const int lf = 31 - __clz(32 / rr);       // 2^lf lanes a row
+    const int fl = 1 << lf;
+    const int cl = (R + fl - 1) >> lf;
+    const int ri = lane >> lf, pi = lane & (fl - 1);
+    const bool act = ri < rr;
+    const int j = nfull + (act ? ri : 0);
+    {
+      const int c0 = act ? min(R, pi * cl) : 0, c1 = act ? min(R, c0 + cl) : 0;
+      const int tj = idx(j);
+      long long hs = 0, ms = 0;
+      int tc = idx(c0);
+#pragma unroll 4
+      for (int c = c0; c < c1; ++c) {
+        const int2 a = A[(c <= j) ? tj + c : tc + j];
+        const int2 w = row[c];
+        hs += (long long)a.y * w.y;
+        ms += (long long)a.y * w.x;
+        ms += (long long)a.x * w.y;
+        tc += c + 1;
+      }
+      for (int o = fl >> 1; o > 0; o >>= 1) {  // the same fl in every lane
+        hs += __shfl_xor_sync(0xffffffffu, hs, o);
+        ms += __shfl_xor_sync(0xffffffffu, ms, o);
+      }
+      ps = 4 * hs + ((ms + (1 << 27)) >> 28);
+    }
+    const bool own = act && pi == 0;  // this lane holds p_j of the split row
+    // ---- K = w^T p / 2
+    long long kh = 0, km = 0;
+    const int2 wf = nfull ? row[lane] : make_int2(0, 0), ws = own ? row[j] : make_int2(0, 0);
+    {
+      const int2 p = split(pf), p2 = split(ps);
+      kh = (long long)p.y * wf.y + (long long)p2.y * ws.y;
+      km = (long long)p.y * wf.x + (long long)p.x * wf.y + (long long)p2.y * ws.x +
+           (long long)p2.x * ws.y;
+    }
+    kh = warp_add(kh);
+    km = warp_add(km);
+    const int2 K = split((4 * kh + (km >> 28)) >> 1);
+    auto q_of = [&](long long p, int2 w) {
+      const long long m = (long long)K.y * w.x + ((long long)K.x * w.y + (1 << 27));
+      return split(p - (4 * ((long long)K.y * w.y) + (m >> 28)));
+    };
+    if (nfull) {
+      const int2 q = q_of(pf, wf);
+      WQ[lane].z = q.x;
+      WQ[lane].w = q.y;
+    }
+    if (own) {
+      const int2 q = q_of(ps, ws);
+      WQ[j].z = q.x;
+      WQ[j].w = q.y;
+    }
+    __syncwarp();
+    // ---- A -= w q^T + q w^T over the packed rows 0 .. l
+    {
+      const int tot = idx(l + 1);
+      int jr = 0, c = lane;
+      while (c > jr) {
+        c -= jr + 1;
+        ++jr;
+      }
+      for (int t = lane; t < tot; t += 32) {
+        const int4 a = WQ[jr], b = WQ[c];
+        const long long hs = (long long)a.y * b.w + (long long)a.w * b.y;
+        long long ms = (long long)a.y * b.z + (1 << 27);
+        ms += (long long)a.x * b.w;
+        ms += (long long)a.w * b.x;
+        ms += (long long)a.z * b.y;
+        A[t] = split(join(A[t]) - 4 * hs - (ms >> 28));
+        c += 32;
+        while (c > jr) {
+          c -= jr + 1;
+          ++jr;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  for (int i = lane; i < n; i += 32) D[i] = to_double(join(A[idx(i) + i]), ex);
+  if (lane == 0) {
+    E[0] = 0.0;
+    H[0] = 0.0;
+  }
+}
+
+void launch_tridiag_in_place(int n, int nsolves, double* C, cudaStream_t stream) {
+  if (nsolves == 0) return;
+  const size_t smem = sizeof(int4) * n + sizeof(int2) * ((size_t)n * (n + 1) / 2);
+  cudaFuncSetAttribute(tridiag_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  tridiag_fixed_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, C);
+}
+
+}  // namespace lg

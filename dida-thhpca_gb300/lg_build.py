@@ -31,6 +31,7 @@ UNITS = {
     "lg_gram_col.cu": [],
     "lg_eig2.cu": [],
     "lg_ft.cu": [],
+    "lg_tri.cu": [],
     "lg_noalloc.cu": [],
     "lg_prepost.cu": [],
     "lg_cube.cu": [],

@@ -73,3 +73,30 @@ def test_analysis_against_the_ql_route(name, ens, monkeypatch):
     i = slice(h, -h)
     inc = np.abs(out[1] - (w.xb + w.axb[..., None]))[i, i].max()
     assert np.abs(out[0] - out[1])[i, i].max() <= 1e-10 * inc
+
+
+@pytest.mark.parametrize("k", [7, 33, 64])
+def test_structured_gram_matrices(k):
+    """Rows that leave the fixed-point reduction (lg_tri.cu) nothing or little to
+    reduce: diagonal, already tridiagonal, zero rows and columns, one dominant
+    row, equal rows, and the same at scales far from one."""
+    rng = np.random.default_rng(1000 + k)
+    eye = np.eye(k)
+    tri = eye + np.diag(rng.standard_normal(k - 1), 1)   # z^T z tridiagonal
+    hole = rng.standard_normal((3 * k, k))
+    hole[:, [0, k // 2, k - 1]] = 0.0
+    spike = rng.standard_normal((2 * k, k))
+    spike[:, k - 2] *= 1e6
+    graded = rng.standard_normal((2 * k, k)) * 2.0 ** -np.arange(k)
+    shapes = [eye * rng.uniform(0.5, 2.0, k), tri, hole, spike, graded, graded[:, ::-1],
+              np.ones((k, k)), np.outer(np.ones(k), rng.standard_normal(k))]
+    cases = []
+    for z in shapes:
+        for scale in (1.0, 2.0 ** -60, 2.0 ** 12):
+            p = z.shape[0]
+            cases.append((np.ascontiguousarray(z * scale), np.ones(p, np.float32),
+                          rng.standard_normal(p), np.ones(p)))
+    st, tr, wb = _batch(cases, 1.1)
+    assert st == 0
+    for c, t, w in zip(cases, tr, wb):
+        _check(c, 1.1, t, w)
