@@ -70,7 +70,8 @@ struct lg_ctx {
   // solve workspace
   // per solve stream: Gram matrices and projected innovations of a chunk, and
   // the lane-parallel eigensolver's scratch (tridiagonal form, eigenvalues,
-  // rotation log, overflow list and count)
+  // rotation log, overflow list and count); in plain FP64 up to 64 members only
+  // lam, which then holds the vectors of the transform
   struct SolveLane {
     double *C = nullptr, *t = nullptr, *tri = nullptr, *lam = nullptr;
     double2* rot_cs = nullptr;
@@ -1208,6 +1209,7 @@ int prepare_capacity(lg_ctx* c) {
     r |= dalloc(&L.C, cap * k * k);
     r |= dalloc(&L.t, cap * k);
     r |= dalloc(&L.ovf_n, 1);
+    if (c->use_ft) r |= dalloc(&L.lam, cap * lg::ft_vec_doubles(geo));
     if (c->use_eig2 && !c->use_ft) {
       r |= dalloc(&L.tri, cap * lg::eig2_tri_doubles(k));
       r |= dalloc(&L.lam, cap * k);
@@ -1492,10 +1494,10 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
         lg::launch_tridiag_in_place(k, b.nsolves, L.C, st);
         CK(record_event(kv[3], st));
         for (int e = 4; e < 6; ++e) CK(record_event(kv[e], st));
-        lg::launch_ft(geo, b, true, L.t, L.C, (size_t)k * k, xb, axb, xa, axa, c->d_trans, nullptr,
+        lg::launch_ft(geo, b, true, L.t, L.C, c->d_trans, xb, axb, xa, axa, nullptr,
                       c->d_status + 1, st);
         CK(record_event(kv[6], st));
-        launches += 3;
+        launches += 6;
       } else {
         lg::launch_eig_apply(geo, b, L.C, L.t, xb, axb, xa, axa, c->d_trans, nullptr,
                              c->d_status + 1, st);
@@ -1608,9 +1610,9 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
         CK(cudaStreamWaitEvent(s_v, c->ev_phase[2][set], 0));
       }
       CK(record_event(kv[5], s_v));
-      lg::launch_ft(geo, b, false, L.t, L.C, (size_t)k * k, xb, axb, xa, axa, nullptr, nullptr,
-                    c->d_status + 1, s_v);
-      launches += 2;
+      lg::launch_ft(geo, b, false, L.t, L.C, L.lam, xb, axb, xa, axa, nullptr, c->d_status + 1,
+                    s_v);
+      launches += 4;
     } else if (c->use_eig2) {
       if (s_q == s_e) {
         lg::launch_eig2(geo, b, L.C, L.t, xb, axb, xa, axa, L.tri, L.lam, L.rot_cs, L.rot_i,
@@ -2364,8 +2366,7 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
     lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
   if (lg::ft_supported(geo)) {
     lg::launch_tridiag_in_place(ens, nbatch, C, st);
-    lg::launch_ft(geo, b, true, t, C, (size_t)ens * ens, nullptr, nullptr, nullptr, nullptr,
-                  d_trans, d_wbar, fail, st);
+    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, fail, st);
   } else {
     lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
                          st);

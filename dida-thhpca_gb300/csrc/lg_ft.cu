@@ -20,13 +20,21 @@
 // Why: the FP64 pipe retires a warp instruction per 17 cycles per SM.  Per
 // 64-member solve the QL iteration takes about 4000 rotations at 24 FP64
 // instructions (one lane each) and their replay 8 per rotation and vector; the
-// shifted solves take 5 per node, element and vector, plus 7 per node and
+// shifted solves take 4 per node, element and vector, plus 8 per node and
 // element for the factors, which the lanes of a solve compute for different
-// nodes.  Measured alone against QL + replay: 921 600 solves of 40 members
-// 233 -> 102 ms, 129 600 of 64 members 93 -> 46 ms; explicit trans against the
-// accumulating solver (lg_eig.cu): 32 768 cubes of 40 members 133 -> 29 ms (with
-// the reduction).  Faster at every size from 7 to 64 members; above, three
-// vectors per lane no longer leave an SM two warps.  Bound by the FP64 pipe.
+// nodes.  The reflections Q^T x and Q z (2 k^2 multiply-adds per vector) leave
+// the FP64 pipe altogether: a vector's norm does not change, so they run in
+// fixed point on the integer pipe as the reduction does (lg_tri.cu), to 2^-58 of
+// the norm per step.  Three kernels, so that the integer ones are not held to
+// the two to four warps per SM that the solves' five arrays leave:
+//   reflect_kernel (Q^T)  vectors in, y out
+//   ft_kernel             f(T) y, and T^-1 y of t
+//   reflect_kernel (Q)    z in; the rows' update, or the columns of W, out
+// and for an explicit trans add_wbar_kernel.  Measured alone against QL + replay:
+// 921 600 solves of 40 members 233 -> 71 ms, 129 600 of 64 members 93 -> 33 ms;
+// explicit trans against the accumulating solver (lg_eig.cu), with the
+// reduction: 32 768 cubes of 40 members 133 -> 15 ms.  Faster at every size from
+// 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
 #include <math.h>
 
@@ -34,6 +42,7 @@
 #include <mutex>
 
 #include "lg_device.cuh"
+#include "lg_fixed.cuh"
 #include "lg_internal.h"
 
 namespace lg {
@@ -128,57 +137,238 @@ __device__ inline void cp_async8(void* dst, const void* src) {
                : "memory");
 }
 
+// Which vectors a call works on: vector v of solve s -- 0: t (kept in the t
+// array's place), v >= 1: the state row v - 1 (analysis; in `vec`, element i at
+// ((s (n + 1) + i) (per - 1) + v - 1), element n being overline_w . x) or the
+// unit vector v - 1 (core; in trans, element i at so n n + i n + v - 1).
+struct Vecs {
+  int core, per;
+  double* t;
+  double* vec;  // or trans
+};
+__device__ inline double* vec_at(const Vecs& z, int n, size_t so, size_t s, int v, int& stride) {
+  if (v == 0) {
+    stride = 1;
+    return z.t + s * n;
+  }
+  stride = z.core ? n : z.per - 1;
+  return (z.core ? z.vec + so * n * n : z.vec + s * (n + 1) * (z.per - 1)) + (v - 1);
+}
+__device__ inline size_t out_index(const SolveBatch& b, int s) {
+  return b.s_col ? (size_t)b.first_solve + s : (size_t)s;
+}
+
+// This lane's vector V (element i at 32 i) from FP64 to integers of 2^(ex):
+// |V| < 2^(ex + 58), held as in lg_tri.cu; false if a value is not finite.
+__device__ inline bool to_fixed(double* V, int n, int& ex) {
+  unsigned emax = 0;
+  for (int i = 0; i < n; ++i)
+    emax = max(emax, ((unsigned)__double2hiint(V[32 * i]) >> 20) & 0x7ffu);
+  float fro = 0.0f;
+  for (int i = 0; i < n; ++i) {
+    const int hi = __double2hiint(V[32 * i]) & 0x7fffffff;
+    const int d = (int)emax - (hi >> 20);
+    const float f =
+        d > 60 ? 0.0f : __int_as_float(((127 - d) << 23) | ((hi & 0xfffff) << 3)) * 1.00001f;
+    fro = fmaf(f, f, fro);
+  }
+  // norm < 2^(emax - 1023) sqrt(fro) 1.001; the power of two above it
+  const int Eb = (int)emax + (int)((__float_as_uint(sqrtf(fro) * 1.001f) >> 23) & 0xffu) - 126;
+  for (int i = 0; i < n; ++i) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(V[32 * i]);
+    const int e = (int)(u >> 52) & 0x7ff;
+    long long x = 0;
+    if (e) {
+      const int sh = min(max(Eb - e, 1), 62);
+      x = (long long)((((u & 0xfffffffffffffull) | 0x10000000000000ull) << 6) + (1ull << (sh - 1))) >> sh;
+      if (u >> 63) x = -x;
+    }
+    reinterpret_cast<int2*>(V)[32 * i] = fixed_split(x);
+  }
+  ex = Eb - 1023 - 58;
+  return emax < 2047;
+}
+
 }  // namespace ft
 
-// Lanes are (slot, vector): slots = 32 / per solves of a warp, per vectors each.
-//   analysis (kCore false): vector 0 is t, vector v >= 1 the solve's state row
-//     v - 1; one warp per block.
-//   kCore: one solve per block, lane j of its ceil(k / 32) warps is the unit
-//     vector e_j; trans and overline_w = W (W t) / (k - 1) come out.
-// Shared memory per warp, [element][lane] so that lanes never conflict: Y (the
-// vector), F (the forward solve), A (the sum over nodes); per block: the
-// factors R of 32 (slot, node) pairs -- in the reductions' phases the same
-// space holds two rows of reflectors per slot -- and T's two diagonals.
-// tri: per solve D[n] | E[n] | H[n] (0: no reflector, else P = I - H u u^T) | U,
-// stride tri_stride.
-template <bool kCore>
-__global__ void ft_kernel(Geometry g, SolveBatch b, const double* tin, const double* tri,
-                          size_t tri_stride, const double* xb, const double* axb, double* xa,
-                          double* axa, double* trans_out, double* wbar_out, int* eig_fail) {
+// y <- Q^T x (kIn; P_{n-1} first) or Q z (P_1 first) of one vector per lane, one
+// warp per block, lanes numbered through the solves' vectors.  Reflector rows of
+// the (up to `slots`) solves that a warp spans come into shared memory a step
+// ahead of their use.
+template <bool kIn, bool kCore>
+__global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, ft::Vecs z,
+                                                     int slots, const double* tri, const double* xb,
+                                                     const double* axb, double* xa, double* axa) {
   const int n = g.ens;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int warps = kCore ? blockDim.x / 32 : 1;
-  const bool vertical = g.vert_dist > 0.0;
-  const int per = kCore ? 32 : 1 + (vertical ? g.n_var : g.n);
-  const int slots = 32 / per;
-  const int q = lane / per, v = lane - q * per;
-  const int s0 = kCore ? (int)blockIdx.x : (int)blockIdx.x * slots;
-  const int nsl = kCore ? 1 : min(slots, b.nsolves - s0);  // solves of this warp
+  const int lane = threadIdx.x;
+  // the rows' update needs no t: its vectors are v = 1 .. per - 1
+  const int v0 = !kIn && !kCore ? 1 : 0;
+  const int per = z.per - v0;
+  const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * per;
+  const int s_first = (int)(id0 / per);
+  const int nsl = (int)((min(id0 + 32, total) - 1) / per) - s_first + 1;
+  const bool mine = id0 + lane < total;
+  const int s = mine ? (int)((id0 + lane) / per) : s_first;
+  const int v = v0 + (mine ? (int)((id0 + lane) - (long long)s * per) : 0);
+  extern __shared__ double sm[];
+  double* const Y = sm + lane;                      // element i at 32 i
+  int2* const Yi = reinterpret_cast<int2*>(Y);
+  double* const ub = sm + 32 * n;                   // two buffers of slots x n
+  const size_t tri_stride = (size_t)n * n;
+  auto fetch = [&](int i, int buf) {
+    if (i >= 1 && i < n)
+      for (int sl = 0; sl < nsl; ++sl) {
+        const double* T = tri + (size_t)(s_first + sl) * tri_stride;
+        const double* u = T + 3 * n + (size_t)i * (i - 1) / 2;
+        double* d = ub + (size_t)(buf * slots + sl) * n;
+        for (int c = lane; c < i; c += 32) ft::cp_async8(d + c, u + c);
+        if (lane == 0) ft::cp_async8(d + n - 1, T + 2 * n + i);  // H (i <= n - 1: free)
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int step = kIn ? -1 : 1, i0 = kIn ? n - 1 : 1;
+  fetch(i0, 0);
+  // ---- the vector
+  int r_state = -1;
+  size_t ci = 0;
+  if (!kCore) {
+    const int col = b.first_col + s / b.levels;
+    const int kk = s % b.levels + 1;
+    const int glat = col % g.num_lat + 1, glon = col / g.num_lat + 1;
+    ci = (size_t)(glat - 1 + g.halo) + (size_t)(g.num_lat + 2 * g.halo) * (size_t)(glon - 1 + g.halo);
+    if (v >= 1) {
+      if (g.vert_dist <= 0.0)
+        r_state = v - 1;
+      else if (g.var_lev[v - 1] > 1)
+        r_state = g.var_start[v - 1] + kk - 1;
+      else if (kk == g.nz)
+        r_state = g.var_start[v - 1];
+    }
+  }
+  const bool row = mine && r_state >= 0;  // analysis: this solve updates the row
+  int vs;
+  double* const out = ft::vec_at(z, n, ft::out_index(b, s), s, v, vs);
+  const double* const xr = xb + (row ? (size_t)n * (r_state + (size_t)g.n * ci) : 0);
+  for (int i = 0; i < n; ++i) {
+    double x = 0.0;
+    if (kIn && kCore)
+      x = v == 0 ? out[i] : (i == v - 1 ? 1.0 : 0.0);
+    else if (kIn)
+      x = v == 0 ? out[i] : (row ? xr[i] : 0.0);
+    else if (kCore || row)
+      x = out[(size_t)i * vs];
+    Y[32 * i] = x;
+  }
+  int ex;
+  const bool finite = ft::to_fixed(Y, n, ex);
+  // ---- reflections: y -= w (w . y)
+  for (int c = 0, i = i0; c < n - 1; ++c, i += step) {
+    fetch(i + step, (c + 1) & 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const double* ud = ub + (size_t)((c & 1) * slots + (s - s_first)) * n;
+    const int2* u = reinterpret_cast<const int2*>(ud);
+    if (__double2hiint(ud[n - 1]) != 0) {
+      long long hs = 0, ms = 1 << 27;
+#pragma unroll 4
+      for (int j = 0; j < i; ++j) {
+        const int2 w = u[j], y = Yi[32 * j];
+        hs += (long long)y.y * w.y;
+        ms += (long long)y.y * w.x;
+        ms += (long long)y.x * w.y;
+      }
+      const int2 D = fixed_split(4 * hs + (ms >> 28));
+      const int D4 = -4 * D.y;  // |D| < 2^58.5
+#pragma unroll 4
+      for (int j = 0; j < i; ++j) {
+        const int2 w = u[j], y = Yi[32 * j];
+        const long long m = (long long)D.y * w.x + ((long long)D.x * w.y + (1 << 27));
+        Yi[32 * j] = fixed_split(fixed_join(y) + (long long)D4 * w.y - (int)(m >> 28));
+      }
+    }
+    __syncwarp();
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  // ---- out
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  if (kIn || kCore) {
+    if (mine)
+      for (int i = 0; i < n; ++i)
+        out[(size_t)i * vs] = finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
+  } else if (row) {
+    // xa = axb + sqrt(rho) x + (W - sqrt(rho) I) x + overline_w . x, recentred
+    const double srho = sqrt(g.inflation);
+    const double ab = axb[r_state + (size_t)g.n * ci];
+    const double dotw = out[(size_t)n * vs];
+    double mean = 0.0;
+    for (int i = 0; i < n; ++i) {
+      const double d = finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
+      const double x = ab + (srho * xr[i] + (d + dotw));
+      Y[32 * i] = x;
+      mean += x;
+    }
+    mean /= (double)n;
+    double* xo = xa + (size_t)n * (r_state + (size_t)g.n * ci);
+    for (int i = 0; i < n; ++i) xo[i] = Y[32 * i] - mean;
+    axa[r_state + (size_t)g.n * ci] = mean;
+  }
+}
+
+// f(T) y per lane, one warp per block.  Analysis: slots = 32 / per solves per
+// warp; v = 0 gives T^-1 y (overline_w in the reduced basis), the rows
+// (f(T) - sqrt(rho)) y and overline_w . x.  Core: lanes numbered through the
+// solves' vectors; unit vectors give f(T) y.
+// Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
+// F (the forward solve), A (the sum over nodes), and for 32 (slot, node) pairs
+// the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
+template <bool kCore>
+__global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
+                                                const double* tri, int* eig_fail) {
+  const int n = g.ens;
+  const int lane = threadIdx.x;
+  const int per = z.per;
+  int s_first, nsl, s, v;
+  bool mine;
+  if (kCore) {
+    const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * per;
+    s_first = (int)(id0 / per);
+    nsl = (int)((min(id0 + 32, total) - 1) / per) - s_first + 1;
+    mine = id0 + lane < total;
+    s = mine ? (int)((id0 + lane) / per) : s_first;
+    v = mine ? (int)((id0 + lane) - (long long)s * per) : 0;
+  } else {
+    s_first = blockIdx.x * slots;
+    nsl = min(slots, b.nsolves - s_first);
+    const int q = lane / per;
+    mine = q < nsl;
+    s = s_first + (mine ? q : 0);
+    v = mine ? lane - q * per : 0;
+  }
+  const int sl = s - s_first;
   extern __shared__ double sm[];
   const int cap = n * 32;
-  double* const Y = sm + (size_t)warp * 3 * cap;
-  double* const F = Y + cap;
-  double* const A = F + cap;
-  double* const R = sm + (size_t)warps * 3 * cap;  // n x 32
-  double* const Dg = R + cap;                      // slots x n: diagonal + shift
-  double* const Eg = Dg + slots * n;               // slots x n: Eg[i] couples i - 1 and i
-#define AT(a, i) (a)[(i) * 32 + lane]
+  double *const Y = sm + lane, *const F = Y + cap, *const A = F + cap;
+  double *const R = sm + 3 * cap, *const L = R + cap;
+  double* const Dg = L + cap;         // slots x n: diagonal + shift
+  double* const Eg = Dg + slots * n;  // slots x n: Eg[i] couples i - 1 and i
   const double shift = (double)(n - 1) / g.inflation;
-  const bool mine = kCore ? warp * 32 + lane < n : q < nsl;
-  const int s = s0 + (kCore ? 0 : q);
+  int vs;
+  double* const io = ft::vec_at(z, n, ft::out_index(b, s), s, v, vs);
+  if (mine)
+    for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
   // T, and per slot the node row (Gershgorin in FP32, rounded up)
-  __shared__ int s_row[32], s_bad[32];
-  for (int sl = warp; sl < nsl; sl += warps) {
-    const double* T = tri + (size_t)(s0 + sl) * tri_stride;
+  __shared__ int s_row[32];
+  for (int q = 0; q < nsl; ++q) {
+    const double* T = tri + (size_t)(s_first + q) * n * n;
     for (int i = lane; i < n; i += 32) {
-      Dg[sl * n + i] = T[i] + shift;
-      Eg[sl * n + i] = T[n + i];
+      Dg[q * n + i] = T[i] + shift;
+      Eg[q * n + i] = T[n + i];
     }
     __syncwarp();
     float mx = 0.0f;
     bool nf = false;
     for (int i = lane; i < n; i += 32) {
-      const double d = Dg[sl * n + i], e0 = Eg[sl * n + i], e1 = i + 1 < n ? Eg[sl * n + i + 1] : 0.0;
+      const double d = Dg[q * n + i], e0 = Eg[q * n + i], e1 = i + 1 < n ? Eg[q * n + i + 1] : 0.0;
       nf |= ((__double2hiint(d) >> 20) & 0x7ff) == 0x7ff || ((__double2hiint(e0) >> 20) & 0x7ff) == 0x7ff;
       mx = fmaxf(mx, fabsf(d2f_bits(d)) + fabsf(d2f_bits(e0)) + fabsf(d2f_bits(e1)));
     }
@@ -187,192 +377,97 @@ __global__ void ft_kernel(Geometry g, SolveBatch b, const double* tin, const dou
     if (lane == 0) {
       // smallest power of two above the bound
       const int ex = (int)((__float_as_uint(mx * (1.0001f / (float)shift)) >> 23) & 0xffu) - 127 + 1;
-      s_row[sl] = nf ? 0 : min(max(ex, 1), ft::kMaxLog);
-      s_bad[sl] = nf;
-      if (nf) atomicAdd(eig_fail, 1);  // as a QL iteration that never converges
+      s_row[q] = nf ? 0 : min(max(ex, 1), ft::kMaxLog);
+      // as a QL iteration that never converges; once per solve
+      if (nf && (!kCore || (long long)(s_first + q) * per >= (long long)blockIdx.x * 32))
+        atomicAdd(eig_fail, 1);
     }
   }
-  // ---- the vectors
-  int r_state = -1;
-  size_t ci = 0;
-  bool work = false;
-  if (kCore) {
-    work = mine;
-    for (int i = 0; i < n; ++i) AT(Y, i) = i == warp * 32 + lane ? 1.0 : 0.0;
-  } else if (mine) {
-    const int col = b.first_col + s / b.levels;
-    const int kk = s % b.levels + 1;
-    const int glat = col % g.num_lat + 1, glon = col / g.num_lat + 1;
-    ci = (size_t)(glat - 1 + g.halo) + (size_t)(g.num_lat + 2 * g.halo) * (size_t)(glon - 1 + g.halo);
-    if (v >= 1) {
-      if (!vertical)
-        r_state = v - 1;
-      else if (g.var_lev[v - 1] > 1)
-        r_state = g.var_start[v - 1] + kk - 1;
-      else if (kk == g.nz)
-        r_state = g.var_start[v - 1];
-    }
-    work = v == 0 || r_state >= 0;
-    const double* x = v == 0 ? tin + (size_t)s * n : xb + (size_t)n * (max(r_state, 0) + (size_t)g.n * ci);
-    for (int i = 0; i < n; ++i) AT(Y, i) = work ? x[i] : 0.0;
-  }
-  if (kCore) __syncthreads(); else __syncwarp();
-  // ---- y <- P_{n-1} first (Q^T) or P_1 first (Q), in place in V.  Row i's
-  // reflectors of every slot come into shared memory a step ahead.
-  double* const ub = R;  // two buffers of slots x n
-  auto fetch = [&](int i, int buf) {
-    if (i >= 1 && i < n)
-      for (int sl = warp; sl < nsl; sl += warps) {
-        const double* T = tri + (size_t)(s0 + sl) * tri_stride;
-        const double* u = T + 3 * n + (size_t)i * (i - 1) / 2;
-        double* d = ub + (size_t)(buf * slots + sl) * n;
-        for (int c = lane; c < i; c += 32) ft::cp_async8(d + c, u + c);
-        if (lane == 0) ft::cp_async8(d + n - 1, T + 2 * n + i);  // H (i <= n - 1: free)
-      }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  auto reflect_all = [&](double* V, bool transposed) {
-    const int step = transposed ? -1 : 1, i0 = transposed ? n - 1 : 1;
-    fetch(i0, 0);
-    for (int c = 0, i = i0; c < n - 1; ++c, i += step) {
-      fetch(i + step, (c + 1) & 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      if (kCore) __syncthreads(); else __syncwarp();
-      const double* u = ub + (size_t)((c & 1) * slots + (kCore ? 0 : min(q, slots - 1))) * n;
-      const double ih = u[n - 1];
-      if (ih != 0.0) {
-        double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0;
-        int j = 0;
-        for (; j + 3 < i; j += 4) {
-          d0 = fma(u[j], AT(V, j), d0);
-          d1 = fma(u[j + 1], AT(V, j + 1), d1);
-          d2 = fma(u[j + 2], AT(V, j + 2), d2);
-          d3 = fma(u[j + 3], AT(V, j + 3), d3);
-        }
-        for (; j < i; ++j) d0 = fma(u[j], AT(V, j), d0);
-        const double dot = -((d0 + d1) + (d2 + d3)) * ih;
-#pragma unroll 4
-        for (j = 0; j < i; ++j) AT(V, j) = fma(u[j], dot, AT(V, j));
-      }
-      if (kCore) __syncthreads(); else __syncwarp();
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (kCore) __syncthreads(); else __syncwarp();
-  };
-  reflect_all(Y, true);
-  // ---- A = sqrt(k - 1) sum_j w_j (T + s_j)^-1 y; the row lanes' last pass
-  // leaves vector 0 (t) with A = T^-1 y
-  const int nb = kCore ? 32 : 32 / slots;  // nodes per batch: lane = slot + slots * node
+  __syncwarp();
+  const int nb = 32 / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
   int nmax = 0;
-  for (int sl = 0; sl < nsl; ++sl) nmax = max(nmax, ft::g_count[s_row[sl]]);
-  const int fs = kCore ? 0 : lane % slots, fj = kCore ? lane : lane / slots;
+  for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
+  const int fs = lane % slots, fj = lane / slots;
   const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
-  for (int i = 0; i < n; ++i) AT(A, i) = 0.0;
+  for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
   auto factor = [&](double sigma) {
-    // R[i] = 1 / (pivot i of T + sigma) for this lane's (slot, node)
+    // T + sigma = U^T diag(1/R) U with U[i-1][i] = L[i], for this lane's pair
     const double *D = Dg + fs * n, *E = Eg + fs * n;
     double r = ft::rcp(D[0] + sigma);
-    AT(R, 0) = r;
+    R[lane] = r;
+#pragma unroll 2
     for (int i = 1; i < n; ++i) {
-      const double e = E[i];
-      r = ft::rcp(fma(-(e * r), e, D[i] + sigma));
-      AT(R, i) = r;
+      const double e = E[i], l = e * r;
+      r = ft::rcp(fma(-l, e, D[i] + sigma));
+      L[32 * i + lane] = l;
+      R[32 * i + lane] = r;
     }
   };
-  auto solve = [&](int rl, double w) {
-    // A += w (T + s)^-1 y with the factors of lane rl
-    const double* E = Eg + (kCore ? 0 : min(q, slots - 1)) * n;
-    const double* Rl = R + rl;
-    double f = Rl[0] * AT(Y, 0);
-    AT(F, 0) = f;
+  auto solve = [&](int pair, double w) {
+    // A += w (T + s)^-1 y with the factors of the pair; each recurrence's chain
+    // is one fused multiply-add per element
+    const double *Rp = R + pair, *Lp = L + pair;
+    double f = Y[0];
+    F[0] = f;
 #pragma unroll 4
     for (int i = 1; i < n; ++i) {
-      f = Rl[i * 32] * fma(-E[i], f, AT(Y, i));
-      AT(F, i) = f;
+      f = fma(-Lp[32 * i], f, Y[32 * i]);
+      F[32 * i] = f;
     }
-    double x = f;
-    AT(A, n - 1) = fma(w, x, AT(A, n - 1));
+    double x = Rp[32 * (n - 1)] * f;
+    A[32 * (n - 1)] = fma(w, x, A[32 * (n - 1)]);
 #pragma unroll 4
     for (int i = n - 2; i >= 0; --i) {
-      x = fma(-Rl[i * 32], E[i + 1] * x, AT(F, i));
-      AT(A, i) = fma(w, x, AT(A, i));
+      x = fma(-Lp[32 * (i + 1)], x, Rp[32 * i] * F[32 * i]);
+      A[32 * i] = fma(w, x, A[32 * i]);
     }
   };
   for (int j0 = 0; j0 < nmax; j0 += nb) {
-    if (warp == 0 && fs < nsl && fj < nb && j0 + fj < nmax)
-      factor(ft::g_nodes[s_row[fs]][j0 + fj].x * shift);
-    if (kCore) __syncthreads(); else __syncwarp();
-    for (int j = 0; j < nb && j0 + j < nmax; ++j) {
-      if (mine) {
-        const int row = s_row[kCore ? 0 : q];
-        solve(kCore ? j : q + slots * j, ft::g_nodes[row][j0 + j].y * wscale);
-      }
-    }
-    if (kCore) __syncthreads(); else __syncwarp();
-  }
-  if (!kCore) {
-    if (lane < nsl) factor(0.0);  // lanes 0 .. slots - 1 are (slot, node 0)
+    if (fs < nsl && fj < nb && j0 + fj < nmax) factor(ft::g_nodes[s_row[fs]][j0 + fj].x * shift);
     __syncwarp();
-    if (mine && v == 0) {
-      for (int i = 0; i < n; ++i) AT(A, i) = 0.0;
-      solve(q, 1.0);
-    }
-    __syncwarp();
-    // dot = overline_w . x in the reduced basis; A becomes (W - sqrt(rho) I) y
-    const double srho = sqrt(g.inflation);
-    double dotw = 0.0;
-    if (mine && v >= 1) {
-      const double* zt = A + q * per;
-      for (int i = 0; i < n; ++i) {
-        const double y = AT(Y, i);
-        dotw = fma(y, zt[i * 32], dotw);
-        AT(A, i) = fma(-srho, y, AT(A, i));
-      }
-    }
-    __syncwarp();
-    reflect_all(A, false);
-    if (work && v >= 1) {
-      // xa = axb + sqrt(rho) x + (W - sqrt(rho) I) x + overline_w . x, recentred
-      const double ab = axb[r_state + (size_t)g.n * ci];
-      const double* xr = xb + (size_t)n * (r_state + (size_t)g.n * ci);
-      double mean = 0.0;
-      for (int i = 0; i < n; ++i) {
-        const double x = ab + (srho * xr[i] + (AT(A, i) + dotw));
-        AT(A, i) = x;
-        mean += x;
-      }
-      mean /= (double)n;
-      double* xo = xa + (size_t)n * (r_state + (size_t)g.n * ci);
-      for (int i = 0; i < n; ++i) xo[i] = AT(A, i) - mean;
-      axa[r_state + (size_t)g.n * ci] = mean;
-    }
-  } else {
-    reflect_all(A, false);  // lane j: column j of W
-    // overline_w = W (W t) / (k - 1): each lane a dot product with its column
-    double* const tv = R;         // t, then W t
-    double* const wt = R + n;
-    const double* t = tin + (size_t)s * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) tv[i] = t[i];
-    __syncthreads();
-    double d = 0.0;
-    if (mine)
-      for (int i = 0; i < n; ++i) d = fma(AT(A, i), tv[i], d);
-    if (mine) wt[warp * 32 + lane] = d;
-    __syncthreads();
-    d = 0.0;
     if (mine) {
-      for (int i = 0; i < n; ++i) d = fma(AT(A, i), wt[i], d);
-      d /= (double)(n - 1);
-      // trans(i, j) = W(i, j) + overline_w(i), column-major; W is symmetric, so
-      // this lane's column is also row i = its index
-      const size_t so = b.s_col ? (size_t)b.first_solve + s : (size_t)s;
-      const int i = warp * 32 + lane;
-      double* To = trans_out + so * n * n;
-      for (int j = 0; j < n; ++j) To[i + (size_t)n * j] = AT(A, j) + d;
-      if (wbar_out) wbar_out[so * n + i] = d;
+      const int rowq = s_row[sl];
+      for (int j = 0; j < nb && j0 + j < nmax; ++j)
+        solve(sl + slots * j, ft::g_nodes[rowq][j0 + j].y * wscale);
     }
+    __syncwarp();
   }
-#undef AT
+  if (lane < nsl) factor(0.0);  // pair (slot, 0)
+  __syncwarp();
+  if (mine && v == 0) {
+    for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
+    solve(sl, 1.0);
+  }
+  __syncwarp();
+  if (!mine) return;
+  if (!kCore && v >= 1) {
+    const double srho = sqrt(g.inflation);
+    const double* zt = sm + 2 * cap + sl * per;  // vector 0's A
+    double dotw = 0.0;
+    for (int i = 0; i < n; ++i) {
+      const double y = Y[32 * i];
+      dotw = fma(y, zt[32 * i], dotw);
+      io[(size_t)i * vs] = fma(-srho, y, A[32 * i]);
+    }
+    io[(size_t)n * vs] = dotw;
+  } else if (kCore) {
+    for (int i = 0; i < n; ++i) io[(size_t)i * vs] = A[32 * i];
+  }
+}
+
+// trans(i, j) = W(i, j) + overline_w(i), column-major; W is symmetric, so its
+// row j comes in place of column j
+__global__ void add_wbar_kernel(int n, SolveBatch b, const double* t, double* trans, double* wbar) {
+  const int s = blockIdx.x;
+  const size_t so = ft::out_index(b, s);
+  const double* w = t + (size_t)s * n;
+  double* To = trans + so * n * n;
+  for (int r = threadIdx.x, i = r % n; r < n * n; r += blockDim.x) {
+    To[r] += w[i];
+    i = (i + blockDim.x) % n;
+  }
+  if (wbar)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) wbar[so * n + i] = w[i];
 }
 
 bool ft_supported(const Geometry& g) {
@@ -381,24 +476,41 @@ bool ft_supported(const Geometry& g) {
   return g.ens >= 7 && g.ens <= 64 && (g.ql_max_iter == 0 || g.ql_max_iter >= 60);
 }
 
-void launch_ft(const Geometry& g, const SolveBatch& b, bool core, const double* t,
-               const double* tri, size_t tri_stride, const double* xb, const double* axb,
-               double* xa, double* axa, double* trans, double* wbar, int* eig_fail,
-               cudaStream_t stream) {
+size_t ft_vec_doubles(const Geometry& g) {
+  return (size_t)(g.ens + 1) * (g.vert_dist > 0.0 ? g.n_var : g.n);
+}
+
+void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, const double* tri,
+               double* vec, const double* xb, const double* axb, double* xa, double* axa,
+               double* wbar, int* eig_fail, cudaStream_t stream) {
   if (b.nsolves == 0) return;
   const int n = g.ens;
-  const bool vertical = g.vert_dist > 0.0;
-  const int slots = core ? 1 : 32 / (1 + (vertical ? g.n_var : g.n));
-  const int warps = core ? (n + 31) / 32 : 1;
-  const size_t smem = sizeof(double) * ((size_t)(3 * warps + 1) * 32 * n + 2 * (size_t)slots * n);
+  const int per = core ? n + 1 : 1 + (g.vert_dist > 0.0 ? g.n_var : g.n);
+  const ft::Vecs z{core ? 1 : 0, per, t, vec};
+  // solves that 32 consecutive vectors can touch
+  auto spans = [](int p) { return (32 + p - 2) / p + 1; };
+  auto blocks = [&](int p) { return (unsigned)(((long long)b.nsolves * p + 31) / 32); };
+  auto reflect = [&](auto kernel, int p) {
+    const int sl = spans(p);
+    const size_t smem = sizeof(double) * ((size_t)32 * n + 2 * (size_t)sl * n);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<blocks(p), 32, smem, stream>>>(g, b, z, sl, tri, xb, axb, xa, axa);
+  };
+  auto solve = [&](auto kernel, int sl, unsigned grid) {
+    const size_t smem = sizeof(double) * ((size_t)5 * 32 * n + 2 * (size_t)sl * n);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<grid, 32, smem, stream>>>(g, b, z, sl, tri, eig_fail);
+  };
   if (core) {
-    cudaFuncSetAttribute(ft_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ft_kernel<true><<<b.nsolves, 32 * warps, smem, stream>>>(g, b, t, tri, tri_stride, xb, axb, xa,
-                                                             axa, trans, wbar, eig_fail);
+    reflect(reflect_kernel<true, true>, per);
+    solve(ft_kernel<true>, spans(per), blocks(per));
+    reflect(reflect_kernel<false, true>, per);
+    add_wbar_kernel<<<b.nsolves, 128, 0, stream>>>(n, b, t, vec, wbar);
   } else {
-    cudaFuncSetAttribute(ft_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ft_kernel<false><<<(b.nsolves + slots - 1) / slots, 32, smem, stream>>>(
-        g, b, t, tri, tri_stride, xb, axb, xa, axa, trans, wbar, eig_fail);
+    const int sl = 32 / per;
+    reflect(reflect_kernel<true, false>, per);
+    solve(ft_kernel<false>, sl, (unsigned)((b.nsolves + sl - 1) / sl));
+    reflect(reflect_kernel<false, false>, per - 1);
   }
 }
 

@@ -52,6 +52,7 @@
 // outside 2^+-400, is marked by a bit pattern in its first Gram element that no
 // other solve can produce, and redone by gram64_kernel.
 #include "lg_device.cuh"
+#include "lg_fixed.cuh"
 #include "lg_internal.h"
 #include "lg_tc.cuh"
 
@@ -129,25 +130,6 @@ __device__ inline void bar_sync(int id, int count) {
 }
 __device__ inline void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-
-// v 2^ex rounded to nearest-even
-__device__ inline double fixed_to_double(long long v, int ex) {
-  if (v == 0) return 0.0;
-  const bool neg = v < 0;
-  const unsigned long long m = neg ? 0ull - (unsigned long long)v : (unsigned long long)v;
-  const int z = __clzll((long long)m);
-  unsigned long long mant;
-  if (z >= 11) {
-    mant = m << (z - 11);
-  } else {
-    const int drop = 11 - z;
-    mant = m >> drop;
-    const unsigned long long rest = m << (64 - drop);
-    mant += (rest > 0x8000000000000000ull || (rest == 0x8000000000000000ull && (mant & 1))) ? 1 : 0;
-  }
-  const unsigned long long bits = ((unsigned long long)(63 - z + ex + 1023 - 1) << 52) + mant;
-  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
 // (hi 2^27 + lo) 2^ex rounded to nearest-even

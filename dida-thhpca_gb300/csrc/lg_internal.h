@@ -283,16 +283,17 @@ void launch_eig_apply(const Geometry& g, const SolveBatch& b, const double* C, c
 size_t eig2_tri_doubles(int n);
 // FP64 transform without eigenvalues (lg_ft.cu), 7 to 64 members: tridiagonal
 // form in the Gram matrices' place (lg_tri.cu: D | E | H | reflectors), then the state
-// rows' update (core false, as launch_eig2's vectors) or explicit trans and
-// overline_w (core true, as launch_eig_apply's modes 1 and cubes).
+// rows' update (core false, as launch_eig2's vectors; vec: ft_vec_doubles per
+// solve of scratch) or explicit trans and overline_w (core true, as
+// launch_eig_apply's modes 1 and cubes; vec: trans).  t is overwritten.
 // prepare_ft_nodes: the node table, once per device, outside stream captures.
 bool ft_supported(const Geometry& g);
 int prepare_ft_nodes();
 void launch_tridiag_in_place(int n, int nsolves, double* C, cudaStream_t stream);
-void launch_ft(const Geometry& g, const SolveBatch& b, bool core, const double* t,
-               const double* tri, size_t tri_stride, const double* xb, const double* axb,
-               double* xa, double* axa, double* trans, double* wbar, int* eig_fail,
-               cudaStream_t stream);
+size_t ft_vec_doubles(const Geometry& g);
+void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, const double* tri,
+               double* vec, const double* xb, const double* axb, double* xa, double* axa,
+               double* wbar, int* eig_fail, cudaStream_t stream);
 bool eig2_supported(const Geometry& g);
 // mixed path, cube solves: explicit trans of each solve from the tridiagonal
 // form and rotation log (solves with rot_n < 0 are left to eig_apply)

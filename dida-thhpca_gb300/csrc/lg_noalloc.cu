@@ -104,8 +104,7 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
     lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
   if (lg::ft_supported(geo)) {
     lg::launch_tridiag_in_place(ens, nbatch, C, st);
-    lg::launch_ft(geo, b, true, t, C, (size_t)ens * ens, nullptr, nullptr, nullptr, nullptr,
-                  d_trans, d_wbar, fail, st);
+    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, fail, st);
   } else {
     lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
                          st);

@@ -22,7 +22,8 @@
 // One warp per matrix, the packed lower triangle in shared memory; lanes take
 // rows (split over lanes where fewer than 32 are left) in A w and elements in
 // the update, as in tridiag_kernel (lg_eig2.cu).  Output in the Gram matrix's
-// place: D[n] | E[n] | H[n] (1: reflector w, 0: none) | w rows (FP64).
+// place: D[n] | E[n] | H[n] (1: reflector w, 0: none) | w rows (w 2^58 as pairs
+// of 32-bit integers).
 // A non-finite C gives a NaN diagonal, which the transform reports.
 //
 // Measured alone against tridiag_kernel: 921 600 matrices of 40 members 116 ->
@@ -30,6 +31,7 @@
 // by instruction issue (0.68 of the slots at 40 members; 0.47 at 64, where the
 // triangles leave twelve warps per SM).
 #include "lg_device.cuh"
+#include "lg_fixed.cuh"
 #include "lg_internal.h"
 
 namespace lg {
@@ -37,34 +39,10 @@ namespace tri {
 
 __device__ inline int idx(int j) { return j * (j + 1) / 2; }
 
-__device__ inline long long join(int2 v) { return (long long)v.y * (1 << 30) + v.x; }
-// x = y 2^30 + x', -2^29 <= x' < 2^29
-__device__ inline int2 split(long long v) {
-  const int h = (int)((v + (1 << 29)) >> 30);
-  return make_int2((int)v - (int)((unsigned)h << 30), h);
-}
-
 __device__ inline long long warp_add(long long v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// v 2^ex (ex from an exponent as 2^(ex)), rounded to nearest-even; results below
-// the normal range become 0
-__device__ inline double to_double(long long v, int ex) {
-  if (v == 0) return 0.0;
-  const bool neg = v < 0;
-  const unsigned long long m = neg ? 0ull - (unsigned long long)v : (unsigned long long)v;
-  const int z = __clzll((long long)m);
-  const unsigned long long t = m << z;  // leading one at bit 63
-  unsigned long long mant = t >> 11;
-  const unsigned rest = (unsigned)t & 0x7ffu;
-  mant += (rest > 0x400u || (rest == 0x400u && (mant & 1))) ? 1 : 0;
-  const int e = 63 - z + ex + 1023 - 1;  // the leading one adds 1
-  if (e < 0) return 0.0;
-  const unsigned long long bits = ((unsigned long long)e << 52) + mant;
-  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
 // For v > 0: v = x 2^(2 r) with x in [1/4, 1); y = 1/sqrt(x) in units of 2^-60
@@ -148,7 +126,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
                         (1ull << (sh - 1))) >> sh;
         if (u >> 63) x = -x;
       }
-      A[t] = split(x);
+      A[t] = fixed_split(x);
       c += 32;
       while (c > j) {
         c -= j + 1;
@@ -162,18 +140,18 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     const int l = i - 1;
     int2* const row = A + idx(i);
     // the row's integers, brought up to [2^56, 2^57) at the largest
-    long long x0 = lane <= l ? join(row[lane]) : 0, x1 = lane + 32 <= l ? join(row[lane + 32]) : 0;
+    long long x0 = lane <= l ? fixed_join(row[lane]) : 0, x1 = lane + 32 <= l ? fixed_join(row[lane + 32]) : 0;
     const unsigned long long m0 = (unsigned long long)llabs(x0), m1 = (unsigned long long)llabs(x1);
     const unsigned long long mm = m0 | m1;  // the leading bit is what counts
     const unsigned mh = __reduce_or_sync(0xffffffffu, (unsigned)(mm >> 32));
     const unsigned ml = __reduce_or_sync(0xffffffffu, (unsigned)mm);
-    double* const u_out = U + (size_t)i * (i - 1) / 2;
+    int2* const u_out = reinterpret_cast<int2*>(U) + (size_t)i * (i - 1) / 2;
     if (l == 0 || (mh | ml) == 0) {
       // nothing to reduce: e is the element beside the diagonal
       const long long e = __shfl_sync(0xffffffffu, l < 32 ? x0 : x1, l & 31);
-      for (int c = lane; c < i; c += 32) u_out[c] = 0.0;
+      for (int c = lane; c < i; c += 32) u_out[c] = make_int2(0, 0);
       if (lane == 0) {
-        E[i] = to_double(e, ex);
+        E[i] = fixed_to_double(e, ex);
         H[i] = 0.0;
       }
       __syncwarp();
@@ -184,7 +162,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     x0 = up >= 0 ? x0 << up : x0 >> -up;
     x1 = up >= 0 ? x1 << up : x1 >> -up;
     // squared norm in units of 2^30
-    const int2 s0 = split(x0), s1 = split(x1);
+    const int2 s0 = fixed_split(x0), s1 = fixed_split(x1);
     long long S1 = (long long)s0.y * s0.y + (long long)s1.y * s1.y;
     long long S2 = 2 * ((long long)s0.y * s0.x + (long long)s1.y * s1.x) +
                    (((long long)s0.x * s0.x + (long long)s1.x * s1.x) >> 30);
@@ -222,21 +200,21 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     };
     const long long w0 = to_w(x0), w1 = to_w(x1);
     if (lane <= l) {
-      const int2 w = split(w0);
+      const int2 w = fixed_split(w0);
       row[lane] = w;
       WQ[lane].x = w.x;
       WQ[lane].y = w.y;
-      u_out[lane] = to_double(w0, -58);
+      u_out[lane] = w;
     }
     if (lane + 32 <= l) {
-      const int2 w = split(w1);
+      const int2 w = fixed_split(w1);
       row[lane + 32] = w;
       WQ[lane + 32].x = w.x;
       WQ[lane + 32].y = w.y;
-      u_out[lane + 32] = to_double(w1, -58);
+      u_out[lane + 32] = w;
     }
     if (lane == 0) {
-      E[i] = to_double(f >= 0 ? -alpha : alpha, ex - up);
+      E[i] = fixed_to_double(f >= 0 ? -alpha : alpha, ex - up);
       H[i] = 1.0;
     }
     __syncwarp();
@@ -291,17 +269,17 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     long long kh = 0, km = 0;
     const int2 wf = nfull ? row[lane] : make_int2(0, 0), ws = own ? row[j] : make_int2(0, 0);
     {
-      const int2 p = split(pf), p2 = split(ps);
+      const int2 p = fixed_split(pf), p2 = fixed_split(ps);
       kh = (long long)p.y * wf.y + (long long)p2.y * ws.y;
       km = (long long)p.y * wf.x + (long long)p.x * wf.y + (long long)p2.y * ws.x +
            (long long)p2.x * ws.y;
     }
     kh = warp_add(kh);
     km = warp_add(km);
-    const int2 K = split((4 * kh + (km >> 28)) >> 1);
+    const int2 K = fixed_split((4 * kh + (km >> 28)) >> 1);
     auto q_of = [&](long long p, int2 w) {
       const long long m = (long long)K.y * w.x + ((long long)K.x * w.y + (1 << 27));
-      return split(p - (4 * ((long long)K.y * w.y) + (m >> 28)));
+      return fixed_split(p - (4 * ((long long)K.y * w.y) + (m >> 28)));
     };
     if (nfull) {
       const int2 q = q_of(pf, wf);
@@ -329,7 +307,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
         ms += (long long)a.x * b.w;
         ms += (long long)a.w * b.x;
         ms += (long long)a.z * b.y;
-        A[t] = split(join(A[t]) - 4 * hs - (ms >> 28));
+        A[t] = fixed_split(fixed_join(A[t]) - 4 * hs - (ms >> 28));
         c += 32;
         while (c > jr) {
           c -= jr + 1;
@@ -339,7 +317,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     }
     __syncwarp();
   }
-  for (int i = lane; i < n; i += 32) D[i] = to_double(join(A[idx(i) + i]), ex);
+  for (int i = lane; i < n; i += 32) D[i] = fixed_to_double(fixed_join(A[idx(i) + i]), ex);
   if (lane == 0) {
     E[0] = 0.0;
     H[0] = 0.0;
