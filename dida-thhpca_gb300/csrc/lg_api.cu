@@ -21,6 +21,7 @@
 #include <initializer_list>
 
 #include <algorithm>
+#include <mutex>
 #include <thread>
 #include <vector>
 
@@ -307,16 +308,21 @@ void neighbour_blocks(const lg_ctx* c, int bx, int by, std::vector<int>& out) {
   }
 }
 
-// Host threads for the observation ingest: one per core, at most 16, and
-// none beyond one per min_per items.  LETKF_GB300_HOST_THREADS sets the count
-// (at most one per item), which the tests use to compare thread counts.
-int host_threads(int64_t n, int64_t min_per) {
-  int hw = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
+// Host threads for the observation ingest of n items: one per 2^13 items, at
+// most four below 2^18 items and one per core, at most 16, from there on.
+// Measured (whole lg_set_obs, 16 Arm cores): four threads cost 0.25 ms to start
+// and join three times, 16 cost 4 ms.  2000 observations 0.3 ms on one thread, 4.2
+// on 16; 60 000: 3.2 on one, 1.7 on four, 4.9 on 16; 250 000: 13.5, 5.5, 6.5 (5.1
+// on eight); 10^6: 55, 22, 15.2.  LETKF_GB300_HOST_THREADS sets the count (at
+// most one per item), which the tests use to compare thread counts.
+int host_threads(int64_t n) {
+  int hw = std::max(1, std::min(n < (1 << 18) ? 4 : 16, (int)std::thread::hardware_concurrency()));
+  int64_t min_per = 1 << 13;
   if (const char* env = getenv("LETKF_GB300_HOST_THREADS")) {
     hw = std::max(1, std::min(64, atoi(env)));
     min_per = 1;
   }
-  return (int)std::max<int64_t>(1, std::min<int64_t>(hw, n / std::max<int64_t>(1, min_per)));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(hw, n / min_per));
 }
 
 // fn(t, begin, end) over [0, n) in nt contiguous ascending ranges (range t on
@@ -735,7 +741,7 @@ int lg_set_obs(lg_ctx* c, const lg_obs_soa* o) {
   // after those of threads < t in every (block, type) segment, so that the
   // copies of a segment ascend by observation as in a serial pass.
   const size_t nbt = (size_t)nb * T;
-  const int nth = host_threads(n, 1 << 15);
+  const int nth = host_threads(n);
   std::vector<std::vector<int>> cnt_t(nth, std::vector<int>(nbt, 0));
   std::vector<int> rows_of(n * 2), cols_of(n * 2);
   std::vector<unsigned char> nrow(n), ncolb(n);
@@ -877,7 +883,7 @@ int lg_set_obs(lg_ctx* c, const lg_obs_soa* o) {
     for (int sg = 0; sg < nseg; ++sg) max_len = std::max(max_len, bt_off[sg + 1] - bt_off[sg]);
     // segments are independent: cells and boxes, then (after the layout of
     // cell_start) the per-segment counting sort, each on host threads
-    const int nts = host_threads(nseg, 1);
+    const int nts = std::min(nseg, host_threads(ncopies));
     run_ranges(nts, nseg, [&](int, int64_t s0, int64_t s1) {
       for (int sg = (int)s0; sg < (int)s1; ++sg) {
         const int j0 = bt_off[sg], j1 = bt_off[sg + 1];
@@ -2321,17 +2327,64 @@ void lg_destroy(lg_ctx* c) {
   delete c;
 }
 
-int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
+namespace {
+// Device memory of the core entry points (one call's Gram matrices, projections
+// and, for lg_letkf_core, its arrays): a stream-ordered pool per device that
+// keeps up to kPoolKeep bytes between calls and returns the rest to the device
+// when a stream is synchronised.  The runtime makes it safe for several threads
+// and streams.  (A cudaMalloc and cudaFree pair per array cost 0.3 ms of a 0.57 ms
+// single-column call.)
+constexpr uint64_t kPoolKeep = (uint64_t)64 << 20;
+cudaMemPool_t core_pool() {
+  constexpr int kMaxDevices = 64;
+  static cudaMemPool_t pools[kMaxDevices] = {};
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      pools[dev] = nullptr;
+    }
+  }
+  return pools[dev];
+}
+
+struct PoolBuf {
+  void* p = nullptr;
+  cudaStream_t st;
+  explicit PoolBuf(cudaStream_t s) : st(s) {}
+  PoolBuf(const PoolBuf&) = delete;
+  int alloc(size_t bytes) {
+    if (bytes > alloc_limit_bytes()) return LG_ERR_NOMEM;
+    const cudaMemPool_t pool = core_pool();
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaErrorUnknown;
+    if (e == cudaSuccess) return LG_OK;
+    fprintf(stderr, "letkf_gb300: device allocation of %zu bytes failed: %s\n", bytes,
+            cudaGetErrorString(e));
+    cudaGetLastError();
+    p = nullptr;
+    return LG_ERR_NOMEM;
+  }
+  ~PoolBuf() {
+    if (p && cudaFreeAsync(p, st) != cudaSuccess) cudaGetLastError();
+  }
+};
+
+// the batched core's kernels on st (C, t: work arrays; *fail: cleared, then the
+// Gram's status or the count of failed eigensolves)
+void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
                   const double* d_hxens, const float* d_rdiaginv, const double* d_dep,
-                  const double* d_rloc, double inflation, int precision, double* d_trans,
-                  double* d_wbar, void* stream_v) {
-  if (ens < 2 || ens > 128 || nbatch < 0 || inflation <= 0.0) return LG_ERR_ARG;
-  if (precision != LG_PREC_FP64 && !lg::mixed_precision(precision)) return LG_ERR_ARG;
-  if (precision == LG_PREC_MIXED_TF32 && !lg::gram_tf32_supported(ens)) return LG_ERR_UNSUPPORTED;
-  if (nbatch == 0) return LG_OK;
-  if (!d_nobsl || !d_off || !d_trans || !d_wbar) return LG_ERR_ARG;
-  if (lg::prepare_ft_nodes() != LG_OK) return LG_ERR_CUDA;
-  cudaStream_t st = (cudaStream_t)stream_v;
+                  const double* d_rloc, double inflation, int precision, double* C, double* t,
+                  int* fail, double* d_trans, double* d_wbar, cudaStream_t st) {
   Geometry geo{};
   geo.ens = ens;
   geo.inflation = inflation;
@@ -2347,14 +2400,6 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   b.b_rdiag = d_rdiaginv;
   b.b_dep = d_dep;
   b.b_rloc = d_rloc;
-  double *C = nullptr, *t = nullptr;
-  int* fail = nullptr;
-  if (dalloc(&C, (size_t)nbatch * ens * ens) != LG_OK || dalloc(&t, (size_t)nbatch * ens) != LG_OK ||
-      dalloc(&fail, 1) != LG_OK) {
-    dfree(C); dfree(t); dfree(fail);
-    return LG_ERR_NOMEM;
-  }
-  int result = LG_OK;
   cudaMemsetAsync(fail, 0, sizeof(int), st);
   lg::HxDev hx{};
   lg::ListDev l{};
@@ -2371,17 +2416,37 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
     lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
                          st);
   }
+}
+
+int core_status(int h_fail) {
+  // negative: a bounded tensor-core wait expired
+  return h_fail < 0 ? LG_ERR_TIMEOUT : h_fail ? LG_ERR_EIG : LG_OK;
+}
+}  // namespace
+
+int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
+                  const double* d_hxens, const float* d_rdiaginv, const double* d_dep,
+                  const double* d_rloc, double inflation, int precision, double* d_trans,
+                  double* d_wbar, void* stream_v) {
+  if (ens < 2 || ens > 128 || nbatch < 0 || inflation <= 0.0) return LG_ERR_ARG;
+  if (precision != LG_PREC_FP64 && !lg::mixed_precision(precision)) return LG_ERR_ARG;
+  if (precision == LG_PREC_MIXED_TF32 && !lg::gram_tf32_supported(ens)) return LG_ERR_UNSUPPORTED;
+  if (nbatch == 0) return LG_OK;
+  if (!d_nobsl || !d_off || !d_trans || !d_wbar) return LG_ERR_ARG;
+  if (lg::prepare_ft_nodes() != LG_OK) return LG_ERR_CUDA;
+  cudaStream_t st = (cudaStream_t)stream_v;
+  PoolBuf C(st), t(st), fail(st);
+  if (C.alloc(sizeof(double) * nbatch * ens * ens) != LG_OK ||
+      t.alloc(sizeof(double) * nbatch * ens) != LG_OK || fail.alloc(sizeof(int)) != LG_OK)
+    return LG_ERR_NOMEM;
+  enqueue_core(ens, nbatch, d_nobsl, d_off, d_hxens, d_rdiaginv, d_dep, d_rloc, inflation,
+               precision, (double*)C.p, (double*)t.p, (int*)fail.p, d_trans, d_wbar, st);
   int h_fail = 0;
   if (cudaGetLastError() != cudaSuccess ||
-      cudaMemcpyAsync(&h_fail, fail, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaMemcpyAsync(&h_fail, fail.p, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
-    result = LG_ERR_CUDA;
-  else if (h_fail < 0)
-    result = LG_ERR_TIMEOUT;  // a bounded tensor-core wait expired
-  else if (h_fail)
-    result = LG_ERR_EIG;
-  dfree(C); dfree(t); dfree(fail);
-  return result;
+    return LG_ERR_CUDA;
+  return core_status(h_fail);
 }
 
 int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiaginv,
@@ -2389,48 +2454,58 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
                   double inflation_factor) {
   if (nanals < 2 || nanals > 128 || nobsl < 0 || !trans || !overline_w) return LG_ERR_ARG;
   if (nobsl > 0 && (!hxens || !rdiaginv || !dep || !rloc)) return LG_ERR_ARG;
-  double *dh = nullptr, *dd = nullptr, *dr = nullptr, *dt = nullptr, *dw = nullptr;
-  float* df = nullptr;
-  int* dn = nullptr;
-  int64_t* doff = nullptr;
+  if (inflation_factor <= 0.0) return LG_ERR_ARG;
+  if (lg::prepare_ft_nodes() != LG_OK) return LG_ERR_CUDA;
+  // One device block, one copy in, one copy out:
+  //   in   offset (8 bytes) | hxens | dep | rloc | rdiaginv | nobsl
+  //   work C | t
+  //   out  trans | overline_w | status
   const size_t p = (size_t)nobsl, k = (size_t)nanals;
-  int r = LG_OK;
-  r |= dalloc(&dh, p * k);
-  r |= dalloc(&df, p);
-  r |= dalloc(&dd, p);
-  r |= dalloc(&dr, p);
-  r |= dalloc(&dt, k * k);
-  r |= dalloc(&dw, k);
-  r |= dalloc(&dn, 1);
-  r |= dalloc(&doff, 1);
-  if (r == LG_OK) {
+  const size_t n_in = 8 + sizeof(double) * p * (k + 2) + sizeof(float) * (p + 1);
+  const size_t in = (n_in + 15) & ~(size_t)15, work = sizeof(double) * (k * k + k);
+  const size_t out = sizeof(double) * (k * k + k) + 8;
+  const cudaStream_t st = nullptr;
+  PoolBuf dev(st);
+  if (dev.alloc(in + work + out) != LG_OK) return LG_ERR_NOMEM;
+  std::vector<unsigned char> host(std::max(n_in, out));
+  {
+    unsigned char* h = host.data();
     const int64_t zero = 0;
-    bool ok = true;
-    if (p) {
-      ok = ok && cudaMemcpy(dh, hxens, sizeof(double) * p * k, cudaMemcpyHostToDevice) == cudaSuccess;
-      ok = ok && cudaMemcpy(df, rdiaginv, sizeof(float) * p, cudaMemcpyHostToDevice) == cudaSuccess;
-      ok = ok && cudaMemcpy(dd, dep, sizeof(double) * p, cudaMemcpyHostToDevice) == cudaSuccess;
-      ok = ok && cudaMemcpy(dr, rloc, sizeof(double) * p, cudaMemcpyHostToDevice) == cudaSuccess;
-    }
-    ok = ok && cudaMemcpy(dn, &nobsl, sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess;
-    ok = ok && cudaMemcpy(doff, &zero, sizeof(int64_t), cudaMemcpyHostToDevice) == cudaSuccess;
-    if (ok) {
-      r = lg_core_batch(nanals, 1, dn, doff, dh, df, dd, dr, inflation_factor, LG_PREC_FP64, dt,
-                        dw, nullptr);
-    } else {
-      cudaGetLastError();
-      r = LG_ERR_CUDA;
-    }
-    if (r == LG_OK || r == LG_ERR_EIG) {
-      if (cudaMemcpy(trans, dt, sizeof(double) * k * k, cudaMemcpyDeviceToHost) != cudaSuccess ||
-          cudaMemcpy(overline_w, dw, sizeof(double) * k, cudaMemcpyDeviceToHost) != cudaSuccess)
-        r = LG_ERR_CUDA;
-    }
-  } else {
-    r = LG_ERR_NOMEM;
+    auto put = [&](const void* src, size_t bytes) {
+      if (bytes) memcpy(h, src, bytes);
+      h += bytes;
+    };
+    put(&zero, 8);
+    put(hxens, sizeof(double) * p * k);
+    put(dep, sizeof(double) * p);
+    put(rloc, sizeof(double) * p);
+    put(rdiaginv, sizeof(float) * p);
+    put(&nobsl, sizeof(int));
   }
-  dfree(dh); dfree(df); dfree(dd); dfree(dr); dfree(dt); dfree(dw); dfree(dn); dfree(doff);
-  return r;
+  unsigned char* const d = (unsigned char*)dev.p;
+  const double* dh = (const double*)(d + 8);
+  const double *dd = dh + p * k, *dr = dd + p;
+  const float* df = (const float*)(dr + p);
+  double* const C = (double*)(d + in);
+  double* const dt = (double*)(d + in + work);
+  int* const fail = (int*)(dt + k * k + k);
+  if (cudaMemcpyAsync(d, host.data(), n_in, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+    cudaGetLastError();
+    return LG_ERR_CUDA;
+  }
+  enqueue_core(nanals, 1, (const int*)(df + p), (const int64_t*)d, dh, df, dd, dr,
+               inflation_factor, LG_PREC_FP64, C, C + k * k, fail, dt, dt + k * k, st);
+  if (cudaGetLastError() != cudaSuccess ||
+      cudaMemcpyAsync(host.data(), dt, out, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess) {
+    cudaGetLastError();
+    return LG_ERR_CUDA;
+  }
+  memcpy(trans, host.data(), sizeof(double) * k * k);
+  memcpy(overline_w, host.data() + sizeof(double) * k * k, sizeof(double) * k);
+  int h_fail = 0;
+  memcpy(&h_fail, host.data() + sizeof(double) * (k * k + k), sizeof(int));
+  return core_status(h_fail);
 }
 
 void letkf_core_(const int* nanals, const int* nobsl, const double* hxens, const float* rdiaginv,
