@@ -27,8 +27,8 @@
 // A non-finite C gives a NaN diagonal, which the transform reports.
 //
 // Measured alone against tridiag_kernel: 921 600 matrices of 40 members 116 ->
-// 65 ms, 129 600 of 64 members 54 -> 34 ms, 2592 of 16 members 81 -> 66 us.  Bound
-// by instruction issue (0.68 of the slots at 40 members; 0.47 at 64, where the
+// 52 ms, 129 600 of 64 members 54 -> 26 ms, 2592 of 16 members 81 -> 52 us; a single
+// matrix of 40 members 94 us.  Bound by instruction issue (at 64 members the
 // triangles leave twelve warps per SM).
 #include "lg_device.cuh"
 #include "lg_fixed.cuh"
@@ -39,30 +39,40 @@ namespace tri {
 
 __device__ inline int idx(int j) { return j * (j + 1) / 2; }
 
+// Sum over the warp (which has to fit 64 bits) by three 32-bit reductions.
 __device__ inline long long warp_add(long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  const unsigned p0 = __reduce_add_sync(0xffffffffu, (unsigned)v & 0x1fffffu);
+  const unsigned p1 = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 21) & 0x1fffffu);
+  const int p2 = __reduce_add_sync(0xffffffffu, (int)(v >> 42));
+  return (long long)p0 + ((long long)p1 << 21) + ((long long)p2 << 42);
 }
 
-// For v > 0: v = x 2^(2 r) with x in [1/4, 1); y = 1/sqrt(x) in units of 2^-60
-// (to about 2^-59), r returned.  y0 from FP32 (error below 2^-22), then
-// y = y0 (1 + e/2 + 3 e^2 / 8), e = 1 - x y0^2; the next term is below 2^-66.
-__device__ inline unsigned long long rsqrt_fixed(unsigned __int128 v, int& r) {
-  const unsigned long long vh = (unsigned long long)(v >> 64);
-  const int z = vh ? __clzll((long long)vh) : 64 + __clzll((long long)(unsigned long long)v);
-  const int p = 128 - z;       // v in [2^(p-1), 2^p)
-  r = (p + 1) >> 1;            // 2^(2r - 2) <= v < 2^(2r)
-  const int up = 128 - 2 * r;  // x = v 2^(-2r): 64-bit fraction = top 64 bits of v << up
-  const unsigned long long x = (unsigned long long)((v << up) >> 64);
+// 1/sqrt(x / 2^64) in units of 2^-60 (to about 2^-59) for x in [2^62, 2^64).
+// y0 from FP32 (error below 2^-22), then y = y0 (1 + e/2 + 3 e^2 / 8), e = 1 -
+// x y0^2; the next term is below 2^-66.
+__device__ inline unsigned long long rsqrt_fixed(unsigned long long x) {
   const float y0f = rsqrtf((float)(unsigned)(x >> 32) * 2.3283064365386963e-10f);
-  const unsigned y0 = (unsigned)(y0f * 1073741824.0f);  // 2^30 y0, at most 2^31
+  const unsigned y0 = (unsigned)(y0f * 1073741824.0f);        // 2^30 y0, at most 2^31
   const unsigned long long y2 = (unsigned long long)y0 * y0;  // 2^60 y0^2
   const long long e = (1ll << 60) - (long long)__umul64hi(x, y2);
   const long long e8 = e >> 8;
   const long long c = (e >> 1) + ((3 * ((e8 * e8) >> 44)) >> 3);
-  return ((unsigned long long)y0 << 30) + (unsigned long long)(long long)(((__int128)c * y0) >> 30);
+  return ((unsigned long long)y0 << 30) +
+         (unsigned long long)((((c >> 6) * (long long)y0) >> 24) +
+                              (long long)(((unsigned long long)(c & 63) * y0) >> 30));
 }
+
+// byte offsets of (row, column) in an array of int4, per element of the packed
+// triangle
+struct Elements {
+  unsigned v[64 * 65 / 2];
+  constexpr Elements() : v() {
+    int t = 0;
+    for (unsigned j = 0; j < 64; ++j)
+      for (unsigned c = 0; c <= j; ++c) v[t++] = (j * 16u) << 16 | (c * 16u);
+  }
+};
+__device__ constexpr Elements g_elements{};
 
 }  // namespace tri
 
@@ -150,10 +160,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
       // nothing to reduce: e is the element beside the diagonal
       const long long e = __shfl_sync(0xffffffffu, l < 32 ? x0 : x1, l & 31);
       for (int c = lane; c < i; c += 32) u_out[c] = make_int2(0, 0);
-      if (lane == 0) {
-        E[i] = fixed_to_double(e, ex);
-        H[i] = 0.0;
-      }
+      if (lane == 0) WQ[i] = make_int4((int)e, (int)(e >> 32), ex, 0);
       __syncwarp();
       continue;
     }
@@ -168,22 +175,23 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
                    (((long long)s0.x * s0.x + (long long)s1.x * s1.x) >> 30);
     S1 = warp_add(S1);
     S2 = warp_add(S2);
-    const unsigned __int128 N = ((unsigned __int128)(unsigned long long)S1 << 30) + (__int128)S2;
-    int r;
-    const unsigned long long yn = rsqrt_fixed(N, r);
-    // norm = sqrt(N 2^30) = N 2^30 / (2^(r + 15) x^(-1/2)...) = x y 2^(r + 15), x = N 2^(-2r)
-    const unsigned long long xn = (unsigned long long)((N << (128 - 2 * r)) >> 64);
-    // x y < 1: a fraction of 2^-60; norm' = (x y) 2^(r + 15), r + 15 in 57 .. 60
-    const unsigned long long rt = __umul64hi(xn, yn);
-    const int ds = 60 - (r + 15);  // 0 .. 3
-    const long long alpha = (long long)((rt + (ds ? 1ull << (ds - 1) : 0ull)) >> ds);
+    // N = |x|^2 / 2^56 in [2^56, 2^64) = xn 2^(-zn), zn even
+    const unsigned long long N =
+        ((unsigned long long)S1 << 4) + (unsigned long long)(S2 >> 26);
+    const int zn = __clzll((long long)N) & ~1;
+    const unsigned long long xn = N << zn;
+    // |x| = sqrt(xn / 2^64) 2^(60 - zn / 2)
+    const unsigned long long rt = __umul64hi(xn, rsqrt_fixed(xn));
+    const long long alpha = (long long)((rt + ((1ull << (zn / 2)) >> 1)) >> (zn / 2));
     const long long f = __shfl_sync(0xffffffffu, l < 32 ? x0 : x1, l & 31);
     const long long af = llabs(f);
-    // u_l = f + sign(f) alpha; h = N + |f| alpha (units of 2^30)
-    const unsigned __int128 hh = N + (((unsigned __int128)(unsigned long long)af *
-                                       (unsigned long long)alpha) >> 30);
-    int rh;
-    const unsigned long long yh = rsqrt_fixed(hh, rh);  // 1/sqrt(h) = yh 2^-60 2^-(rh + 15)
+    // u_l = f + sign(f) alpha; h = |x|^2 + |f| alpha = hh 2^57 = xh 2^(57 - zh), zh odd
+    const unsigned long long hh =
+        (N >> 1) + __umul64hi((unsigned long long)af << 6, (unsigned long long)alpha << 1);
+    const int zh = ((__clzll((long long)hh) + 1) & ~1) - 1;
+    const unsigned long long xh = zh < 0 ? hh >> 1 : hh << zh;
+    const int rh = (121 - zh) >> 1;  // sqrt(h) = sqrt(xh / 2^64) 2^rh
+    const long long yh = (long long)(rsqrt_fixed(xh) << 1);
     const long long ul = f >= 0 ? f + alpha : f - alpha;
     if (lane == (l & 31)) {
       if (l < 32)
@@ -191,13 +199,8 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
       else
         x1 = ul;
     }
-    // w 2^58 = u yh 2^(58 - 60 - rh - 15): (u 2^3)(yh) / 2^64 is u yh 2^-61, so a
-    // further shift by rh + 15 + 2 - 61 = rh - 44 (13 to 17: rh + 15 in 57 .. 61)
-    auto to_w = [&](long long x) -> long long {
-      const __int128 t = (__int128)x * (long long)yh;
-      const int sh = rh + 17;
-      return (long long)((t + ((__int128)1 << (sh - 1))) >> sh);
-    };
+    // w 2^58 = u 2^(58 - rh) yh 2^-61; |u| < 2^(rh + 0.5), so u 2^(62 - rh) fits
+    auto to_w = [&](long long x) { return (__mul64hi(x << (62 - rh), yh) + 1) >> 1; };
     const long long w0 = to_w(x0), w1 = to_w(x1);
     if (lane <= l) {
       const int2 w = fixed_split(w0);
@@ -214,8 +217,8 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
       u_out[lane + 32] = w;
     }
     if (lane == 0) {
-      E[i] = fixed_to_double(f >= 0 ? -alpha : alpha, ex - up);
-      H[i] = 1.0;
+      const long long e = f >= 0 ? -alpha : alpha;
+      WQ[i] = make_int4((int)e, (int)(e >> 32), ex - up, 1);  // column i is done with
     }
     __syncwarp();
     // ---- p = A w: rows 0 .. nfull - 1 a lane each, the rest split over f lanes
@@ -295,32 +298,44 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     // ---- A -= w q^T + q w^T over the packed rows 0 .. l
     {
       const int tot = idx(l + 1);
-      int jr = 0, c = lane;
-      while (c > jr) {
-        c -= jr + 1;
-        ++jr;
-      }
-      for (int t = lane; t < tot; t += 32) {
-        const int4 a = WQ[jr], b = WQ[c];
+      const unsigned char* const wq = reinterpret_cast<const unsigned char*>(WQ);
+      auto updated = [](int4 a, int4 b, int2 x) {
         const long long hs = (long long)a.y * b.w + (long long)a.w * b.y;
         long long ms = (long long)a.y * b.z + (1 << 27);
         ms += (long long)a.x * b.w;
         ms += (long long)a.w * b.x;
         ms += (long long)a.z * b.y;
-        A[t] = fixed_split(fixed_join(A[t]) - 4 * hs - (ms >> 28));
-        c += 32;
-        while (c > jr) {
-          c -= jr + 1;
-          ++jr;
-        }
+        return fixed_split(fixed_join(x) - 4 * hs - (ms >> 28));
+      };
+      int t = lane;
+      for (; t + 32 < tot; t += 64) {  // two elements a lane, loaded together
+        const unsigned o0 = g_elements.v[t], o1 = g_elements.v[t + 32];
+        const int4 a0 = *reinterpret_cast<const int4*>(wq + (o0 >> 16));
+        const int4 b0 = *reinterpret_cast<const int4*>(wq + (o0 & 0xffffu));
+        const int4 a1 = *reinterpret_cast<const int4*>(wq + (o1 >> 16));
+        const int4 b1 = *reinterpret_cast<const int4*>(wq + (o1 & 0xffffu));
+        const int2 e0 = A[t], e1 = A[t + 32];
+        A[t] = updated(a0, b0, e0);
+        A[t + 32] = updated(a1, b1, e1);
+      }
+      if (t < tot) {
+        const unsigned o = g_elements.v[t];
+        A[t] = updated(*reinterpret_cast<const int4*>(wq + (o >> 16)),
+                       *reinterpret_cast<const int4*>(wq + (o & 0xffffu)), A[t]);
       }
     }
     __syncwarp();
   }
-  for (int i = lane; i < n; i += 32) D[i] = fixed_to_double(fixed_join(A[idx(i) + i]), ex);
-  if (lane == 0) {
-    E[0] = 0.0;
-    H[0] = 0.0;
+  for (int i = lane; i < n; i += 32) {
+    D[i] = fixed_to_double(fixed_join(A[idx(i) + i]), ex);
+    double e = 0.0, h = 0.0;
+    if (i > 0) {
+      const int4 w = WQ[i];
+      e = fixed_to_double((long long)w.y << 32 | (unsigned)w.x, w.z);
+      h = w.w ? 1.0 : 0.0;
+    }
+    E[i] = e;
+    H[i] = h;
   }
 }
 
