@@ -28,25 +28,21 @@
 // 2^-54 of the chunk's largest |z| times |z| per entry, adding up as a random
 // walk; a chain of FP64 additions loses 2^-53 of the partial sum at each.
 //
-// One persistent CTA per SM (the accumulators fill tensor memory), 20 warps in
-// three roles that work on neighbouring chunks of up to 1536 entries.  Seven
-// warps drop the candidates whose vertical weight cannot be non-zero by an
-// integer compare of |ln p - ln p_e|, queue the others in list order, and weigh
-// the queue densely (the only FP64 work, some 35 instructions per kept entry).
-// Twelve warps convert 64 entries at a time by integer arithmetic into one of
-// two operand buffers, take finished sums out of tensor memory and write C and
-// t.  One warp issues the MMAs (a converting warp that issued them was late for
-// its next stage by the MMAs' own time, 2500 cycles).  The rows' largest values
-// and the levels' ln p come from small kernels before this one.
-//
-// Measured alone (one stream), against gram64_kernel: 921 600 solves of 40
-// members with 379 kept entries each (of 1562 candidates) 727 -> 128 ms;
-// 129 600 solves of 64 members with 954 kept entries 595 -> 58 ms; 82 944
-// solves of 40 members with 24 entries 5.6 -> 4.1 ms; 2592 of 16 members with
-// 51 entries 0.18 -> 0.10 ms.  It wins at every size measured, so up to 64
-// members (the tensor-memory columns' limit) every solve comes here.  Bound by
-// the converting warps: some 50 instructions per element at three warps per
-// scheduler, then taking the sums out (once per 256 entries).
+// One persistent CTA per SM (the accumulators fill tensor memory), 28 warps in
+// four roles that work on neighbouring chunks of up to 1536 entries:
+//   weighing (7 warps)    drop the candidates whose vertical weight cannot be
+//     non-zero by an integer compare of |ln p - ln p_e|, queue the others in list
+//     order, and weigh the queue densely (the only FP64 work, some 35
+//     instructions per kept entry);
+//   converting (12)       64 entries at a time by integer arithmetic into one of
+//     two operand buffers;
+//   issuing (1)           the MMAs (a converting warp that issued them was late
+//     for its next stage by the MMAs' own time, 2500 cycles);
+//   adding up (8)         finished sums out of tensor memory, C and t.
+// The rows' largest values and the levels' ln p come from small kernels before
+// this one.  Roles meet at mbarriers with bounded waits; the first that runs out
+// raises s_abort, every role leaves its loop and the launch reports
+// LG_ERR_TIMEOUT.
 //
 // A solve with a non-finite weight, row or innovation, or with magnitudes
 // outside 2^+-400, is marked by a bit pattern in its first Gram element that no
@@ -59,11 +55,11 @@
 namespace lg {
 namespace g64 {
 
-constexpr int kPWarps = 7, kXWarps = 12;              // weighing; converting and adding up
+constexpr int kPWarps = 7, kXWarps = 12, kDWarps = 8;  // weighing, converting, adding up
 constexpr int kMmaWarp = kPWarps;                     // issues the MMAs
-constexpr int kX0 = kMmaWarp + 1;                     // first converting warp (a multiple of 4)
-constexpr int kPThreads = 32 * kPWarps, kXThreads = 32 * kXWarps;
-constexpr int kThreads = 32 * (kX0 + kXWarps);
+constexpr int kX0 = kMmaWarp + 1, kD0 = kX0 + kXWarps;  // first warps (multiples of 4)
+constexpr int kPThreads = 32 * kPWarps, kXThreads = 32 * kXWarps, kDThreads = 32 * kDWarps;
+constexpr int kThreads = 32 * (kD0 + kDWarps);
 constexpr int kStage = 64;                            // entries per stage (4 K = 16 chunks)
 constexpr int kSlice = 64 * 16 * 2;                   // 2048 B: 64 rows x K = 16 FP16
 constexpr int kTileD = 7 * kSlice;                    // the d~ tile after zero and six slices
@@ -78,10 +74,8 @@ constexpr int kSmem = 2 * kStageBytes + 2 * kQueueBytes + 64 * 65 * 8;
 // C's exact sums are kept in units of 2^-51 of the largest product times 2^-1:
 // twice the sum of 1536 products stays below 2^63
 constexpr int kDrop = 10;
-// named barriers: the converting and the weighing warps' own; queue full and
-// queue empty, operand buffer converted (two each); tensor memory drained
-constexpr int kBarX = 1, kBarP = 2, kBarFull = 3, kBarEmpty = 5, kBarStage = 7, kBarDrain = 9;
-constexpr int kXMma = kXThreads + 32;
+// named barriers: the weighing and the adding warps' own
+constexpr int kBarP = 1, kBarD = 2;
 constexpr int kTmemCols = 512;
 constexpr int kColD = 448;                            // first column of the d~ products
 constexpr int kExLimit = 400;
@@ -128,8 +122,8 @@ __device__ inline void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.alig
 __device__ inline void bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
-__device__ inline void bar_arrive(int id, int count) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+__device__ inline void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
 }
 
 // (hi 2^27 + lo) 2^ex rounded to nearest-even
@@ -271,35 +265,44 @@ struct QueueHead {
 };
 
 // kR: units (member, 4 entries) of a stage per converting thread -- 2 up to 48
-// members, 3 above -- and with it the columns of a warp quadruple (8 kR)
+// members, 3 above
 template <int kR>
 __global__ void __launch_bounds__(g64::kThreads, 1)
     gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, double* Cout, double* tout,
                      int* err) {
   using namespace g64;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ uint64_t mbar[2];
+  // operand buffer multiplied, converted; queue full, empty; exact sum complete,
+  // taken out (one phase per group of stages: the adding warps wait for no stage
+  // in between, so a stage barrier's parity would not tell them which phase it is)
+  __shared__ uint64_t m_mma[2], m_conv[2], m_full[2], m_empty[2], m_sum, m_drain;
   __shared__ uint32_t tmem_base_sh;
   __shared__ int s_wcnt[2][kPWarps];
   __shared__ longlong2 s_t[2][64];
   __shared__ int s_kmax, s_dmax, s_nf;
+  __shared__ volatile int s_abort;
+  __shared__ int s_stop[2];  // s_abort as the weighing and the adding warps agree on it
   __shared__ QueueHead s_head[2];
 
   const int k = g.ens;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool batch = b.mode == 1;
-  // the zero slices of the two operand buffers
-  auto zero_blocks = [&](int t, int nt) {
-    for (int i = t; i < 8 * kSlice / 16; i += nt)
-      *reinterpret_cast<uint4*>(smem_raw + (i / (kSlice / 16)) * kChunkBytes +
-                                i % (kSlice / 16) * 16) = make_uint4(0, 0, 0, 0);
-  };
   if (tid == 0) {
-    tc::mbar_init(&mbar[0], 1);
-    tc::mbar_init(&mbar[1], 1);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&m_mma[i], 1);
+      tc::mbar_init(&m_conv[i], kXWarps);
+      tc::mbar_init(&m_full[i], kPThreads);
+      tc::mbar_init(&m_empty[i], kXWarps + 1 + kDWarps);
+    }
+    tc::mbar_init(&m_sum, 1);
+    tc::mbar_init(&m_drain, kDWarps);
+    s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  zero_blocks(tid, kThreads);
+  // the zero slices of the two operand buffers
+  for (int i = tid; i < 8 * kSlice / 16; i += kThreads)
+    *reinterpret_cast<uint4*>(smem_raw + (i / (kSlice / 16)) * kChunkBytes +
+                              i % (kSlice / 16) * 16) = make_uint4(0, 0, 0, 0);
   tc::fence_proxy_async();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -315,10 +318,16 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     return reinterpret_cast<int4*>(smem_raw + 2 * kStageBytes + qb * kQueueBytes);
   };
   auto q_d = [&](int qb) { return reinterpret_cast<long long*>(q_par(qb) + kQueue); };
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    if (!s_abort && !tc::mbar_wait(bar, parity)) s_abort = 1;
+    __syncwarp();
+  };
+  // s_abort, the same for the lanes of a warp
+  auto stopped = [&]() { return __any_sync(0xffffffffu, s_abort != 0); };
 
   if (warp < kX0) {
-  // registers: 256 x 48 + 384 x 128 within the launch's 640 x 96
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+  // registers: 256 x 56 + 384 x 80 + 256 x 72 within the launch's 896 x 72
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp < kPWarps) {
     // ================= weighing warps
     const bool vertical = !batch && g.vert_dist > 0.0;
@@ -329,16 +338,21 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     const double inv_vd = 1.0 / g.vert_dist;
     int work = 0;
     unsigned nq = 0;  // queues filled so far
-    auto fill = [&](int s, int64_t base, int p, double al, int& scan, bool& first) -> bool {
+    // 1: a queue is filled; 0: the solve is left to gram64_kernel; -1: stop
+    auto fill = [&](int s, int64_t base, int p, double al, int& scan, bool& first) -> int {
       const int qb = nq & 1;
       int4* const par = q_par(qb);
       long long* const qd = q_d(qb);
-      if (nq >= 2) bar_sync(kBarEmpty + qb, kThreads);
+      if (nq >= 2) wait(&m_empty[qb], ((nq - 2) >> 1) & 1);
+      bar_sync(kBarP, kPThreads);  // every thread has read the last queue's maxima
       if (tid == 0) {
         s_kmax = 0;
         s_dmax = 0;
         s_nf = 0;
+        s_stop[0] = s_abort;
       }
+      bar_sync(kBarP, kPThreads);
+      if (s_stop[0]) return -1;
       int qn = 0;
       while (qn <= kQueue - kRefill && scan < p) {
         int ent[kPer];
@@ -393,50 +407,66 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       // weights, densely (FP64): rr into par, d~ into qd
       int kmax = 0, dmax = 0, cnt = 0;
       bool nf = false;
-      for (int q = tid; q < qn; q += kPThreads) {
-        const int4 c = par[q];
-        const int ent = c.w;
-        const int64_t i = base + c.z;
-        double rl, rdg, dep;
-        int e;
-        if (batch) {
-          rl = b.b_rloc[i];
-          rdg = (double)b.b_rdiag[i];
-          dep = b.b_dep[i];
-          const double* y = b.b_hx + (size_t)i * k;
-          unsigned em = 0;
-          for (int j = 0; j < k; ++j) em = max(em, (unsigned)__double2hiint(y[j]) & 0x7fffffffu);
-          e = (int)em;
-        } else {
-          rl = l.rloc[i];
-          rdg = (double)hx.rdiag[ent];
-          dep = hx.dis[ent];
-          e = hx.yexp[ent];
-          if (vertical) {
-            const double z = fabs(__hiloint2double(c.y, c.x)) * inv_vd;
-            rl = rl * (g.gc_filter_vertical ? taper_fast(z) : schr(z));
-          }
-        }
-        double w = sqrt(rdg * rl), d = 0.0;
-        if (w != 0.0) {
-          d = w * dep;
-          const int ew = (__double2hiint(w) >> 20) & 0x7ff;
-          const int ed = (__double2hiint(d) >> 20) & 0x7ff;
-          ++cnt;
-          nf |= (e >> 20) == 2047 || ew == 2047 || ed == 2047;
-          if (e >> 20) {
-            // the bound |z| < 2^(kz - 1022): the product of the mantissas (each
-            // rounded up, so at most 4) decides whether it carries
-            const double fy = __hiloint2double((e & 0xfffff) | 0x3ff00000, -1);
-            const double fw = __hiloint2double((__double2hiint(w) & 0xfffff) | 0x3ff00000, -1);
-            kmax = max(kmax, (e >> 20) + ew + ((__double2hiint(fy * fw) >> 20) - 1023));
-            dmax = max(dmax, ed);
+      for (int q0 = tid; q0 < qn; q0 += 2 * kPThreads) {
+        // two entries at a time: their loads are in flight together
+        double rl[2], dep[2], dz[2];
+        float rdg[2];
+        int e[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int q = q0 + r * kPThreads;
+          rl[r] = dep[r] = dz[r] = 0.0;
+          rdg[r] = 0.0f;
+          e[r] = 0;
+          if (q >= qn) continue;
+          const int4 c = par[q];
+          const int64_t i = base + c.z;
+          dz[r] = __hiloint2double(c.y, c.x);
+          if (batch) {
+            rl[r] = b.b_rloc[i];
+            rdg[r] = b.b_rdiag[i];
+            dep[r] = b.b_dep[i];
+            const double* y = b.b_hx + (size_t)i * k;
+            unsigned em = 0;
+            for (int j = 0; j < k; ++j) em = max(em, (unsigned)__double2hiint(y[j]) & 0x7fffffffu);
+            e[r] = (int)em;
           } else {
-            w = 0.0;  // a row of zeros
+            rl[r] = l.rloc[i];
+            rdg[r] = hx.rdiag[c.w];
+            dep[r] = hx.dis[c.w];
+            e[r] = hx.yexp[c.w];
           }
         }
-        *reinterpret_cast<double*>(&par[q]) = w;
-        qd[q] = __double_as_longlong(d);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int q = q0 + r * kPThreads;
+          if (q >= qn) continue;
+          double x = rl[r];
+          if (vertical) {
+            const double z = fabs(dz[r]) * inv_vd;
+            x = x * (g.gc_filter_vertical ? taper_fast(z) : schr(z));
+          }
+          double w = sqrt((double)rdg[r] * x), d = 0.0;
+          if (w != 0.0) {
+            d = w * dep[r];
+            const int ew = (__double2hiint(w) >> 20) & 0x7ff;
+            const int ed = (__double2hiint(d) >> 20) & 0x7ff;
+            ++cnt;
+            nf |= (e[r] >> 20) == 2047 || ew == 2047 || ed == 2047;
+            if (e[r] >> 20) {
+              // the bound |z| < 2^(kz - 1022): the product of the mantissas (each
+              // rounded up, so at most 4) decides whether it carries
+              const double fy = __hiloint2double((e[r] & 0xfffff) | 0x3ff00000, -1);
+              const double fw = __hiloint2double((__double2hiint(w) & 0xfffff) | 0x3ff00000, -1);
+              kmax = max(kmax, (e[r] >> 20) + ew + ((__double2hiint(fy * fw) >> 20) - 1023));
+              dmax = max(dmax, ed);
+            } else {
+              w = 0.0;  // a row of zeros
+            }
+          }
+          *reinterpret_cast<double*>(&par[q]) = w;
+          qd[q] = __double_as_longlong(d);
+        }
       }
       kmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)kmax);
       dmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)dmax);
@@ -482,10 +512,10 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         qd[q] = ((dq & 0x7fffffffffffffffll) + bias()) * 32 | (dq & (1ll << 63));
       }
       if (tid == 0) s_head[qb] = QueueHead{s, qr / kStage, S, Sd, first ? 1 : 0, bad ? 1 : 0};
-      bar_arrive(kBarFull + qb, kThreads);
+      mbar_arrive(&m_full[qb]);
       ++nq;
       first = false;
-      return !bad;
+      return bad ? 0 : 1;
     };
     for (int s = blockIdx.x; s < b.nsolves; s += gridDim.x) {
       int64_t base;
@@ -501,69 +531,71 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       const double al = vertical ? tout[(size_t)s * k] : 0.0;
       int scan = 0;
       bool first = true;
-      while (fill(s, base, p, al, scan, first) && scan < p) {
-      }
+      int r = 1;
+      do {
+        r = fill(s, base, p, al, scan, first);
+      } while (r > 0 && scan < p);
+      if (r < 0) break;
     }
     const int qb = nq & 1;
-    if (nq >= 2) bar_sync(kBarEmpty + qb, kThreads);
+    if (nq >= 2) wait(&m_empty[qb], ((nq - 2) >> 1) & 1);
     if (tid == 0) s_head[qb] = QueueHead{-1, 0, 0, 0, 0, 0};
-    bar_arrive(kBarFull + qb, kThreads);
+    mbar_arrive(&m_full[qb]);
     work = (int)__reduce_add_sync(0xffffffffu, (unsigned)work);
     if (b.work && lane == 0 && work) atomicAdd(b.work, (unsigned long long)work);
-  } else if (warp == kMmaWarp) {
+  } else {
     // ================= the issuing warp
-    unsigned n = 0;  // stages issued (buffer n & 1)
-    bool started = false;
+    const uint64_t desc0 = tc::make_desc(tc::smem_u32(smem_raw), 128, 256);
+    unsigned n = 0, groups = 0;  // stages issued (buffer n & 1), exact sums begun
     for (unsigned nq = 0;; ++nq) {
       const int qb = nq & 1;
-      bar_sync(kBarFull + qb, kThreads);
-      const int stages = s_head[qb].s < 0 ? -1 : s_head[qb].stages;
-      if (stages < 0) break;
-      bar_arrive(kBarEmpty + qb, kThreads);
+      wait(&m_full[qb], (nq >> 1) & 1);
+      if (stopped() || s_head[qb].s < 0) break;
+      const int stages = s_head[qb].stages;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&m_empty[qb]);
       for (int st = 0; st < stages; ++st, ++n) {
-        bar_sync(kBarStage + (n & 1), kXMma);
+        wait(&m_conv[n & 1], (n >> 1) & 1);
         if (st % kGroup == 0) {
           // a new exact sum: the finished one is out of tensor memory
-          if (started) bar_sync(kBarDrain, kXMma);
-          started = true;
+          if (groups > 0) wait(&m_drain, (groups - 1) & 1);
+          ++groups;
         }
+        if (stopped()) break;
         if (lane == 0) {
           tc::fence_after();
-          const uint32_t sb = tc::smem_u32(smem_raw) + (n & 1) * kStageBytes;
+          // descriptors of an operand at `off` bytes into the buffer: its address is
+          // in the low 14 bits, in units of 16 bytes
+          const uint32_t lo = (uint32_t)desc0 + (n & 1) * (kStageBytes / 16);
+          const uint32_t hi = (uint32_t)(desc0 >> 32);
+          auto at = [&](int off) { return (uint64_t)hi << 32 | (lo + (uint32_t)off / 16); };
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            auto at = [&](int pos) {
-              return tc::make_desc(sb + c * kChunkBytes + pos * kSlice, 128, 256);
-            };
-            const uint64_t dt = tc::make_desc(sb + c * kChunkBytes + kTileD, 128, 256);
+            const int o = c * kChunkBytes;
             const uint32_t more = (st % kGroup > 0 || c > 0) ? 1u : 0u;
-            mma(tmem, at(1), at(2), idesc(64), more);         // [5;0] x 0
-            mma(tmem + 64, at(2), at(3), idesc(256), more);   // [0;1] x 1 3 2 4
-            mma(tmem + 320, at(4), at(4), idesc(64), more);   // [3;2] x 3
-            mma(tmem + 384, at(5), at(5), idesc(64), more);   // [2;4] x 2
-            mma(tmem + 384, at(0), at(3), idesc(64), 1u);     // [zero;5] x 1
-            mma(tmem + kColD, at(1), dt, idesc(16), more);
-            mma(tmem + kColD + 16, at(3), dt, idesc(16), more);
-            mma(tmem + kColD + 32, at(5), dt, idesc(16), more);
+            mma(tmem, at(o + kSlice), at(o + 2 * kSlice), idesc(64), more);           // [5;0] x 0
+            mma(tmem + 64, at(o + 2 * kSlice), at(o + 3 * kSlice), idesc(256), more); // [0;1] x 1 3 2 4
+            mma(tmem + 320, at(o + 4 * kSlice), at(o + 4 * kSlice), idesc(64), more); // [3;2] x 3
+            mma(tmem + 384, at(o + 5 * kSlice), at(o + 5 * kSlice), idesc(64), more); // [2;4] x 2
+            mma(tmem + 384, at(o), at(o + 3 * kSlice), idesc(64), 1u);                // [zero;5] x 1
+            mma(tmem + kColD, at(o + kSlice), at(o + kTileD), idesc(16), more);
+            mma(tmem + kColD + 16, at(o + 3 * kSlice), at(o + kTileD), idesc(16), more);
+            mma(tmem + kColD + 32, at(o + 5 * kSlice), at(o + kTileD), idesc(16), more);
           }
-          tc::mma_commit(&mbar[n & 1]);
+          tc::mma_commit(&m_mma[n & 1]);
+          if (st % kGroup == kGroup - 1 || st == stages - 1) tc::mma_commit(&m_sum);
         }
         __syncwarp();
       }
     }
-    if (started) bar_sync(kBarDrain, kXMma);
+    // every MMA issued here is complete before tensor memory is given back (the
+    // bounded wait itself, whatever s_abort says)
+    if (n > 0 && !tc::mbar_wait(&m_mma[(n - 1) & 1], ((n - 1) >> 1) & 1)) s_abort = 1;
   }
-  } else {
+  } else if (warp < kD0) {
     // ================= converting warps
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     const int xt = tid - 32 * kX0;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const bool low = (warp & 3) < 2;         // accumulator rows 0..63: the first slice of A
-    const int row = (warp & 1) * 32 + lane;  // member of this thread's accumulator row
-    constexpr int kW = kR == 2 ? 8 : 4;      // accumulator columns taken out at a time
-    constexpr int cw = kR;                   // octets of columns of each warp quadruple
-    const int j0 = (warp - kX0) / 4 * 8 * cw;
-    const int noct = max(0, min(cw, (k - j0 + 7) / 8));  // uniform in a warp
     // unit u of a stage: entries 4 (u & 1) .. + 3 of the 8-entry group u / 2k, member
     // (u / 2) % k -- two lanes fill the 16 bytes of an operand row.  This thread's
     // units: member, first entry (< 0: none), place in the operand buffer
@@ -576,61 +608,131 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       ud[r] = (ug >> 1) * kChunkBytes + (um[r] >> 3) * 256 + (ug & 1) * 128 + (um[r] & 7) * 16 +
               (u & 1) * 8;
     }
-    // the chunk's sums, 64 x 65
-    long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + 2 * kQueueBytes);
-    bool ok = true;
-    unsigned n = 0, nq = 0;  // stages issued (buffer n & 1), queues taken
-    for (;; ++nq) {
+    unsigned n = 0;  // stages converted (buffer n & 1)
+    for (unsigned nq = 0;; ++nq) {
       const int qb = nq & 1;
-      bar_sync(kBarFull + qb, kThreads);
-      const QueueHead h = s_head[qb];
-      if (h.s < 0) break;
+      wait(&m_full[qb], (nq >> 1) & 1);
+      if (stopped() || s_head[qb].s < 0) break;
+      const int stages = s_head[qb].stages;
       const int4* const par = q_par(qb);
       const long long* const qd = q_d(qb);
+      const double* const ysrc = batch ? b.b_hx + (size_t)b.b_off[s_head[qb].s] * k : hx.yb;
+      uint2 y[kR][4];
+      auto load = [&](int st, int r) {
+        if (uq[r] < 0) return;
+        const int q0 = st * kStage + uq[r];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          y[r][e] = __ldg(reinterpret_cast<const uint2*>(ysrc + (size_t)par[q0 + e].w * k + um[r]));
+      };
+      if (stages > 0) {
+#pragma unroll
+        for (int r = 0; r < kR; ++r) load(0, r);
+      }
+      for (int st = 0; st < stages; ++st, ++n) {
+        unsigned char* const buf = smem_raw + (n & 1) * kStageBytes;
+        if (n >= 2) wait(&m_mma[n & 1], ((n - 2) >> 1) & 1);
+        if (stopped()) break;
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+          if (uq[r] < 0) continue;
+          const int q0 = st * kStage + uq[r];
+          uint32_t o[2][6];
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            digit_pairs(digits_of(y[r][2 * e].y, y[r][2 * e].x, par[q0 + 2 * e]),
+                        digits_of(y[r][2 * e + 1].y, y[r][2 * e + 1].x, par[q0 + 2 * e + 1]),
+                        y[r][2 * e].y, y[r][2 * e + 1].y, o[e]);
+          if (st + 1 < stages) load(st + 1, r);  // in flight beside the rest of this stage
+          unsigned char* const dst = buf + ud[r];
+#pragma unroll
+          for (int a = 0; a < 6; ++a)
+            *reinterpret_cast<uint2*>(dst + slice_pos(a) * kSlice) = make_uint2(o[0][a], o[1][a]);
+        }
+        if (warp == kD0 - 1) {
+          // d~ slices: row b of the 16-row tile, two entries per lane
+          const int q0 = st * kStage + 2 * lane;
+          uint32_t o[6];
+          const unsigned long long d0 = (unsigned long long)qd[q0], d1 = (unsigned long long)qd[q0 + 1];
+          digit_pairs(d0 & ~(1ull << 63), d1 & ~(1ull << 63), (unsigned)(d0 >> 32),
+                      (unsigned)(d1 >> 32), o);
+          unsigned char* const dst = buf + (lane >> 3) * kChunkBytes + kTileD +
+                                     ((lane >> 2) & 1) * 128 + (lane & 3) * 4;
+#pragma unroll
+          for (int a = 0; a < 6; ++a) *reinterpret_cast<uint32_t*>(dst + a * 16) = o[a];
+        }
+        tc::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&m_conv[n & 1]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&m_empty[qb]);
+    }
+  } else {
+    // ================= adding warps
+    const int xt = tid - 32 * kD0;
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool low = (warp & 3) < 2;         // accumulator rows 0..63: the first slice of A
+    const int row = (warp & 1) * 32 + lane;  // member of this thread's accumulator row
+    // columns of this warp quadruple: groups of four, from j0
+    const int cw = (k + 7) / 8 * 4;
+    const int j0 = (warp - kD0) / 4 * cw;
+    const int ng = (cw + 3) / 4, h0 = (ng + 1) / 2;
+    // the chunk's sums, 64 x 65
+    long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + 2 * kQueueBytes);
+    unsigned groups = 0;  // exact sums taken out
+    for (unsigned nq = 0;; ++nq) {
+      const int qb = nq & 1;
+      wait(&m_full[qb], (nq >> 1) & 1);
+      const QueueHead h = s_head[qb];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&m_empty[qb]);
+      bar_sync(kBarD, kDThreads);  // the chunk before is written
+      if (xt == 0) s_stop[1] = s_abort;
+      bar_sync(kBarD, kDThreads);
+      if (s_stop[1] || h.s < 0) break;
       double* const C = Cout + (size_t)h.s * k * k;
       double* const tv = tout + (size_t)h.s * k;
-      long long acc[8 * cw], thi = 0, tlo = 0;
+      long long thi = 0, tlo = 0;
+      // four columns of this half's exact FP32 sums as one integer each, written or
+      // added to U
+      auto columns = [&](int g4, bool add) {
+        const int j = j0 + 4 * g4;
+        float v[7][4];
 #pragma unroll
-      for (int j = 0; j < 8 * cw; ++j) acc[j] = 0;
-      auto drain = [&](unsigned last) {
-        // the exact FP32 sums of the stages up to `last`, added as integers
-        if (ok && !tc::mbar_wait(&mbar[last & 1], (last >> 1) & 1)) ok = false;
-        tc::fence_after();
+        for (int m = 0; m < 7; ++m) tmem_ld4(lane_addr + 64u * m + (uint32_t)j, v[m]);
+        tmem_wait_ld();
+        long long* const u = U + row * 65 + j;
 #pragma unroll
-        for (int o = 0; o < cw * (8 / kW); ++o) {
-          if (o >= noct * (8 / kW)) continue;
-          float v[7][kW];
+        for (int c = 0; c < 4; ++c) {
+          int x[7];
 #pragma unroll
-          for (int m = 0; m < 7; ++m) {
-            const uint32_t at = lane_addr + 64u * m + (uint32_t)(j0 + kW * o);
-            if constexpr (kW == 8)
-              tmem_ld8(at, v[m]);
-            else
-              tmem_ld4(at, v[m]);
+          for (int m = 0; m < 7; ++m) x[m] = __float2int_rn(v[m][c]);
+          // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
+          // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
+          long long A = add ? u[c] : 0;
+          if (low) {  // 50 01 03 02 04 33 22
+            A += (long long)x[1] * (1 << 27);
+            A += (long long)x[3] * (1 << 18);
+            A += (long long)x[2] * (1 << 9);
+            const int y = 2 * x[4] + x[6] + ((x[0] + (x[5] >> 10) + 128) >> 8);
+            A += (y + 1) >> 1;
+          } else {    // 00 11 13 12 14 23 42+51
+            A += (long long)((unsigned long long)(unsigned)(x[0] * 8) << 32);
+            A += (long long)x[1] * (1 << 17);
+            A += (long long)x[3] * (1 << 9);
+            A += x[2] + ((x[4] + x[5] + ((x[6] + 256) >> 9) + 256) >> 9);
           }
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < kW; ++j) {
-            int x[7];
-#pragma unroll
-            for (int m = 0; m < 7; ++m) x[m] = __float2int_rn(v[m][j]);
-            // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
-            // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
-            long long& A = acc[kW * o + j];
-            if (low) {  // 50 01 03 02 04 33 22
-              A += (long long)x[1] * (1 << 27);
-              A += (long long)x[3] * (1 << 18);
-              A += (long long)x[2] * (1 << 9);
-              const int y = 2 * x[4] + x[6] + ((x[0] + (x[5] >> 10) + 128) >> 8);
-              A += (y + 1) >> 1;
-            } else {    // 00 11 13 12 14 23 42+51
-              A += (long long)((unsigned long long)(unsigned)(x[0] * 8) << 32);
-              A += (long long)x[1] * (1 << 17);
-              A += (long long)x[3] * (1 << 9);
-              A += x[2] + ((x[4] + x[5] + ((x[6] + 256) >> 9) + 256) >> 9);
-            }
-          }
+          u[c] = A;
         }
+      };
+      for (int st = 0; st < h.stages; st += kGroup, ++groups) {
+        wait(&m_sum, groups & 1);
+        tc::fence_after();
+        // The two halves' sums meet in U: one half takes the first columns while the
+        // other takes the rest, then they change over
+        const bool fresh = st == 0;
+        for (int q = low ? 0 : h0; q < (low ? h0 : ng); ++q) columns(q, !fresh);
         if (j0 == 0) {
           float v[3][8];
 #pragma unroll
@@ -657,102 +759,47 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
           }
           tlo += (w6 + 256) >> 9;
         }
+        bar_sync(kBarD, kDThreads);
+        for (int q = low ? h0 : 0; q < (low ? ng : h0); ++q) columns(q, true);
         tc::fence_before();
-        bar_arrive(kBarDrain, kXMma);
-      };
-      const double* const ysrc = batch ? b.b_hx + (size_t)b.b_off[h.s] * k : hx.yb;
-      uint2 y[kR][4];
-      auto load = [&](int st, int r) {
-        if (uq[r] < 0) return;
-        const int q0 = st * kStage + uq[r];
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          y[r][e] = __ldg(reinterpret_cast<const uint2*>(ysrc + (size_t)par[q0 + e].w * k + um[r]));
-      };
-      if (h.stages > 0) {
-#pragma unroll
-        for (int r = 0; r < kR; ++r) load(0, r);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&m_drain);
+        if (st + kGroup < h.stages) bar_sync(kBarD, kDThreads);  // U's columns change hands again
       }
-      for (int st = 0; st < h.stages; ++st, ++n) {
-        unsigned char* const buf = smem_raw + (n & 1) * kStageBytes;
-        if (n >= 2 && ok && !tc::mbar_wait(&mbar[n & 1], ((n - 2) >> 1) & 1)) ok = false;
-#pragma unroll
-        for (int r = 0; r < kR; ++r) {
-          if (uq[r] < 0) continue;
-          const int q0 = st * kStage + uq[r];
-          uint32_t o[2][6];
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-            digit_pairs(digits_of(y[r][2 * e].y, y[r][2 * e].x, par[q0 + 2 * e]),
-                        digits_of(y[r][2 * e + 1].y, y[r][2 * e + 1].x, par[q0 + 2 * e + 1]),
-                        y[r][2 * e].y, y[r][2 * e + 1].y, o[e]);
-          if (st + 1 < h.stages) load(st + 1, r);  // in flight beside the rest of this stage
-          unsigned char* const dst = buf + ud[r];
-#pragma unroll
-          for (int a = 0; a < 6; ++a)
-            *reinterpret_cast<uint2*>(dst + slice_pos(a) * kSlice) = make_uint2(o[0][a], o[1][a]);
-        }
-        if (warp == kX0 + kXWarps - 1) {
-          // d~ slices: row b of the 16-row tile, two entries per lane
-          const int q0 = st * kStage + 2 * lane;
-          uint32_t o[6];
-          const unsigned long long d0 = (unsigned long long)qd[q0], d1 = (unsigned long long)qd[q0 + 1];
-          digit_pairs(d0 & ~(1ull << 63), d1 & ~(1ull << 63), (unsigned)(d0 >> 32),
-                      (unsigned)(d1 >> 32), o);
-          unsigned char* const dst = buf + (lane >> 3) * kChunkBytes + kTileD +
-                                     ((lane >> 2) & 1) * 128 + (lane & 3) * 4;
-#pragma unroll
-          for (int a = 0; a < 6; ++a) *reinterpret_cast<uint32_t*>(dst + a * 16) = o[a];
-        }
-        tc::fence_proxy_async();
-        bar_arrive(kBarStage + (n & 1), kXMma);
-        // a new exact sum starts with this stage: take the finished one out
-        if (st > 0 && st % kGroup == 0) drain(n - 1);
-      }
-      bar_arrive(kBarEmpty + qb, kThreads);  // this thread is done with the queue
       if (h.bad) {
-        bar_sync(kBarX, kXThreads);  // an earlier chunk's C is written
+        // (an earlier chunk's C is written: the barrier at the top)
         if (xt == 0) C[0] = __longlong_as_double((long long)kGramMark);
         continue;
       }
       if (h.stages == 0 && !h.first) continue;
-      if (h.stages > 0) {
-        drain(n - 1);
-        // the two row halves meet in shared memory
-        if (!low) {
-#pragma unroll
-          for (int j = 0; j < 8 * cw; ++j)
-            if (j < 8 * noct) U[row * 65 + j0 + j] = acc[j];
-        }
-        if (j0 == 0) s_t[low ? 0 : 1][row] = make_longlong2(thi, tlo);
-        bar_sync(kBarX, kXThreads);
-        if (low) {
-#pragma unroll
-          for (int j = 0; j < 8 * cw; ++j)
-            if (j < 8 * noct) U[row * 65 + j0 + j] += acc[j];
-        }
-        bar_sync(kBarX, kXThreads);
-      }
+      if (j0 == 0) s_t[low ? 0 : 1][row] = make_longlong2(thi, tlo);
+      bar_sync(kBarD, kDThreads);
       const int ex2 = 2 * h.S - 62 + kDrop, ext = h.S + h.Sd - 61;
       // C = (U + U^T) / 2 in place (rows i and k - 1 - i of the triangle share one
       // row of k + 1 elements), then out in rows
       if (h.stages > 0) {
-        for (int r = xt; r < (k + 1) / 2 * (k + 1); r += kXThreads) {
-          const int a = r / (k + 1), c = r - a * (k + 1);
-          if (2 * a == k - 1 && c > a) continue;  // odd k: the middle row meets itself
+        for (int r = xt, a = xt / (k + 1), c = xt - a * (k + 1); r < (k + 1) / 2 * (k + 1);
+             r += kDThreads) {
           const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
-          const long long v =
-              __double_as_longlong(fixed_to_double(U[i * 65 + j] + U[j * 65 + i], ex2));
-          U[i * 65 + j] = v;
-          U[j * 65 + i] = v;
+          if (!(2 * a == k - 1 && c > a)) {  // odd k: the middle row meets itself
+            const long long v =
+                __double_as_longlong(fixed_to_double(U[i * 65 + j] + U[j * 65 + i], ex2));
+            U[i * 65 + j] = v;
+            U[j * 65 + i] = v;
+          }
+          c += kDThreads;
+          while (c > k) {
+            c -= k + 1;
+            ++a;
+          }
         }
-        bar_sync(kBarX, kXThreads);
+        bar_sync(kBarD, kDThreads);
       }
-      for (int r = xt, j = xt / k, i = xt - j * k; r < k * k; r += kXThreads) {
+      for (int r = xt, j = xt / k, i = xt - j * k; r < k * k; r += kDThreads) {
         double v = h.stages > 0 ? __longlong_as_double(U[j * 65 + i]) : 0.0;
         if (!h.first) v += C[r];
         C[r] = v;
-        i += kXThreads;
+        i += kDThreads;
         while (i >= k) {
           i -= k;
           ++j;
@@ -764,16 +811,14 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
           v = wide_to_double(s_t[0][xt].x + s_t[1][xt].x, s_t[0][xt].y + s_t[1][xt].y, ext);
         tv[xt] = h.first ? v : tv[xt] + v;
       }
-      if (h.stages > 0) bar_sync(kBarX, kXThreads);  // U and s_t are free again
     }
-    if (n > 0 && !tc::mbar_wait(&mbar[(n - 1) & 1], ((n - 1) >> 1) & 1)) ok = false;
-    if (!ok) atomicExch(err, LG_ERR_TIMEOUT);
   }
   tc::fence_before();
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kTmemCols));
+  if (tid == 0 && s_abort) atomicExch(err, LG_ERR_TIMEOUT);
 }
 
 bool gram64_tc_supported(int ens) { return ens <= 64; }
