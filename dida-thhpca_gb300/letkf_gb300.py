@@ -280,8 +280,11 @@ def gmcore_to_da(ps, u_half, v_half, pt, area_subcell, area_cell, halo: int, str
     import torch
     lib = load_library()
     nz, num_lat, num_lon, ens = u_half.shape
-    xb = torch.zeros((num_lon + 2 * halo, num_lat + 2 * halo, 1 + 3 * nz, ens),
+    xb = torch.empty((num_lon + 2 * halo, num_lat + 2 * halo, 1 + 3 * nz, ens),
                      dtype=torch.float64, device=ps.device)
+    if halo > 0:  # every other point is written by the kernel
+        xb[:, :halo].zero_()
+        xb[:, -halo:].zero_()
     args = [t.contiguous() for t in (ps, u_half, v_half, pt, area_subcell, area_cell)]
     check(lib.lg_gmcore_to_da_device(ens, num_lat, num_lon, nz, halo,
                                      *[C.c_void_p(t.data_ptr()) for t in args],
