@@ -20,21 +20,27 @@
 // Why: the FP64 pipe retires a warp instruction per 17 cycles per SM.  Per
 // 64-member solve the QL iteration takes about 4000 rotations at 24 FP64
 // instructions (one lane each) and their replay 8 per rotation and vector; the
-// shifted solves take 4 per node, element and vector, plus 8 per node and
+// shifted solves take 4 per node, element and vector, plus 7 per node and
 // element for the factors, which the lanes of a solve compute for different
-// nodes.  The reflections Q^T x and Q z (2 k^2 multiply-adds per vector) leave
-// the FP64 pipe altogether: a vector's norm does not change, so they run in
-// fixed point on the integer pipe as the reduction does (lg_tri.cu), to 2^-58 of
-// the norm per step.  Three kernels, so that the integer ones are not held to
-// the two to four warps per SM that the solves' five arrays leave:
-//   reflect_kernel (Q^T)  vectors in, y out
-//   ft_kernel             f(T) y, and T^-1 y of t
-//   reflect_kernel (Q)    z in; the rows' update, or the columns of W, out
-// and for an explicit trans add_wbar_kernel.  Measured alone against QL + replay:
-// 921 600 solves of 40 members 233 -> 71 ms, 129 600 of 64 members 93 -> 33 ms;
-// explicit trans against the accumulating solver (lg_eig.cu), with the
-// reduction: 32 768 cubes of 40 members 133 -> 15 ms.  Faster at every size from
-// 7 to 64 members; above, five arrays leave an SM one warp.
+// nodes.  overline_w . x = (T^(-1/2) y) . (T^(-1/2) Q^T t) needs no solve of its
+// own.  The reflections (2 k^2 multiply-adds per vector) leave the FP64 pipe
+// altogether: a vector's norm does not change, so they run in fixed point on the
+// integer pipe as the reduction does (lg_tri.cu), to 2^-58 of the norm per step.
+//   rows (analysis): reflect_kernel (Q^T), ft_kernel, reflect_kernel (Q) with the
+//     rows' update -- three kernels, so that the integer ones are not held to the
+//     two to four warps per SM that the solves' five arrays leave;
+//   explicit trans: ft_matrix_kernel forms F = f(T) itself, whose upper triangle
+//     takes 2 FP64 instructions per node and element (no right-hand side: with
+//     T + s = L D L^T, G = (T + s)^-1 has G_jj = 1/D_j + L_{j+1}^2 G_{j+1,j+1} and
+//     G_ij = -L_{i+1} G_{i+1,j} above it), then W = Q F Q^T by two reflect_kernel
+//     passes and overline_w = W (W t) / (k - 1) in add_wbar_kernel.  A solve per
+//     unit vector instead made this step 12.9 ms where it is 7.7 (32 768 cubes of
+//     40 members).
+// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 66 ms,
+// 129 600 of 64 members 93 -> 31 ms; explicit trans against the accumulating
+// solver (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 9.6
+// ms.  Faster at every size from 7 to 64 members; above, five arrays leave an SM
+// one warp.
 #include <float.h>
 #include <math.h>
 
@@ -137,22 +143,22 @@ __device__ inline void cp_async8(void* dst, const void* src) {
                : "memory");
 }
 
-// Which vectors a call works on: vector v of solve s -- 0: t (kept in the t
-// array's place), v >= 1: the state row v - 1 (analysis; in `vec`, element i at
-// ((s (n + 1) + i) (per - 1) + v - 1), element n being overline_w . x) or the
-// unit vector v - 1 (core; in trans, element i at so n n + i n + v - 1).
+// Vectors of an analysis call: vector v of solve s -- 0: t (kept in the t array's
+// place), v >= 1: the state row v - 1 (in `vec`, element i at
+// ((s (n + 1) + i) (per - 1) + v - 1), element n being overline_w . x).  Core
+// calls: column v of the solve's n x n matrix in `vec` (trans).
 struct Vecs {
-  int core, per;
+  int per;
   double* t;
-  double* vec;  // or trans
+  double* vec;
 };
-__device__ inline double* vec_at(const Vecs& z, int n, size_t so, size_t s, int v, int& stride) {
+__device__ inline double* vec_at(const Vecs& z, int n, size_t s, int v, int& stride) {
   if (v == 0) {
     stride = 1;
     return z.t + s * n;
   }
-  stride = z.core ? n : z.per - 1;
-  return (z.core ? z.vec + so * n * n : z.vec + s * (n + 1) * (z.per - 1)) + (v - 1);
+  stride = z.per - 1;
+  return z.vec + s * (n + 1) * (z.per - 1) + (v - 1);
 }
 __device__ inline size_t out_index(const SolveBatch& b, int s) {
   return b.s_col ? (size_t)b.first_solve + s : (size_t)s;
@@ -191,18 +197,22 @@ __device__ inline bool to_fixed(double* V, int n, int& ex) {
 
 }  // namespace ft
 
-// y <- Q^T x (kIn; P_{n-1} first) or Q z (P_1 first) of one vector per lane, one
-// warp per block, lanes numbered through the solves' vectors.  Reflector rows of
-// the (up to `slots`) solves that a warp spans come into shared memory a step
-// ahead of their use.
-template <bool kIn, bool kCore>
+// One vector per lane, one warp per block, lanes numbered through the solves'
+// vectors.  Analysis: y <- Q^T x (kFirst; P_{n-1} first) or Q z (P_1 first) with
+// the rows' update.  Core, W = Q F Q^T: the first pass takes column j of the
+// symmetric F from row j of the matrix and leaves Q F's column j there (the
+// matrix then holds (Q F)^T); the second takes column j -- row j of Q F -- and
+// leaves W's column j there, so that no lane reads what another one writes.
+// Reflector rows of the (up to `slots`) solves that a warp spans come into shared
+// memory a step ahead of their use.
+template <bool kFirst, bool kCore>
 __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, ft::Vecs z,
                                                      int slots, const double* tri, const double* xb,
                                                      const double* axb, double* xa, double* axa) {
   const int n = g.ens;
   const int lane = threadIdx.x;
   // the rows' update needs no t: its vectors are v = 1 .. per - 1
-  const int v0 = !kIn && !kCore ? 1 : 0;
+  const int v0 = !kFirst && !kCore ? 1 : 0;
   const int per = z.per - v0;
   const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * per;
   const int s_first = (int)(id0 / per);
@@ -226,12 +236,19 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
       }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  const int step = kIn ? -1 : 1, i0 = kIn ? n - 1 : 1;
+  constexpr bool kDown = kFirst && !kCore;  // Q^T
+  const int step = kDown ? -1 : 1, i0 = kDown ? n - 1 : 1;
   fetch(i0, 0);
   // ---- the vector
   int r_state = -1;
   size_t ci = 0;
-  if (!kCore) {
+  double* out;
+  int vs;
+  if (kCore) {
+    out = z.vec + ft::out_index(b, s) * n * n + (kFirst ? (size_t)v * n : (size_t)v);
+    vs = kFirst ? 1 : n;
+  } else {
+    out = ft::vec_at(z, n, s, v, vs);
     const int col = b.first_col + s / b.levels;
     const int kk = s % b.levels + 1;
     const int glat = col % g.num_lat + 1, glon = col / g.num_lat + 1;
@@ -246,16 +263,14 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
     }
   }
   const bool row = mine && r_state >= 0;  // analysis: this solve updates the row
-  int vs;
-  double* const out = ft::vec_at(z, n, ft::out_index(b, s), s, v, vs);
   const double* const xr = xb + (row ? (size_t)n * (r_state + (size_t)g.n * ci) : 0);
   for (int i = 0; i < n; ++i) {
     double x = 0.0;
-    if (kIn && kCore)
-      x = v == 0 ? out[i] : (i == v - 1 ? 1.0 : 0.0);
-    else if (kIn)
+    if (kCore)
+      x = out[(size_t)i * vs];
+    else if (kFirst)
       x = v == 0 ? out[i] : (row ? xr[i] : 0.0);
-    else if (kCore || row)
+    else if (row)
       x = out[(size_t)i * vs];
     Y[32 * i] = x;
   }
@@ -291,7 +306,7 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   // ---- out
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  if (kIn || kCore) {
+  if (kFirst || kCore) {
     if (mine)
       for (int i = 0; i < n; ++i)
         out[(size_t)i * vs] = finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
@@ -314,50 +329,15 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   }
 }
 
-// f(T) y per lane, one warp per block.  Analysis: slots = 32 / per solves per
-// warp; v = 0 gives T^-1 y (overline_w in the reduced basis), the rows
-// (f(T) - sqrt(rho)) y and overline_w . x.  Core: lanes numbered through the
-// solves' vectors; unit vectors give f(T) y.
-// Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
-// F (the forward solve), A (the sum over nodes), and for 32 (slot, node) pairs
-// the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
-template <bool kCore>
-__global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
-                                                const double* tri, int* eig_fail) {
-  const int n = g.ens;
+namespace ft {
+
+// One warp: T's diagonals of the solves s_first .. + nsl - 1 into Dg (with the
+// shift) and Eg, and each one's row of the node table (Gershgorin in FP32,
+// rounded up).  A non-finite T counts in *eig_fail, as a QL iteration that never
+// converges, if its first vector id is not below id0.
+__device__ inline void load_t(int n, const double* tri, int s_first, int nsl, double shift, double* Dg,
+                              double* Eg, int* s_row, int per, long long id0, int* eig_fail) {
   const int lane = threadIdx.x;
-  const int per = z.per;
-  int s_first, nsl, s, v;
-  bool mine;
-  if (kCore) {
-    const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * per;
-    s_first = (int)(id0 / per);
-    nsl = (int)((min(id0 + 32, total) - 1) / per) - s_first + 1;
-    mine = id0 + lane < total;
-    s = mine ? (int)((id0 + lane) / per) : s_first;
-    v = mine ? (int)((id0 + lane) - (long long)s * per) : 0;
-  } else {
-    s_first = blockIdx.x * slots;
-    nsl = min(slots, b.nsolves - s_first);
-    const int q = lane / per;
-    mine = q < nsl;
-    s = s_first + (mine ? q : 0);
-    v = mine ? lane - q * per : 0;
-  }
-  const int sl = s - s_first;
-  extern __shared__ double sm[];
-  const int cap = n * 32;
-  double *const Y = sm + lane, *const F = Y + cap, *const A = F + cap;
-  double *const R = sm + 3 * cap, *const L = R + cap;
-  double* const Dg = L + cap;         // slots x n: diagonal + shift
-  double* const Eg = Dg + slots * n;  // slots x n: Eg[i] couples i - 1 and i
-  const double shift = (double)(n - 1) / g.inflation;
-  int vs;
-  double* const io = ft::vec_at(z, n, ft::out_index(b, s), s, v, vs);
-  if (mine)
-    for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
-  // T, and per slot the node row (Gershgorin in FP32, rounded up)
-  __shared__ int s_row[32];
   for (int q = 0; q < nsl; ++q) {
     const double* T = tri + (size_t)(s_first + q) * n * n;
     for (int i = lane; i < n; i += 32) {
@@ -377,32 +357,64 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
     if (lane == 0) {
       // smallest power of two above the bound
       const int ex = (int)((__float_as_uint(mx * (1.0001f / (float)shift)) >> 23) & 0xffu) - 127 + 1;
-      s_row[q] = nf ? 0 : min(max(ex, 1), ft::kMaxLog);
-      // as a QL iteration that never converges; once per solve
-      if (nf && (!kCore || (long long)(s_first + q) * per >= (long long)blockIdx.x * 32))
-        atomicAdd(eig_fail, 1);
+      s_row[q] = nf ? 0 : min(max(ex, 1), kMaxLog);
+      if (nf && (long long)(s_first + q) * per >= id0) atomicAdd(eig_fail, 1);
     }
   }
   __syncwarp();
+}
+
+// reciprocal pivots R and multipliers L of T + sigma = L D L^T for this lane's
+// (slot, node) pair
+__device__ inline void factor(int n, const double* D, const double* E, double sigma, double* R,
+                              double* L) {
+  double r = rcp(D[0] + sigma);
+  R[0] = r;
+#pragma unroll 2
+  for (int i = 1; i < n; ++i) {
+    const double e = E[i], l = e * r;
+    r = rcp(fma(-l, e, D[i] + sigma));
+    L[32 * i] = l;
+    R[32 * i] = r;
+  }
+}
+
+}  // namespace ft
+
+// f(T) y per lane, one warp per block, slots = 32 / per solves per warp: t gives
+// sqrt(k-1) T^(-1/2) y, the rows (f(T) - sqrt(rho)) y and overline_w . x.
+// Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
+// F (the forward solve), A (the sum over nodes), and for 32 (slot, node) pairs
+// the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
+__global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
+                                                const double* tri, int* eig_fail) {
+  const int n = g.ens;
+  const int lane = threadIdx.x;
+  const int per = z.per;
+  const int s_first = blockIdx.x * slots;
+  const int nsl = min(slots, b.nsolves - s_first);
+  const bool mine = lane / per < nsl;
+  const int sl = mine ? lane / per : 0, s = s_first + sl;
+  const int v = mine ? lane - sl * per : 0;
+  extern __shared__ double sm[];
+  const int cap = n * 32;
+  double *const Y = sm + lane, *const F = Y + cap, *const A = F + cap;
+  double *const R = sm + 3 * cap, *const L = R + cap;
+  double* const Dg = L + cap;         // slots x n: diagonal + shift
+  double* const Eg = Dg + slots * n;  // slots x n: Eg[i] couples i - 1 and i
+  __shared__ int s_row[32];
+  const double shift = (double)(n - 1) / g.inflation;
+  int vs;
+  double* const io = ft::vec_at(z, n, s, v, vs);
+  if (mine)
+    for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
+  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, 1, 0, eig_fail);
   const int nb = 32 / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
   int nmax = 0;
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
   const int fs = lane % slots, fj = lane / slots;
   const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
   for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
-  auto factor = [&](double sigma) {
-    // T + sigma = U^T diag(1/R) U with U[i-1][i] = L[i], for this lane's pair
-    const double *D = Dg + fs * n, *E = Eg + fs * n;
-    double r = ft::rcp(D[0] + sigma);
-    R[lane] = r;
-#pragma unroll 2
-    for (int i = 1; i < n; ++i) {
-      const double e = E[i], l = e * r;
-      r = ft::rcp(fma(-l, e, D[i] + sigma));
-      L[32 * i + lane] = l;
-      R[32 * i + lane] = r;
-    }
-  };
   auto solve = [&](int pair, double w) {
     // A += w (T + s)^-1 y with the factors of the pair; each recurrence's chain
     // is one fused multiply-add per element
@@ -423,7 +435,9 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
     }
   };
   for (int j0 = 0; j0 < nmax; j0 += nb) {
-    if (fs < nsl && fj < nb && j0 + fj < nmax) factor(ft::g_nodes[s_row[fs]][j0 + fj].x * shift);
+    if (fs < nsl && fj < nb && j0 + fj < nmax)
+      ft::factor(n, Dg + fs * n, Eg + fs * n, ft::g_nodes[s_row[fs]][j0 + fj].x * shift, R + lane,
+                 L + lane);
     __syncwarp();
     if (mine) {
       const int rowq = s_row[sl];
@@ -432,42 +446,113 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
     }
     __syncwarp();
   }
-  if (lane < nsl) factor(0.0);  // pair (slot, 0)
-  __syncwarp();
-  if (mine && v == 0) {
-    for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
-    solve(sl, 1.0);
+  if (!mine || v == 0) return;
+  const double srho = sqrt(g.inflation);
+  const double* zt = sm + 2 * cap + sl * per;  // vector 0's A
+  double dotw = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double a = A[32 * i];
+    dotw = fma(a, zt[32 * i], dotw);
+    io[(size_t)i * vs] = fma(-srho, Y[32 * i], a);
   }
-  __syncwarp();
-  if (!mine) return;
-  if (!kCore && v >= 1) {
-    const double srho = sqrt(g.inflation);
-    const double* zt = sm + 2 * cap + sl * per;  // vector 0's A
-    double dotw = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const double y = Y[32 * i];
-      dotw = fma(y, zt[32 * i], dotw);
-      io[(size_t)i * vs] = fma(-srho, y, A[32 * i]);
+  io[(size_t)n * vs] = dotw / (double)(n - 1);
+}
+
+// F = f(T) of each solve, symmetric, into its n x n matrix: one column per lane,
+// lanes numbered through the solves' columns, one warp per block.  Shared memory
+// as in ft_kernel: A (the column), and per (slot, node) pair L and the diagonal G
+// of (T + s)^-1 (R first).
+__global__ void __launch_bounds__(32) ft_matrix_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
+                                                       const double* tri, int* eig_fail) {
+  const int n = g.ens;
+  const int lane = threadIdx.x;
+  const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * n;
+  const int s_first = (int)(id0 / n);
+  const int nsl = (int)((min(id0 + 32, total) - 1) / n) - s_first + 1;
+  const bool mine = id0 + lane < total;
+  const int s = mine ? (int)((id0 + lane) / n) : s_first, sl = s - s_first;
+  const int v = mine ? (int)((id0 + lane) - (long long)s * n) : 0;
+  extern __shared__ double sm[];
+  const int cap = n * 32;
+  double *const A = sm + lane, *const G = sm + cap, *const L = G + cap;
+  double* const Dg = L + cap;
+  double* const Eg = Dg + slots * n;
+  __shared__ int s_row[32];
+  const double shift = (double)(n - 1) / g.inflation;
+  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, n, id0, eig_fail);
+  const int nb = 32 / slots;
+  int nmax = 0;
+  for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
+  const int fs = lane % slots, fj = lane / slots;
+  const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
+  for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
+  const int vmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)v);
+  for (int j0 = 0; j0 < nmax; j0 += nb) {
+    if (fs < nsl && fj < nb && j0 + fj < nmax) {
+      const double2 node = ft::g_nodes[s_row[fs]][j0 + fj];
+      ft::factor(n, Dg + fs * n, Eg + fs * n, node.x * shift, G + lane, L + lane);
+      // the weighted diagonal w G_jj, from the last element up, in R's place
+      const double w = node.y * wscale;
+      double gd = w * G[32 * (n - 1) + lane];
+      G[32 * (n - 1) + lane] = gd;
+      for (int i = n - 2; i >= 0; --i) {
+        const double l = L[32 * (i + 1) + lane];
+        gd = fma(l, l * gd, w * G[32 * i + lane]);
+        G[32 * i + lane] = gd;
+      }
     }
-    io[(size_t)n * vs] = dotw;
-  } else if (kCore) {
-    for (int i = 0; i < n; ++i) io[(size_t)i * vs] = A[32 * i];
+    __syncwarp();
+    for (int j = 0; j < nb && j0 + j < nmax; ++j) {
+      const int pair = sl + slots * j;
+      const double *Gp = G + pair, *Lp = L + pair;
+      double x = 0.0;
+#pragma unroll 4
+      for (int i = vmax; i >= 0; --i) {
+        // above the diagonal x is not begun yet, on it it starts
+        const double step = i < n - 1 ? -Lp[32 * (i + 1)] * x : 0.0;
+        x = i == v ? Gp[32 * i] : step;
+        if (i <= v) A[32 * i] += x;
+      }
+    }
+    __syncwarp();
+  }
+  if (!mine) return;
+  double* const out = z.vec + ft::out_index(b, s) * n * n;
+  for (int i = 0; i <= v; ++i) {
+    const double x = A[32 * i];
+    out[(size_t)i * n + v] = x;
+    out[(size_t)v * n + i] = x;
   }
 }
 
-// trans(i, j) = W(i, j) + overline_w(i), column-major; W is symmetric, so its
-// row j comes in place of column j
-__global__ void add_wbar_kernel(int n, SolveBatch b, const double* t, double* trans, double* wbar) {
-  const int s = blockIdx.x;
+// overline_w = W (W t) / (k - 1), trans(i, j) = W(i, j) + overline_w(i),
+// column-major (W is symmetric)
+__global__ void __launch_bounds__(128) add_wbar_kernel(int n, SolveBatch b, const double* tin,
+                                                       double* trans, double* wbar) {
+  const int s = blockIdx.x, tid = threadIdx.x;
   const size_t so = ft::out_index(b, s);
-  const double* w = t + (size_t)s * n;
   double* To = trans + so * n * n;
-  for (int r = threadIdx.x, i = r % n; r < n * n; r += blockDim.x) {
-    To[r] += w[i];
-    i = (i + blockDim.x) % n;
+  __shared__ double t[64], u[64], w[64];
+  if (tid < n) t[tid] = tin[(size_t)s * n + tid];
+  __syncthreads();
+  if (tid < n) {
+    double d = 0.0;
+    for (int j = 0; j < n; ++j) d = fma(To[tid + (size_t)n * j], t[j], d);
+    u[tid] = d;
   }
-  if (wbar)
-    for (int i = threadIdx.x; i < n; i += blockDim.x) wbar[so * n + i] = w[i];
+  __syncthreads();
+  if (tid < n) {
+    double d = 0.0;
+    for (int j = 0; j < n; ++j) d = fma(To[tid + (size_t)n * j], u[j], d);
+    d /= (double)(n - 1);
+    w[tid] = d;
+    if (wbar) wbar[so * n + tid] = d;
+  }
+  __syncthreads();
+  for (int r = tid, i = tid % n; r < n * n; r += 128) {
+    To[r] += w[i];
+    i = (i + 128) % n;
+  }
 }
 
 bool ft_supported(const Geometry& g) {
@@ -485,8 +570,8 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
                double* wbar, int* eig_fail, cudaStream_t stream) {
   if (b.nsolves == 0) return;
   const int n = g.ens;
-  const int per = core ? n + 1 : 1 + (g.vert_dist > 0.0 ? g.n_var : g.n);
-  const ft::Vecs z{core ? 1 : 0, per, t, vec};
+  const int per = core ? n : 1 + (g.vert_dist > 0.0 ? g.n_var : g.n);
+  const ft::Vecs z{per, t, vec};
   // solves that 32 consecutive vectors can touch
   auto spans = [](int p) { return (32 + p - 2) / p + 1; };
   auto blocks = [&](int p) { return (unsigned)(((long long)b.nsolves * p + 31) / 32); };
@@ -496,20 +581,20 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kernel<<<blocks(p), 32, smem, stream>>>(g, b, z, sl, tri, xb, axb, xa, axa);
   };
-  auto solve = [&](auto kernel, int sl, unsigned grid) {
-    const size_t smem = sizeof(double) * ((size_t)5 * 32 * n + 2 * (size_t)sl * n);
+  auto solve = [&](auto kernel, int arrays, int sl, unsigned grid) {
+    const size_t smem = sizeof(double) * ((size_t)arrays * 32 * n + 2 * (size_t)sl * n);
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kernel<<<grid, 32, smem, stream>>>(g, b, z, sl, tri, eig_fail);
   };
   if (core) {
-    reflect(reflect_kernel<true, true>, per);
-    solve(ft_kernel<true>, spans(per), blocks(per));
-    reflect(reflect_kernel<false, true>, per);
+    solve(ft_matrix_kernel, 3, spans(n), blocks(n));
+    reflect(reflect_kernel<true, true>, n);
+    reflect(reflect_kernel<false, true>, n);
     add_wbar_kernel<<<b.nsolves, 128, 0, stream>>>(n, b, t, vec, wbar);
   } else {
     const int sl = 32 / per;
     reflect(reflect_kernel<true, false>, per);
-    solve(ft_kernel<false>, sl, (unsigned)((b.nsolves + sl - 1) / sl));
+    solve(ft_kernel, 5, sl, (unsigned)((b.nsolves + sl - 1) / sl));
     reflect(reflect_kernel<false, false>, per - 1);
   }
 }
