@@ -36,11 +36,11 @@
 //     passes and overline_w = W (W t) / (k - 1) in add_wbar_kernel.  A solve per
 //     unit vector instead made this step 12.9 ms where it is 7.7 (32 768 cubes of
 //     40 members).
-// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 66 ms,
-// 129 600 of 64 members 93 -> 31 ms; explicit trans against the accumulating
-// solver (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 9.6
-// ms.  Faster at every size from 7 to 64 members; above, five arrays leave an SM
-// one warp.
+// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 62 ms,
+// 129 600 of 64 members 93 -> 29 ms (66 and 31 with the elimination from one
+// end); explicit trans against the accumulating solver (lg_eig.cu), with the
+// reduction: 32 768 cubes of 40 members 133 -> 9.6 ms.  Faster at every size
+// from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
 #include <math.h>
 
@@ -364,8 +364,8 @@ __device__ inline void load_t(int n, const double* tri, int s_first, int nsl, do
   __syncwarp();
 }
 
-// reciprocal pivots R and multipliers L of T + sigma = L D L^T for this lane's
-// (slot, node) pair
+// reciprocal pivots R and multipliers L (L[32 i] of the edge i - 1, i) of T +
+// sigma = L D L^T for this lane's (slot, node) pair
 __device__ inline void factor(int n, const double* D, const double* E, double sigma, double* R,
                               double* L) {
   double r = rcp(D[0] + sigma);
@@ -377,6 +377,36 @@ __device__ inline void factor(int n, const double* D, const double* E, double si
     L[32 * i] = l;
     R[32 * i] = r;
   }
+}
+
+// The same elimination from both ends, meeting at element m = n / 2: as many
+// operations in two independent chains of half the length.
+__device__ inline void factor_twisted(int n, const double* D, const double* E, double sigma, double* R,
+                                      double* L) {
+  const int m = n / 2, nd = n - 1 - m;  // nd elements below m, m >= nd above
+  double r = rcp(D[0] + sigma), q = rcp(D[n - 1] + sigma);
+  R[0] = r;
+  R[32 * (n - 1)] = q;
+  for (int c = 1; c < nd; ++c) {
+    const int b = n - 1 - c;
+    const double e = E[c], l = e * r, h = E[b + 1], k = h * q;
+    r = rcp(fma(-l, e, D[c] + sigma));
+    q = rcp(fma(-k, h, D[b] + sigma));
+    L[32 * c] = l;
+    R[32 * c] = r;
+    L[32 * (b + 1)] = k;
+    R[32 * b] = q;
+  }
+  if (m > nd) {
+    const double e = E[m - 1], l = e * r;
+    r = rcp(fma(-l, e, D[m - 1] + sigma));
+    L[32 * (m - 1)] = l;
+    R[32 * (m - 1)] = r;
+  }
+  const double e = E[m], l = e * r, h = E[m + 1], k = h * q;
+  L[32 * m] = l;
+  L[32 * (m + 1)] = k;
+  R[32 * m] = rcp(fma(-k, h, fma(-l, e, D[m] + sigma)));
 }
 
 }  // namespace ft
@@ -415,29 +445,67 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
   const int fs = lane % slots, fj = lane / slots;
   const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
   for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
+  const int m = n / 2, nd = n - 1 - m;
   auto solve = [&](int pair, double w) {
-    // A += w (T + s)^-1 y with the factors of the pair; each recurrence's chain
-    // is one fused multiply-add per element
+    // A += w (T + s)^-1 y with the pair's twisted factors: inwards, then outwards
+    // from element m, both chains one fused multiply-add per element; the next
+    // element's operands are read ahead of the chains' stores
     const double *Rp = R + pair, *Lp = L + pair;
-    double f = Y[0];
+    double f = Y[0], h = Y[32 * (n - 1)];
     F[0] = f;
+    F[32 * (n - 1)] = h;
+    double lf = Lp[32], yf = Y[32], lh = Lp[32 * (n - 1)], yh = Y[32 * (n - 2)];
 #pragma unroll 4
-    for (int i = 1; i < n; ++i) {
-      f = fma(-Lp[32 * i], f, Y[32 * i]);
-      F[32 * i] = f;
+    for (int c = 1; c < nd; ++c) {
+      const int b = n - 1 - c;
+      f = fma(-lf, f, yf);
+      h = fma(-lh, h, yh);
+      lf = Lp[32 * (c + 1)];
+      yf = Y[32 * (c + 1)];
+      lh = Lp[32 * b];
+      yh = Y[32 * (b - 1)];
+      F[32 * c] = f;
+      F[32 * b] = h;
     }
-    double x = Rp[32 * (n - 1)] * f;
-    A[32 * (n - 1)] = fma(w, x, A[32 * (n - 1)]);
+    if (m > nd) {
+      f = fma(-lf, f, yf);
+      F[32 * (m - 1)] = f;
+    }
+    double u = Rp[32 * m] * fma(-Lp[32 * (m + 1)], h, fma(-Lp[32 * m], f, Y[32 * m]));
+    A[32 * m] = fma(w, u, A[32 * m]);
+    double d = u;
+    int iu = m - 1, id = m + 1;
+    double lu = Lp[32 * m], gu = Rp[32 * iu] * F[32 * iu], au = A[32 * iu];
+    double ld = Lp[32 * id], gd = Rp[32 * id] * F[32 * id], ad = A[32 * id];
 #pragma unroll 4
-    for (int i = n - 2; i >= 0; --i) {
-      x = fma(-Lp[32 * (i + 1)], x, Rp[32 * i] * F[32 * i]);
-      A[32 * i] = fma(w, x, A[32 * i]);
+    for (int c = 1; c < nd; ++c) {
+      u = fma(-lu, u, gu);
+      d = fma(-ld, d, gd);
+      const double xu = fma(w, u, au), xd = fma(w, d, ad);
+      const int ju = iu - 1, jd = id + 1;
+      lu = Lp[32 * iu];
+      gu = Rp[32 * ju] * F[32 * ju];
+      au = A[32 * ju];
+      ld = Lp[32 * jd];
+      gd = Rp[32 * jd] * F[32 * jd];
+      ad = A[32 * jd];
+      A[32 * iu] = xu;
+      A[32 * id] = xd;
+      iu = ju;
+      id = jd;
+    }
+    u = fma(-lu, u, gu);
+    A[32 * iu] = fma(w, u, au);
+    A[32 * id] = fma(w, fma(-ld, d, gd), ad);
+    if (m > nd) {
+      u = fma(-Lp[32], u, Rp[0] * F[0]);
+      A[0] = fma(w, u, A[0]);
     }
   };
   for (int j0 = 0; j0 < nmax; j0 += nb) {
     if (fs < nsl && fj < nb && j0 + fj < nmax)
-      ft::factor(n, Dg + fs * n, Eg + fs * n, ft::g_nodes[s_row[fs]][j0 + fj].x * shift, R + lane,
-                 L + lane);
+      ft::factor_twisted(n, Dg + fs * n, Eg + fs * n, ft::g_nodes[s_row[fs]][j0 + fj].x * shift,
+                         R + lane, L + lane);
     __syncwarp();
     if (mine) {
       const int rowq = s_row[sl];
