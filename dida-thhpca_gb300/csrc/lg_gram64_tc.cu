@@ -17,14 +17,21 @@
 // entries are exact integers; they are combined in 64-bit integers.  Pairs of
 // slices (a, b) with a + b >= 7 (below 2^-63 of the largest product) are left
 // out, and of the rest only one of (a, b) and (b, a) is formed (C is symmetric).
-// Slices lie in shared memory as [zero 5 0 1 3 2 4], 64 rows each, so that two
-// neighbours make one M = 128 operand (rows "first | second"):
+// Up to 40 members three slices make one M = 128 operand.  They lie as [zero zero
+// 3 4 5 0 1 2], 40 rows each, followed by the slices of d~ as rows of their own:
+//   A = [0;1;2] x B = [8 rows of zero, 3 4 5 0 1 2, d~] (N = 256)   01 .. 25, d~
+//   A = [3;4;5] x B = d~ (N = 16), into the first 8 columns         d~
+//   A = [zero;zero;3] x B = [3] (N = 48), onto 20                   33
+// 256 tensor-memory columns, so two buffers alternate and the sums of one are
+// taken out while the next is filled.  From 41 members on the slices lie as [zero
+// 5 0 1 3 2 4], 64 rows each, and two neighbours make an operand ("first | second"):
 //   block 0   A = [5;0] x B = [0]              50 | 00
 //   1..4      A = [0;1] x B = [1 3 2 4]        01 03 02 04 | 11 13 12 14
 //   5         A = [3;2] x B = [3]              33 | 23
 //   6         A = [2;4] x B = [2], + [zero;5] x [1]   22 | 42 + 51
 //   d~        A = [5;0], [1;3], [2;4] x B = the six slices of d~ (N = 16)
-// 448 + 48 of the 512 tensor-memory columns.  An element's error is about
+// 448 + 48 of the 512 tensor-memory columns: the sums are taken out before the
+// next ones begin.  An element's error is about
 // 2^-54 of the chunk's largest |z| times |z| per entry, adding up as a random
 // walk; a chain of FP64 additions loses 2^-53 of the partial sum at each.
 //
@@ -44,14 +51,16 @@
 // raises s_abort, every role leaves its loop and the launch reports
 // LG_ERR_TIMEOUT.
 //
-// Bound: an MMA of M = 128 takes max(46, N / 2) cycles, the eight of a K = 16
-// chunk 432 alone and about 800 beside the conversions, which share the shared
-// memory's bandwidth with the operands (50 KB a chunk); a stage of conversions
-// is about 3000 cycles of the twelve warps.  Measured alone against gram64_kernel:
-// 921 600 solves of 40 members and 379 entries (of 1562 candidates) 727 -> 126
-// ms; 129 600 of 64 members, 954 entries 595 -> 54 ms; 82 944 of 40 members, 24
-// entries 5.6 -> 3.6 ms; 2592 of 16 members, 51 entries 0.18 -> 0.08 ms.  It wins
-// at every size, so up to 64 members there is no other path.
+// Bound: the conversions, about 3000 issue slots of twelve warps a stage, beside
+// the MMAs -- max(46, N / 2) cycles each, 220 a K = 16 chunk with three slices per
+// operand, 432 with two, and about 800 while the conversions share the shared
+// memory's bandwidth with their operands (22 and 50 KB a chunk).  Two slices per
+// operand and one buffer at 40 members left the MMAs waiting for the sums to be
+// taken out; measured alone (gram64_kernel -> two slices -> three slices): 921 600
+// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 126 -> 104 ms;
+// 82 944 of 40 members, 24 entries 5.6 -> 3.6 -> 3.6 ms; 2592 of 16 members, 51
+// entries 0.18 -> 0.085 -> 0.077 ms; 129 600 of 64 members, 954 entries 595 -> 54
+// ms.  It wins at every size, so up to 64 members there is no other path.
 // A solve with a non-finite weight, row or innovation, or with magnitudes
 // outside 2^+-400, is marked by a bit pattern in its first Gram element that no
 // other solve can produce, and redone by gram64_kernel.
@@ -69,16 +78,30 @@ constexpr int kX0 = kMmaWarp + 1, kD0 = kX0 + kXWarps;  // first warps (multiple
 constexpr int kPThreads = 32 * kPWarps, kXThreads = 32 * kXWarps, kDThreads = 32 * kDWarps;
 constexpr int kThreads = 32 * (kD0 + kDWarps);
 constexpr int kStage = 64;                            // entries per stage (4 K = 16 chunks)
-constexpr int kSlice = 64 * 16 * 2;                   // 2048 B: 64 rows x K = 16 FP16
-constexpr int kTileD = 7 * kSlice;                    // the d~ tile after zero and six slices
-constexpr int kChunkBytes = kTileD + 16 * 16 * 2;
-constexpr int kStageBytes = 4 * kChunkBytes;          // 59392 B
 constexpr int kQueue = 1536;                          // entries of a chunk (one scale)
 constexpr int kPer = 4;                               // candidates per thread and refill
 constexpr int kRefill = kPer * kPThreads;
 constexpr int kGroup = 4;                             // stages per exact FP32 sum (256 entries)
 constexpr int kQueueBytes = kQueue * (16 + 8);
-constexpr int kSmem = 2 * kStageBytes + 2 * kQueueBytes + 64 * 65 * 8;
+// Operands and sums in shared memory.  A slice is kRows rows x K = 16 FP16.
+template <bool kThree>
+struct Layout {
+  static constexpr int kRows = kThree ? 40 : 64;
+  static constexpr int kSlice = kRows * 16 * 2;
+  // [zero zero 3 4 5 0 1 2], d~ (8 rows), d~ again (16 rows); [zero 5 0 1 3 2 4], d~ (16)
+  static constexpr int kTileD = (kThree ? 8 : 7) * kSlice;
+  static constexpr int kTileD2 = kTileD + 8 * 16 * 2;
+  static constexpr int kChunk = kThree ? kTileD2 + 16 * 16 * 2 : kTileD + 16 * 16 * 2;
+  static constexpr int kStageBytes = 4 * kChunk;
+  static constexpr int kUStride = kThree ? 41 : 65;
+  static constexpr int kURows = kThree ? 120 : 64;  // a row per accumulator row, or per member
+  static constexpr int kSmem = 2 * kStageBytes + 2 * kQueueBytes + kURows * kUStride * 8;
+  // memory position of slice a
+  static __host__ __device__ constexpr int pos(int a) {
+    return kThree ? (a >= 3 ? a - 1 : a + 5)
+                  : a == 5 ? 1 : a == 0 ? 2 : a == 1 ? 3 : a == 3 ? 4 : a == 2 ? 5 : 6;
+  }
+};
 // C's exact sums are kept in units of 2^-51 of the largest product times 2^-1:
 // twice the sum of 1536 products stays below 2^63
 constexpr int kDrop = 10;
@@ -200,10 +223,6 @@ __device__ inline void digit_pairs(unsigned long long z0, unsigned long long z1,
   out[1] = pack(a1 >> 9, b1 << 7, 0x01ff01ffu);
   out[0] = pack(a1 >> 18, b1 >> 2, 0x03ff03ffu);
 }
-// memory position of slice a in [zero 5 0 1 3 2 4]
-__host__ __device__ constexpr int slice_pos(int a) {
-  return a == 5 ? 1 : a == 0 ? 2 : a == 1 ? 3 : a == 3 ? 4 : a == 2 ? 5 : 6;
-}
 
 // Gaspari-Cohn as schr2 (lg_device.cuh) without its divisions: the same
 // polynomial with fused multiply-adds, 1/12 rounded once and 1/ri by two
@@ -273,20 +292,25 @@ struct QueueHead {
 };
 
 // kR: units (member, 4 entries) of a stage per converting thread -- 2 up to 48
-// members, 3 above
-template <int kR>
+// members, 3 above.  kThree: three slices in an operand's 128 rows (up to 40
+// members).
+template <int kR, bool kThree>
 __global__ void __launch_bounds__(g64::kThreads, 1)
     gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, double* Cout, double* tout,
                      int* err) {
   using namespace g64;
+  using L = Layout<kThree>;
+  constexpr int kSlice = L::kSlice, kTileD = L::kTileD, kChunkBytes = L::kChunk,
+                kStageBytes = L::kStageBytes, kUStride = L::kUStride;
+  constexpr int kBufs = kThree ? 2 : 1;  // accumulator buffers in tensor memory
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // operand buffer multiplied, converted; queue full, empty; exact sum complete,
   // taken out (one phase per group of stages: the adding warps wait for no stage
   // in between, so a stage barrier's parity would not tell them which phase it is)
-  __shared__ uint64_t m_mma[2], m_conv[2], m_full[2], m_empty[2], m_sum, m_drain;
+  __shared__ uint64_t m_mma[2], m_conv[2], m_full[2], m_empty[2], m_sum[2], m_drain[2];
   __shared__ uint32_t tmem_base_sh;
   __shared__ int s_wcnt[2][kPWarps];
-  __shared__ longlong2 s_t[2][64];
+  __shared__ longlong2 s_t[kThree ? 3 : 2][64];
   __shared__ int s_kmax, s_dmax, s_nf;
   __shared__ volatile int s_abort;
   __shared__ int s_stop[2];  // s_abort as the weighing and the adding warps agree on it
@@ -301,16 +325,16 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       tc::mbar_init(&m_conv[i], kXWarps);
       tc::mbar_init(&m_full[i], kPThreads);
       tc::mbar_init(&m_empty[i], kXWarps + 1 + kDWarps);
+      tc::mbar_init(&m_sum[i], 1);
+      tc::mbar_init(&m_drain[i], kDWarps);
     }
-    tc::mbar_init(&m_sum, 1);
-    tc::mbar_init(&m_drain, kDWarps);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // the zero slices of the two operand buffers
-  for (int i = tid; i < 8 * kSlice / 16; i += kThreads)
-    *reinterpret_cast<uint4*>(smem_raw + (i / (kSlice / 16)) * kChunkBytes +
-                              i % (kSlice / 16) * 16) = make_uint4(0, 0, 0, 0);
+  // the operand buffers' rows that stay zero: zero slices, members above k, the
+  // d~ tiles' other rows
+  for (int i = tid; i < 2 * kStageBytes / 16; i += kThreads)
+    reinterpret_cast<uint4*>(smem_raw)[i] = make_uint4(0, 0, 0, 0);
   tc::fence_proxy_async();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -566,7 +590,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         wait(&m_conv[n & 1], (n >> 1) & 1);
         if (st % kGroup == 0) {
           // a new exact sum: the finished one is out of tensor memory
-          if (groups > 0) wait(&m_drain, (groups - 1) & 1);
+          if (groups >= kBufs)
+            wait(&m_drain[(groups - kBufs) % kBufs], ((groups - kBufs) / kBufs) & 1);
           ++groups;
         }
         if (stopped()) break;
@@ -581,17 +606,25 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
           for (int c = 0; c < 4; ++c) {
             const int o = c * kChunkBytes;
             const uint32_t more = (st % kGroup > 0 || c > 0) ? 1u : 0u;
-            mma(tmem, at(o + kSlice), at(o + 2 * kSlice), idesc(64), more);           // [5;0] x 0
-            mma(tmem + 64, at(o + 2 * kSlice), at(o + 3 * kSlice), idesc(256), more); // [0;1] x 1 3 2 4
-            mma(tmem + 320, at(o + 4 * kSlice), at(o + 4 * kSlice), idesc(64), more); // [3;2] x 3
-            mma(tmem + 384, at(o + 5 * kSlice), at(o + 5 * kSlice), idesc(64), more); // [2;4] x 2
-            mma(tmem + 384, at(o), at(o + 3 * kSlice), idesc(64), 1u);                // [zero;5] x 1
-            mma(tmem + kColD, at(o + kSlice), at(o + kTileD), idesc(16), more);
-            mma(tmem + kColD + 16, at(o + 3 * kSlice), at(o + kTileD), idesc(16), more);
-            mma(tmem + kColD + 32, at(o + 5 * kSlice), at(o + kTileD), idesc(16), more);
+            if constexpr (kThree) {
+              const uint32_t d = tmem + ((groups - 1) & 1) * 256;
+              // [0;1;2] x [zero 3 4 5 0 1 2 d~], [3;4;5] x d~, [zero;zero;3] x 3
+              mma(d, at(o + 5 * kSlice), at(o + 2 * kSlice - 256), idesc(256), more);
+              mma(d, at(o + 2 * kSlice), at(o + L::kTileD2), idesc(16), 1u);
+              mma(d + 128, at(o), at(o + 2 * kSlice), idesc(48), 1u);
+            } else {
+              mma(tmem, at(o + kSlice), at(o + 2 * kSlice), idesc(64), more);           // [5;0] x 0
+              mma(tmem + 64, at(o + 2 * kSlice), at(o + 3 * kSlice), idesc(256), more); // [0;1] x 1 3 2 4
+              mma(tmem + 320, at(o + 4 * kSlice), at(o + 4 * kSlice), idesc(64), more); // [3;2] x 3
+              mma(tmem + 384, at(o + 5 * kSlice), at(o + 5 * kSlice), idesc(64), more); // [2;4] x 2
+              mma(tmem + 384, at(o), at(o + 3 * kSlice), idesc(64), 1u);                // [zero;5] x 1
+              mma(tmem + kColD, at(o + kSlice), at(o + kTileD), idesc(16), more);
+              mma(tmem + kColD + 16, at(o + 3 * kSlice), at(o + kTileD), idesc(16), more);
+              mma(tmem + kColD + 32, at(o + 5 * kSlice), at(o + kTileD), idesc(16), more);
+            }
           }
           tc::mma_commit(&m_mma[n & 1]);
-          if (st % kGroup == kGroup - 1 || st == stages - 1) tc::mma_commit(&m_sum);
+          if (st % kGroup == kGroup - 1 || st == stages - 1) tc::mma_commit(&m_sum[(groups - 1) % kBufs]);
         }
         __syncwarp();
       }
@@ -655,7 +688,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
           unsigned char* const dst = buf + ud[r];
 #pragma unroll
           for (int a = 0; a < 6; ++a)
-            *reinterpret_cast<uint2*>(dst + slice_pos(a) * kSlice) = make_uint2(o[0][a], o[1][a]);
+            *reinterpret_cast<uint2*>(dst + L::pos(a) * kSlice) = make_uint2(o[0][a], o[1][a]);
         }
         if (warp == kD0 - 1) {
           // d~ slices: row b of the 16-row tile, two entries per lane
@@ -668,6 +701,10 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
                                      ((lane >> 2) & 1) * 128 + (lane & 3) * 4;
 #pragma unroll
           for (int a = 0; a < 6; ++a) *reinterpret_cast<uint32_t*>(dst + a * 16) = o[a];
+          if constexpr (kThree)
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+              *reinterpret_cast<uint32_t*>(dst + L::kTileD2 - kTileD + a * 16) = o[a];
         }
         tc::fence_proxy_async();
         __syncwarp();
@@ -680,14 +717,31 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     // ================= adding warps
     const int xt = tid - 32 * kD0;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const bool low = (warp & 3) < 2;         // accumulator rows 0..63: the first slice of A
-    const int row = (warp & 1) * 32 + lane;  // member of this thread's accumulator row
+    // this thread's accumulator row: slice of the operand and member
+    const int arow = (warp & 3) * 32 + lane;
+    const int blk = kThree ? arow / 40 : arow / 64;
+    const int row = kThree ? arow - 40 * blk : arow - 64 * blk;
+    const bool low = blk == 0;
     // columns of this warp quadruple: groups of four, from j0
     const int cw = (k + 7) / 8 * 4;
     const int j0 = (warp - kD0) / 4 * cw;
     const int ng = (cw + 3) / 4, h0 = (ng + 1) / 2;
-    // the chunk's sums, 64 x 65
+    // the chunk's sums: per member, or (kThree) per accumulator row
     long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + 2 * kQueueBytes);
+    // kThree: an off-diagonal pair counts twice, weight 2^(90 - 9 (a + b)) in units
+    // of 2^(45 + kDrop); slice blk against slices 0 (times 2^32), 1, 2, 3, and
+    // below a unit, times 2^-19, against 0, 2, 3, 4, 5.  33 shares its sum with 20,
+    // which 02 takes off again: (U + U^T) sees 20 and 02 alike.
+    //   0   00 2^35, 01 2^27, 02 2^18 - 2^-19, 03 2^9, 04 1, 05 2^-9
+    //   1   11 2^17, 12 2^9, 13 1, 14 2^-9, 15 2^-18
+    //   2   20+33 2^-19, 22 2^-1, 23 2^-9, 24 2^-18
+    const int c00 = blk == 0 ? 8 : 0, h1 = blk == 0 ? 1 << 27 : blk == 1 ? 1 << 17 : 0;
+    const int h2 = blk == 0 ? 1 << 18 : blk == 1 ? 1 << 9 : 0;
+    const int h3 = blk == 0 ? 1 << 9 : blk == 1 ? 1 : 0;
+    const int f0 = blk == 2 ? 1 : 0, f2 = blk == 0 ? -1 : blk == 1 ? 0 : 1 << 18;
+    const int f3 = blk == 2 ? 1 << 10 : 0;
+    const int f4 = blk == 0 ? 1 << 19 : blk == 1 ? 1 << 10 : 2;
+    const int f5 = blk == 0 ? 1 << 10 : blk == 1 ? 2 : 0;
     unsigned groups = 0;  // exact sums taken out
     for (unsigned nq = 0;; ++nq) {
       const int qb = nq & 1;
@@ -706,73 +760,134 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       // added to U
       auto columns = [&](int g4, bool add) {
         const int j = j0 + 4 * g4;
-        float v[7][4];
+        if constexpr (kThree) {
+          const uint32_t at = lane_addr + (groups & 1) * 256 + 8u + (uint32_t)j;
+          float v[6][4];
 #pragma unroll
-        for (int m = 0; m < 7; ++m) tmem_ld4(lane_addr + 64u * m + (uint32_t)j, v[m]);
-        tmem_wait_ld();
-        long long* const u = U + row * 65 + j;
+          for (int m = 0; m < 6; ++m) tmem_ld4(at + 40u * m, v[m]);
+          tmem_wait_ld();
+          long long* const u = U + arow * kUStride + j;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          int x[7];
+          for (int c = 0; c < 4; ++c) {
+            int x[6];  // against slices 3 4 5 0 1 2
 #pragma unroll
-          for (int m = 0; m < 7; ++m) x[m] = __float2int_rn(v[m][c]);
-          // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
-          // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
-          long long A = add ? u[c] : 0;
-          if (low) {  // 50 01 03 02 04 33 22
-            A += (long long)x[1] * (1 << 27);
-            A += (long long)x[3] * (1 << 18);
-            A += (long long)x[2] * (1 << 9);
-            const int y = 2 * x[4] + x[6] + ((x[0] + (x[5] >> 10) + 128) >> 8);
-            A += (y + 1) >> 1;
-          } else {    // 00 11 13 12 14 23 42+51
-            A += (long long)((unsigned long long)(unsigned)(x[0] * 8) << 32);
-            A += (long long)x[1] * (1 << 17);
-            A += (long long)x[3] * (1 << 9);
-            A += x[2] + ((x[4] + x[5] + ((x[6] + 256) >> 9) + 256) >> 9);
+            for (int m = 0; m < 6; ++m) x[m] = __float2int_rn(v[m][c]);
+            long long A = add && arow < 120 ? u[c] : 0;
+            A += (long long)((unsigned long long)(unsigned)(x[3] * c00) << 32);
+            A += (long long)x[4] * h1;
+            A += (long long)x[5] * h2;
+            A += (long long)x[0] * h3;
+            // below a unit, in units of 2^-19
+            long long f = (long long)x[3] * f0 + (1 << 18);
+            f += (long long)x[5] * f2;
+            f += (long long)x[0] * f3;
+            f += (long long)x[1] * f4;
+            f += (long long)x[2] * f5;
+            if (arow < 120) u[c] = A + (f >> 19);
           }
-          u[c] = A;
+        } else {
+          float v[7][4];
+#pragma unroll
+          for (int m = 0; m < 7; ++m) tmem_ld4(lane_addr + 64u * m + (uint32_t)j, v[m]);
+          tmem_wait_ld();
+          long long* const u = U + row * kUStride + j;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            int x[7];
+#pragma unroll
+            for (int m = 0; m < 7; ++m) x[m] = __float2int_rn(v[m][c]);
+            // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
+            // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
+            long long A = add ? u[c] : 0;
+            if (low) {  // 50 01 03 02 04 33 22
+              A += (long long)x[1] * (1 << 27);
+              A += (long long)x[3] * (1 << 18);
+              A += (long long)x[2] * (1 << 9);
+              const int y = 2 * x[4] + x[6] + ((x[0] + (x[5] >> 10) + 128) >> 8);
+              A += (y + 1) >> 1;
+            } else {    // 00 11 13 12 14 23 42+51
+              A += (long long)((unsigned long long)(unsigned)(x[0] * 8) << 32);
+              A += (long long)x[1] * (1 << 17);
+              A += (long long)x[3] * (1 << 9);
+              A += x[2] + ((x[4] + x[5] + ((x[6] + 256) >> 9) + 256) >> 9);
+            }
+            u[c] = A;
+          }
         }
       };
       for (int st = 0; st < h.stages; st += kGroup, ++groups) {
-        wait(&m_sum, groups & 1);
+        wait(&m_sum[groups % kBufs], (groups / kBufs) & 1);
         tc::fence_after();
-        // The two halves' sums meet in U: one half takes the first columns while the
-        // other takes the rest, then they change over
-        const bool fresh = st == 0;
-        for (int q = low ? 0 : h0; q < (low ? h0 : ng); ++q) columns(q, !fresh);
-        if (j0 == 0) {
-          float v[3][8];
+        if constexpr (kThree) {
+          for (int q = 0; q < ng; ++q) columns(q, st > 0);
+          if (j0 == 0) {
+            const uint32_t at = lane_addr + (groups & 1) * 256;
+            float v[8], z[4];
+            tmem_ld8(at + 248u, v);
+            tmem_ld4(at, z);
+            tmem_wait_ld();
+            long long x[6], y[4];  // slice blk, and blk + 3, against d~ slices 0..
 #pragma unroll
-          for (int m = 0; m < 3; ++m) tmem_ld8(lane_addr + kColD + 16u * m, v[m]);
-          tmem_wait_ld();
-          long long x[3][6];
+            for (int j = 0; j < 6; ++j) x[j] = __float2int_rn(v[j]);
 #pragma unroll
-          for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int j = 0; j < 6; ++j) x[m][j] = __float2int_rn(v[m][j]);
-          // rows 5|0, 1|3, 2|4 of z against d~ slices 0..5, a + b <= 6; thi in
-          // units of weight 2, tlo of weight 5
-          long long w6;
-          if (low) {
-            thi += (x[1][0] << 9) + x[1][1] + x[2][0];
-            tlo += (x[1][2] << 18) + (x[1][3] << 9) + x[1][4] + (x[2][1] << 18) + (x[2][2] << 9) +
-                   x[2][3] + x[0][0];
-            w6 = x[0][1] + x[1][5] + x[2][4];
-          } else {
-            thi += (x[0][0] << 18) + (x[0][1] << 9) + x[0][2];
-            tlo += (x[0][3] << 18) + (x[0][4] << 9) + x[0][5] + (x[1][0] << 18) + (x[1][1] << 9) +
-                   x[1][2] + (x[2][0] << 9) + x[2][1];
-            w6 = x[1][3] + x[2][2];
+            for (int j = 0; j < 4; ++j) y[j] = __float2int_rn(z[j]);
+            long long w6;
+            if (blk == 0) {
+              thi += (x[0] << 18) + (x[1] << 9) + x[2];
+              tlo += (x[3] << 18) + (x[4] << 9) + x[5] + (y[0] << 18) + (y[1] << 9) + y[2];
+              w6 = y[3];
+            } else if (blk == 1) {
+              thi += (x[0] << 9) + x[1];
+              tlo += (x[2] << 18) + (x[3] << 9) + x[4] + (y[0] << 9) + y[1];
+              w6 = x[5] + y[2];
+            } else {
+              thi += x[0];
+              tlo += (x[1] << 18) + (x[2] << 9) + x[3] + y[0];
+              w6 = x[4] + y[1];
+            }
+            tlo += (w6 + 256) >> 9;
           }
-          tlo += (w6 + 256) >> 9;
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&m_drain[groups & 1]);
+        } else {
+          // The two halves' sums meet in U: one half takes the first columns while the
+          // other takes the rest, then they change over
+          const bool fresh = st == 0;
+          for (int q = low ? 0 : h0; q < (low ? h0 : ng); ++q) columns(q, !fresh);
+          if (j0 == 0) {
+            float v[3][8];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) tmem_ld8(lane_addr + kColD + 16u * m, v[m]);
+            tmem_wait_ld();
+            long long x[3][6];
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+#pragma unroll
+              for (int j = 0; j < 6; ++j) x[m][j] = __float2int_rn(v[m][j]);
+            // rows 5|0, 1|3, 2|4 of z against d~ slices 0..5, a + b <= 6; thi in
+            // units of weight 2, tlo of weight 5
+            long long w6;
+            if (low) {
+              thi += (x[1][0] << 9) + x[1][1] + x[2][0];
+              tlo += (x[1][2] << 18) + (x[1][3] << 9) + x[1][4] + (x[2][1] << 18) + (x[2][2] << 9) +
+                     x[2][3] + x[0][0];
+              w6 = x[0][1] + x[1][5] + x[2][4];
+            } else {
+              thi += (x[0][0] << 18) + (x[0][1] << 9) + x[0][2];
+              tlo += (x[0][3] << 18) + (x[0][4] << 9) + x[0][5] + (x[1][0] << 18) + (x[1][1] << 9) +
+                     x[1][2] + (x[2][0] << 9) + x[2][1];
+              w6 = x[1][3] + x[2][2];
+            }
+            tlo += (w6 + 256) >> 9;
+          }
+          bar_sync(kBarD, kDThreads);
+          for (int q = low ? h0 : 0; q < (low ? ng : h0); ++q) columns(q, true);
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&m_drain[0]);
+          if (st + kGroup < h.stages) bar_sync(kBarD, kDThreads);  // U's columns change hands again
         }
-        bar_sync(kBarD, kDThreads);
-        for (int q = low ? h0 : 0; q < (low ? ng : h0); ++q) columns(q, true);
-        tc::fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&m_drain);
-        if (st + kGroup < h.stages) bar_sync(kBarD, kDThreads);  // U's columns change hands again
       }
       if (h.bad) {
         // (an earlier chunk's C is written: the barrier at the top)
@@ -780,7 +895,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         continue;
       }
       if (h.stages == 0 && !h.first) continue;
-      if (j0 == 0) s_t[low ? 0 : 1][row] = make_longlong2(thi, tlo);
+      if (j0 == 0 && arow < (kThree ? 120 : 128)) s_t[blk][row] = make_longlong2(thi, tlo);
       bar_sync(kBarD, kDThreads);
       const int ex2 = 2 * h.S - 62 + kDrop, ext = h.S + h.Sd - 61;
       // C = (U + U^T) / 2 in place (rows i and k - 1 - i of the triangle share one
@@ -790,10 +905,13 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
              r += kDThreads) {
           const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
           if (!(2 * a == k - 1 && c > a)) {  // odd k: the middle row meets itself
-            const long long v =
-                __double_as_longlong(fixed_to_double(U[i * 65 + j] + U[j * 65 + i], ex2));
-            U[i * 65 + j] = v;
-            U[j * 65 + i] = v;
+            long long u = U[i * kUStride + j] + U[j * kUStride + i];
+            if constexpr (kThree)
+              u += U[(40 + i) * kUStride + j] + U[(40 + j) * kUStride + i] +
+                   U[(80 + i) * kUStride + j] + U[(80 + j) * kUStride + i];
+            const long long v = __double_as_longlong(fixed_to_double(u, ex2));
+            U[i * kUStride + j] = v;
+            U[j * kUStride + i] = v;
           }
           c += kDThreads;
           while (c > k) {
@@ -804,7 +922,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         bar_sync(kBarD, kDThreads);
       }
       for (int r = xt, j = xt / k, i = xt - j * k; r < k * k; r += kDThreads) {
-        double v = h.stages > 0 ? __longlong_as_double(U[j * 65 + i]) : 0.0;
+        double v = h.stages > 0 ? __longlong_as_double(U[j * kUStride + i]) : 0.0;
         if (!h.first) v += C[r];
         C[r] = v;
         i += kDThreads;
@@ -815,8 +933,14 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       }
       if (xt < k) {
         double v = 0.0;
-        if (h.stages > 0)
-          v = wide_to_double(s_t[0][xt].x + s_t[1][xt].x, s_t[0][xt].y + s_t[1][xt].y, ext);
+        if (h.stages > 0) {
+          long long hi = s_t[0][xt].x + s_t[1][xt].x, lo = s_t[0][xt].y + s_t[1][xt].y;
+          if constexpr (kThree) {
+            hi += s_t[2][xt].x;
+            lo += s_t[2][xt].y;
+          }
+          v = wide_to_double(hi, lo, ext);
+        }
         tv[xt] = h.first ? v : tv[xt] + v;
       }
     }
@@ -837,14 +961,16 @@ void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, cons
   const int grid = b.nsolves < 152 ? b.nsolves : 152;
   if (b.mode == 0 && g.vert_dist > 0.0)
     level_lnp_kernel<<<(b.nsolves + 127) / 128, 128, 0, stream>>>(g, b, axb, t);
-  auto run = [&](auto kernel) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g64::kSmem);
-    kernel<<<grid, g64::kThreads, g64::kSmem, stream>>>(g, hx, l, b, C, t, err);
+  auto run = [&](auto kernel, int smem) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    kernel<<<grid, g64::kThreads, smem, stream>>>(g, hx, l, b, C, t, err);
   };
-  if (g.ens <= 48)
-    run(gram64_tc_kernel<2>);
+  if (g.ens <= 40)
+    run(gram64_tc_kernel<2, true>, g64::Layout<true>::kSmem);
+  else if (g.ens <= 48)
+    run(gram64_tc_kernel<2, false>, g64::Layout<false>::kSmem);
   else
-    run(gram64_tc_kernel<3>);
+    run(gram64_tc_kernel<3, false>, g64::Layout<false>::kSmem);
 }
 
 }  // namespace lg

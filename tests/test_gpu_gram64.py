@@ -106,3 +106,22 @@ def test_values_left_to_the_fp64_kernel():
     assert np.allclose(tr[2], np.sqrt(1.05) * np.eye(k), rtol=0, atol=1e-13)
     _, wt = _reference(*tiny, 1.05)
     assert np.allclose(wb[2], wt, rtol=1e-11, atol=0)
+
+
+@pytest.mark.parametrize("k", [3, 23, 32, 39, 40, 41])
+def test_three_slices_per_operand(k):
+    """Up to 40 members three slices share an operand's 128 rows and two
+    accumulator buffers alternate: list lengths around one to four of the exact
+    sums that change them, and weights of one sign (the largest sums)."""
+    rng = np.random.default_rng(300 + k)
+    sizes = [1, 256, 257, 511, 512, 513, 769, 1025, 1793, 2049]
+    cases = [_case(rng, k, p) for p in sizes]
+    same = _case(rng, k, 1024)
+    same[0][:] = same[0][0] * rng.uniform(0.99, 1.0, 1024)[:, None]  # nearly one row 1024 times
+    cases.append(same)
+    st, tr, wb = _batch(cases, 1.05)
+    assert st == 0
+    for c, t, w, p in zip(cases, tr, wb, sizes + ["same"]):
+        t0, w0 = _reference(*c, 1.05)
+        assert np.allclose(t, t0, rtol=1e-11, atol=1e-11), p
+        assert np.allclose(w, w0, rtol=1e-11, atol=1e-11), p
