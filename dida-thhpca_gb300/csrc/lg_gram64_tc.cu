@@ -56,11 +56,12 @@
 // operand, 432 with two, and about 800 while the conversions share the shared
 // memory's bandwidth with their operands (22 and 50 KB a chunk).  Two slices per
 // operand and one buffer at 40 members left the MMAs waiting for the sums to be
-// taken out; measured alone (gram64_kernel -> two slices -> three slices): 921 600
-// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 126 -> 104 ms;
-// 82 944 of 40 members, 24 entries 5.6 -> 3.6 -> 3.6 ms; 2592 of 16 members, 51
-// entries 0.18 -> 0.085 -> 0.077 ms; 129 600 of 64 members, 954 entries 595 -> 54
-// ms.  It wins at every size, so up to 64 members there is no other path.
+// taken out, and each sum's conversion to integers (16 lanes a cycle and SM) is
+// kept to four or five per element.  Measured alone against gram64_kernel: 921 600
+// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 95 ms (126 with
+// two slices per operand); 82 944 of 40 members, 24 entries 5.6 -> 3.0 ms; 2592 of
+// 16 members, 51 entries 0.18 -> 0.08 ms; 129 600 of 64 members, 954 entries 595 ->
+// 49 ms.  It wins at every size, so up to 64 members there is no other path.
 // A solve with a non-finite weight, row or innovation, or with magnitudes
 // outside 2^+-400, is marked by a bit pattern in its first Gram element that no
 // other solve can produce, and redone by gram64_kernel.
@@ -729,19 +730,22 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     // the chunk's sums: per member, or (kThree) per accumulator row
     long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + 2 * kQueueBytes);
     // kThree: an off-diagonal pair counts twice, weight 2^(90 - 9 (a + b)) in units
-    // of 2^(45 + kDrop); slice blk against slices 0 (times 2^32), 1, 2, 3, and
-    // below a unit, times 2^-19, against 0, 2, 3, 4, 5.  33 shares its sum with 20,
+    // of 2^(45 + kDrop); slice blk against slices 0 (times 2^32), 1, 2, 3 as
+    // integers, and against 0, 2, 3, 4, 5 as the FP32 part.  33 shares its sum with 20,
     // which 02 takes off again: (U + U^T) sees 20 and 02 alike.
     //   0   00 2^35, 01 2^27, 02 2^18 - 2^-19, 03 2^9, 04 1, 05 2^-9
     //   1   11 2^17, 12 2^9, 13 1, 14 2^-9, 15 2^-18
     //   2   20+33 2^-19, 22 2^-1, 23 2^-9, 24 2^-18
     const int c00 = blk == 0 ? 8 : 0, h1 = blk == 0 ? 1 << 27 : blk == 1 ? 1 << 17 : 0;
     const int h2 = blk == 0 ? 1 << 18 : blk == 1 ? 1 << 9 : 0;
-    const int h3 = blk == 0 ? 1 << 9 : blk == 1 ? 1 : 0;
-    const int f0 = blk == 2 ? 1 : 0, f2 = blk == 0 ? -1 : blk == 1 ? 0 : 1 << 18;
-    const int f3 = blk == 2 ? 1 << 10 : 0;
-    const int f4 = blk == 0 ? 1 << 19 : blk == 1 ? 1 << 10 : 2;
-    const int f5 = blk == 0 ? 1 << 10 : blk == 1 ? 2 : 0;
+    const int h3 = blk == 0 ? 1 << 9 : 0;
+    const float f0 = blk == 2 ? 0x1p-19f : 0.0f, f2 = blk == 0 ? -0x1p-19f : blk == 1 ? 0.0f : 0.5f;
+    const float f3 = blk == 0 ? 0.0f : blk == 1 ? 1.0f : 0x1p-9f;
+    const float f4 = blk == 0 ? 1.0f : blk == 1 ? 0x1p-9f : 0x1p-18f;
+    const float f5 = blk == 0 ? 0x1p-9f : blk == 1 ? 0x1p-18f : 0.0f;
+    // kDThreads elements further on in rows of k + 1, and of k
+    const int step_a = kDThreads / (k + 1), step_c = kDThreads - step_a * (k + 1);
+    const int step_j = kDThreads / k, step_i = kDThreads - step_j * k;
     unsigned groups = 0;  // exact sums taken out
     for (unsigned nq = 0;; ++nq) {
       const int qb = nq & 1;
@@ -756,70 +760,66 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       double* const C = Cout + (size_t)h.s * k * k;
       double* const tv = tout + (size_t)h.s * k;
       long long thi = 0, tlo = 0;
-      // four columns of this half's exact FP32 sums as one integer each, written or
-      // added to U
+      // four columns of the exact FP32 sums as one integer each, written or added to
+      // U.  The products worth a unit or less (below 2^-50 of the largest product)
+      // come together in FP32 first: 24 bits of at most 2^24 units.
+      auto columns3 = [&](int g4, bool add) {
+        const uint32_t at = lane_addr + (groups & 1) * 256 + 8u + (uint32_t)(j0 + 4 * g4);
+        float v[6][4];  // against slices 3 4 5 0 1 2
+#pragma unroll
+        for (int m = 0; m < 6; ++m) tmem_ld4(at + 40u * m, v[m]);
+        tmem_wait_ld();
+        long long* const u = U + arow * kUStride + j0 + 4 * g4;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float f = fmaf(f0, v[3][c], fmaf(f5, v[2][c], fmaf(f4, v[1][c],
+                          fmaf(f3, v[0][c], f2 * v[5][c]))));
+          long long A = add && arow < 120 ? u[c] : 0;
+          A += __float2int_rn(f);
+          if ((warp & 3) < 3) {  // the last warp's rows are all slice 2
+            A += (long long)__float2int_rn(v[4][c]) * h1;
+            A += (long long)__float2int_rn(v[5][c]) * h2;
+          }
+          if ((warp & 3) < 2) {
+            A += (long long)__float2int_rn(v[0][c]) * h3;
+            A += (long long)((unsigned long long)(unsigned)(__float2int_rn(v[3][c]) * c00) << 32);
+          }
+          if (arow < 120) u[c] = A;
+        }
+      };
       auto columns = [&](int g4, bool add) {
         const int j = j0 + 4 * g4;
-        if constexpr (kThree) {
-          const uint32_t at = lane_addr + (groups & 1) * 256 + 8u + (uint32_t)j;
-          float v[6][4];
+        float v[7][4];
 #pragma unroll
-          for (int m = 0; m < 6; ++m) tmem_ld4(at + 40u * m, v[m]);
-          tmem_wait_ld();
-          long long* const u = U + arow * kUStride + j;
+        for (int m = 0; m < 7; ++m) tmem_ld4(lane_addr + 64u * m + (uint32_t)j, v[m]);
+        tmem_wait_ld();
+        long long* const u = U + row * kUStride + j;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            int x[6];  // against slices 3 4 5 0 1 2
-#pragma unroll
-            for (int m = 0; m < 6; ++m) x[m] = __float2int_rn(v[m][c]);
-            long long A = add && arow < 120 ? u[c] : 0;
-            A += (long long)((unsigned long long)(unsigned)(x[3] * c00) << 32);
-            A += (long long)x[4] * h1;
-            A += (long long)x[5] * h2;
-            A += (long long)x[0] * h3;
-            // below a unit, in units of 2^-19
-            long long f = (long long)x[3] * f0 + (1 << 18);
-            f += (long long)x[5] * f2;
-            f += (long long)x[0] * f3;
-            f += (long long)x[1] * f4;
-            f += (long long)x[2] * f5;
-            if (arow < 120) u[c] = A + (f >> 19);
+        for (int c = 0; c < 4; ++c) {
+          // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
+          // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
+          long long A = add ? u[c] : 0;
+          if (low) {  // 50 01 03 02 04 33 22
+            A += (long long)__float2int_rn(v[1][c]) * (1 << 27);
+            A += (long long)__float2int_rn(v[3][c]) * (1 << 18);
+            A += (long long)__float2int_rn(v[2][c]) * (1 << 9);
+            A += __float2int_rn(
+                fmaf(0x1p-19f, v[5][c], fmaf(0x1p-9f, v[0][c], fmaf(0.5f, v[6][c], v[4][c]))));
+          } else {    // 00 11 13 12 14 23 42+51
+            A += (long long)((unsigned long long)(unsigned)(__float2int_rn(v[0][c]) * 8) << 32);
+            A += (long long)__float2int_rn(v[1][c]) * (1 << 17);
+            A += (long long)__float2int_rn(v[3][c]) * (1 << 9);
+            A += __float2int_rn(
+                fmaf(0x1p-18f, v[6][c], fmaf(0x1p-9f, v[4][c], fmaf(0x1p-9f, v[5][c], v[2][c]))));
           }
-        } else {
-          float v[7][4];
-#pragma unroll
-          for (int m = 0; m < 7; ++m) tmem_ld4(lane_addr + 64u * m + (uint32_t)j, v[m]);
-          tmem_wait_ld();
-          long long* const u = U + row * kUStride + j;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            int x[7];
-#pragma unroll
-            for (int m = 0; m < 7; ++m) x[m] = __float2int_rn(v[m][c]);
-            // an off-diagonal pair counts twice (C = (U + U^T) / 2); weight
-            // 2^(90 - 9 (a + b)) in units of 2^(45 + kDrop)
-            long long A = add ? u[c] : 0;
-            if (low) {  // 50 01 03 02 04 33 22
-              A += (long long)x[1] * (1 << 27);
-              A += (long long)x[3] * (1 << 18);
-              A += (long long)x[2] * (1 << 9);
-              const int y = 2 * x[4] + x[6] + ((x[0] + (x[5] >> 10) + 128) >> 8);
-              A += (y + 1) >> 1;
-            } else {    // 00 11 13 12 14 23 42+51
-              A += (long long)((unsigned long long)(unsigned)(x[0] * 8) << 32);
-              A += (long long)x[1] * (1 << 17);
-              A += (long long)x[3] * (1 << 9);
-              A += x[2] + ((x[4] + x[5] + ((x[6] + 256) >> 9) + 256) >> 9);
-            }
-            u[c] = A;
-          }
+          u[c] = A;
         }
       };
       for (int st = 0; st < h.stages; st += kGroup, ++groups) {
         wait(&m_sum[groups % kBufs], (groups / kBufs) & 1);
         tc::fence_after();
         if constexpr (kThree) {
-          for (int q = 0; q < ng; ++q) columns(q, st > 0);
+          for (int q = 0; q < ng; ++q) columns3(q, st > 0);
           if (j0 == 0) {
             const uint32_t at = lane_addr + (groups & 1) * 256;
             float v[8], z[4];
@@ -899,49 +899,80 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       bar_sync(kBarD, kDThreads);
       const int ex2 = 2 * h.S - 62 + kDrop, ext = h.S + h.Sd - 61;
       // C = (U + U^T) / 2 in place (rows i and k - 1 - i of the triangle share one
-      // row of k + 1 elements), then out in rows
+      // row of k + 1 elements), four elements' loads in flight; t by the threads
+      // with the fewest elements
       if (h.stages > 0) {
-        for (int r = xt, a = xt / (k + 1), c = xt - a * (k + 1); r < (k + 1) / 2 * (k + 1);
-             r += kDThreads) {
-          const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
-          if (!(2 * a == k - 1 && c > a)) {  // odd k: the middle row meets itself
-            long long u = U[i * kUStride + j] + U[j * kUStride + i];
-            if constexpr (kThree)
-              u += U[(40 + i) * kUStride + j] + U[(40 + j) * kUStride + i] +
-                   U[(80 + i) * kUStride + j] + U[(80 + j) * kUStride + i];
-            const long long v = __double_as_longlong(fixed_to_double(u, ex2));
-            U[i * kUStride + j] = v;
-            U[j * kUStride + i] = v;
+        const int total = (k + 1) / 2 * (k + 1);
+        int a = xt / (k + 1), c = xt - a * (k + 1);
+        for (int r0 = xt; r0 < total; r0 += 4 * kDThreads) {
+          int at[4], ta[4];
+          long long u[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
+            // odd k: the middle row meets itself
+            const bool mine = r0 + e * kDThreads < total && !(2 * a == k - 1 && c > a);
+            at[e] = mine ? i * kUStride + j : -1;
+            ta[e] = j * kUStride + i;
+            u[e] = 0;
+            if (mine) {
+              u[e] = U[at[e]] + U[ta[e]];
+              if constexpr (kThree)
+                u[e] += U[at[e] + 40 * kUStride] + U[ta[e] + 40 * kUStride] +
+                        U[at[e] + 80 * kUStride] + U[ta[e] + 80 * kUStride];
+            }
+            a += step_a;
+            c += step_c;
+            if (c > k) {
+              c -= k + 1;
+              ++a;
+            }
           }
-          c += kDThreads;
-          while (c > k) {
-            c -= k + 1;
-            ++a;
-          }
-        }
-        bar_sync(kBarD, kDThreads);
-      }
-      for (int r = xt, j = xt / k, i = xt - j * k; r < k * k; r += kDThreads) {
-        double v = h.stages > 0 ? __longlong_as_double(U[j * kUStride + i]) : 0.0;
-        if (!h.first) v += C[r];
-        C[r] = v;
-        i += kDThreads;
-        while (i >= k) {
-          i -= k;
-          ++j;
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (at[e] >= 0) {
+              const long long v = __double_as_longlong(fixed_to_double(u[e], ex2));
+              U[at[e]] = v;
+              U[ta[e]] = v;
+            }
         }
       }
-      if (xt < k) {
+      if (kDThreads - 1 - xt < k) {
+        const int i = kDThreads - 1 - xt;
         double v = 0.0;
         if (h.stages > 0) {
-          long long hi = s_t[0][xt].x + s_t[1][xt].x, lo = s_t[0][xt].y + s_t[1][xt].y;
+          long long hi = s_t[0][i].x + s_t[1][i].x, lo = s_t[0][i].y + s_t[1][i].y;
           if constexpr (kThree) {
-            hi += s_t[2][xt].x;
-            lo += s_t[2][xt].y;
+            hi += s_t[2][i].x;
+            lo += s_t[2][i].y;
           }
           v = wide_to_double(hi, lo, ext);
         }
-        tv[xt] = h.first ? v : tv[xt] + v;
+        tv[i] = h.first ? v : tv[i] + v;
+      }
+      bar_sync(kBarD, kDThreads);
+      // out in rows
+      int j = xt / k, i = xt - j * k;
+      for (int r0 = xt; r0 < k * k; r0 += 4 * kDThreads) {
+        double v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = r0 + e * kDThreads;
+          v[e] = 0.0;
+          if (r < k * k) {
+            if (h.stages > 0) v[e] = __longlong_as_double(U[j * kUStride + i]);
+            if (!h.first) v[e] += C[r];
+          }
+          j += step_j;
+          i += step_i;
+          if (i >= k) {
+            i -= k;
+            ++j;
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (r0 + e * kDThreads < k * k) C[r0 + e * kDThreads] = v[e];
       }
     }
   }
