@@ -36,7 +36,7 @@
 // walk; a chain of FP64 additions loses 2^-53 of the partial sum at each.
 //
 // One persistent CTA per SM (the accumulators fill tensor memory), 28 warps in
-// four roles that work on neighbouring chunks of up to 1536 entries:
+// four roles that work on neighbouring chunks of up to 1344 or 1536 entries:
 //   weighing (7 warps)    drop the candidates whose vertical weight cannot be
 //     non-zero by an integer compare of |ln p - ln p_e|, queue the others in list
 //     order, and weigh the queue densely (the only FP64 work, some 35
@@ -79,11 +79,9 @@ constexpr int kX0 = kMmaWarp + 1, kD0 = kX0 + kXWarps;  // first warps (multiple
 constexpr int kPThreads = 32 * kPWarps, kXThreads = 32 * kXWarps, kDThreads = 32 * kDWarps;
 constexpr int kThreads = 32 * (kD0 + kDWarps);
 constexpr int kStage = 64;                            // entries per stage (4 K = 16 chunks)
-constexpr int kQueue = 1536;                          // entries of a chunk (one scale)
 constexpr int kPer = 4;                               // candidates per thread and refill
 constexpr int kRefill = kPer * kPThreads;
 constexpr int kGroup = 4;                             // stages per exact FP32 sum (256 entries)
-constexpr int kQueueBytes = kQueue * (16 + 8);
 // Operands and sums in shared memory.  A slice is kRows rows x K = 16 FP16.
 template <bool kThree>
 struct Layout {
@@ -96,7 +94,13 @@ struct Layout {
   static constexpr int kStageBytes = 4 * kChunk;
   static constexpr int kUStride = kThree ? 41 : 65;
   static constexpr int kURows = kThree ? 120 : 64;  // a row per accumulator row, or per member
-  static constexpr int kSmem = 2 * kStageBytes + 2 * kQueueBytes + kURows * kUStride * 8;
+  // entries of a chunk (one scale), and chunks in flight between the roles: one more
+  // where the operands leave room for it, so that solves of different lengths even
+  // out
+  static constexpr int kQueue = kThree ? 1344 : 1536, kDepth = kThree ? 3 : 2;
+  static constexpr int kQueueBytes = kQueue * (16 + 8);
+  static constexpr int kSmem =
+      2 * kStageBytes + kDepth * kQueueBytes + kURows * kUStride * 8;
   // memory position of slice a
   static __host__ __device__ constexpr int pos(int a) {
     return kThree ? (a >= 3 ? a - 1 : a + 5)
@@ -302,20 +306,21 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
   using namespace g64;
   using L = Layout<kThree>;
   constexpr int kSlice = L::kSlice, kTileD = L::kTileD, kChunkBytes = L::kChunk,
-                kStageBytes = L::kStageBytes, kUStride = L::kUStride;
+                kStageBytes = L::kStageBytes, kUStride = L::kUStride, kQueue = L::kQueue,
+                kQueueBytes = L::kQueueBytes, kDepth = L::kDepth;
   constexpr int kBufs = kThree ? 2 : 1;  // accumulator buffers in tensor memory
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // operand buffer multiplied, converted; queue full, empty; exact sum complete,
   // taken out (one phase per group of stages: the adding warps wait for no stage
   // in between, so a stage barrier's parity would not tell them which phase it is)
-  __shared__ uint64_t m_mma[2], m_conv[2], m_full[2], m_empty[2], m_sum[2], m_drain[2];
+  __shared__ uint64_t m_mma[2], m_conv[2], m_sum[2], m_drain[2], m_full[kDepth], m_empty[kDepth];
   __shared__ uint32_t tmem_base_sh;
   __shared__ int s_wcnt[2][kPWarps];
   __shared__ longlong2 s_t[kThree ? 3 : 2][64];
   __shared__ int s_kmax, s_dmax, s_nf;
   __shared__ volatile int s_abort;
   __shared__ int s_stop[2];  // s_abort as the weighing and the adding warps agree on it
-  __shared__ QueueHead s_head[2];
+  __shared__ QueueHead s_head[kDepth];
 
   const int k = g.ens;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -324,10 +329,12 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&m_mma[i], 1);
       tc::mbar_init(&m_conv[i], kXWarps);
-      tc::mbar_init(&m_full[i], kPThreads);
-      tc::mbar_init(&m_empty[i], kXWarps + 1 + kDWarps);
       tc::mbar_init(&m_sum[i], 1);
       tc::mbar_init(&m_drain[i], kDWarps);
+    }
+    for (int i = 0; i < kDepth; ++i) {
+      tc::mbar_init(&m_full[i], kPThreads);
+      tc::mbar_init(&m_empty[i], kXWarps + 1 + kDWarps);
     }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -373,10 +380,10 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     unsigned nq = 0;  // queues filled so far
     // 1: a queue is filled; 0: the solve is left to gram64_kernel; -1: stop
     auto fill = [&](int s, int64_t base, int p, double al, int& scan, bool& first) -> int {
-      const int qb = nq & 1;
+      const int qb = nq % kDepth;
       int4* const par = q_par(qb);
       long long* const qd = q_d(qb);
-      if (nq >= 2) wait(&m_empty[qb], ((nq - 2) >> 1) & 1);
+      if (nq >= kDepth) wait(&m_empty[qb], (nq / kDepth - 1) & 1);
       bar_sync(kBarP, kPThreads);  // every thread has read the last queue's maxima
       if (tid == 0) {
         s_kmax = 0;
@@ -570,8 +577,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       } while (r > 0 && scan < p);
       if (r < 0) break;
     }
-    const int qb = nq & 1;
-    if (nq >= 2) wait(&m_empty[qb], ((nq - 2) >> 1) & 1);
+    const int qb = nq % kDepth;
+    if (nq >= kDepth) wait(&m_empty[qb], (nq / kDepth - 1) & 1);
     if (tid == 0) s_head[qb] = QueueHead{-1, 0, 0, 0, 0, 0};
     mbar_arrive(&m_full[qb]);
     work = (int)__reduce_add_sync(0xffffffffu, (unsigned)work);
@@ -581,8 +588,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     const uint64_t desc0 = tc::make_desc(tc::smem_u32(smem_raw), 128, 256);
     unsigned n = 0, groups = 0;  // stages issued (buffer n & 1), exact sums begun
     for (unsigned nq = 0;; ++nq) {
-      const int qb = nq & 1;
-      wait(&m_full[qb], (nq >> 1) & 1);
+      const int qb = nq % kDepth;
+      wait(&m_full[qb], (nq / kDepth) & 1);
       if (stopped() || s_head[qb].s < 0) break;
       const int stages = s_head[qb].stages;
       __syncwarp();
@@ -652,8 +659,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     }
     unsigned n = 0;  // stages converted (buffer n & 1)
     for (unsigned nq = 0;; ++nq) {
-      const int qb = nq & 1;
-      wait(&m_full[qb], (nq >> 1) & 1);
+      const int qb = nq % kDepth;
+      wait(&m_full[qb], (nq / kDepth) & 1);
       if (stopped() || s_head[qb].s < 0) break;
       const int stages = s_head[qb].stages;
       const int4* const par = q_par(qb);
@@ -728,7 +735,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     const int j0 = (warp - kD0) / 4 * cw;
     const int ng = (cw + 3) / 4, h0 = (ng + 1) / 2;
     // the chunk's sums: per member, or (kThree) per accumulator row
-    long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + 2 * kQueueBytes);
+    long long* const U = reinterpret_cast<long long*>(smem_raw + 2 * kStageBytes + kDepth * kQueueBytes);
     // kThree: an off-diagonal pair counts twice, weight 2^(90 - 9 (a + b)) in units
     // of 2^(45 + kDrop); slice blk against slices 0 (times 2^32), 1, 2, 3 as
     // integers, and against 0, 2, 3, 4, 5 as the FP32 part.  33 shares its sum with 20,
@@ -748,8 +755,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     const int step_j = kDThreads / k, step_i = kDThreads - step_j * k;
     unsigned groups = 0;  // exact sums taken out
     for (unsigned nq = 0;; ++nq) {
-      const int qb = nq & 1;
-      wait(&m_full[qb], (nq >> 1) & 1);
+      const int qb = nq % kDepth;
+      wait(&m_full[qb], (nq / kDepth) & 1);
       const QueueHead h = s_head[qb];
       __syncwarp();
       if (lane == 0) mbar_arrive(&m_empty[qb]);
