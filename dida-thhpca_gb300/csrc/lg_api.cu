@@ -1476,7 +1476,8 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
       else if (mixed_tc)
         lg::launch_gram_tc_stream(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, rec, st);
       else
-        lg::launch_gram64(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, st);
+        lg::launch_gram64(geo, c->hx, c->lists, b, axb, !cube_trans_fp32(c) && lg::ft_supported(geo),
+                          L.C, L.t, c->d_status, st);
       CK(record_event(kv[1], st));
       CK(record_event(kv[2], st));
       if (cube_trans_fp32(c)) {
@@ -1599,7 +1600,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
     else if (mixed_tc)
       lg::launch_gram_tc(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, s_g, &rec);
     else
-      lg::launch_gram64(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, s_g);
+      lg::launch_gram64(geo, c->hx, c->lists, b, axb, c->use_ft, L.C, L.t, c->d_status, s_g);
     CK(cudaMemsetAsync(L.ovf_n, 0, sizeof(int), s_g));
     CK(record_event(kv[1], s_g));
     if (nl >= 3) {
@@ -2408,7 +2409,7 @@ void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   else if (precision == LG_PREC_MIXED && lg::gram_tc_supported(ens))
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
   else
-    lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
+    lg::launch_gram64(geo, hx, l, b, nullptr, lg::ft_supported(geo), C, t, fail, st);
   if (lg::ft_supported(geo)) {
     lg::launch_tridiag_in_place(ens, nbatch, C, st);
     lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, fail, st);

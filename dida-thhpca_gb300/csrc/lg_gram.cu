@@ -242,12 +242,13 @@ __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
 }
 
 void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
-                   const double* axb, double* C, double* t, int* err, cudaStream_t stream) {
+                   const double* axb, bool lower, double* C, double* t, int* err,
+                   cudaStream_t stream) {
   if (b.nsolves == 0) return;
   // up to 64 members: exact slices on the tensor cores, then the solves they
   // cannot hold (non-finite or extreme values) here
   const int marked = gram64_tc_supported(g.ens) && (b.mode == 1 || hx.yexp) ? 1 : 0;
-  if (marked) launch_gram64_tc(g, hx, l, b, axb, C, t, err, stream);
+  if (marked) launch_gram64_tc(g, hx, l, b, axb, lower, C, t, err, stream);
   const int grid = marked ? (b.nsolves + kGramThreads - 1) / kGramThreads : b.nsolves;
   const int kp = (g.ens + 3) & ~3;
   const int nb = kp / 4;

@@ -58,10 +58,10 @@
 // operand and one buffer at 40 members left the MMAs waiting for the sums to be
 // taken out, and each sum's conversion to integers (16 lanes a cycle and SM) is
 // kept to four or five per element.  Measured alone against gram64_kernel: 921 600
-// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 95 ms (126 with
-// two slices per operand); 82 944 of 40 members, 24 entries 5.6 -> 3.0 ms; 2592 of
+// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 93 ms (126 with
+// two slices per operand); 82 944 of 40 members, 24 entries 5.6 -> 2.7 ms; 2592 of
 // 16 members, 51 entries 0.18 -> 0.08 ms; 129 600 of 64 members, 954 entries 595 ->
-// 49 ms.  It wins at every size, so up to 64 members there is no other path.
+// 48 ms.  It wins at every size, so up to 64 members there is no other path.
 // A solve with a non-finite weight, row or innovation, or with magnitudes
 // outside 2^+-400, is marked by a bit pattern in its first Gram element that no
 // other solve can produce, and redone by gram64_kernel.
@@ -301,8 +301,8 @@ struct QueueHead {
 // members).
 template <int kR, bool kThree>
 __global__ void __launch_bounds__(g64::kThreads, 1)
-    gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, double* Cout, double* tout,
-                     int* err) {
+    gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, int lower, double* Cout,
+                     double* tout, int* err) {
   using namespace g64;
   using L = Layout<kThree>;
   constexpr int kSlice = L::kSlice, kTileD = L::kTileD, kChunkBytes = L::kChunk,
@@ -750,9 +750,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     const float f3 = blk == 0 ? 0.0f : blk == 1 ? 1.0f : 0x1p-9f;
     const float f4 = blk == 0 ? 1.0f : blk == 1 ? 0x1p-9f : 0x1p-18f;
     const float f5 = blk == 0 ? 0x1p-9f : blk == 1 ? 0x1p-18f : 0.0f;
-    // kDThreads elements further on in rows of k + 1, and of k
+    // kDThreads elements further on in rows of k + 1
     const int step_a = kDThreads / (k + 1), step_c = kDThreads - step_a * (k + 1);
-    const int step_j = kDThreads / k, step_i = kDThreads - step_j * k;
     unsigned groups = 0;  // exact sums taken out
     for (unsigned nq = 0;; ++nq) {
       const int qb = nq % kDepth;
@@ -905,44 +904,44 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       if (j0 == 0 && arow < (kThree ? 120 : 128)) s_t[blk][row] = make_longlong2(thi, tlo);
       bar_sync(kBarD, kDThreads);
       const int ex2 = 2 * h.S - 62 + kDrop, ext = h.S + h.Sd - 61;
-      // C = (U + U^T) / 2 in place (rows i and k - 1 - i of the triangle share one
-      // row of k + 1 elements), four elements' loads in flight; t by the threads
-      // with the fewest elements
-      if (h.stages > 0) {
-        const int total = (k + 1) / 2 * (k + 1);
-        int a = xt / (k + 1), c = xt - a * (k + 1);
-        for (int r0 = xt; r0 < total; r0 += 4 * kDThreads) {
-          int at[4], ta[4];
-          long long u[4];
+      // C = (U + U^T) / 2 out, the lower triangle in rows (rows i and k - 1 - i of it
+      // share one row of k + 1 elements), four elements' loads in flight; t by the
+      // threads with the fewest elements
+      const int total = (k + 1) / 2 * (k + 1);
+      int a = xt / (k + 1), c = xt - a * (k + 1);
+      for (int r0 = xt; r0 < total; r0 += 4 * kDThreads) {
+        int ci[4], cj[4];
+        long long u[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
-            // odd k: the middle row meets itself
-            const bool mine = r0 + e * kDThreads < total && !(2 * a == k - 1 && c > a);
-            at[e] = mine ? i * kUStride + j : -1;
-            ta[e] = j * kUStride + i;
-            u[e] = 0;
-            if (mine) {
-              u[e] = U[at[e]] + U[ta[e]];
-              if constexpr (kThree)
-                u[e] += U[at[e] + 40 * kUStride] + U[ta[e] + 40 * kUStride] +
-                        U[at[e] + 80 * kUStride] + U[ta[e] + 80 * kUStride];
-            }
-            a += step_a;
-            c += step_c;
-            if (c > k) {
-              c -= k + 1;
-              ++a;
-            }
+        for (int e = 0; e < 4; ++e) {
+          const int i = c <= a ? a : k - 1 - a, j = c <= a ? c : c - a - 1;
+          // odd k: the middle row meets itself
+          const bool mine = r0 + e * kDThreads < total && !(2 * a == k - 1 && c > a);
+          ci[e] = mine ? i : -1;
+          cj[e] = j;
+          u[e] = 0;
+          if (mine && h.stages > 0) {
+            const int at = i * kUStride + j, ta = j * kUStride + i;
+            u[e] = U[at] + U[ta];
+            if constexpr (kThree)
+              u[e] += U[at + 40 * kUStride] + U[ta + 40 * kUStride] + U[at + 80 * kUStride] +
+                      U[ta + 80 * kUStride];
           }
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (at[e] >= 0) {
-              const long long v = __double_as_longlong(fixed_to_double(u[e], ex2));
-              U[at[e]] = v;
-              U[ta[e]] = v;
-            }
+          a += step_a;
+          c += step_c;
+          if (c > k) {
+            c -= k + 1;
+            ++a;
+          }
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (ci[e] >= 0) {
+            double v = fixed_to_double(u[e], ex2);
+            if (!h.first) v += C[ci[e] * k + cj[e]];
+            C[ci[e] * k + cj[e]] = v;
+            if (!lower) C[cj[e] * k + ci[e]] = v;
+          }
       }
       if (kDThreads - 1 - xt < k) {
         const int i = kDThreads - 1 - xt;
@@ -957,30 +956,6 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         }
         tv[i] = h.first ? v : tv[i] + v;
       }
-      bar_sync(kBarD, kDThreads);
-      // out in rows
-      int j = xt / k, i = xt - j * k;
-      for (int r0 = xt; r0 < k * k; r0 += 4 * kDThreads) {
-        double v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int r = r0 + e * kDThreads;
-          v[e] = 0.0;
-          if (r < k * k) {
-            if (h.stages > 0) v[e] = __longlong_as_double(U[j * kUStride + i]);
-            if (!h.first) v[e] += C[r];
-          }
-          j += step_j;
-          i += step_i;
-          if (i >= k) {
-            i -= k;
-            ++j;
-          }
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (r0 + e * kDThreads < k * k) C[r0 + e * kDThreads] = v[e];
-      }
     }
   }
   tc::fence_before();
@@ -994,14 +969,15 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
 bool gram64_tc_supported(int ens) { return ens <= 64; }
 
 void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
-                      const double* axb, double* C, double* t, int* err, cudaStream_t stream) {
+                      const double* axb, bool lower, double* C, double* t, int* err,
+                      cudaStream_t stream) {
   if (b.nsolves == 0) return;
   const int grid = b.nsolves < 152 ? b.nsolves : 152;
   if (b.mode == 0 && g.vert_dist > 0.0)
     level_lnp_kernel<<<(b.nsolves + 127) / 128, 128, 0, stream>>>(g, b, axb, t);
   auto run = [&](auto kernel, int smem) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    kernel<<<grid, g64::kThreads, smem, stream>>>(g, hx, l, b, C, t, err);
+    kernel<<<grid, g64::kThreads, smem, stream>>>(g, hx, l, b, lower ? 1 : 0, C, t, err);
   };
   if (g.ens <= 40)
     run(gram64_tc_kernel<2, true>, g64::Layout<true>::kSmem);

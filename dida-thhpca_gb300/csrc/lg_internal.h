@@ -212,10 +212,12 @@ size_t scan_tmp_bytes(int n);
 // FP64 Gram matrices and projections: exact slices on the tensor cores up to 64
 // members (lg_gram64_tc.cu; mode 0 needs hx.yexp), the FP64 pipe otherwise
 void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
-                   const double* axb, double* C, double* t, int* err, cudaStream_t stream);
+                   const double* axb, bool lower, double* C, double* t, int* err,
+                   cudaStream_t stream);
 bool gram64_tc_supported(int ens);
 void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
-                      const double* axb, double* C, double* t, int* err, cudaStream_t stream);
+                      const double* axb, bool lower, double* C, double* t, int* err,
+                      cudaStream_t stream);
 void launch_row_exponents(int ens, int64_t rows, const double* yb, int* yexp, cudaStream_t stream);
 // first Gram element of a solve that gram64_tc_kernel leaves to gram64_kernel:
 // a NaN with a payload no arithmetic here produces

@@ -101,7 +101,7 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
   if (precision == LG_PREC_MIXED && lg::gram_tc_supported(ens))
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
   else
-    lg::launch_gram64(geo, hx, l, b, nullptr, C, t, fail, st);
+    lg::launch_gram64(geo, hx, l, b, nullptr, lg::ft_supported(geo), C, t, fail, st);
   if (lg::ft_supported(geo)) {
     lg::launch_tridiag_in_place(ens, nbatch, C, st);
     lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, fail, st);

@@ -89,9 +89,25 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
   // ---- scale: 2^E just above the Frobenius norm (FP32 sum relative to the
   // largest exponent, rounded up)
   unsigned emax = 0;
-  for (int t = lane; t < n * n; t += 32)
-    emax = max(emax, ((unsigned)__double2hiint(M[t]) >> 20) & 0x7ffu);
+  {
+    int j = 0, c = lane;
+    while (c > j) {
+      c -= j + 1;
+      ++j;
+    }
+    for (int t = lane; t < np; t += 32) {
+      const double a = M[(size_t)j * n + c];
+      A[t] = make_int2(__double2loint(a), __double2hiint(a));
+      emax = max(emax, ((unsigned)__double2hiint(a) >> 20) & 0x7ffu);
+      c += 32;
+      while (c > j) {
+        c -= j + 1;
+        ++j;
+      }
+    }
+  }
   emax = __reduce_max_sync(0xffffffffu, emax);
+  __syncwarp();
   double* const D = M;
   double* const E = M + n;
   double* const H = M + 2 * n;
@@ -106,43 +122,38 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     return;
   }
   float fro = 0.0f;
-  for (int t = lane; t < n * n; t += 32) {
-    const int hi = __double2hiint(M[t]) & 0x7fffffff;
+  auto rough = [&](int t) {  // mantissa to 20 bits, rounded up, at 2^-d
+    const int hi = A[t].y & 0x7fffffff;
     const int d = (int)emax - (hi >> 20);
-    // mantissa to 20 bits, rounded up, at 2^-d
-    const float f = d > 60 ? 0.0f
-                           : __int_as_float(((127 - d) << 23) | ((hi & 0xfffff) << 3)) * 1.00001f;
+    return d > 60 ? 0.0f : __int_as_float(((127 - d) << 23) | ((hi & 0xfffff) << 3)) * 1.00001f;
+  };
+  for (int t = lane; t < np; t += 32) {
+    const float f = rough(t);
     fro = fmaf(f, f, fro);
+  }
+  fro *= 2.0f;  // both triangles; the diagonal once
+  for (int j = lane; j < n; j += 32) {
+    const float f = rough(idx(j) + j);
+    fro = fmaf(-f, f, fro);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
+  __syncwarp();
   // |C|_F < 2^(emax - 1023) sqrt(fro) 1.001; E = the exponent above
   const int ef = (int)((__float_as_uint(sqrtf(fro) * 1.001f) >> 23) & 0xffu) - 127 + 1;
   const int Eb = (int)emax + ef;  // E + 1023
-  {
-    int j = 0, c = lane;
-    while (c > j) {
-      c -= j + 1;
-      ++j;
+  for (int t = lane; t < np; t += 32) {
+    const int2 a = A[t];
+    const unsigned long long u = (unsigned long long)(unsigned)a.y << 32 | (unsigned)a.x;
+    const int e = (int)(u >> 52) & 0x7ff;
+    long long x = 0;
+    if (e) {
+      const int sh = min(Eb - e, 62);  // >= 1
+      x = (long long)((((u & 0xfffffffffffffull) | 0x10000000000000ull) << 7) +
+                      (1ull << (sh - 1))) >> sh;
+      if (u >> 63) x = -x;
     }
-    for (int t = lane; t < np; t += 32) {
-      const double a = M[(size_t)j * n + c];
-      const unsigned long long u = (unsigned long long)__double_as_longlong(a);
-      const int e = (int)(u >> 52) & 0x7ff;
-      long long x = 0;
-      if (e) {
-        const int sh = min(Eb - e, 62);  // >= 1
-        x = (long long)((((u & 0xfffffffffffffull) | 0x10000000000000ull) << 7) +
-                        (1ull << (sh - 1))) >> sh;
-        if (u >> 63) x = -x;
-      }
-      A[t] = fixed_split(x);
-      c += 32;
-      while (c > j) {
-        c -= j + 1;
-        ++j;
-      }
-    }
+    A[t] = fixed_split(x);
   }
   __syncwarp();
   const int ex = Eb - 1023 - 59;  // a = X 2^ex
