@@ -1516,7 +1516,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
     CK(cudaStreamWaitEvent(st, c->ev_join, 0));
     const lg::CubeDev cd{g.cube_n, g.cube_nz, g.cube_n - g.overlap, c->cube_ngroups,
                          (g.vert_dist > 0.0 && g.overlap == 0) ? 1 : 0, c->d_cube_off};
-    lg::launch_cube_apply(geo, cd, c->d_trans, xb, axb, xa, axa, st);
+    lg::launch_cube_apply(geo, cd, ns, c->d_trans, xb, axb, xa, axa, st);
     launches += 1;
     if (io) {
       CK(cudaEventRecord(c->ev_phase[3][0], st));

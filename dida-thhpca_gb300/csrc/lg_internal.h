@@ -270,7 +270,7 @@ struct CubeDev {
   int grouped;          // vertical path without overlap: level groups of cube_nz levels
   const int* cube_off;  // nblocks + 1: first cube of each block
 };
-void launch_cube_apply(const Geometry& g, const CubeDev& cd, const double* trans,
+void launch_cube_apply(const Geometry& g, const CubeDev& cd, int nsolves, const double* trans,
                        const double* xb, const double* axb, double* xa, double* axa,
                        cudaStream_t stream);
 
