@@ -42,6 +42,7 @@
 // reduction: 32 768 cubes of 40 members 133 -> 9.6 ms.  Faster at every size
 // from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
+#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
@@ -411,21 +412,26 @@ __device__ inline void factor_twisted(int n, const double* D, const double* E, d
 
 }  // namespace ft
 
-// f(T) y per lane, one warp per block, slots = 32 / per solves per warp: t gives
-// sqrt(k-1) T^(-1/2) y, the rows (f(T) - sqrt(rho)) y and overline_w . x.
+// f(T) y per lane, one warp per block: t gives sqrt(k-1) T^(-1/2) y, the rows
+// (f(T) - sqrt(rho)) y and overline_w . x.  A warp takes `slots` solves with `rows`
+// rows and t each; a solve of more than 31 rows is spread over `parts` warps, each
+// with a t of its own.
 // Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
 // F (the forward solve), A (the sum over nodes), and for 32 (slot, node) pairs
 // the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
 __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
-                                                const double* tri, int* eig_fail) {
+                                                int rows, int parts, const double* tri,
+                                                int* eig_fail) {
   const int n = g.ens;
   const int lane = threadIdx.x;
-  const int per = z.per;
-  const int s_first = blockIdx.x * slots;
+  const int lanes = rows + 1;  // of a solve
+  const int s_first = parts > 1 ? (int)blockIdx.x / parts : (int)blockIdx.x * slots;
   const int nsl = min(slots, b.nsolves - s_first);
-  const bool mine = lane / per < nsl;
-  const int sl = mine ? lane / per : 0, s = s_first + sl;
-  const int v = mine ? lane - sl * per : 0;
+  const int part = parts > 1 ? (int)blockIdx.x - s_first * parts : 0;
+  const int sl = lane / lanes < nsl ? lane / lanes : 0, s = s_first + sl;
+  const int vl = lane - sl * lanes;  // 0: t
+  const bool mine = lane / lanes < nsl && (vl == 0 || part * rows + vl < z.per);
+  const int v = mine && vl > 0 ? part * rows + vl : 0;
   extern __shared__ double sm[];
   const int cap = n * 32;
   double *const Y = sm + lane, *const F = Y + cap, *const A = F + cap;
@@ -438,7 +444,7 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
   double* const io = ft::vec_at(z, n, s, v, vs);
   if (mine)
     for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
-  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, 1, 0, eig_fail);
+  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, 1, part == 0 ? 0 : LLONG_MAX, eig_fail);
   const int nb = 32 / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
   int nmax = 0;
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
@@ -516,7 +522,7 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
   }
   if (!mine || v == 0) return;
   const double srho = sqrt(g.inflation);
-  const double* zt = sm + 2 * cap + sl * per;  // vector 0's A
+  const double* zt = sm + 2 * cap + sl * lanes;  // vector 0's A
   double dotw = 0.0;
   for (int i = 0; i < n; ++i) {
     const double a = A[32 * i];
@@ -649,20 +655,24 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kernel<<<blocks(p), 32, smem, stream>>>(g, b, z, sl, tri, xb, axb, xa, axa);
   };
-  auto solve = [&](auto kernel, int arrays, int sl, unsigned grid) {
+  auto solve_smem = [&](auto kernel, int arrays, int sl) {
     const size_t smem = sizeof(double) * ((size_t)arrays * 32 * n + 2 * (size_t)sl * n);
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kernel<<<grid, 32, smem, stream>>>(g, b, z, sl, tri, eig_fail);
+    return smem;
   };
   if (core) {
-    solve(ft_matrix_kernel, 3, spans(n), blocks(n));
+    const int sl = spans(n);
+    ft_matrix_kernel<<<blocks(n), 32, solve_smem(ft_matrix_kernel, 3, sl), stream>>>(g, b, z, sl, tri,
+                                                                                     eig_fail);
     reflect(reflect_kernel<true, true>, n);
     reflect(reflect_kernel<false, true>, n);
     add_wbar_kernel<<<b.nsolves, 128, 0, stream>>>(n, b, t, vec, wbar);
   } else {
-    const int sl = 32 / per;
+    const int parts = (per + 29) / 31, rows = (per - 1 + parts - 1) / parts, sl = 32 / (rows + 1);
+    const unsigned grid = parts > 1 ? (unsigned)b.nsolves * parts : (unsigned)((b.nsolves + sl - 1) / sl);
     reflect(reflect_kernel<true, false>, per);
-    solve(ft_kernel, 5, sl, (unsigned)((b.nsolves + sl - 1) / sl));
+    ft_kernel<<<grid, 32, solve_smem(ft_kernel, 5, sl), stream>>>(g, b, z, sl, rows, parts, tri,
+                                                                  eig_fail);
     reflect(reflect_kernel<false, false>, per - 1);
   }
 }

@@ -100,3 +100,27 @@ def test_structured_gram_matrices(k):
     assert st == 0
     for c, t, w in zip(cases, tr, wb):
         _check(c, 1.1, t, w)
+
+
+@pytest.mark.parametrize("nz", [10, 11, 21, 32])
+def test_every_row_in_one_solve(nz, monkeypatch):
+    """Without vertical localisation a solve transforms every row of its column:
+    31 (a warp with t), 34, 64 and 97 rows (more than a warp), against the QL
+    route with the tolerance above."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset("tiny3d").replace(nz=nz, vert_dist=-1.0)
+    w = synth.make_workload(cfg)
+    out = []
+    for limit in (None, "59"):
+        if limit:
+            monkeypatch.setenv("LETKF_GB300_QL_ITERS", limit)
+        ctx = lg.Letkf(cfg)
+        ctx.set_obs(w.obs)
+        xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+        ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+        ctx.letkf_final()
+        out.append(xa + axa[..., None])
+    i = slice(cfg.halo, -cfg.halo)
+    inc = np.abs(out[1] - (w.xb + w.axb[..., None]))[i, i].max()
+    assert np.abs(out[0] - out[1])[i, i].max() <= 1e-10 * inc
