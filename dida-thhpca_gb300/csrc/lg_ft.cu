@@ -20,7 +20,7 @@
 // Why: the FP64 pipe retires a warp instruction per 17 cycles per SM.  Per
 // 64-member solve the QL iteration takes about 4000 rotations at 24 FP64
 // instructions (one lane each) and their replay 8 per rotation and vector; the
-// shifted solves take 4 per node, element and vector, plus 7 per node and
+// shifted solves take 3 per node, element and vector, plus 8 per node and
 // element for the factors, which the lanes of a solve compute for different
 // nodes.  overline_w . x = (T^(-1/2) y) . (T^(-1/2) Q^T t) needs no solve of its
 // own.  The reflections (2 k^2 multiply-adds per vector) leave the FP64 pipe
@@ -30,23 +30,26 @@
 //     rows' update -- three kernels, so that the integer ones are not held to the
 //     two to four warps per SM that the solves' five arrays leave;
 //   explicit trans: ft_matrix_kernel forms F = f(T) itself, whose upper triangle
-//     takes 2 FP64 instructions per node and element (no right-hand side: with
+//     takes 1 FP64 instruction per node and element (no right-hand side: with
 //     T + s = L D L^T, G = (T + s)^-1 has G_jj = 1/D_j + L_{j+1}^2 G_{j+1,j+1} and
 //     G_ij = -L_{i+1} G_{i+1,j} above it), then W = Q F Q^T by two reflect_kernel
 //     passes and overline_w = W (W t) / (k - 1) in add_wbar_kernel.  A solve per
-//     unit vector instead made this step 12.9 ms where it is 7.7 (32 768 cubes of
+//     unit vector instead made this step 12.9 ms where it is 7.2 (32 768 cubes of
 //     40 members).
-// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 62 ms,
-// 129 600 of 64 members 93 -> 29 ms (66 and 31 with the elimination from one
-// end); explicit trans against the accumulating solver (lg_eig.cu), with the
-// reduction: 32 768 cubes of 40 members 133 -> 9.6 ms.  Faster at every size
-// from 7 to 64 members; above, five arrays leave an SM one warp.
+// The sum over the nodes is kept in 64-bit integers: off the FP64 pipe, and the same
+// in any order, so that a vector may be spread over several lanes (launch_ft) and the
+// result does not depend on how many solves a launch has.
+// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 57 ms,
+// 129 600 of 64 members 93 -> 24 ms; explicit trans against the accumulating solver
+// (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 9.1 ms.  Faster at
+// every size from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
 #include <limits.h>
 #include <math.h>
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "lg_device.cuh"
 #include "lg_fixed.cuh"
@@ -165,23 +168,76 @@ __device__ inline size_t out_index(const SolveBatch& b, int s) {
   return b.s_col ? (size_t)b.first_solve + s : (size_t)s;
 }
 
-// This lane's vector V (element i at 32 i) from FP64 to integers of 2^(ex):
-// |V| < 2^(ex + 58), held as in lg_tri.cu; false if a value is not finite.
-__device__ inline bool to_fixed(double* V, int n, int& ex) {
-  unsigned emax = 0;
-  for (int i = 0; i < n; ++i)
-    emax = max(emax, ((unsigned)__double2hiint(V[32 * i]) >> 20) & 0x7ffu);
-  float fro = 0.0f;
-  for (int i = 0; i < n; ++i) {
-    const int hi = __double2hiint(V[32 * i]) & 0x7fffffff;
-    const int d = (int)emax - (hi >> 20);
-    const float f =
-        d > 60 ? 0.0f : __int_as_float(((127 - d) << 23) | ((hi & 0xfffff) << 3)) * 1.00001f;
-    fro = fmaf(f, f, fro);
+// A vector of n elements over kL neighbouring lanes: lane part p holds elements
+// p, p + kL, .. at 0, 32, 64, ..; own(n) of them.  All lanes of the warp call it.
+template <int kL>
+__device__ inline int own(int n, int part) {
+  return kL == 1 ? n : (n - part + kL - 1) / kL;
+}
+template <int kL, typename T>
+__device__ inline T sum_parts(T x) {
+#pragma unroll
+  for (int o = 1; o < kL; o *= 2) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// Sum of f(i) over a vector's elements (i: this lane's, of m) in an order that does
+// not depend on kL: eight sums of the elements equal modulo 8, joined as a tree.
+template <int kL, typename F>
+__device__ inline double sum_elements(int m, F f) {
+  constexpr int kC = 8 / kL;
+  double c[kC];
+#pragma unroll
+  for (int q = 0; q < kC; ++q) c[q] = 0.0;
+  for (int i = 0; i < m; i += kC) {
+#pragma unroll
+    for (int q = 0; q < kC; ++q)
+      if (i + q < m) c[q] += f(i + q);
   }
-  // norm < 2^(emax - 1023) sqrt(fro) 1.001; the power of two above it
-  const int Eb = (int)emax + (int)((__float_as_uint(sqrtf(fro) * 1.001f) >> 23) & 0xffu) - 126;
-  for (int i = 0; i < n; ++i) {
+#pragma unroll
+  for (int q = 0; q < kC; ++q) c[q] = sum_parts<kL>(c[q]);
+#pragma unroll
+  for (int o = 1; o < kC; o *= 2)
+#pragma unroll
+    for (int q = 0; q < kC; q += 2 * o) c[q] += c[q + o];
+  return c[0];
+}
+
+// a += x in units of 2^(top - 62), for |x| < 2^top, Eb = top + 1022: sums of
+// the nodes' terms, exact in any order and off the FP64 pipe
+__device__ inline void add_fixed(long long& a, double x, int Eb) {
+  const int hi = __double2hiint(x);
+  const unsigned long long m =
+      ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(x)) << 9;
+  const long long v = (long long)(m >> min(max(Eb - ((hi >> 20) & 0x7ff), 0), 63));
+  a += hi < 0 ? -v : v;
+}
+// power of two above f(T)'s norm, sqrt(rho) at most
+__device__ inline int f_top(double inflation) {
+  return ((__double2hiint(1.01 * sqrt(inflation)) >> 20) & 0x7ff) - 1022;
+}
+
+// This vector V from FP64 to integers of 2^(ex): |V| < 2^(ex + 58), held as in
+// lg_tri.cu; false if a value is not finite.  m: this lane's elements.
+template <int kL>
+__device__ inline bool to_fixed(double* V, int m, int& ex) {
+  unsigned emax = 0;
+  for (int i = 0; i < m; ++i)
+    emax = max(emax, ((unsigned)__double2hiint(V[32 * i]) >> 20) & 0x7ffu);
+#pragma unroll
+  for (int o = 1; o < kL; o *= 2) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+  // norm < 2^(emax - 1043) sqrt(squares), in integers (any order); the power of two
+  // above it
+  unsigned long long squares = 0;
+  for (int i = 0; i < m; ++i) {
+    const int hi = __double2hiint(V[32 * i]) & 0x7fffffff;
+    const unsigned f =
+        ((((unsigned)hi & 0xfffffu) | 0x100000u) + 1 >> min((int)emax - (hi >> 20), 31)) + 1;
+    squares += (unsigned long long)f * f;
+  }
+  squares = sum_parts<kL>(squares);
+  const int Eb = (int)emax - 20 + (65 - __clzll((long long)squares)) / 2;
+  for (int i = 0; i < m; ++i) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(V[32 * i]);
     const int e = (int)(u >> 52) & 0x7ff;
     long long x = 0;
@@ -198,7 +254,7 @@ __device__ inline bool to_fixed(double* V, int n, int& ex) {
 
 }  // namespace ft
 
-// One vector per lane, one warp per block, lanes numbered through the solves'
+// One vector over kL lanes, one warp per block, lanes numbered through the solves'
 // vectors.  Analysis: y <- Q^T x (kFirst; P_{n-1} first) or Q z (P_1 first) with
 // the rows' update.  Core, W = Q F Q^T: the first pass takes column j of the
 // symmetric F from row j of the matrix and leaves Q F's column j there (the
@@ -206,7 +262,7 @@ __device__ inline bool to_fixed(double* V, int n, int& ex) {
 // leaves W's column j there, so that no lane reads what another one writes.
 // Reflector rows of the (up to `slots`) solves that a warp spans come into shared
 // memory a step ahead of their use.
-template <bool kFirst, bool kCore>
+template <bool kFirst, bool kCore, int kL>
 __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, ft::Vecs z,
                                                      int slots, const double* tri, const double* xb,
                                                      const double* axb, double* xa, double* axa) {
@@ -215,16 +271,19 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   // the rows' update needs no t: its vectors are v = 1 .. per - 1
   const int v0 = !kFirst && !kCore ? 1 : 0;
   const int per = z.per - v0;
-  const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * per;
+  constexpr int kV = 32 / kL;  // vectors of a warp
+  const long long id0 = (long long)blockIdx.x * kV, total = (long long)b.nsolves * per;
   const int s_first = (int)(id0 / per);
-  const int nsl = (int)((min(id0 + 32, total) - 1) / per) - s_first + 1;
-  const bool mine = id0 + lane < total;
-  const int s = mine ? (int)((id0 + lane) / per) : s_first;
-  const int v = v0 + (mine ? (int)((id0 + lane) - (long long)s * per) : 0);
+  const int nsl = (int)((min(id0 + kV, total) - 1) / per) - s_first + 1;
+  const long long id = id0 + lane / kL;
+  const int part = kL == 1 ? 0 : lane % kL, m = ft::own<kL>(n, part);
+  const bool mine = id < total;
+  const int s = mine ? (int)(id / per) : s_first;
+  const int v = v0 + (mine ? (int)(id - (long long)s * per) : 0);
   extern __shared__ double sm[];
-  double* const Y = sm + lane;                      // element i at 32 i
+  double* const Y = sm + lane;                      // element part + kL i at 32 i
   int2* const Yi = reinterpret_cast<int2*>(Y);
-  double* const ub = sm + 32 * n;                   // two buffers of slots x n
+  double* const ub = sm + 32 * ((n + kL - 1) / kL);  // two buffers of slots x n
   const size_t tri_stride = (size_t)n * n;
   auto fetch = [&](int i, int buf) {
     if (i >= 1 && i < n)
@@ -265,42 +324,58 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   }
   const bool row = mine && r_state >= 0;  // analysis: this solve updates the row
   const double* const xr = xb + (row ? (size_t)n * (r_state + (size_t)g.n * ci) : 0);
-  for (int i = 0; i < n; ++i) {
+  for (int i = 0; i < m; ++i) {
+    const int e = part + kL * i;
     double x = 0.0;
     if (kCore)
-      x = out[(size_t)i * vs];
+      x = out[(size_t)e * vs];
     else if (kFirst)
-      x = v == 0 ? out[i] : (row ? xr[i] : 0.0);
+      x = v == 0 ? out[e] : (row ? xr[e] : 0.0);
     else if (row)
-      x = out[(size_t)i * vs];
+      x = out[(size_t)e * vs];
     Y[32 * i] = x;
   }
   int ex;
-  const bool finite = ft::to_fixed(Y, n, ex);
+  const bool finite = ft::to_fixed<kL>(Y, m, ex);
   // ---- reflections: y -= w (w . y)
   for (int c = 0, i = i0; c < n - 1; ++c, i += step) {
     fetch(i + step, (c + 1) & 1);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
     const double* ud = ub + (size_t)((c & 1) * slots + (s - s_first)) * n;
-    const int2* u = reinterpret_cast<const int2*>(ud);
-    if (__double2hiint(ud[n - 1]) != 0) {
-      long long hs = 0, ms = 1 << 27;
+    const int2* u = reinterpret_cast<const int2*>(ud) + part;
+    const bool reflect = __double2hiint(ud[n - 1]) != 0;
+    const int mi = ft::own<kL>(i, part);
+    long long hs = 0, ms = part == 0 ? 1 << 27 : 0;  // rounds the sum's cut
+    auto dot = [&]() {
 #pragma unroll 4
-      for (int j = 0; j < i; ++j) {
-        const int2 w = u[j], y = Yi[32 * j];
+      for (int j = 0; j < mi; ++j) {
+        const int2 w = u[kL * j], y = Yi[32 * j];
         hs += (long long)y.y * w.y;
         ms += (long long)y.y * w.x;
         ms += (long long)y.x * w.y;
       }
+    };
+    auto update = [&]() {
       const int2 D = fixed_split(4 * hs + (ms >> 28));
       const int D4 = -4 * D.y;  // |D| < 2^58.5
 #pragma unroll 4
-      for (int j = 0; j < i; ++j) {
-        const int2 w = u[j], y = Yi[32 * j];
-        const long long m = (long long)D.y * w.x + ((long long)D.x * w.y + (1 << 27));
-        Yi[32 * j] = fixed_split(fixed_join(y) + (long long)D4 * w.y - (int)(m >> 28));
+      for (int j = 0; j < mi; ++j) {
+        const int2 w = u[kL * j], y = Yi[32 * j];
+        const long long c2 = (long long)D.y * w.x + ((long long)D.x * w.y + (1 << 27));
+        Yi[32 * j] = fixed_split(fixed_join(y) + (long long)D4 * w.y - (int)(c2 >> 28));
       }
+    };
+    if (kL == 1) {
+      if (reflect) {
+        dot();
+        update();
+      }
+    } else {
+      if (reflect) dot();
+      hs = ft::sum_parts<kL>(hs);
+      ms = ft::sum_parts<kL>(ms);
+      if (reflect) update();
     }
     __syncwarp();
   }
@@ -309,25 +384,26 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   if (kFirst || kCore) {
     if (mine)
-      for (int i = 0; i < n; ++i)
-        out[(size_t)i * vs] = finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
-  } else if (row) {
-    // xa = axb + sqrt(rho) x + (W - sqrt(rho) I) x + overline_w . x, recentred
-    const double srho = sqrt(g.inflation);
-    const double ab = axb[r_state + (size_t)g.n * ci];
-    const double dotw = out[(size_t)n * vs];
-    double mean = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const double d = finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
-      const double x = ab + (srho * xr[i] + (d + dotw));
-      Y[32 * i] = x;
-      mean += x;
-    }
-    mean /= (double)n;
-    double* xo = xa + (size_t)n * (r_state + (size_t)g.n * ci);
-    for (int i = 0; i < n; ++i) xo[i] = Y[32 * i] - mean;
-    axa[r_state + (size_t)g.n * ci] = mean;
+      for (int i = 0; i < m; ++i)
+        out[(size_t)(part + kL * i) * vs] =
+            finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
+    return;
   }
+  // xa = axb + sqrt(rho) x + (W - sqrt(rho) I) x + overline_w . x, recentred
+  const double srho = sqrt(g.inflation);
+  const double ab = row ? axb[r_state + (size_t)g.n * ci] : 0.0;
+  const double dotw = row ? out[(size_t)n * vs] : 0.0;
+  const double mean = ft::sum_elements<kL>(m, [&](int i) {
+    if (!row) return 0.0;
+    const double d = finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
+    const double x = ab + (srho * xr[part + kL * i] + (d + dotw));
+    Y[32 * i] = x;
+    return x;
+  }) / (double)n;
+  if (!row) return;
+  double* xo = xa + (size_t)n * (r_state + (size_t)g.n * ci);
+  for (int i = 0; i < m; ++i) xo[part + kL * i] = Y[32 * i] - mean;
+  if (part == 0) axa[r_state + (size_t)g.n * ci] = mean;
 }
 
 namespace ft {
@@ -337,7 +413,8 @@ namespace ft {
 // rounded up).  A non-finite T counts in *eig_fail, as a QL iteration that never
 // converges, if its first vector id is not below id0.
 __device__ inline void load_t(int n, const double* tri, int s_first, int nsl, double shift, double* Dg,
-                              double* Eg, int* s_row, int per, long long id0, int* eig_fail) {
+                              double* Eg, int* s_row, bool* s_nan, int per, long long id0,
+                              int* eig_fail) {
   const int lane = threadIdx.x;
   for (int q = 0; q < nsl; ++q) {
     const double* T = tri + (size_t)(s_first + q) * n * n;
@@ -359,6 +436,7 @@ __device__ inline void load_t(int n, const double* tri, int s_first, int nsl, do
       // smallest power of two above the bound
       const int ex = (int)((__float_as_uint(mx * (1.0001f / (float)shift)) >> 23) & 0xffu) - 127 + 1;
       s_row[q] = nf ? 0 : min(max(ex, 1), kMaxLog);
+      s_nan[q] = nf;
       if (nf && (long long)(s_first + q) * per >= id0) atomicAdd(eig_fail, 1);
     }
   }
@@ -382,32 +460,33 @@ __device__ inline void factor(int n, const double* D, const double* E, double si
 
 // The same elimination from both ends, meeting at element m = n / 2: as many
 // operations in two independent chains of half the length.
-__device__ inline void factor_twisted(int n, const double* D, const double* E, double sigma, double* R,
-                                      double* L) {
+// R is scaled by the node's weight w, which makes the solution w (T + sigma)^-1 y.
+__device__ inline void factor_twisted(int n, const double* D, const double* E, double sigma, double w,
+                                      double* R, double* L) {
   const int m = n / 2, nd = n - 1 - m;  // nd elements below m, m >= nd above
   double r = rcp(D[0] + sigma), q = rcp(D[n - 1] + sigma);
-  R[0] = r;
-  R[32 * (n - 1)] = q;
+  R[0] = w * r;
+  R[32 * (n - 1)] = w * q;
   for (int c = 1; c < nd; ++c) {
     const int b = n - 1 - c;
     const double e = E[c], l = e * r, h = E[b + 1], k = h * q;
     r = rcp(fma(-l, e, D[c] + sigma));
     q = rcp(fma(-k, h, D[b] + sigma));
     L[32 * c] = l;
-    R[32 * c] = r;
+    R[32 * c] = w * r;
     L[32 * (b + 1)] = k;
-    R[32 * b] = q;
+    R[32 * b] = w * q;
   }
   if (m > nd) {
     const double e = E[m - 1], l = e * r;
     r = rcp(fma(-l, e, D[m - 1] + sigma));
     L[32 * (m - 1)] = l;
-    R[32 * (m - 1)] = r;
+    R[32 * (m - 1)] = w * r;
   }
   const double e = E[m], l = e * r, h = E[m + 1], k = h * q;
   L[32 * m] = l;
   L[32 * (m + 1)] = k;
-  R[32 * m] = rcp(fma(-k, h, fma(-l, e, D[m] + sigma)));
+  R[32 * m] = w * rcp(fma(-k, h, fma(-l, e, D[m] + sigma)));
 }
 
 }  // namespace ft
@@ -419,40 +498,51 @@ __device__ inline void factor_twisted(int n, const double* D, const double* E, d
 // Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
 // F (the forward solve), A (the sum over nodes), and for 32 (slot, node) pairs
 // the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
+template <int kL>
 __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
                                                 int rows, int parts, const double* tri,
                                                 int* eig_fail) {
   const int n = g.ens;
   const int lane = threadIdx.x;
-  const int lanes = rows + 1;  // of a solve
+  const int lanes = (rows + 1) * kL;  // of a solve
   const int s_first = parts > 1 ? (int)blockIdx.x / parts : (int)blockIdx.x * slots;
   const int nsl = min(slots, b.nsolves - s_first);
-  const int part = parts > 1 ? (int)blockIdx.x - s_first * parts : 0;
+  const int first_row = parts > 1 ? ((int)blockIdx.x - s_first * parts) * rows : 0;
   const int sl = lane / lanes < nsl ? lane / lanes : 0, s = s_first + sl;
-  const int vl = lane - sl * lanes;  // 0: t
-  const bool mine = lane / lanes < nsl && (vl == 0 || part * rows + vl < z.per);
-  const int v = mine && vl > 0 ? part * rows + vl : 0;
+  const int vl = (lane - sl * lanes) / kL;  // 0: t
+  const int part = lane % kL;               // this lane's nodes: part, part + kL, ..
+  const bool mine = lane / lanes < nsl && (vl == 0 || first_row + vl < z.per);
+  const int v = mine && vl > 0 ? first_row + vl : 0;
   extern __shared__ double sm[];
   const int cap = n * 32;
-  double *const Y = sm + lane, *const F = Y + cap, *const A = F + cap;
+  double *const Y = sm + lane, *const F = Y + cap;
+  long long* const A = reinterpret_cast<long long*>(F + cap);  // in units of 2^(top - 62)
   double *const R = sm + 3 * cap, *const L = R + cap;
   double* const Dg = L + cap;         // slots x n: diagonal + shift
   double* const Eg = Dg + slots * n;  // slots x n: Eg[i] couples i - 1 and i
   __shared__ int s_row[32];
+  __shared__ bool s_nan[32];
   const double shift = (double)(n - 1) / g.inflation;
   int vs;
   double* const io = ft::vec_at(z, n, s, v, vs);
   if (mine)
+#pragma unroll 4
     for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
-  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, 1, part == 0 ? 0 : LLONG_MAX, eig_fail);
+  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, s_nan, 1, first_row == 0 ? 0 : LLONG_MAX, eig_fail);
   const int nb = 32 / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
   int nmax = 0;
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
   const int fs = lane % slots, fj = lane / slots;
   const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
-  for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
+  // |f(T) y| < 2^top
+  unsigned emax = 0;
+  for (int i = 0; i < n; ++i) {
+    A[32 * i] = 0;
+    if (mine) emax = max(emax, ((unsigned)__double2hiint(Y[32 * i]) >> 20) & 0x7ffu);
+  }
+  const int top = (int)emax - 1022 + 3 + ft::f_top(g.inflation), Eb = top + 1022;
   const int m = n / 2, nd = n - 1 - m;
-  auto solve = [&](int pair, double w) {
+  auto solve = [&](int pair) {
     // A += w (T + s)^-1 y with the pair's twisted factors: inwards, then outwards
     // from element m, both chains one fused multiply-add per element; the next
     // element's operands are read ahead of the chains' stores
@@ -478,88 +568,98 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
       F[32 * (m - 1)] = f;
     }
     double u = Rp[32 * m] * fma(-Lp[32 * (m + 1)], h, fma(-Lp[32 * m], f, Y[32 * m]));
-    A[32 * m] = fma(w, u, A[32 * m]);
+    ft::add_fixed(A[32 * m], u, Eb);
     double d = u;
     int iu = m - 1, id = m + 1;
-    double lu = Lp[32 * m], gu = Rp[32 * iu] * F[32 * iu], au = A[32 * iu];
-    double ld = Lp[32 * id], gd = Rp[32 * id] * F[32 * id], ad = A[32 * id];
+    double lu = Lp[32 * m], gu = Rp[32 * iu] * F[32 * iu];
+    double ld = Lp[32 * id], gd = Rp[32 * id] * F[32 * id];
 #pragma unroll 4
     for (int c = 1; c < nd; ++c) {
       u = fma(-lu, u, gu);
       d = fma(-ld, d, gd);
-      const double xu = fma(w, u, au), xd = fma(w, d, ad);
       const int ju = iu - 1, jd = id + 1;
       lu = Lp[32 * iu];
       gu = Rp[32 * ju] * F[32 * ju];
-      au = A[32 * ju];
       ld = Lp[32 * jd];
       gd = Rp[32 * jd] * F[32 * jd];
-      ad = A[32 * jd];
-      A[32 * iu] = xu;
-      A[32 * id] = xd;
+      ft::add_fixed(A[32 * iu], u, Eb);
+      ft::add_fixed(A[32 * id], d, Eb);
       iu = ju;
       id = jd;
     }
     u = fma(-lu, u, gu);
-    A[32 * iu] = fma(w, u, au);
-    A[32 * id] = fma(w, fma(-ld, d, gd), ad);
-    if (m > nd) {
-      u = fma(-Lp[32], u, Rp[0] * F[0]);
-      A[0] = fma(w, u, A[0]);
-    }
+    ft::add_fixed(A[32 * iu], u, Eb);
+    ft::add_fixed(A[32 * id], fma(-ld, d, gd), Eb);
+    if (m > nd) ft::add_fixed(A[0], fma(-Lp[32], u, Rp[0] * F[0]), Eb);
   };
   for (int j0 = 0; j0 < nmax; j0 += nb) {
-    if (fs < nsl && fj < nb && j0 + fj < nmax)
-      ft::factor_twisted(n, Dg + fs * n, Eg + fs * n, ft::g_nodes[s_row[fs]][j0 + fj].x * shift,
-                         R + lane, L + lane);
-    __syncwarp();
-    if (mine) {
-      const int rowq = s_row[sl];
-      for (int j = 0; j < nb && j0 + j < nmax; ++j)
-        solve(sl + slots * j, ft::g_nodes[rowq][j0 + j].y * wscale);
+    if (fs < nsl && fj < nb && j0 + fj < nmax) {
+      const double2 node = ft::g_nodes[s_row[fs]][j0 + fj];
+      ft::factor_twisted(n, Dg + fs * n, Eg + fs * n, node.x * shift, node.y * wscale, R + lane,
+                         L + lane);
     }
     __syncwarp();
+    if (mine)
+      for (int j = part; j < nb && j0 + j < nmax; j += kL) solve(sl + slots * j);
+    __syncwarp();
   }
-  if (!mine || v == 0) return;
+  // ---- out
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const bool finite = emax < 2047u && !s_nan[sl];
+  double* const Af = reinterpret_cast<double*>(A);
+  for (int i = 0; i < n; ++i) {
+    const long long a = ft::sum_parts<kL>(A[32 * i]);
+    Af[32 * i] = finite ? fixed_to_double(a, top - 62) : nan;
+  }
+  __syncwarp();
+  const bool row = mine && v > 0;
   const double srho = sqrt(g.inflation);
   const double* zt = sm + 2 * cap + sl * lanes;  // vector 0's A
-  double dotw = 0.0;
-  for (int i = 0; i < n; ++i) {
-    const double a = A[32 * i];
-    dotw = fma(a, zt[32 * i], dotw);
+  const double dotw = ft::sum_elements<kL>(ft::own<kL>(n, part), [&](int q) {
+    if (!row) return 0.0;
+    const int i = part + kL * q;
+    const double a = Af[32 * i];
     io[(size_t)i * vs] = fma(-srho, Y[32 * i], a);
-  }
-  io[(size_t)n * vs] = dotw / (double)(n - 1);
+    return a * zt[32 * i];
+  });
+  if (row && part == 0) io[(size_t)n * vs] = dotw / (double)(n - 1);
 }
 
 // F = f(T) of each solve, symmetric, into its n x n matrix: one column per lane,
 // lanes numbered through the solves' columns, one warp per block.  Shared memory
 // as in ft_kernel: A (the column), and per (slot, node) pair L and the diagonal G
 // of (T + s)^-1 (R first).
+template <int kL>
 __global__ void __launch_bounds__(32) ft_matrix_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
                                                        const double* tri, int* eig_fail) {
   const int n = g.ens;
   const int lane = threadIdx.x;
-  const long long id0 = (long long)blockIdx.x * 32, total = (long long)b.nsolves * n;
+  constexpr int kV = 32 / kL;  // columns of a warp
+  const long long id0 = (long long)blockIdx.x * kV, total = (long long)b.nsolves * n;
   const int s_first = (int)(id0 / n);
-  const int nsl = (int)((min(id0 + 32, total) - 1) / n) - s_first + 1;
-  const bool mine = id0 + lane < total;
-  const int s = mine ? (int)((id0 + lane) / n) : s_first, sl = s - s_first;
-  const int v = mine ? (int)((id0 + lane) - (long long)s * n) : 0;
+  const int nsl = (int)((min(id0 + kV, total) - 1) / n) - s_first + 1;
+  const long long id = id0 + lane / kL;
+  const int part = lane % kL;  // this lane's nodes: part, part + kL, ..
+  const bool mine = id < total;
+  const int s = mine ? (int)(id / n) : s_first, sl = s - s_first;
+  const int v = mine ? (int)(id - (long long)s * n) : 0;
   extern __shared__ double sm[];
   const int cap = n * 32;
-  double *const A = sm + lane, *const G = sm + cap, *const L = G + cap;
+  long long* const A = reinterpret_cast<long long*>(sm) + lane;  // in units of 2^(top - 62)
+  double *const G = sm + cap, *const L = G + cap;
   double* const Dg = L + cap;
   double* const Eg = Dg + slots * n;
   __shared__ int s_row[32];
+  __shared__ bool s_nan[32];
   const double shift = (double)(n - 1) / g.inflation;
-  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, n, id0, eig_fail);
+  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, s_nan, n, id0, eig_fail);
   const int nb = 32 / slots;
   int nmax = 0;
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
   const int fs = lane % slots, fj = lane / slots;
   const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
-  for (int i = 0; i < n; ++i) A[32 * i] = 0.0;
+  for (int i = 0; i < n; ++i) A[32 * i] = 0;
+  const int top = ft::f_top(g.inflation), Eb = top + 1022;
   const int vmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)v);
   for (int j0 = 0; j0 < nmax; j0 += nb) {
     if (fs < nsl && fj < nb && j0 + fj < nmax) {
@@ -576,7 +676,7 @@ __global__ void __launch_bounds__(32) ft_matrix_kernel(Geometry g, SolveBatch b,
       }
     }
     __syncwarp();
-    for (int j = 0; j < nb && j0 + j < nmax; ++j) {
+    for (int j = part; j < nb && j0 + j < nmax; j += kL) {
       const int pair = sl + slots * j;
       const double *Gp = G + pair, *Lp = L + pair;
       double x = 0.0;
@@ -585,15 +685,19 @@ __global__ void __launch_bounds__(32) ft_matrix_kernel(Geometry g, SolveBatch b,
         // above the diagonal x is not begun yet, on it it starts
         const double step = i < n - 1 ? -Lp[32 * (i + 1)] * x : 0.0;
         x = i == v ? Gp[32 * i] : step;
-        if (i <= v) A[32 * i] += x;
+        if (i <= v) ft::add_fixed(A[32 * i], x, Eb);
       }
     }
     __syncwarp();
   }
+  if (kL > 1)
+    for (int i = 0; i <= vmax; ++i) A[32 * i] = ft::sum_parts<kL>(A[32 * i]);
   if (!mine) return;
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const bool finite = !s_nan[sl];
   double* const out = z.vec + ft::out_index(b, s) * n * n;
-  for (int i = 0; i <= v; ++i) {
-    const double x = A[32 * i];
+  for (int i = part; i <= v; i += kL) {
+    const double x = finite ? fixed_to_double(A[32 * i], top - 62) : nan;
     out[(size_t)i * n + v] = x;
     out[(size_t)v * n + i] = x;
   }
@@ -646,35 +750,87 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
   const int n = g.ens;
   const int per = core ? n : 1 + (g.vert_dist > 0.0 ? g.n_var : g.n);
   const ft::Vecs z{per, t, vec};
-  // solves that 32 consecutive vectors can touch
-  auto spans = [](int p) { return (32 + p - 2) / p + 1; };
-  auto blocks = [&](int p) { return (unsigned)(((long long)b.nsolves * p + 31) / 32); };
-  auto reflect = [&](auto kernel, int p) {
-    const int sl = spans(p);
-    const size_t smem = sizeof(double) * ((size_t)32 * n + 2 * (size_t)sl * n);
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kernel<<<blocks(p), 32, smem, stream>>>(g, b, z, sl, tri, xb, axb, xa, axa);
+  auto with = [](int lanes, auto f) {
+    switch (lanes) {
+      case 8: f(std::integral_constant<int, 8>()); break;
+      case 4: f(std::integral_constant<int, 4>()); break;
+      case 2: f(std::integral_constant<int, 2>()); break;
+      default: f(std::integral_constant<int, 1>());
+    }
   };
-  auto solve_smem = [&](auto kernel, int arrays, int sl) {
-    const size_t smem = sizeof(double) * ((size_t)arrays * 32 * n + 2 * (size_t)sl * n);
+  auto smem_of = [&](auto kernel, size_t doubles) {
+    const size_t smem = sizeof(double) * doubles;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return smem;
   };
+  // solves that the vectors of a warp can touch, p to a solve, and warps
+  auto spans = [](int p, int vectors) { return (vectors + p - 2) / p + 1; };
+  auto blocks = [&](int p, int vectors) {
+    return (unsigned)(((long long)b.nsolves * p + vectors - 1) / vectors);
+  };
+  auto reflect = [&](auto first, int p, int lanes) {
+    with(lanes, [&](auto l) {
+      constexpr int kL = decltype(l)::value, kV = 32 / kL;
+      constexpr bool kFirst = decltype(first)::value;
+      const int sl = spans(p, kV);
+      const size_t doubles = 32 * (size_t)((n + kL - 1) / kL) + 2 * (size_t)sl * n;
+      auto run = [&](auto kernel) {
+        kernel<<<blocks(p, kV), 32, smem_of(kernel, doubles), stream>>>(g, b, z, sl, tri, xb, axb, xa,
+                                                                       axa);
+      };
+      if (core)
+        run(reflect_kernel<kFirst, true, kL>);
+      else
+        run(reflect_kernel<kFirst, false, kL>);
+    });
+  };
+  // Lanes per vector, for the solves (lf, which share its nodes) and the reflections
+  // (lr, its elements).  Few vectors leave most schedulers idle and the time is one
+  // lane's chain; many vectors fill the chip and the shares cost their sums -- except
+  // that an analysis's reflections gain occupancy from a smaller array per warp at
+  // every size (core ones read columns, which two lanes coalesce worse).  By warps of
+  // vectors at one lane each; measured, us of a core call of 40 members with lf at 8 /
+  // 4 / 2 / 1: 20 warps 312 / 315 / 324 / 346, 160 warps 349 / 322 / 326 / 344, 320
+  // warps 411 / 374 / 354 / 371, 640 warps 520 / 446 / 423 / 408; with lr: 160 warps
+  // 285 / 291 / 320 / 369, 640 warps 456 / 410 / 423 / 463, 2880 warps 1479 / 1277 /
+  // 1204 / 1252, 41 000 warps 18.9 / 15.8 / 14.5 / 14.1 ms.  Analysis of 16 members, lf:
+  // 324 warps 122 / 123 / 143 / 188, 1296 warps 210 / 205 / 190 / 204, 2500 warps 321 /
+  // 293 / 289 / 283; lr: 324 warps 73 / 92 / 122 / 198, 2500 warps 289 / 281 / 293 /
+  // 365; of 40 members, 144 000 warps in eleven launches, lr 70.9 / 62.9 / 59.2 / 63.0 ms.
+  const long long warps = ((long long)b.nsolves * per + 31) / 32;  // (never INT_MAX)
+  auto lanes_for = [&](int w8, int w4, int w2) {
+    return warps < w8 ? 8 : warps < w4 ? 4 : warps < w2 ? 2 : 1;
+  };
+  using First = std::true_type;
+  using Second = std::false_type;
   if (core) {
-    const int sl = spans(n);
-    ft_matrix_kernel<<<blocks(n), 32, solve_smem(ft_matrix_kernel, 3, sl), stream>>>(g, b, z, sl, tri,
-                                                                                     eig_fail);
-    reflect(reflect_kernel<true, true>, n);
-    reflect(reflect_kernel<false, true>, n);
+    const int lf = lanes_for(40, 200, 450), lr = lanes_for(200, 800, 6000);
+    with(lf, [&](auto l) {
+      constexpr int kL = decltype(l)::value, kV = 32 / kL;
+      const int sl = spans(n, kV);
+      const size_t smem = smem_of(ft_matrix_kernel<kL>, 3 * 32 * (size_t)n + 2 * (size_t)sl * n);
+      ft_matrix_kernel<kL><<<blocks(n, kV), 32, smem, stream>>>(g, b, z, sl, tri, eig_fail);
+    });
+    reflect(First(), n, lr);
+    reflect(Second(), n, lr);
     add_wbar_kernel<<<b.nsolves, 128, 0, stream>>>(n, b, t, vec, wbar);
-  } else {
-    const int parts = (per + 29) / 31, rows = (per - 1 + parts - 1) / parts, sl = 32 / (rows + 1);
-    const unsigned grid = parts > 1 ? (unsigned)b.nsolves * parts : (unsigned)((b.nsolves + sl - 1) / sl);
-    reflect(reflect_kernel<true, false>, per);
-    ft_kernel<<<grid, 32, solve_smem(ft_kernel, 5, sl), stream>>>(g, b, z, sl, rows, parts, tri,
-                                                                  eig_fail);
-    reflect(reflect_kernel<false, false>, per - 1);
+    return;
   }
+  int lf = lanes_for(400, 700, 2000);
+  const int lr = lanes_for(700, 2000, INT_MAX);
+  // a solve's vectors have to fit a warp, nearly filling it
+  while (lf > 1 && (per * lf > 32 || 32 % (per * lf) > 4)) lf /= 2;
+  const int parts = (per + 29) / 31, rows = (per - 1 + parts - 1) / parts;
+  reflect(First(), per, lr);
+  with(lf, [&](auto l) {
+    constexpr int kL = decltype(l)::value;
+    const int sl = 32 / ((rows + 1) * kL);
+    const size_t smem = smem_of(ft_kernel<kL>, 5 * 32 * (size_t)n + 2 * (size_t)sl * n);
+    const unsigned grid =
+        parts > 1 ? (unsigned)b.nsolves * parts : (unsigned)((b.nsolves + sl - 1) / sl);
+    ft_kernel<kL><<<grid, 32, smem, stream>>>(g, b, z, sl, rows, parts, tri, eig_fail);
+  });
+  reflect(Second(), per - 1, lr);
 }
 
 }  // namespace lg

@@ -124,3 +124,18 @@ def test_every_row_in_one_solve(nz, monkeypatch):
     i = slice(cfg.halo, -cfg.halo)
     inc = np.abs(out[1] - (w.xb + w.axb[..., None]))[i, i].max()
     assert np.abs(out[0] - out[1])[i, i].max() <= 1e-10 * inc
+
+
+@pytest.mark.parametrize("k,nb", [(7, 1), (9, 3), (40, 1), (41, 100), (64, 70), (40, 400), (33, 700)])
+def test_lanes_per_vector(k, nb):
+    """Batches from one solve to some hundred: 8, 4, 2 and 1 lanes per vector,
+    member counts that leave lanes without elements."""
+    rng = np.random.default_rng(17 * k + nb)
+    base = [_case(rng, k, p) for p in (0, 5, 3 * k)]
+    cases = [base[i % 3] for i in range(nb)]
+    st, tr, wb = _batch(cases, 1.05)
+    assert st == 0
+    for i in sorted({0, 1, 2, nb // 2, nb - 3, nb - 2, nb - 1} & set(range(nb))):
+        _check(cases[i], 1.05, tr[i], wb[i])
+    for i in range(3, nb):  # a solve's result does not depend on its place
+        assert np.array_equal(tr[i], tr[i % 3]) and np.array_equal(wb[i], wb[i % 3])
