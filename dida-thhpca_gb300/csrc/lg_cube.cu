@@ -75,10 +75,10 @@ __device__ inline double scaled(long long p, int ex) {
 // rounded once to 2^-58 of their (Frobenius) norms, and by Cauchy-Schwarz no sum
 // leaves 64 bits.  The mean is the mean of the products, so axb stays out of the
 // perturbations.  Measured, 32 768
-// solves of 40 members over 7200 columns of 97 rows: 4.4 -> 1.5 ms (a block per
+// solves of 40 members over 7200 columns of 97 rows: 4.4 -> 1.3 ms (a block per
 // column, 1.8 ms; FP64 at full lanes would take 2.3).
-constexpr int kThreads = 256;
-__global__ void __launch_bounds__(kThreads, 3)
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 768 / kThreads)
     cube_apply_kernel(Geometry g, CubeDev cd, const double* trans, const double* xb, const double* axb,
                       double* xa, double* axa) {
   const int k = g.ens, n = g.n, LDT = k + 1;  // odd stride for even k: few conflicts in staging
@@ -319,11 +319,23 @@ void launch_cube_apply(const Geometry& g, const CubeDev& cd, int nsolves, const 
                        const double* xb, const double* axb, double* xa, double* axa,
                        cudaStream_t stream) {
   const int k = g.ens;
-  const size_t batch = 2 * (kThreads / k);
-  const size_t smem = 8 * ((size_t)k * (k + 1) + batch * (((k + 1) & ~1) + k + 3));
-  const int grid = cd.stride == cd.cube_n ? nsolves : g.num_lat * g.num_lon;
-  cudaFuncSetAttribute(cube_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cube_apply_kernel<<<grid, kThreads, smem, stream>>>(g, cd, trans, xb, axb, xa, axa);
+  const bool per_solve = cd.stride == cd.cube_n;
+  const int grid = per_solve ? nsolves : g.num_lat * g.num_lon;
+  auto run = [&](auto kernel, int threads) {
+    const size_t batch = 2 * (threads / k);
+    const size_t smem = 8 * ((size_t)k * (k + 1) + batch * (((k + 1) & ~1) + k + 3));
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<grid, threads, smem, stream>>>(g, cd, trans, xb, axb, xa, axa);
+  };
+  // Smaller blocks hide the steps between barriers better; above 64 members 128 threads
+  // hold a single row each time and idle, unless there are few rows.  At 128 / 256
+  // threads: 32 768 solves of 28 rows of 40 members 1.28 / 1.52 ms; single levels, 12
+  // rows of 15 members 19 / 24 us, 12 of 70 30 / 33 us, 27 of 85 84 / 56 us.
+  const int rows = (cd.grouped ? g.n_var * cd.cube_nz : g.n) * (per_solve ? cd.cube_n * cd.cube_n : 1);
+  if (k <= 64 || rows * k <= 1024)
+    run(cube_apply_kernel<128>, 128);
+  else
+    run(cube_apply_kernel<256>, 256);
 }
 
 }  // namespace lg
