@@ -82,15 +82,16 @@ constexpr int kHalfLevels = 256;    // levels the search passes in FP32
 __global__ void __launch_bounds__(128) hx_kernel(Geometry g, ObsDev ob, const double* xb,
                                                  const double* axb, HxDev hx, int* err,
                                                  int64_t j0, int64_t j1) {
-  // half_ph(kk) = x + y (ps - ptop), FP32
+  // half_ph(kk) = x + y (ps - ptop), FP32 (a handful of levels is not worth it)
   __shared__ float2 s_half[kHalfLevels];
-  for (int kk = threadIdx.x; kk < min(g.nz, kHalfLevels); kk += blockDim.x) {
+  const int passed = g.nz < 8 ? 0 : min(g.nz, kHalfLevels);
+  for (int kk = threadIdx.x; kk < passed; kk += blockDim.x) {
     const bool sigma = g.vcoord == LG_VCOORD_SIGMA;
     const double a = 0.5 * (g.ca[kk] + g.ca[kk + 1]), b = 0.5 * (g.cb[kk] + g.cb[kk + 1]);
     s_half[kk] = sigma ? make_float2((float)g.ptop, (float)a)
                        : make_float2((float)(a * (g.p0 - g.ptop) + g.ptop), (float)b);
   }
-  __syncthreads();
+  if (passed) __syncthreads();
   const int64_t j = j0 + (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x / 32);
   if (j >= j1) return;
   const unsigned lane = threadIdx.x & 31u;
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(128) hx_kernel(Geometry g, ObsDev ob, const do
     psd[q] = __dsub_rn(ps[q], g.ptop);
     hp[q] = hpm[q] = 0.0;
   }
-  bool has3d = false;  // the log-p weights are needed only for 3-D variables
+  bool has3d = false;  // levels and log-p weights are needed only for 3-D variables
   for (int kv = 0; kv < onv; ++kv) has3d |= g.var_lev[c_types.var[ti][kv]] > 1;
   for (int l = 0; l < onz; ++l) {
     const double po = oph[l];
@@ -194,12 +195,12 @@ __global__ void __launch_bounds__(128) hx_kernel(Geometry g, ObsDev ob, const do
 #pragma unroll
     for (int q = 0; q < kMaxMemberSlots; ++q) {
       const int e = (int)lane + 32 * q;
-      if (e < k) {
+      if (has3d && e < k) {
         // while (jj <= nz && po > half_ph(jj)) jj++; half_ph(nz + 1) is
         // half_ph(nz), so hp needs no update when jj reaches nz + 1
         int j = max(jj[q], 1);
         const float pf = (float)psd[q];
-        for (; j <= min(g.nz, kHalfLevels); ++j) {
+        for (; j <= passed; ++j) {
           const float2 h = s_half[j - 1];
           const float far = 1e-6f * (fabsf(h.x) + fabsf(h.y * pf) + fabsf(pof));
           if (!(pof - fmaf(h.y, pf, h.x) > far)) break;
