@@ -525,6 +525,12 @@ int lg_create(lg_ctx** out, const lg_config* cfg) {
   // localisation, whatever da_vert_distance is (letkf.F90:227-235)
   if (g.overlap > 0) c->cfg.vert_dist = 0.0;
   c->cubes = g.cube_n > 1 || g.overlap > 0 || (g.cube_nz > 1 && c->cfg.vert_dist > 0.0);
+  // Solves per chunk: one lane of the QL kernel takes a matrix, so a launch with fewer
+  // than 384 warps takes as long as a full one.  1 GiB of Gram matrices holds that many
+  // solves up to 104 members; above, the workspace grows to hold them.  128 members,
+  // 36 864 solves, on the default streams: 206 .. 214 ms at 1024 MiB (8192 solves), 188
+  // at 1536 (12 288), 187 .. 202 at 2048 and 3072.
+  c->tune.chunk_mb = std::max(1024, (int)((12288 * 8 * (size_t)g.ens * g.ens + (1 << 20) - 1) >> 20));
   c->vec64 = getenv("LETKF_GB300_VEC64") != nullptr;
   if (lg::prepare_ft_nodes() != LG_OK) {
     delete c;
