@@ -1111,7 +1111,7 @@ int prepare_capacity(lg_ctx* c) {
   if (cells)
     lg::launch_search_cells(geo, c->obs, c->cells, lcount, 0, c->d_band, st);
   else
-    lg::launch_search(geo, c->obs, lcount, 0, c->d_band, st);
+    lg::launch_search(geo, c->obs, lcount, 0, false, c->d_band, st);
   lg::launch_scan_counts(c->lists.cnt, c->lists.off, ncol, c->d_scan_tmp, c->scan_tmp_bytes, st);
   if (cells) CK(cudaMemsetAsync(c->d_fresh, 1, sizeof(int), st));  // done by the sync below
   CK(cudaGetLastError());
@@ -1411,14 +1411,14 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
   if (cells)
     lg::launch_search_cells(geo, c->obs, c->cells, lcount, 0, c->d_band, st, c->d_fresh);
   else
-    lg::launch_search(geo, c->obs, lcount, 0, c->d_band, st);
+    lg::launch_search(geo, c->obs, lcount, 0, false, c->d_band, st);
   CK(cudaMemsetAsync(c->d_fresh, 0, sizeof(int), st));  // later analyses count again
   lg::launch_scan_counts(c->lists.cnt, c->lists.off, ncol, c->d_scan_tmp, c->scan_tmp_bytes, st);
   launches += 3;  // count pass + the scan's init and scan kernels
   if (cells)
     lg::launch_search_cells(geo, c->obs, c->cells, c->lists, 1, nullptr, st);
   else
-    lg::launch_search(geo, c->obs, c->lists, 1, nullptr, st);
+    lg::launch_search(geo, c->obs, c->lists, 1, g.precision == LG_PREC_FP64, nullptr, st);
   launches += 1;
   CK(record_event(c->ev[5], st));
   CK(cudaStreamWaitEvent(st, c->ev_hx, 0));
@@ -1872,7 +1872,7 @@ int lg_list_counts(lg_ctx* c, int* counts, int64_t* total) {
   if (c->have_cells && !getenv("LETKF_GB300_LINEAR_SEARCH"))
     lg::launch_search_cells(c->geo, c->obs, c->cells, l, 0, nullptr, st);
   else
-    lg::launch_search(c->geo, c->obs, l, 0, nullptr, st);
+    lg::launch_search(c->geo, c->obs, l, 0, false, nullptr, st);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(counts, l.cnt, sizeof(int) * ncol, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));

@@ -43,17 +43,45 @@ __device__ inline double schr(double ri) { return ri > 2.0 ? 0.0 : 1.0; }
 
 __device__ inline double loc_fn(double ri, int gc) { return gc ? schr2(ri) : schr(ri); }
 
+// Gaspari-Cohn as schr2 without its divisions: the same
+// polynomial with fused multiply-adds, 1/12 rounded once and 1/ri by two
+// Newton steps from the hardware approximation; agrees to a few ulp of 1.
+__device__ inline double taper_fast(double ri) {
+  if (ri > 2.0) return 0.0;
+  if (ri > 1.0) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ri));
+    r = fma(r, fma(-ri, r, 1.0), r);
+    r = fma(r, fma(-ri, r, 1.0), r);
+    double t = fma(ri, 1.0 / 12.0, -0.5);
+    t = fma(t, ri, 0.625);
+    t = fma(t, ri, (double)1.666667f);
+    t = fma(t, ri, -5.0);
+    t = fma(t, ri, 4.0);
+    return fma(-(double)0.6666667f, r, t);
+  }
+  if (ri > 0.0) {
+    const double t = fma(fma(-0.25, ri, 0.5), ri, 0.625);
+    return fma(fma(t, ri, -(double)1.666667f), ri * ri, 1.0);
+  }
+  return 1.0;
+}
+
 // x/180*pi with the reference's two roundings
 __device__ inline double deg2rad_r8(double x) { return __dmul_rn(__ddiv_rn(x, 180.0), pi_r4()); }
 
 // latlon_dist_r8 (pro_info.F90:149-161) from precomputed per-point terms:
 // cx = cos(x/180*pi), sx = sin(x/180*pi), yr = y/180*pi, point 1 = observation.
-__device__ inline double latlon_dist_pre(double cx1, double sx1, double yr1, double cx2,
-                                         double sx2, double yr2) {
+__device__ inline double latlon_angle_pre(double cx1, double sx1, double yr1, double cx2,
+                                          double sx2, double yr2) {
   double c3 = cos(__dsub_rn(yr1, yr2));
   double v = __dadd_rn(__dmul_rn(__dmul_rn(cx1, cx2), c3), __dmul_rn(sx1, sx2));
   if (!(v < 1.0)) v = (v != v) ? v : 1.0;
-  return __dmul_rn(earth_r4(), acos(v));
+  return acos(v);
+}
+__device__ inline double latlon_dist_pre(double cx1, double sx1, double yr1, double cx2,
+                                         double sx2, double yr2) {
+  return __dmul_rn(earth_r4(), latlon_angle_pre(cx1, sx1, yr1, cx2, sx2, yr2));
 }
 
 __device__ inline unsigned lane_id() { return threadIdx.x & 31u; }

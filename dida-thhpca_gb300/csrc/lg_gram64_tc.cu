@@ -229,30 +229,6 @@ __device__ inline void digit_pairs(unsigned long long z0, unsigned long long z1,
   out[0] = pack(a1 >> 18, b1 >> 2, 0x03ff03ffu);
 }
 
-// Gaspari-Cohn as schr2 (lg_device.cuh) without its divisions: the same
-// polynomial with fused multiply-adds, 1/12 rounded once and 1/ri by two
-// Newton steps from the hardware approximation; agrees to a few ulp of 1.
-__device__ inline double taper_fast(double ri) {
-  if (ri > 2.0) return 0.0;
-  if (ri > 1.0) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ri));
-    r = fma(r, fma(-ri, r, 1.0), r);
-    r = fma(r, fma(-ri, r, 1.0), r);
-    double t = fma(ri, 1.0 / 12.0, -0.5);
-    t = fma(t, ri, 0.625);
-    t = fma(t, ri, (double)1.666667f);
-    t = fma(t, ri, -5.0);
-    t = fma(t, ri, 4.0);
-    return fma(-(double)0.6666667f, r, t);
-  }
-  if (ri > 0.0) {
-    const double t = fma(fma(-0.25, ri, 0.5), ri, 0.625);
-    return fma(fma(t, ri, -(double)1.666667f), ri * ri, 1.0);
-  }
-  return 1.0;
-}
-
 }  // namespace g64
 
 // High word of the largest |y| of each H(x) row: its biased exponent from bit 20

@@ -194,7 +194,7 @@ void launch_hx_export(int ens, int64_t e0, int64_t e1, const HxDev& hx, double* 
                       cudaStream_t stream);
 void launch_hx_import(int ens, int64_t e0, int64_t e1, HxDev hx, const double* rows,
                       cudaStream_t stream);
-void launch_search(const Geometry& g, const ObsDev& o, ListDev l, int fill,
+void launch_search(const Geometry& g, const ObsDev& o, ListDev l, int fill, bool fp64,
                    unsigned long long* band, cudaStream_t stream);
 // skip (count pass only, may be null): when *skip is non-zero the launch does
 // nothing -- the counts and statistics are already those of this selection
