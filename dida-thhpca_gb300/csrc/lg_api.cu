@@ -1510,7 +1510,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
         lg::launch_ft(geo, b, true, L.t, L.C, c->d_trans, xb, axb, xa, axa, nullptr,
                       c->d_status + 1, st);
         CK(record_event(kv[6], st));
-        launches += 6;
+        launches += 7;
       } else {
         lg::launch_eig_apply(geo, b, L.C, L.t, xb, axb, xa, axa, c->d_trans, nullptr,
                              c->d_status + 1, st);
@@ -1625,7 +1625,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
       CK(record_event(kv[5], s_v));
       lg::launch_ft(geo, b, false, L.t, L.C, L.lam, xb, axb, xa, axa, nullptr, c->d_status + 1,
                     s_v);
-      launches += 4;
+      launches += 5;
     } else if (c->use_eig2) {
       if (s_q == s_e) {
         lg::launch_eig2(geo, b, L.C, L.t, xb, axb, xa, axa, L.tri, L.lam, L.rot_cs, L.rot_i,
