@@ -25,7 +25,9 @@
 // nodes.  overline_w . x = (T^(-1/2) y) . (T^(-1/2) Q^T t) needs no solve of its
 // own.  The reflections (2 k^2 multiply-adds per vector) leave the FP64 pipe
 // altogether: a vector's norm does not change, so they run in fixed point on the
-// integer pipe as the reduction does (lg_tri.cu), to 2^-58 of the norm per step.
+// integer pipe as the reduction does (lg_tri.cu), to 2^-58 of the norm per step, two
+// reflectors at a time (reading and rounding the vector once for both took the
+// explicit trans of those cubes from 7.2 to 6.6 ms).
 //   rows (analysis): reflect_kernel (Q^T), ft_kernel, reflect_kernel (Q) with the
 //     rows' update -- three kernels, so that the integer ones are not held to the
 //     two to four warps per SM that the solves' five arrays leave;
@@ -34,14 +36,14 @@
 //     T + s = L D L^T, G = (T + s)^-1 has G_jj = 1/D_j + L_{j+1}^2 G_{j+1,j+1} and
 //     G_ij = -L_{i+1} G_{i+1,j} above it), then W = Q F Q^T by two reflect_kernel
 //     passes and overline_w = W (W t) / (k - 1) in add_wbar_kernel.  A solve per
-//     unit vector instead made this step 12.9 ms where it is 7.2 (32 768 cubes of
+//     unit vector instead made this step 12.9 ms where it is 6.6 (32 768 cubes of
 //     40 members).
 // The sum over the nodes is kept in 64-bit integers: off the FP64 pipe, and the same
 // in any order, so that a vector may be spread over several lanes (launch_ft) and the
 // result does not depend on how many solves a launch has.
-// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 57 ms,
-// 129 600 of 64 members 93 -> 24 ms; explicit trans against the accumulating solver
-// (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 9.1 ms.  Faster at
+// Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 55 ms,
+// 129 600 of 64 members 93 -> 23 ms; explicit trans against the accumulating solver
+// (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 8.5 ms.  Faster at
 // every size from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
 #include <limits.h>
@@ -261,7 +263,7 @@ __device__ inline bool to_fixed(double* V, int m, int& ex) {
 // matrix then holds (Q F)^T); the second takes column j -- row j of Q F -- and
 // leaves W's column j there, so that no lane reads what another one writes.
 // Reflector rows of the (up to `slots`) solves that a warp spans come into shared
-// memory a step ahead of their use.
+// memory, two at a time, a step ahead of their use.
 template <bool kFirst, bool kCore, int kL>
 __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, ft::Vecs z,
                                                      int slots, const double* tri, const double* xb,
@@ -283,22 +285,37 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   extern __shared__ double sm[];
   double* const Y = sm + lane;                      // element part + kL i at 32 i
   int2* const Yi = reinterpret_cast<int2*>(Y);
-  double* const ub = sm + 32 * ((n + kL - 1) / kL);  // two buffers of slots x n
+  double* const ub = sm + 32 * ((n + kL - 1) / kL);  // two buffers of slots x 2 n
   const size_t tri_stride = (size_t)n * n;
-  auto fetch = [&](int i, int buf) {
-    if (i >= 1 && i < n)
+  // pair m, 1 .. n / 2: reflectors 2 m and 2 m - 1 as rows A and B, B padded with a
+  // zero, and w_A . w_B behind A; for even n the last pair is reflector n - 1 alone
+  auto fetch = [&](int m, int buf) {
+    if (m >= 1 && m <= n / 2)
       for (int sl = 0; sl < nsl; ++sl) {
         const double* T = tri + (size_t)(s_first + sl) * tri_stride;
-        const double* u = T + 3 * n + (size_t)i * (i - 1) / 2;
-        double* d = ub + (size_t)(buf * slots + sl) * n;
-        for (int c = lane; c < i; c += 32) ft::cp_async8(d + c, u + c);
-        if (lane == 0) ft::cp_async8(d + n - 1, T + 2 * n + i);  // H (i <= n - 1: free)
+        double* d = ub + (size_t)(buf * slots + sl) * 2 * n;
+        const bool two = 2 * m < n;
+        const int la = two ? 2 * m : n - 1;
+        const double* u = T + 3 * n + (size_t)la * (la - 1) / 2;
+        for (int c = lane; c < la; c += 32) {
+          ft::cp_async8(d + c, u + c);
+          if (two && c < la - 1)
+            ft::cp_async8(d + n + c, u - (la - 1) + c);
+          else
+            d[n + c] = 0.0;
+        }
+        if (lane == 0) {
+          if (two)
+            ft::cp_async8(d + n - 1, T + 2 * n + la);
+          else
+            d[n - 1] = 0.0;
+        }
       }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   constexpr bool kDown = kFirst && !kCore;  // Q^T
-  const int step = kDown ? -1 : 1, i0 = kDown ? n - 1 : 1;
-  fetch(i0, 0);
+  const int step = kDown ? -1 : 1, m0 = kDown ? n / 2 : 1;
+  fetch(m0, 0);
   // ---- the vector
   int r_state = -1;
   size_t ci = 0;
@@ -337,45 +354,43 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   }
   int ex;
   const bool finite = ft::to_fixed<kL>(Y, m, ex);
-  // ---- reflections: y -= w (w . y)
-  for (int c = 0, i = i0; c < n - 1; ++c, i += step) {
-    fetch(i + step, (c + 1) & 1);
+  // ---- two reflections at a time: y -= w1 d1 + w2 d2, d1 = w1 . y, d2 = w2 . y -
+  // (w1 . w2) d1, so that y is read twice and rounded once for both
+  for (int c = 0, mp = m0; c < n / 2; ++c, mp += step) {
+    fetch(mp + step, (c + 1) & 1);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    const double* ud = ub + (size_t)((c & 1) * slots + (s - s_first)) * n;
-    const int2* u = reinterpret_cast<const int2*>(ud) + part;
-    const bool reflect = __double2hiint(ud[n - 1]) != 0;
-    const int mi = ft::own<kL>(i, part);
-    long long hs = 0, ms = part == 0 ? 1 << 27 : 0;  // rounds the sum's cut
-    auto dot = [&]() {
+    const int2* const ud =
+        reinterpret_cast<const int2*>(ub + (size_t)((c & 1) * slots + (s - s_first)) * 2 * n);
+    const int2 *uA = ud + part, *uB = ud + n + part;
+    const int2 g2 = ud[n - 1];
+    const int mi = ft::own<kL>(min(2 * mp, n - 1), part);
+    long long hA = 0, hB = 0, mA = part == 0 ? 1 << 27 : 0, mB = mA;  // rounds the sum's cut
 #pragma unroll 4
-      for (int j = 0; j < mi; ++j) {
-        const int2 w = u[kL * j], y = Yi[32 * j];
-        hs += (long long)y.y * w.y;
-        ms += (long long)y.y * w.x;
-        ms += (long long)y.x * w.y;
-      }
-    };
-    auto update = [&]() {
-      const int2 D = fixed_split(4 * hs + (ms >> 28));
-      const int D4 = -4 * D.y;  // |D| < 2^58.5
+    for (int j = 0; j < mi; ++j) {
+      const int2 y = Yi[32 * j], w = uA[kL * j], x = uB[kL * j];
+      hA += (long long)y.y * w.y;
+      mA += (long long)y.y * w.x;
+      mA += (long long)y.x * w.y;
+      hB += (long long)y.y * x.y;
+      mB += (long long)y.y * x.x;
+      mB += (long long)y.x * x.y;
+    }
+    long long dA = 4 * ft::sum_parts<kL>(hA) + (ft::sum_parts<kL>(mA) >> 28);
+    long long dB = 4 * ft::sum_parts<kL>(hB) + (ft::sum_parts<kL>(mB) >> 28);
+    const int2 D1 = fixed_split(kDown ? dA : dB);
+    const long long cross = 4 * ((long long)D1.y * g2.y) +
+                            (((long long)D1.y * g2.x + (long long)D1.x * g2.y + (1 << 27)) >> 28);
+    const int2 D2 = fixed_split((kDown ? dB : dA) - cross);
+    const int2 DA = kDown ? D1 : D2, DB = kDown ? D2 : D1;
+    const int A4 = -4 * DA.y, B4 = -4 * DB.y;  // |D| < 2^58.5
 #pragma unroll 4
-      for (int j = 0; j < mi; ++j) {
-        const int2 w = u[kL * j], y = Yi[32 * j];
-        const long long c2 = (long long)D.y * w.x + ((long long)D.x * w.y + (1 << 27));
-        Yi[32 * j] = fixed_split(fixed_join(y) + (long long)D4 * w.y - (int)(c2 >> 28));
-      }
-    };
-    if (kL == 1) {
-      if (reflect) {
-        dot();
-        update();
-      }
-    } else {
-      if (reflect) dot();
-      hs = ft::sum_parts<kL>(hs);
-      ms = ft::sum_parts<kL>(ms);
-      if (reflect) update();
+    for (int j = 0; j < mi; ++j) {
+      const int2 w = uA[kL * j], x = uB[kL * j], y = Yi[32 * j];
+      long long c2 = (long long)DA.y * w.x + ((long long)DA.x * w.y + (1 << 27));
+      c2 += (long long)DB.y * x.x;
+      c2 += (long long)DB.x * x.y;
+      Yi[32 * j] = fixed_split(fixed_join(y) + (long long)A4 * w.y + (long long)B4 * x.y - (c2 >> 28));
     }
     __syncwarp();
   }
@@ -773,7 +788,7 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
       constexpr int kL = decltype(l)::value, kV = 32 / kL;
       constexpr bool kFirst = decltype(first)::value;
       const int sl = spans(p, kV);
-      const size_t doubles = 32 * (size_t)((n + kL - 1) / kL) + 2 * (size_t)sl * n;
+      const size_t doubles = 32 * (size_t)((n + kL - 1) / kL) + 4 * (size_t)sl * n;
       auto run = [&](auto kernel) {
         kernel<<<blocks(p, kV), 32, smem_of(kernel, doubles), stream>>>(g, b, z, sl, tri, xb, axb, xa,
                                                                        axa);

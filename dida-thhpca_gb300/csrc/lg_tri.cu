@@ -22,12 +22,13 @@
 // One warp per matrix, the packed lower triangle in shared memory; lanes take
 // rows (split over lanes where fewer than 32 are left) in A w and elements in
 // the update, as in tridiag_kernel (lg_eig2.cu).  Output in the Gram matrix's
-// place: D[n] | E[n] | H[n] (1: reflector w, 0: none) | w rows (w 2^58 as pairs
-// of 32-bit integers).
+// place: D[n] | E[n] | G[n] (even i: w_i . w_{i-1}, for the transform, which applies
+// two reflectors at a time) | w rows, zero where there is none (w and G in units of
+// 2^-58 as pairs of 32-bit integers).
 // A non-finite C gives a NaN diagonal, which the transform reports.
 //
 // Measured alone against tridiag_kernel: 921 600 matrices of 40 members 116 ->
-// 52 ms, 129 600 of 64 members 54 -> 26 ms, 2592 of 16 members 81 -> 52 us; a single
+// 52 ms, 129 600 of 64 members 54 -> 27 ms, 2592 of 16 members 81 -> 52 us; a single
 // matrix of 40 members 94 us.  Bound by instruction issue (at 64 members the
 // triangles leave twelve warps per SM).
 #include "lg_device.cuh"
@@ -110,15 +111,16 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
   __syncwarp();
   double* const D = M;
   double* const E = M + n;
-  double* const H = M + 2 * n;
+  int2* const G = reinterpret_cast<int2*>(M + 2 * n);
   double* const U = M + 3 * n;
   if (emax == 0 || emax >= 2047u - 8u) {  // all zero, or not representable: NaN
     __syncwarp();
     for (int i = lane; i < n; i += 32) {
       D[i] = emax ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
       E[i] = 0.0;
-      H[i] = 0.0;
+      G[i] = make_int2(0, 0);
     }
+    for (int t = lane; t < n * (n - 1) / 2; t += 32) U[t] = 0.0;
     return;
   }
   float fro = 0.0f;
@@ -339,14 +341,26 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
   }
   for (int i = lane; i < n; i += 32) {
     D[i] = fixed_to_double(fixed_join(A[idx(i) + i]), ex);
-    double e = 0.0, h = 0.0;
+    double e = 0.0;
     if (i > 0) {
       const int4 w = WQ[i];
       e = fixed_to_double((long long)w.y << 32 | (unsigned)w.x, w.z);
-      h = w.w ? 1.0 : 0.0;
     }
     E[i] = e;
-    H[i] = h;
+  }
+  // w_i . w_{i-1}, a pair per lane (rows i - 1 and i follow each other)
+  for (int i = 2 * lane + 2; i < n; i += 64) {
+    const int2* const y = reinterpret_cast<const int2*>(U) + (size_t)i * (i - 1) / 2;
+    const int2* const x = y - (i - 1);
+    long long hs = 0, ms = 1 << 27;
+#pragma unroll 8
+    for (int c = 0; c < i - 1; ++c) {
+      const int2 a = x[c], b = y[c];
+      hs += (long long)a.y * b.y;
+      ms += (long long)a.y * b.x;
+      ms += (long long)a.x * b.y;
+    }
+    G[i] = fixed_split(4 * hs + (ms >> 28));
   }
 }
 
