@@ -36,14 +36,14 @@
 //     T + s = L D L^T, G = (T + s)^-1 has G_jj = 1/D_j + L_{j+1}^2 G_{j+1,j+1} and
 //     G_ij = -L_{i+1} G_{i+1,j} above it), then W = Q F Q^T by two reflect_kernel
 //     passes and overline_w = W (W t) / (k - 1) in add_wbar_kernel.  A solve per
-//     unit vector instead made this step 12.9 ms where it is 6.6 (32 768 cubes of
+//     unit vector instead made this step 12.9 ms where it is 6.4 (32 768 cubes of
 //     40 members).
 // The sum over the nodes is kept in 64-bit integers: off the FP64 pipe, and the same
 // in any order, so that a vector may be spread over several lanes (launch_ft) and the
 // result does not depend on how many solves a launch has.
 // Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 55 ms,
 // 129 600 of 64 members 93 -> 23 ms; explicit trans against the accumulating solver
-// (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 8.5 ms.  Faster at
+// (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 8.3 ms.  Faster at
 // every size from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
 #include <limits.h>
@@ -691,16 +691,28 @@ __global__ void __launch_bounds__(32) ft_matrix_kernel(Geometry g, SolveBatch b,
       }
     }
     __syncwarp();
-    for (int j = part; j < nb && j0 + j < nmax; j += kL) {
-      const int pair = sl + slots * j;
-      const double *Gp = G + pair, *Lp = L + pair;
-      double x = 0.0;
+    // two nodes' chains at a time, one read of A for both (32 768 cubes 6.57 -> 6.40
+    // ms); one past the last keeps x = 0
+    const int nn = min(nb, nmax - j0);
+    for (int j = part; j < nn; j += 2 * kL) {
+      const bool two = j + kL < nn;
+      const int p0 = sl + slots * j, p1 = two ? p0 + slots * kL : p0;
+      const double *L0 = L + p0, *L1 = L + p1;
+      const double g0 = G[32 * v + p0], g1 = two ? G[32 * v + p1] : 0.0;
+      double x0 = 0.0, x1 = 0.0;
 #pragma unroll 4
       for (int i = vmax; i >= 0; --i) {
         // above the diagonal x is not begun yet, on it it starts
-        const double step = i < n - 1 ? -Lp[32 * (i + 1)] * x : 0.0;
-        x = i == v ? Gp[32 * i] : step;
-        if (i <= v) ft::add_fixed(A[32 * i], x, Eb);
+        const double s0 = i < n - 1 ? -L0[32 * (i + 1)] * x0 : 0.0;
+        const double s1 = i < n - 1 ? -L1[32 * (i + 1)] * x1 : 0.0;
+        x0 = i == v ? g0 : s0;
+        x1 = i == v ? g1 : s1;
+        if (i <= v) {
+          long long a = A[32 * i];
+          ft::add_fixed(a, x0, Eb);
+          ft::add_fixed(a, x1, Eb);
+          A[32 * i] = a;
+        }
       }
     }
     __syncwarp();
