@@ -476,32 +476,33 @@ __device__ inline void factor(int n, const double* D, const double* E, double si
 // The same elimination from both ends, meeting at element m = n / 2: as many
 // operations in two independent chains of half the length.
 // R is scaled by the node's weight w, which makes the solution w (T + sigma)^-1 y.
+template <int kPW>
 __device__ inline void factor_twisted(int n, const double* D, const double* E, double sigma, double w,
                                       double* R, double* L) {
   const int m = n / 2, nd = n - 1 - m;  // nd elements below m, m >= nd above
   double r = rcp(D[0] + sigma), q = rcp(D[n - 1] + sigma);
   R[0] = w * r;
-  R[32 * (n - 1)] = w * q;
+  R[kPW * (n - 1)] = w * q;
   for (int c = 1; c < nd; ++c) {
     const int b = n - 1 - c;
     const double e = E[c], l = e * r, h = E[b + 1], k = h * q;
     r = rcp(fma(-l, e, D[c] + sigma));
     q = rcp(fma(-k, h, D[b] + sigma));
-    L[32 * c] = l;
-    R[32 * c] = w * r;
-    L[32 * (b + 1)] = k;
-    R[32 * b] = w * q;
+    L[kPW * c] = l;
+    R[kPW * c] = w * r;
+    L[kPW * (b + 1)] = k;
+    R[kPW * b] = w * q;
   }
   if (m > nd) {
     const double e = E[m - 1], l = e * r;
     r = rcp(fma(-l, e, D[m - 1] + sigma));
-    L[32 * (m - 1)] = l;
-    R[32 * (m - 1)] = w * r;
+    L[kPW * (m - 1)] = l;
+    R[kPW * (m - 1)] = w * r;
   }
   const double e = E[m], l = e * r, h = E[m + 1], k = h * q;
-  L[32 * m] = l;
-  L[32 * (m + 1)] = k;
-  R[32 * m] = w * rcp(fma(-k, h, fma(-l, e, D[m] + sigma)));
+  L[kPW * m] = l;
+  L[kPW * (m + 1)] = k;
+  R[kPW * m] = w * rcp(fma(-k, h, fma(-l, e, D[m] + sigma)));
 }
 
 }  // namespace ft
@@ -511,9 +512,9 @@ __device__ inline void factor_twisted(int n, const double* D, const double* E, d
 // rows and t each; a solve of more than 31 rows is spread over `parts` warps, each
 // with a t of its own.
 // Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
-// F (the forward solve), A (the sum over nodes), and for 32 (slot, node) pairs
+// F (the forward solve), A (the sum over nodes), and for kPW (slot, node) pairs
 // the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
-template <int kL>
+template <int kL, int kPW>
 __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
                                                 int rows, int parts, const double* tri,
                                                 int* eig_fail) {
@@ -532,8 +533,8 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
   const int cap = n * 32;
   double *const Y = sm + lane, *const F = Y + cap;
   long long* const A = reinterpret_cast<long long*>(F + cap);  // in units of 2^(top - 62)
-  double *const R = sm + 3 * cap, *const L = R + cap;
-  double* const Dg = L + cap;         // slots x n: diagonal + shift
+  double *const R = sm + 3 * cap, *const L = R + kPW * n;
+  double* const Dg = L + kPW * n;         // slots x n: diagonal + shift
   double* const Eg = Dg + slots * n;  // slots x n: Eg[i] couples i - 1 and i
   __shared__ int s_row[32];
   __shared__ bool s_nan[32];
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
 #pragma unroll 4
     for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
   ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, s_nan, 1, first_row == 0 ? 0 : LLONG_MAX, eig_fail);
-  const int nb = 32 / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
+  const int nb = kPW / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
   int nmax = 0;
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
   const int fs = lane % slots, fj = lane / slots;
@@ -565,15 +566,15 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
     double f = Y[0], h = Y[32 * (n - 1)];
     F[0] = f;
     F[32 * (n - 1)] = h;
-    double lf = Lp[32], yf = Y[32], lh = Lp[32 * (n - 1)], yh = Y[32 * (n - 2)];
+    double lf = Lp[kPW], yf = Y[32], lh = Lp[kPW * (n - 1)], yh = Y[32 * (n - 2)];
 #pragma unroll 4
     for (int c = 1; c < nd; ++c) {
       const int b = n - 1 - c;
       f = fma(-lf, f, yf);
       h = fma(-lh, h, yh);
-      lf = Lp[32 * (c + 1)];
+      lf = Lp[kPW * (c + 1)];
       yf = Y[32 * (c + 1)];
-      lh = Lp[32 * b];
+      lh = Lp[kPW * b];
       yh = Y[32 * (b - 1)];
       F[32 * c] = f;
       F[32 * b] = h;
@@ -582,21 +583,21 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
       f = fma(-lf, f, yf);
       F[32 * (m - 1)] = f;
     }
-    double u = Rp[32 * m] * fma(-Lp[32 * (m + 1)], h, fma(-Lp[32 * m], f, Y[32 * m]));
+    double u = Rp[kPW * m] * fma(-Lp[kPW * (m + 1)], h, fma(-Lp[kPW * m], f, Y[32 * m]));
     ft::add_fixed(A[32 * m], u, Eb);
     double d = u;
     int iu = m - 1, id = m + 1;
-    double lu = Lp[32 * m], gu = Rp[32 * iu] * F[32 * iu];
-    double ld = Lp[32 * id], gd = Rp[32 * id] * F[32 * id];
+    double lu = Lp[kPW * m], gu = Rp[kPW * iu] * F[32 * iu];
+    double ld = Lp[kPW * id], gd = Rp[kPW * id] * F[32 * id];
 #pragma unroll 4
     for (int c = 1; c < nd; ++c) {
       u = fma(-lu, u, gu);
       d = fma(-ld, d, gd);
       const int ju = iu - 1, jd = id + 1;
-      lu = Lp[32 * iu];
-      gu = Rp[32 * ju] * F[32 * ju];
-      ld = Lp[32 * jd];
-      gd = Rp[32 * jd] * F[32 * jd];
+      lu = Lp[kPW * iu];
+      gu = Rp[kPW * ju] * F[32 * ju];
+      ld = Lp[kPW * jd];
+      gd = Rp[kPW * jd] * F[32 * jd];
       ft::add_fixed(A[32 * iu], u, Eb);
       ft::add_fixed(A[32 * id], d, Eb);
       iu = ju;
@@ -605,12 +606,12 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
     u = fma(-lu, u, gu);
     ft::add_fixed(A[32 * iu], u, Eb);
     ft::add_fixed(A[32 * id], fma(-ld, d, gd), Eb);
-    if (m > nd) ft::add_fixed(A[0], fma(-Lp[32], u, Rp[0] * F[0]), Eb);
+    if (m > nd) ft::add_fixed(A[0], fma(-Lp[kPW], u, Rp[0] * F[0]), Eb);
   };
   for (int j0 = 0; j0 < nmax; j0 += nb) {
     if (fs < nsl && fj < nb && j0 + fj < nmax) {
       const double2 node = ft::g_nodes[s_row[fs]][j0 + fj];
-      ft::factor_twisted(n, Dg + fs * n, Eg + fs * n, node.x * shift, node.y * wscale, R + lane,
+      ft::factor_twisted<kPW>(n, Dg + fs * n, Eg + fs * n, node.x * shift, node.y * wscale, R + lane,
                          L + lane);
     }
     __syncwarp();
@@ -863,10 +864,19 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
   with(lf, [&](auto l) {
     constexpr int kL = decltype(l)::value;
     const int sl = 32 / ((rows + 1) * kL);
-    const size_t smem = smem_of(ft_kernel<kL>, 5 * 32 * (size_t)n + 2 * (size_t)sl * n);
     const unsigned grid =
         parts > 1 ? (unsigned)b.nsolves * parts : (unsigned)((b.nsolves + sl - 1) / sl);
-    ft_kernel<kL><<<grid, 32, smem, stream>>>(g, b, z, sl, rows, parts, tri, eig_fail);
+    auto run = [&](auto kernel, int pairs) {
+      const size_t doubles = (3 * 32 + 2 * (size_t)pairs) * n + 2 * (size_t)sl * n;
+      kernel<<<grid, 32, smem_of(kernel, doubles), stream>>>(g, b, z, sl, rows, parts, tri, eig_fail);
+    };
+    // factors of 32 (solve, node) pairs at a time; from 57 members on that leaves an SM
+    // two warps where 16 pairs leave three: 129 600 solves of 64 members 23.4 / 22.4 ms
+    // at 32 / 16, 921 600 of 40 members 55.0 / 61.2
+    if (n > 56)
+      run(ft_kernel<kL, 16>, 16);
+    else
+      run(ft_kernel<kL, 32>, 32);
   });
   reflect(Second(), per - 1, lr);
 }

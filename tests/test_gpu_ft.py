@@ -139,3 +139,10 @@ def test_lanes_per_vector(k, nb):
         _check(cases[i], 1.05, tr[i], wb[i])
     for i in range(3, nb):  # a solve's result does not depend on its place
         assert np.array_equal(tr[i], tr[i % 3]) and np.array_equal(wb[i], wb[i % 3])
+
+
+@pytest.mark.parametrize("name,ens", [("tiny2d", 56), ("tiny2d", 57), ("tiny3d", 57), ("tiny2d", 64)])
+def test_factors_of_half_a_warp(name, ens, monkeypatch):
+    """From 57 members on a warp factors 16 (solve, node) pairs at a time, below
+    32: both sides of the line against the QL route, tolerance as above."""
+    test_analysis_against_the_ql_route(name, ens, monkeypatch)
