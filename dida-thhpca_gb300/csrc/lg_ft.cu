@@ -42,7 +42,7 @@
 // in any order, so that a vector may be spread over several lanes (launch_ft) and the
 // result does not depend on how many solves a launch has.
 // Measured alone against QL + replay: 921 600 solves of 40 members 233 -> 55 ms,
-// 129 600 of 64 members 93 -> 23 ms; explicit trans against the accumulating solver
+// 129 600 of 64 members 93 -> 22 ms; explicit trans against the accumulating solver
 // (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 8.3 ms.  Faster at
 // every size from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
