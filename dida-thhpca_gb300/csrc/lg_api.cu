@@ -1176,13 +1176,13 @@ int prepare_capacity(lg_ctx* c) {
       r |= dalloc(&L.C, cap * k * k);
       r |= dalloc(&L.t, cap * k);
       r |= dalloc(&L.ovf_n, 1);
+      r |= dalloc(&L.ovf_list, cap);
       if (eig2) {
         r |= dalloc(&L.tri, cap * lg::eig2_tri_doubles(k));
         r |= dalloc(&L.lam, cap * k);
         r |= dalloc(&L.rot_cs, (cap * (size_t)c->rot_cap + 1) / 2);  // float2 entries
         r |= dalloc(&L.rot_i, cap * (size_t)c->rot_cap);
         r |= dalloc(&L.rot_n, cap);
-        r |= dalloc(&L.ovf_list, cap);
       }
       if (r != LG_OK) return LG_ERR_NOMEM;
       L.cap = cap;
@@ -1221,6 +1221,7 @@ int prepare_capacity(lg_ctx* c) {
     r |= dalloc(&L.C, cap * k * k);
     r |= dalloc(&L.t, cap * k);
     r |= dalloc(&L.ovf_n, 1);
+    r |= dalloc(&L.ovf_list, cap);
     if (c->use_ft) r |= dalloc(&L.lam, cap * lg::ft_vec_doubles(geo));
     if (c->use_eig2 && !c->use_ft) {
       r |= dalloc(&L.tri, cap * lg::eig2_tri_doubles(k));
@@ -1229,7 +1230,6 @@ int prepare_capacity(lg_ctx* c) {
                                  rot_pairs_per_slot);
       r |= dalloc(&L.rot_i, cap * (size_t)c->rot_cap);
       r |= dalloc(&L.rot_n, cap);
-      r |= dalloc(&L.ovf_list, cap);
     }
     if (r != LG_OK) return LG_ERR_NOMEM;
     L.cap = cap;
@@ -1504,13 +1504,20 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
         CK(record_event(kv[6], st));
         launches += 5;
       } else if (lg::ft_supported(geo)) {
-        lg::launch_tridiag_in_place(k, b.nsolves, L.C, st);
+        CK(cudaMemsetAsync(L.ovf_n, 0, sizeof(int), st));
+        lg::launch_tridiag_in_place(geo, b.nsolves, L.C, L.ovf_list, L.ovf_n, st);
         CK(record_event(kv[3], st));
         for (int e = 4; e < 6; ++e) CK(record_event(kv[e], st));
         lg::launch_ft(geo, b, true, L.t, L.C, c->d_trans, xb, axb, xa, axa, nullptr,
                       c->d_status + 1, st);
+        lg::SolveBatch fb = b;  // spectra beyond the transform's range
+        fb.solve_list = L.ovf_list;
+        fb.solve_count = L.ovf_n;
+        fb.left = 1;
+        lg::launch_eig_apply(geo, fb, L.C, L.t, xb, axb, xa, axa, c->d_trans, nullptr,
+                             c->d_status + 1, st);
         CK(record_event(kv[6], st));
-        launches += 7;
+        launches += 8;
       } else {
         lg::launch_eig_apply(geo, b, L.C, L.t, xb, axb, xa, axa, c->d_trans, nullptr,
                              c->d_status + 1, st);
@@ -1615,7 +1622,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
     }
     CK(record_event(kv[2], s_e));
     if (c->use_ft) {
-      lg::launch_tridiag_in_place(k, b.nsolves, L.C, s_e);
+      lg::launch_tridiag_in_place(geo, b.nsolves, L.C, L.ovf_list, L.ovf_n, s_e);
       CK(record_event(kv[3], s_e));
       CK(record_event(kv[4], s_e));
       if (nl >= 3) {
@@ -1625,7 +1632,13 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
       CK(record_event(kv[5], s_v));
       lg::launch_ft(geo, b, false, L.t, L.C, L.lam, xb, axb, xa, axa, nullptr, c->d_status + 1,
                     s_v);
-      launches += 5;
+      lg::SolveBatch fb = b;  // spectra beyond the transform's range
+      fb.solve_list = L.ovf_list;
+      fb.solve_count = L.ovf_n;
+      fb.left = 1;
+      lg::launch_eig_apply(geo, fb, L.C, L.t, xb, axb, xa, axa, nullptr, nullptr,
+                           c->d_status + 1, s_v);
+      launches += 6;
     } else if (c->use_eig2) {
       if (s_q == s_e) {
         lg::launch_eig2(geo, b, L.C, L.t, xb, axb, xa, axa, L.tri, L.lam, L.rot_cs, L.rot_i,
@@ -2386,12 +2399,13 @@ struct PoolBuf {
   }
 };
 
-// the batched core's kernels on st (C, t: work arrays; *fail: cleared, then the
-// Gram's status or the count of failed eigensolves)
+// The batched core's kernels on st (C, t: work arrays; status: two words, cleared, then
+// the Gram's status or the count of failed eigensolves, and the count of solves left to
+// the eigenvalue route).  left: that route for those solves, after their count was read.
 void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
                   const double* d_hxens, const float* d_rdiaginv, const double* d_dep,
                   const double* d_rloc, double inflation, int precision, double* C, double* t,
-                  int* fail, double* d_trans, double* d_wbar, cudaStream_t st) {
+                  int* status, double* d_trans, double* d_wbar, bool left, cudaStream_t st) {
   Geometry geo{};
   geo.ens = ens;
   geo.inflation = inflation;
@@ -2407,20 +2421,27 @@ void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   b.b_rdiag = d_rdiaginv;
   b.b_dep = d_dep;
   b.b_rloc = d_rloc;
-  cudaMemsetAsync(fail, 0, sizeof(int), st);
+  if (left) {
+    b.left = 1;
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, status,
+                         st);
+    return;
+  }
+  cudaMemsetAsync(status, 0, 2 * sizeof(int), st);
   lg::HxDev hx{};
   lg::ListDev l{};
   if (precision == LG_PREC_MIXED_TF32)
-    lg::launch_gram_tf32(geo, hx, l, b, nullptr, C, t, fail, lg::RecDev{}, st);
+    lg::launch_gram_tf32(geo, hx, l, b, nullptr, C, t, status, lg::RecDev{}, st);
   else if (precision == LG_PREC_MIXED && lg::gram_tc_supported(ens))
-    lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, fail, st);
+    lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, status, st);
   else
-    lg::launch_gram64(geo, hx, l, b, nullptr, lg::ft_supported(geo), C, t, fail, st);
+    lg::launch_gram64(geo, hx, l, b, nullptr, lg::ft_supported(geo), C, t, status, st);
   if (lg::ft_supported(geo)) {
-    lg::launch_tridiag_in_place(ens, nbatch, C, st);
-    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, fail, st);
+    lg::launch_tridiag_in_place(geo, nbatch, C, nullptr, status + 1, st);
+    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, status,
+                  st);
   } else {
-    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, fail,
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, status,
                          st);
   }
 }
@@ -2442,18 +2463,21 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   if (!d_nobsl || !d_off || !d_trans || !d_wbar) return LG_ERR_ARG;
   if (lg::prepare_ft_nodes() != LG_OK) return LG_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream_v;
-  PoolBuf C(st), t(st), fail(st);
+  PoolBuf C(st), t(st), status(st);
   if (C.alloc(sizeof(double) * nbatch * ens * ens) != LG_OK ||
-      t.alloc(sizeof(double) * nbatch * ens) != LG_OK || fail.alloc(sizeof(int)) != LG_OK)
+      t.alloc(sizeof(double) * nbatch * ens) != LG_OK || status.alloc(2 * sizeof(int)) != LG_OK)
     return LG_ERR_NOMEM;
-  enqueue_core(ens, nbatch, d_nobsl, d_off, d_hxens, d_rdiaginv, d_dep, d_rloc, inflation,
-               precision, (double*)C.p, (double*)t.p, (int*)fail.p, d_trans, d_wbar, st);
-  int h_fail = 0;
-  if (cudaGetLastError() != cudaSuccess ||
-      cudaMemcpyAsync(&h_fail, fail.p, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return LG_ERR_CUDA;
-  return core_status(h_fail);
+  int h[2] = {0, 0};
+  for (const bool left : {false, true}) {
+    enqueue_core(ens, nbatch, d_nobsl, d_off, d_hxens, d_rdiaginv, d_dep, d_rloc, inflation,
+                 precision, (double*)C.p, (double*)t.p, (int*)status.p, d_trans, d_wbar, left, st);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(h, status.p, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+      return LG_ERR_CUDA;
+    if (h[0] < 0 || h[1] == 0) break;
+  }
+  return core_status(h[0]);
 }
 
 int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiaginv,
@@ -2495,24 +2519,27 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
   const float* df = (const float*)(dr + p);
   double* const C = (double*)(d + in);
   double* const dt = (double*)(d + in + work);
-  int* const fail = (int*)(dt + k * k + k);
+  int* const status = (int*)(dt + k * k + k);
   if (cudaMemcpyAsync(d, host.data(), n_in, cudaMemcpyHostToDevice, st) != cudaSuccess) {
     cudaGetLastError();
     return LG_ERR_CUDA;
   }
-  enqueue_core(nanals, 1, (const int*)(df + p), (const int64_t*)d, dh, df, dd, dr,
-               inflation_factor, LG_PREC_FP64, C, C + k * k, fail, dt, dt + k * k, st);
-  if (cudaGetLastError() != cudaSuccess ||
-      cudaMemcpyAsync(host.data(), dt, out, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess) {
-    cudaGetLastError();
-    return LG_ERR_CUDA;
+  int h[2] = {0, 0};
+  for (const bool left : {false, true}) {
+    enqueue_core(nanals, 1, (const int*)(df + p), (const int64_t*)d, dh, df, dd, dr,
+                 inflation_factor, LG_PREC_FP64, C, C + k * k, status, dt, dt + k * k, left, st);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(host.data(), dt, out, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
+      cudaGetLastError();
+      return LG_ERR_CUDA;
+    }
+    memcpy(h, host.data() + sizeof(double) * (k * k + k), sizeof h);
+    if (h[0] < 0 || h[1] == 0) break;
   }
   memcpy(trans, host.data(), sizeof(double) * k * k);
   memcpy(overline_w, host.data() + sizeof(double) * k * k, sizeof(double) * k);
-  int h_fail = 0;
-  memcpy(&h_fail, host.data() + sizeof(double) * (k * k + k), sizeof(int));
-  return core_status(h_fail);
+  return core_status(h[0]);
 }
 
 void letkf_core_(const int* nanals, const int* nobsl, const double* hxens, const float* rdiaginv,

@@ -60,6 +60,8 @@ __global__ void __launch_bounds__(NT) eig_apply_kernel(Geometry g, SolveBatch b,
     s = ii;
   }
   const int n = g.ens;
+  const double* C = Cin + (size_t)s * n * n;
+  if (b.left && (unsigned long long)__double_as_longlong(C[1]) != kLeftMark) continue;
   const int LD = n | 1;  // odd row stride
   const int tid = threadIdx.x;
   extern __shared__ double sm[];
@@ -73,10 +75,9 @@ __global__ void __launch_bounds__(NT) eig_apply_kernel(Geometry g, SolveBatch b,
   double* red = x + n;             // 8
   __shared__ int s_fail;
 
-  const double* C = Cin + (size_t)s * n * n;
   for (int idx = tid; idx < n * n; idx += NT) {
-    const int i = idx % n, j = idx / n;  // C column-major
-    a[i * LD + j] = C[idx];
+    const int i = idx % n, j = idx / n;  // C column-major; left: its lower rows only
+    a[i * LD + j] = C[b.left && i > j ? i * n + j : idx];
   }
   for (int i = tid; i < n; i += NT) tv[i] = tin[(size_t)s * n + i];
   if (tid == 0) s_fail = 0;
@@ -362,7 +363,7 @@ void launch_eig_apply(const Geometry& g, const SolveBatch& b, const double* C, c
   const int n = g.ens;
   const int LD = n | 1;
   const size_t smem = sizeof(double) * ((size_t)n * LD + 6 * n + 8);
-  const int grid = b.solve_list ? std::min(b.nsolves, 152 * 6) : b.nsolves;
+  const int grid = b.solve_list || b.left ? std::min(b.nsolves, 152 * 6) : b.nsolves;
   if (n <= 64) {
     // one warp per matrix: the QL rotations are broadcast by shuffles, no block barriers
     cudaFuncSetAttribute(eig_apply_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -60,8 +60,9 @@
 namespace lg {
 namespace ft {
 
-constexpr int kMaxLog = 80;    // M/m up to 2^80
-constexpr int kMaxNodes = 128;  // nodes per row of the table, padded with zero weight
+// M/m up to 2^43: Gershgorin's bound is below 3 |C| + m, |C| at most 2^(kFtLog + 1) m
+constexpr int kMaxLog = kFtLog + 3;
+constexpr int kMaxNodes = 72;  // nodes per row of the table (65 at 2^43), padded with zero weight
 // [log2(M/m)][node]: (s_j / m, w_j / sqrt(m))
 __device__ double2 g_nodes[kMaxLog + 1][kMaxNodes];
 __device__ int g_count[kMaxLog + 1];
@@ -256,6 +257,13 @@ __device__ inline bool to_fixed(double* V, int m, int& ex) {
 
 }  // namespace ft
 
+namespace ft {
+// T of a solve that the reduction left to the eigenvalue route
+__device__ inline bool left_alone(const double* T) {
+  return (unsigned long long)__double_as_longlong(T[1]) == kLeftMark;
+}
+}  // namespace ft
+
 // One vector over kL lanes, one warp per block, lanes numbered through the solves'
 // vectors.  Analysis: y <- Q^T x (kFirst; P_{n-1} first) or Q z (P_1 first) with
 // the rows' update.  Core, W = Q F Q^T: the first pass takes column j of the
@@ -281,6 +289,8 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   const int part = kL == 1 ? 0 : lane % kL, m = ft::own<kL>(n, part);
   const bool mine = id < total;
   const int s = mine ? (int)(id / per) : s_first;
+  // a solve left to the eigenvalue route: its t and its rows stay as they are
+  const bool left = !kCore && ft::left_alone(tri + (size_t)s * n * n);
   const int v = v0 + (mine ? (int)(id - (long long)s * per) : 0);
   extern __shared__ double sm[];
   double* const Y = sm + lane;                      // element part + kL i at 32 i
@@ -330,7 +340,7 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
     const int kk = s % b.levels + 1;
     const int glat = col % g.num_lat + 1, glon = col / g.num_lat + 1;
     ci = (size_t)(glat - 1 + g.halo) + (size_t)(g.num_lat + 2 * g.halo) * (size_t)(glon - 1 + g.halo);
-    if (v >= 1) {
+    if (v >= 1 && !left) {
       if (g.vert_dist <= 0.0)
         r_state = v - 1;
       else if (g.var_lev[v - 1] > 1)
@@ -398,7 +408,7 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   // ---- out
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   if (kFirst || kCore) {
-    if (mine)
+    if (mine && !left)
       for (int i = 0; i < m; ++i)
         out[(size_t)(part + kL * i) * vs] =
             finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
@@ -426,7 +436,8 @@ namespace ft {
 // One warp: T's diagonals of the solves s_first .. + nsl - 1 into Dg (with the
 // shift) and Eg, and each one's row of the node table (Gershgorin in FP32,
 // rounded up).  A non-finite T counts in *eig_fail, as a QL iteration that never
-// converges, if its first vector id is not below id0.
+// converges, if its first vector id is not below id0 (a solve left alone has the mark
+// for its second diagonal element: NaN, but not counted).
 __device__ inline void load_t(int n, const double* tri, int s_first, int nsl, double shift, double* Dg,
                               double* Eg, int* s_row, bool* s_nan, int per, long long id0,
                               int* eig_fail) {
@@ -452,7 +463,7 @@ __device__ inline void load_t(int n, const double* tri, int s_first, int nsl, do
       const int ex = (int)((__float_as_uint(mx * (1.0001f / (float)shift)) >> 23) & 0xffu) - 127 + 1;
       s_row[q] = nf ? 0 : min(max(ex, 1), kMaxLog);
       s_nan[q] = nf;
-      if (nf && (long long)(s_first + q) * per >= id0) atomicAdd(eig_fail, 1);
+      if (nf && (long long)(s_first + q) * per >= id0 && !left_alone(T)) atomicAdd(eig_fail, 1);
     }
   }
   __syncwarp();

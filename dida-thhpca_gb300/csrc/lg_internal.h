@@ -154,6 +154,9 @@ struct SolveBatch {
   // optional: process only the solves listed in solve_list[0 .. *solve_count)
   const int* solve_list;
   const int* solve_count;
+  // eig_apply: only solves that the fixed-point reduction left alone (kLeftMark in the
+  // second element of C, which then holds the lower triangle's rows)
+  int left;
   // mode 0 with cubes: solve s of the batch is solve first_solve + s of the
   // analysis, at centre column s_col[.] and centre level s_kk[.] (1-based);
   // its trans goes to eig_apply's trans output
@@ -289,9 +292,15 @@ size_t eig2_tri_doubles(int n);
 // solve of scratch) or explicit trans and overline_w (core true, as
 // launch_eig_apply's modes 1 and cubes; vec: trans).  t is overwritten.
 // prepare_ft_nodes: the node table, once per device, outside stream captures.
+// The reduction leaves alone a solve whose C is beyond 2^kFtLog times (k - 1) / rho: it
+// marks it and, where given, appends it to list and counts it in *count; launch_ft
+// writes nothing of its own for it, and launch_eig_apply (left) does it afterwards.
+constexpr int kFtLog = 40;
+constexpr unsigned long long kLeftMark = 0x7ff96c6566745f21ull;
 bool ft_supported(const Geometry& g);
 int prepare_ft_nodes();
-void launch_tridiag_in_place(int n, int nsolves, double* C, cudaStream_t stream);
+void launch_tridiag_in_place(const Geometry& g, int nsolves, double* C, int* list, int* count,
+                             cudaStream_t stream);
 size_t ft_vec_doubles(const Geometry& g);
 void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, const double* tri,
                double* vec, const double* xb, const double* axb, double* xa, double* axa,

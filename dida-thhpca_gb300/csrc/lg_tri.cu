@@ -25,12 +25,17 @@
 // place: D[n] | E[n] | G[n] (even i: w_i . w_{i-1}, for the transform, which applies
 // two reflectors at a time) | w rows, zero where there is none (w and G in units of
 // 2^-58 as pairs of 32-bit integers).
-// A non-finite C gives a NaN diagonal, which the transform reports.
+// A non-finite C gives a NaN diagonal, which the transform reports.  A finite one beyond
+// 2^kFtLog times (k - 1) / rho is marked and left for the eigenvalue route: f(T) is
+// formed in units of 2^-62 of sqrt(rho), so a C of full rank would lose half the bits of
+// that ratio, and beyond 2^59 its rounding would reach the shift (k - 1) / rho itself.
 //
 // Measured alone against tridiag_kernel: 921 600 matrices of 40 members 116 ->
 // 52 ms, 129 600 of 64 members 54 -> 27 ms, 2592 of 16 members 81 -> 52 us; a single
 // matrix of 40 members 94 us.  Bound by instruction issue (at 64 members the
 // triangles leave twelve warps per SM).
+#include <math.h>
+
 #include "lg_device.cuh"
 #include "lg_fixed.cuh"
 #include "lg_internal.h"
@@ -77,7 +82,8 @@ __device__ constexpr Elements g_elements{};
 
 }  // namespace tri
 
-__global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, double* C) {
+__global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, int Eb_max, double* C,
+                                                          int* list, int* count) {
   using namespace tri;
   const int s = blockIdx.x;
   if (s >= nsolves) return;
@@ -113,7 +119,15 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
   double* const E = M + n;
   int2* const G = reinterpret_cast<int2*>(M + 2 * n);
   double* const U = M + 3 * n;
-  if (emax == 0 || emax >= 2047u - 8u) {  // all zero, or not representable: NaN
+  auto leave = [&]() {  // to the eigenvalue route: C as it is, marked
+    __syncwarp();
+    if (lane == 0) {
+      M[1] = __longlong_as_double((long long)kLeftMark);
+      const int at = atomicAdd(count, 1);
+      if (list) list[at] = s;
+    }
+  };
+  if (emax == 0 || emax == 2047u) {  // all zero, or not finite: NaN
     __syncwarp();
     for (int i = lane; i < n; i += 32) {
       D[i] = emax ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
@@ -123,6 +137,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
     for (int t = lane; t < n * (n - 1) / 2; t += 32) U[t] = 0.0;
     return;
   }
+  if (emax >= 2047u - 8u) return leave();
   float fro = 0.0f;
   auto rough = [&](int t) {  // mantissa to 20 bits, rounded up, at 2^-d
     const int hi = A[t].y & 0x7fffffff;
@@ -144,6 +159,7 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
   // |C|_F < 2^(emax - 1023) sqrt(fro) 1.001; E = the exponent above
   const int ef = (int)((__float_as_uint(sqrtf(fro) * 1.001f) >> 23) & 0xffu) - 127 + 1;
   const int Eb = (int)emax + ef;  // E + 1023
+  if (Eb > Eb_max) return leave();
   for (int t = lane; t < np; t += 32) {
     const int2 a = A[t];
     const unsigned long long u = (unsigned long long)(unsigned)a.y << 32 | (unsigned)a.x;
@@ -364,11 +380,15 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, d
   }
 }
 
-void launch_tridiag_in_place(int n, int nsolves, double* C, cudaStream_t stream) {
+void launch_tridiag_in_place(const Geometry& g, int nsolves, double* C, int* list, int* count,
+                             cudaStream_t stream) {
   if (nsolves == 0) return;
+  const int n = g.ens;
+  // 2^E beyond 2^kFtLog times the power of two below (k - 1) / rho
+  const int Eb_max = 1023 + ilogb((double)(n - 1) / g.inflation) + kFtLog;
   const size_t smem = sizeof(int4) * n + sizeof(int2) * ((size_t)n * (n + 1) / 2);
   cudaFuncSetAttribute(tridiag_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  tridiag_fixed_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, C);
+  tridiag_fixed_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, Eb_max, C, list, count);
 }
 
 }  // namespace lg

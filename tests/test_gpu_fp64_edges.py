@@ -1,0 +1,94 @@
+"""Edges of the plain-FP64 path: spectra and magnitudes outside its kernels' ranges,
+zero rows, boundaries of the localisation, and what its entry points keep and report.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from test_gpu_ft import _check
+from test_gpu_gram64 import LG_ERR_EIG, _batch, _case, _reference
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("k", [7, 40, 64])
+def test_core_spectra_beyond_the_node_table(k):
+    """Full-rank Gram matrices up to 2^400 times (k - 1) / rho: beyond 2^40 the
+    eigenvalue route answers.  f(T) in units of 2^-62 of sqrt(rho) leaves W some 2^-40 of
+    itself at that line, 1e-12, beside k 2^-53 of the reference; 1e-9 has room for both."""
+    rng = np.random.default_rng(40 + k)
+    cases = []
+    for scale in (2.0 ** 14, 2.0 ** 20, 2.0 ** 45, 2.0 ** 120, 2.0 ** 200):
+        hx = rng.standard_normal((6 * k, k))  # of full rank: the members' mean stays
+        cases.append((hx * scale, np.ones(6 * k, np.float32), rng.standard_normal(6 * k),
+                      rng.uniform(0.5, 1.0, 6 * k)))
+    cases.append(_case(rng, k, 300))
+    st, tr, wb = _batch(cases, 1.05)
+    assert st == 0
+    _check(cases.pop(), 1.05, tr[-1], wb[-1])
+    for c, t, w in zip(cases, tr, wb):
+        lam = np.linalg.eigvalsh((c[0] * c[3][:, None]).T @ c[0])
+        size = np.sqrt((k - 1) / max(lam.min(), (k - 1) / 1.05))  # of W, for this full-rank C
+        t0, w0 = _reference(*c, 1.05)
+        assert np.abs(w - w0).max() <= 1e-9 * max(np.abs(w0).max(), 1e-300)
+        assert np.abs((t - w) - (t0.T - w0[:, None]).T).max() <= 1e-9 * size
+
+
+@pytest.mark.parametrize("name,ens,more", [
+    ("tiny3d", 16, {}), ("tiny3d", 64, {}), ("tiny2d", 8, {}),
+    ("tiny3d", 16, {"cube_n": 2, "cube_nz": 2}), ("tiny3d", 16, {"cube_n": 3, "overlap": 1})])
+def test_analysis_spectra_beyond_the_node_table(name, ens, more, monkeypatch):
+    """Observation errors of 1e-18: every column's Gram matrix is far beyond the table, so
+    the analysis is the accumulating eigenvalue solver's bit for bit -- the solver that a
+    lowered sweep limit with a rotation log of one octet gives (cubes: the limit alone)."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset(name).replace(ens=ens, local_dist=9000.0, vert_dist=3.0 if "3d" in name else -1.0,
+                                  **more)
+    w = synth.make_workload(cfg)
+    w.obs.rinv[:] = 1e36
+    out = []
+    for old in (False, True):
+        if old:
+            monkeypatch.setenv("LETKF_GB300_QL_ITERS", "59")
+            monkeypatch.setenv("LETKF_GB300_ROT_CAP", "8")
+        ctx = lg.Letkf(cfg)
+        ctx.set_obs(w.obs)
+        xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+        st = 0
+        try:
+            ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+        except RuntimeError as e:
+            st = str(e)
+        out.append((xa, axa, st, ctx.stats()["n_eig_fail"]))
+        ctx.letkf_final()
+    assert out[0][2:] == out[1][2:]
+    assert np.array_equal(out[0][0], out[1][0], equal_nan=True)
+    assert np.array_equal(out[0][1], out[1][1], equal_nan=True)
+
+
+def test_spectra_beyond_the_node_table_at_every_core_entry():
+    """lg_letkf_core and lg_core_batch_noalloc answer such a solve as lg_core_batch does, a
+    usual one beside it too."""
+    import torch
+    import letkf_gb300 as lg
+    L = lg.load_library()
+    rng = np.random.default_rng(3)
+    k, p = 24, 150
+    cases = [_case(rng, k, p), (rng.standard_normal((p, k)) * 2.0 ** 45, np.ones(p, np.float32),
+                                rng.standard_normal(p), np.ones(p))]
+    st, tr, wb = _batch(cases, 1.05)
+    assert st == 0
+    for c, t, w in zip(cases, tr, wb):
+        t1, w1 = lg.letkf_core(*c, 1.05)
+        assert np.array_equal(t1, t) and np.array_equal(w1, w)
+    dev = [torch.from_numpy(np.array([p, p], np.int32)).cuda(), torch.tensor([0, p]).cuda()]
+    dev += [torch.from_numpy(np.concatenate([c[i] for c in cases])).cuda() for i in range(4)]
+    outs = [torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((2, k, k), (2, k))]
+    P = lambda x: C.c_void_p(x.data_ptr())  # noqa: E731
+    L.lg_core_batch_noalloc.argtypes = L.lg_core_batch.argtypes
+    assert L.lg_core_batch_noalloc(k, 2, *[P(d) for d in dev], 1.05, 0, P(outs[0]), P(outs[1]),
+                                   None) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(outs[0].cpu().numpy(), tr) and np.array_equal(outs[1].cpu().numpy(), wb)
