@@ -206,7 +206,7 @@ __device__ inline double sum_elements(int m, F f) {
   return c[0];
 }
 
-// a += x in units of 2^(top - 62), for |x| < 2^top, Eb = top + 1022: sums of
+// a += x in units of 2^(top - 62), for |x| < 2^top, Eb = top + 1022 >= 62: sums of
 // the nodes' terms, exact in any order and off the FP64 pipe
 __device__ inline void add_fixed(long long& a, double x, int Eb) {
   const int hi = __double2hiint(x);
@@ -567,7 +567,9 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
     A[32 * i] = 0;
     if (mine) emax = max(emax, ((unsigned)__double2hiint(Y[32 * i]) >> 20) & 0x7ffu);
   }
-  const int top = (int)emax - 1022 + 3 + ft::f_top(g.inflation), Eb = top + 1022;
+  // at least 64, so that add_fixed shifts a zero's leading one out: a vector of zeros
+  // (a state row without spread, t of an empty list) stays exactly zero
+  const int Eb = max((int)emax + 3 + ft::f_top(g.inflation), 64), top = Eb - 1022;
   const int m = n / 2, nd = n - 1 - m;
   auto solve = [&](int pair) {
     // A += w (T + s)^-1 y with the pair's twisted factors: inwards, then outwards

@@ -92,3 +92,24 @@ def test_spectra_beyond_the_node_table_at_every_core_entry():
                                    None) == 0
     torch.cuda.synchronize()
     assert np.array_equal(outs[0].cpu().numpy(), tr) and np.array_equal(outs[1].cpu().numpy(), wb)
+
+
+@pytest.mark.parametrize("name,ens", [("tiny2d", 8), ("tiny3d", 16), ("tiny3d", 64)])
+def test_a_variable_that_is_zero_stays_zero(name, ens):
+    """Members without spread around a zero mean: every term of such a row's analysis is
+    zero, so xa and axa are exactly zero."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset(name).replace(ens=ens)
+    w = synth.make_workload(cfg)
+    rows = slice(0, 1) if cfg.nz == 1 else slice(1 + cfg.nz, 1 + 2 * cfg.nz)  # x, or v
+    w.xb[:, :, rows] = 0.0
+    w.axb[:, :, rows] = 0.0
+    xa, axa = np.full_like(w.xb, np.nan), np.full_like(w.axb, np.nan)
+    ctx = lg.Letkf(cfg)
+    ctx.set_obs(w.obs)
+    ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+    ctx.letkf_final()
+    i = slice(cfg.halo, -cfg.halo)
+    assert not axa[i, i, rows].any()
+    assert not xa[i, i, rows].any()
