@@ -1623,6 +1623,12 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
     CK(record_event(kv[2], s_e));
     if (c->use_ft) {
       lg::launch_tridiag_in_place(geo, b.nsolves, L.C, L.ovf_list, L.ovf_n, s_e);
+      lg::SolveBatch fb = b;  // spectra beyond the transform's range
+      fb.solve_list = L.ovf_list;
+      fb.solve_count = L.ovf_n;
+      fb.left = 1;
+      lg::launch_eig_apply(geo, fb, L.C, L.t, xb, axb, xa, axa, nullptr, nullptr,
+                           c->d_status + 1, s_e);
       CK(record_event(kv[3], s_e));
       CK(record_event(kv[4], s_e));
       if (nl >= 3) {
@@ -1632,12 +1638,6 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
       CK(record_event(kv[5], s_v));
       lg::launch_ft(geo, b, false, L.t, L.C, L.lam, xb, axb, xa, axa, nullptr, c->d_status + 1,
                     s_v);
-      lg::SolveBatch fb = b;  // spectra beyond the transform's range
-      fb.solve_list = L.ovf_list;
-      fb.solve_count = L.ovf_n;
-      fb.left = 1;
-      lg::launch_eig_apply(geo, fb, L.C, L.t, xb, axb, xa, axa, nullptr, nullptr,
-                           c->d_status + 1, s_v);
       launches += 6;
     } else if (c->use_eig2) {
       if (s_q == s_e) {

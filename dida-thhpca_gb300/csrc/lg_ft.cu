@@ -289,8 +289,6 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   const int part = kL == 1 ? 0 : lane % kL, m = ft::own<kL>(n, part);
   const bool mine = id < total;
   const int s = mine ? (int)(id / per) : s_first;
-  // a solve left to the eigenvalue route: its t and its rows stay as they are
-  const bool left = !kCore && ft::left_alone(tri + (size_t)s * n * n);
   const int v = v0 + (mine ? (int)(id - (long long)s * per) : 0);
   extern __shared__ double sm[];
   double* const Y = sm + lane;                      // element part + kL i at 32 i
@@ -340,7 +338,7 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
     const int kk = s % b.levels + 1;
     const int glat = col % g.num_lat + 1, glon = col / g.num_lat + 1;
     ci = (size_t)(glat - 1 + g.halo) + (size_t)(g.num_lat + 2 * g.halo) * (size_t)(glon - 1 + g.halo);
-    if (v >= 1 && !left) {
+    if (v >= 1) {
       if (g.vert_dist <= 0.0)
         r_state = v - 1;
       else if (g.var_lev[v - 1] > 1)
@@ -408,7 +406,7 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
   // ---- out
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   if (kFirst || kCore) {
-    if (mine && !left)
+    if (mine)
       for (int i = 0; i < m; ++i)
         out[(size_t)(part + kL * i) * vs] =
             finite ? fixed_to_double(fixed_join(Yi[32 * i]), ex) : nan;
@@ -426,6 +424,9 @@ __global__ void __launch_bounds__(32) reflect_kernel(Geometry g, SolveBatch b, f
     return x;
   }) / (double)n;
   if (!row) return;
+  // ft_kernel made the rows of a solve left to the eigenvalue route NaN: they stay as that
+  // route wrote them
+  if (!finite && ft::left_alone(tri + (size_t)s * tri_stride)) return;
   double* xo = xa + (size_t)n * (r_state + (size_t)g.n * ci);
   for (int i = 0; i < m; ++i) xo[part + kL * i] = Y[32 * i] - mean;
   if (part == 0) axa[r_state + (size_t)g.n * ci] = mean;
@@ -561,15 +562,14 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
   const int fs = lane % slots, fj = lane / slots;
   const double wscale = sqrt((double)(n - 1) * shift);  // sqrt(k - 1) sqrt(m)
-  // |f(T) y| < 2^top
-  unsigned emax = 0;
+  // |f(T) y| < 2^top.  From 128 on, so that add_fixed shifts a zero's leading one out: a
+  // vector of zeros (a state row without spread, t of an empty list) stays exactly zero.
+  unsigned emax = 128;
   for (int i = 0; i < n; ++i) {
     A[32 * i] = 0;
     if (mine) emax = max(emax, ((unsigned)__double2hiint(Y[32 * i]) >> 20) & 0x7ffu);
   }
-  // at least 64, so that add_fixed shifts a zero's leading one out: a vector of zeros
-  // (a state row without spread, t of an empty list) stays exactly zero
-  const int Eb = max((int)emax + 3 + ft::f_top(g.inflation), 64), top = Eb - 1022;
+  const int top = (int)emax - 1022 + 3 + ft::f_top(g.inflation), Eb = top + 1022;
   const int m = n / 2, nd = n - 1 - m;
   auto solve = [&](int pair) {
     // A += w (T + s)^-1 y with the pair's twisted factors: inwards, then outwards

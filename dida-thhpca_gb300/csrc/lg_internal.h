@@ -292,9 +292,10 @@ size_t eig2_tri_doubles(int n);
 // solve of scratch) or explicit trans and overline_w (core true, as
 // launch_eig_apply's modes 1 and cubes; vec: trans).  t is overwritten.
 // prepare_ft_nodes: the node table, once per device, outside stream captures.
-// The reduction leaves alone a solve whose C is beyond 2^kFtLog times (k - 1) / rho: it
-// marks it and, where given, appends it to list and counts it in *count; launch_ft
-// writes nothing of its own for it, and launch_eig_apply (left) does it afterwards.
+// The reduction leaves alone a solve whose C may be beyond 2^kFtLog times (k - 1) / rho: it
+// marks it, counts it in *count and, where given, appends it to list.  launch_eig_apply
+// (left) does it: before launch_ft with state rows, which overwrites t but not such a
+// solve's rows, after launch_ft with an explicit trans, which overwrites that.
 constexpr int kFtLog = 40;
 constexpr unsigned long long kLeftMark = 0x7ff96c6566745f21ull;
 bool ft_supported(const Geometry& g);

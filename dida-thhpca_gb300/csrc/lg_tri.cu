@@ -25,8 +25,8 @@
 // place: D[n] | E[n] | G[n] (even i: w_i . w_{i-1}, for the transform, which applies
 // two reflectors at a time) | w rows, zero where there is none (w and G in units of
 // 2^-58 as pairs of 32-bit integers).
-// A non-finite C gives a NaN diagonal, which the transform reports.  A finite one beyond
-// 2^kFtLog times (k - 1) / rho is marked and left for the eigenvalue route: f(T) is
+// A non-finite C gives a NaN diagonal, which the transform reports.  A finite one that may
+// be beyond 2^kFtLog times (k - 1) / rho (by its largest element) is marked and left for the eigenvalue route: f(T) is
 // formed in units of 2^-62 of sqrt(rho), so a C of full rank would lose half the bits of
 // that ratio, and beyond 2^59 its rounding would reach the shift (k - 1) / rho itself.
 //
@@ -35,6 +35,8 @@
 // matrix of 40 members 94 us.  Bound by instruction issue (at 64 members the
 // triangles leave twelve warps per SM).
 #include <math.h>
+
+#include <algorithm>
 
 #include "lg_device.cuh"
 #include "lg_fixed.cuh"
@@ -82,7 +84,7 @@ __device__ constexpr Elements g_elements{};
 
 }  // namespace tri
 
-__global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, int Eb_max, double* C,
+__global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, int e_max, double* C,
                                                           int* list, int* count) {
   using namespace tri;
   const int s = blockIdx.x;
@@ -119,16 +121,16 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, i
   double* const E = M + n;
   int2* const G = reinterpret_cast<int2*>(M + 2 * n);
   double* const U = M + 3 * n;
-  auto leave = [&]() {  // to the eigenvalue route: C as it is, marked
+  if (emax == 0 || (int)emax >= e_max) {  // all zero, not finite: NaN, or left alone
     __syncwarp();
-    if (lane == 0) {
-      M[1] = __longlong_as_double((long long)kLeftMark);
-      const int at = atomicAdd(count, 1);
-      if (list) list[at] = s;
+    if (emax && emax < 2047u) {
+      if (lane == 0) {
+        M[1] = __longlong_as_double((long long)kLeftMark);
+        const int at = atomicAdd(count, 1);
+        if (list) list[at] = s;
+      }
+      return;
     }
-  };
-  if (emax == 0 || emax == 2047u) {  // all zero, or not finite: NaN
-    __syncwarp();
     for (int i = lane; i < n; i += 32) {
       D[i] = emax ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
       E[i] = 0.0;
@@ -137,7 +139,6 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, i
     for (int t = lane; t < n * (n - 1) / 2; t += 32) U[t] = 0.0;
     return;
   }
-  if (emax >= 2047u - 8u) return leave();
   float fro = 0.0f;
   auto rough = [&](int t) {  // mantissa to 20 bits, rounded up, at 2^-d
     const int hi = A[t].y & 0x7fffffff;
@@ -159,7 +160,6 @@ __global__ void __launch_bounds__(32) tridiag_fixed_kernel(int n, int nsolves, i
   // |C|_F < 2^(emax - 1023) sqrt(fro) 1.001; E = the exponent above
   const int ef = (int)((__float_as_uint(sqrtf(fro) * 1.001f) >> 23) & 0xffu) - 127 + 1;
   const int Eb = (int)emax + ef;  // E + 1023
-  if (Eb > Eb_max) return leave();
   for (int t = lane; t < np; t += 32) {
     const int2 a = A[t];
     const unsigned long long u = (unsigned long long)(unsigned)a.y << 32 | (unsigned)a.x;
@@ -384,11 +384,12 @@ void launch_tridiag_in_place(const Geometry& g, int nsolves, double* C, int* lis
                              cudaStream_t stream) {
   if (nsolves == 0) return;
   const int n = g.ens;
-  // 2^E beyond 2^kFtLog times the power of two below (k - 1) / rho
-  const int Eb_max = 1023 + ilogb((double)(n - 1) / g.inflation) + kFtLog;
+  // the first biased exponent of an element at which |C|, less than 64 times the largest
+  // element, may be beyond 2^kFtLog (k - 1) / rho, or is not representable
+  const int e_max = std::min(1023 + ilogb((double)(n - 1) / g.inflation) + kFtLog - 6, 2047 - 8);
   const size_t smem = sizeof(int4) * n + sizeof(int2) * ((size_t)n * (n + 1) / 2);
   cudaFuncSetAttribute(tridiag_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  tridiag_fixed_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, Eb_max, C, list, count);
+  tridiag_fixed_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, e_max, C, list, count);
 }
 
 }  // namespace lg
