@@ -347,10 +347,13 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
   if (warp < kPWarps) {
     // ================= weighing warps
     const bool vertical = !batch && g.vert_dist > 0.0;
-    // |al - ln p| beyond this (one part in 2^50 above 2 vert_dist) has z > 2, so
-    // weight zero; compared on the bit pattern, a NaN stays a candidate
-    const long long lim_bits =
-        __double_as_longlong(2.0 * g.vert_dist * (1.0 + 8.8817841970012523e-16));
+    // |al - ln p| / vert_dist rounds to more than 2 exactly where |al - ln p| > 2
+    // vert_dist, and to more than 1 where it is > vert_dist: the sides of the
+    // localisation's boundaries are taken from these, not from the product with the
+    // rounded reciprocal.  Compared on the bit patterns; a NaN stays a candidate.
+    const long long lim_bits = __double_as_longlong(2.0 * g.vert_dist);
+    const long long one_bits = __double_as_longlong(g.vert_dist);
+    // (a product differs by less than two roundings from the quotient)
     const double inv_vd = 1.0 / g.vert_dist;
     int work = 0;
     unsigned nq = 0;  // queues filled so far
@@ -459,7 +462,15 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
           if (q >= qn) continue;
           double x = rl[r];
           if (vertical) {
-            const double z = fabs(dz[r]) * inv_vd;
+            double z = fabs(dz[r]) * inv_vd;
+            if ((unsigned)__double2loint(z) + 4u < 8u) {  // within four roundings of 1 or 2
+              const long long a = __double_as_longlong(fabs(dz[r])), b = __double_as_longlong(z);
+              if (a <= one_bits)
+                z = __longlong_as_double(min(b, 0x3ff0000000000000ll));  // at most 1
+              else if (a <= lim_bits)
+                z = __longlong_as_double(
+                    min(max(b, 0x3ff0000000000001ll), 0x4000000000000000ll));  // in (1, 2]
+            }
             x = x * (g.gc_filter_vertical ? taper_fast(z) : schr(z));
           }
           double w = sqrt((double)rdg[r] * x), d = 0.0;

@@ -113,3 +113,40 @@ def test_a_variable_that_is_zero_stays_zero(name, ens):
     i = slice(cfg.halo, -cfg.halo)
     assert not axa[i, i, rows].any()
     assert not xa[i, i, rows].any()
+
+
+def test_box_localisation_at_exactly_two_scales():
+    """An observation whose |ln p - ln p_e| / vert_dist is exactly 2 belongs to the box
+    (weight 1), and with the next smaller vert_dist it does not.  Twelve levels, each with a
+    vert_dist of half its own distance; with that next one the product with the rounded
+    reciprocal would still be 2 for some."""
+    import torch
+    import letkf_gb300 as lg
+    import synth
+    base = lg.preset("tiny3d").replace(nz=12, gc_filter=0, gc_filter_vertical=0, n_obs=40)
+    w = synth.make_workload(base)
+    w.axb[:, :, 0] = 1e5
+    w.obs.type[:] = 0  # ps: no level search in H(x)
+    w.obs.ph[:] = 2e4
+    w.obs.yo[:] = 1e5 + 500.0
+    a, b, p0, ptop = lg.vertical_coord(base)
+    lev = a * (p0 - ptop) + b * (1e5 - ptop) + ptop
+    dz = (torch.log(torch.from_numpy(0.5 * (lev[:-1] + lev[1:])).cuda())
+          - torch.log(torch.tensor(2e4, dtype=torch.float64, device="cuda"))).abs().cpu().numpy()
+    within = 0
+    for kk in range(base.nz):
+        cfg = base.replace(vert_dist=float(dz[kk] / 2.0))
+        less = np.nextafter(cfg.vert_dist, 0.0)
+        assert dz[kk] / cfg.vert_dist == 2.0 < dz[kk] / less
+        within += dz[kk] * (1.0 / less) <= 2.0
+        out = []
+        for vd in (cfg.vert_dist, less):
+            ctx = lg.Letkf(cfg.replace(vert_dist=float(vd)))
+            ctx.set_obs(w.obs)
+            xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+            ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+            ctx.letkf_final()
+            out.append(axa[1:-1, 1:-1, 1 + kk] - w.axb[1:-1, 1:-1, 1 + kk])
+        assert np.abs(out[0]).max() > 1e-6    # u at this level is analysed from the observations
+        assert np.abs(out[1]).max() < 1e-9    # one rounding further: outside
+    assert within > 0
