@@ -34,8 +34,13 @@ struct SearchArgs {
 // A copy kept by the exact test has ri <= 2; rounding beyond it is clamped.
 __device__ inline double kept_weight(const Geometry& g, const ObsDev& ob, int o, double ccx,
                                      double csx, double cyr, double per_rad) {
-  const double ri =
-      fmin(latlon_angle_pre(ob.dcx[o], ob.dsx[o], ob.dyr[o], ccx, csx, cyr) * per_rad, 2.0);
+  const double angle = latlon_angle_pre(ob.dcx[o], ob.dsx[o], ob.dyr[o], ccx, csx, cyr);
+  double ri = angle * per_rad;
+  // within four roundings of 1 the quotient decides which polynomial it is (they differ by
+  // 6e-7 there)
+  if ((unsigned)__double2loint(ri) + 4u < 8u)
+    ri = __ddiv_rn(__dmul_rn(earth_r4(), angle), g.local_dist);
+  ri = fmin(ri, 2.0);
   return g.gc_filter ? taper_fast(ri) : schr(ri);
 }
 

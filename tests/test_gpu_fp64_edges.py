@@ -150,3 +150,54 @@ def test_box_localisation_at_exactly_two_scales():
         assert np.abs(out[0]).max() > 1e-6    # u at this level is analysed from the observations
         assert np.abs(out[1]).max() < 1e-9    # one rounding further: outside
     assert within > 0
+
+
+@pytest.mark.parametrize("linear", [False, True])
+def test_weights_at_exactly_one_localisation_distance(linear, monkeypatch):
+    """The two polynomials of the taper differ by 6e-7 at ri = 1 (their REAL(4) literals); the
+    side is that of the quotient distance / local_dist, for local_dist within two roundings
+    of the distance of a column from an observation.  The expected distance is formed by the
+    reference's operations with the GPU's cos, sin and acos."""
+    import torch
+    import letkf_gb300 as lg
+    import synth
+    if linear:
+        monkeypatch.setenv("LETKF_GB300_LINEAR_SEARCH", "1")
+    base = lg.preset("tiny2d").replace(n_obs=1)
+    w = synth.make_workload(base)
+    lat, lon = lg.model_grid(base)
+    w.obs.lat[:], w.obs.lon[:] = 12.34375, 100.71875
+    pi = float(np.float32(3.14159274101257324))
+    earth = float(np.float32(6371.393))
+    rad = lambda x: torch.tensor(x / 180.0 * pi, dtype=torch.float64, device="cuda")  # noqa: E731
+    x1, y1 = rad(12.34375), rad(100.71875)
+
+    def taper(ri):
+        if ri > 1.0:
+            rj = (ri / 12.0 - 0.5) * ri + 0.625
+            rj = rj * ri + float(np.float32(1.666667))
+            return (rj * ri - 5.0) * ri + 4.0 - float(np.float32(0.6666667)) / ri
+        rj = (-0.25 * ri + 0.5) * ri + 0.625
+        return (rj * ri - float(np.float32(1.666667))) * (ri * ri) + 1.0
+
+    other = 0
+    for i, j in ((9, 11), (11, 10), (8, 9), (12, 12), (10, 8), (10, 13)):
+        x2, y2 = rad(float(lat[i])), rad(float(lon[j]))
+        v = torch.cos(x1) * torch.cos(x2) * torch.cos(y1 - y2) + torch.sin(x1) * torch.sin(x2)
+        angle = float(torch.acos(v))
+        dist = earth * angle
+        col = j * base.num_lat + i
+        for step in (-2, -1, 0, 1, 2):
+            ld = dist
+            for _ in range(abs(step)):
+                ld = float(np.nextafter(ld, np.inf if step > 0 else 0.0))
+            ctx = lg.Letkf(base.replace(local_dist=ld))
+            ctx.set_obs(w.obs)
+            xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+            ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+            _, rloc = ctx.column_list(col)
+            ctx.letkf_final()
+            assert rloc.size == 1
+            assert abs(rloc[0] - taper(dist / ld)) < 1e-13, (i, j, step)
+            other += (angle * (earth / ld) > 1.0) != (dist / ld > 1.0)
+    assert other > 0  # the product with the rounded reciprocal would take the other side
