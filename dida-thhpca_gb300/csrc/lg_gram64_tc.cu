@@ -648,11 +648,14 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     for (unsigned nq = 0;; ++nq) {
       const int qb = nq % kDepth;
       wait(&m_full[qb], (nq / kDepth) & 1);
-      if (stopped() || s_head[qb].s < 0) break;
+      // the solve is read once: after an expired wait the weighing warps may put -1 here
+      // between two reads, and it indexes b_off
+      const int s = *(volatile const int*)&s_head[qb].s;
+      if (stopped() || s < 0) break;
       const int stages = s_head[qb].stages;
       const int4* const par = q_par(qb);
       const long long* const qd = q_d(qb);
-      const double* const ysrc = batch ? b.b_hx + (size_t)b.b_off[s_head[qb].s] * k : hx.yb;
+      const double* const ysrc = batch ? b.b_hx + (size_t)b.b_off[s] * k : hx.yb;
       uint2 y[kR][4];
       auto load = [&](int st, int r) {
         if (uq[r] < 0) return;
