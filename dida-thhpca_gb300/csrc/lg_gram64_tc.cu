@@ -47,8 +47,8 @@
 //     for its next stage by the MMAs' own time, 2500 cycles);
 //   adding up (8)         finished sums out of tensor memory, C and t.
 // The rows' largest values and the levels' ln p come from small kernels before
-// this one.  Roles meet at mbarriers with bounded waits; the first that runs out
-// raises s_abort, every role leaves its loop and the launch reports
+// this one.  Roles meet at mbarriers with bounded waits (lg_set_wait_limit); the first
+// that runs out raises s_abort, every role leaves its loop and the launch reports
 // LG_ERR_TIMEOUT.
 //
 // Bound: the conversions, about 3000 issue slots of twelve warps a stage, beside
@@ -274,11 +274,12 @@ struct QueueHead {
 
 // kR: units (member, 4 entries) of a stage per converting thread -- 2 up to 48
 // members, 3 above.  kThree: three slices in an operand's 128 rows (up to 40
-// members).
-template <int kR, bool kThree>
+// members).  kLimited: waits end after wait_ns (a clock in the waits of every launch
+// would cost them registers).
+template <int kR, bool kThree, bool kLimited>
 __global__ void __launch_bounds__(g64::kThreads, 1)
-    gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, int lower, double* Cout,
-                     double* tout, int* err) {
+    gram64_tc_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, int lower, long long wait_ns,
+                     double* Cout, double* tout, int* err) {
   using namespace g64;
   using L = Layout<kThree>;
   constexpr int kSlice = L::kSlice, kTileD = L::kTileD, kChunkBytes = L::kChunk,
@@ -335,7 +336,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
   };
   auto q_d = [&](int qb) { return reinterpret_cast<long long*>(q_par(qb) + kQueue); };
   auto wait = [&](uint64_t* bar, uint32_t parity) {
-    if (!s_abort && !tc::mbar_wait(bar, parity)) s_abort = 1;
+    if (!s_abort && !(kLimited ? tc::mbar_wait_ns(bar, parity, wait_ns) : tc::mbar_wait(bar, parity)))
+      s_abort = 1;
     __syncwarp();
   };
   // s_abort, the same for the lanes of a warp
@@ -624,8 +626,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         __syncwarp();
       }
     }
-    // every MMA issued here is complete before tensor memory is given back (the
-    // bounded wait itself, whatever s_abort says)
+    // every MMA issued here is complete before tensor memory is given back (the wait with
+    // its full bound, whatever s_abort says)
     if (n > 0 && !tc::mbar_wait(&m_mma[(n - 1) & 1], ((n - 1) >> 1) & 1)) s_abort = 1;
   }
   } else if (warp < kD0) {
@@ -967,14 +969,19 @@ void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, cons
     level_lnp_kernel<<<(b.nsolves + 127) / 128, 128, 0, stream>>>(g, b, axb, t);
   auto run = [&](auto kernel, int smem) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    kernel<<<grid, g64::kThreads, smem, stream>>>(g, hx, l, b, lower ? 1 : 0, C, t, err);
+    kernel<<<grid, g64::kThreads, smem, stream>>>(g, hx, l, b, lower ? 1 : 0,
+                                                  (long long)g.tc_wait_ns, C, t, err);
   };
+  const bool limited = g.tc_wait_ns > 0;
   if (g.ens <= 40)
-    run(gram64_tc_kernel<2, true>, g64::Layout<true>::kSmem);
+    run(limited ? gram64_tc_kernel<2, true, true> : gram64_tc_kernel<2, true, false>,
+        g64::Layout<true>::kSmem);
   else if (g.ens <= 48)
-    run(gram64_tc_kernel<2, false>, g64::Layout<false>::kSmem);
+    run(limited ? gram64_tc_kernel<2, false, true> : gram64_tc_kernel<2, false, false>,
+        g64::Layout<false>::kSmem);
   else
-    run(gram64_tc_kernel<3, false>, g64::Layout<false>::kSmem);
+    run(limited ? gram64_tc_kernel<3, false, true> : gram64_tc_kernel<3, false, false>,
+        g64::Layout<false>::kSmem);
 }
 
 }  // namespace lg

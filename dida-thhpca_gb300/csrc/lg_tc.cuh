@@ -85,6 +85,23 @@ __device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// the same for at most limit_ns of wall-clock time (test_wait never suspends)
+__device__ inline bool mbar_wait_ns(uint64_t* bar, uint32_t parity, long long limit_ns) {
+  const uint64_t t0 = global_ns();
+  do {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  } while (global_ns() - t0 <= (uint64_t)limit_ns);
+  return false;
+}
+
 __device__ inline void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"

@@ -296,8 +296,9 @@ int lg_gmcore_to_da_device(int ens, int num_lat, int num_lon, int nz, int halo,
                            const double* d_area_cell, double* d_xb, void* stream);
 
 /* Wall-clock limit [ns] of the tensor-core Gram's pipeline waits (the column
- * Gram's mbarrier waits between its producer, converter and MMA warps);
- * 0 restores the default of 2 s.  On expiry a CTA raises LG_ERR_TIMEOUT,
+ * Gram's mbarrier waits between its producer, converter and MMA warps, and the
+ * FP64 Gram's of up to 64 members between its roles);
+ * 0 restores the default of about 2 s.  On expiry a CTA raises LG_ERR_TIMEOUT,
  * waits (with the full bound) for its own MMAs and copies, frees its tensor
  * memory and returns, and the analysis returns LG_ERR_TIMEOUT.  For tests of
  * that path and for diagnosing a stalled device; no reference counterpart. */

@@ -201,3 +201,30 @@ def test_weights_at_exactly_one_localisation_distance(linear, monkeypatch):
             assert abs(rloc[0] - taper(dist / ld)) < 1e-13, (i, j, step)
             other += (angle * (earth / ld) > 1.0) != (dist / ld > 1.0)
     assert other > 0  # the product with the rounded reciprocal would take the other side
+
+
+@pytest.mark.parametrize("name,ens", [("tiny3d", 16), ("small3d", 40), ("tiny3d", 64)])
+def test_wait_limit_reports_timeout_and_context_recovers(name, ens):
+    """A wait limit of 1 ns makes the first wait between the FP64 Gram's roles run out: every
+    role leaves, the issuing warp waits (with its full bound) for its own MMAs, the CTAs free
+    their tensor memory and return, and the analysis reports LG_ERR_TIMEOUT.  With the
+    default limit back the same context's next analysis is a fresh context's bit for bit."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset(name).replace(ens=ens)
+    w = synth.make_workload(cfg)
+    xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+    ctx = lg.Letkf(cfg)
+    ctx.set_obs(w.obs)
+    ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+    want = xa.copy(), axa.copy()
+    ctx.letkf_final()
+    ctx = lg.Letkf(cfg)
+    ctx.set_obs(w.obs)
+    ctx.set_wait_limit(1)
+    with pytest.raises(RuntimeError, match="LG_ERR_TIMEOUT"):
+        ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+    ctx.set_wait_limit(0)
+    ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+    ctx.letkf_final()
+    assert np.array_equal(xa, want[0]) and np.array_equal(axa, want[1])
