@@ -180,6 +180,13 @@ int ql_iter_limit() {
   return e ? std::max(1, atoi(e)) : 60;
 }
 
+// test hook: LETKF_GB300_WAIT_NS=n bounds the core entry points' tensor-core waits as
+// lg_set_wait_limit does an analysis's (which has a context to ask)
+long long core_wait_limit() {
+  const char* e = getenv("LETKF_GB300_WAIT_NS");
+  return e ? std::max(0, atoi(e)) : 0;
+}
+
 template <typename T>
 int dalloc(T** p, size_t n) {
   *p = nullptr;
@@ -2399,9 +2406,12 @@ struct PoolBuf {
   }
 };
 
-// The batched core's kernels on st (C, t: work arrays; status: two words, cleared, then
-// the Gram's status or the count of failed eigensolves, and the count of solves left to
+// The batched core's kernels on st (C, t: work arrays; status: kCoreStatus words, cleared,
+// then the Gram's status, the count of failed eigensolves and the count of solves left to
 // the eigenvalue route).  left: that route for those solves, after their count was read.
+// Words of their own: after an expired wait of the Gram the matrices that it did not
+// write may well count as failed.
+constexpr int kCoreStatus = 3;
 void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
                   const double* d_hxens, const float* d_rdiaginv, const double* d_dep,
                   const double* d_rloc, double inflation, int precision, double* C, double* t,
@@ -2411,6 +2421,7 @@ void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   geo.inflation = inflation;
   geo.vert_dist = -1.0;
   geo.ql_max_iter = ql_iter_limit();
+  geo.tc_wait_ns = core_wait_limit();
   lg::SolveBatch b{};
   b.mode = 1;
   b.nsolves = nbatch;
@@ -2423,11 +2434,11 @@ void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   b.b_rloc = d_rloc;
   if (left) {
     b.left = 1;
-    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, status,
-                         st);
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar,
+                         status + 1, st);
     return;
   }
-  cudaMemsetAsync(status, 0, 2 * sizeof(int), st);
+  cudaMemsetAsync(status, 0, kCoreStatus * sizeof(int), st);
   lg::HxDev hx{};
   lg::ListDev l{};
   if (precision == LG_PREC_MIXED_TF32)
@@ -2437,18 +2448,18 @@ void enqueue_core(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   else
     lg::launch_gram64(geo, hx, l, b, nullptr, lg::ft_supported(geo), C, t, status, st);
   if (lg::ft_supported(geo)) {
-    lg::launch_tridiag_in_place(geo, nbatch, C, nullptr, status + 1, st);
-    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, status,
-                  st);
+    lg::launch_tridiag_in_place(geo, nbatch, C, nullptr, status + 2, st);
+    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar,
+                  status + 1, st);
   } else {
-    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, status,
-                         st);
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar,
+                         status + 1, st);
   }
 }
 
-int core_status(int h_fail) {
-  // negative: a bounded tensor-core wait expired
-  return h_fail < 0 ? LG_ERR_TIMEOUT : h_fail ? LG_ERR_EIG : LG_OK;
+int core_status(const int* h) {
+  // the Gram's word first: negative, a bounded tensor-core wait expired
+  return h[0] < 0 ? LG_ERR_TIMEOUT : h[1] ? LG_ERR_EIG : LG_OK;
 }
 }  // namespace
 
@@ -2465,9 +2476,10 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   cudaStream_t st = (cudaStream_t)stream_v;
   PoolBuf C(st), t(st), status(st);
   if (C.alloc(sizeof(double) * nbatch * ens * ens) != LG_OK ||
-      t.alloc(sizeof(double) * nbatch * ens) != LG_OK || status.alloc(2 * sizeof(int)) != LG_OK)
+      t.alloc(sizeof(double) * nbatch * ens) != LG_OK || 
+      status.alloc(kCoreStatus * sizeof(int)) != LG_OK)
     return LG_ERR_NOMEM;
-  int h[2] = {0, 0};
+  int h[kCoreStatus] = {};
   for (const bool left : {false, true}) {
     enqueue_core(ens, nbatch, d_nobsl, d_off, d_hxens, d_rdiaginv, d_dep, d_rloc, inflation,
                  precision, (double*)C.p, (double*)t.p, (int*)status.p, d_trans, d_wbar, left, st);
@@ -2475,9 +2487,9 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
         cudaMemcpyAsync(h, status.p, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       return LG_ERR_CUDA;
-    if (h[0] < 0 || h[1] == 0) break;
+    if (h[0] < 0 || h[2] == 0) break;
   }
-  return core_status(h[0]);
+  return core_status(h);
 }
 
 int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiaginv,
@@ -2494,7 +2506,7 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
   const size_t p = (size_t)nobsl, k = (size_t)nanals;
   const size_t n_in = 8 + sizeof(double) * p * (k + 2) + sizeof(float) * (p + 1);
   const size_t in = (n_in + 15) & ~(size_t)15, work = sizeof(double) * (k * k + k);
-  const size_t out = sizeof(double) * (k * k + k) + 8;
+  const size_t out = sizeof(double) * (k * k + k) + sizeof(int) * kCoreStatus;
   const cudaStream_t st = nullptr;
   PoolBuf dev(st);
   if (dev.alloc(in + work + out) != LG_OK) return LG_ERR_NOMEM;
@@ -2524,7 +2536,7 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
     cudaGetLastError();
     return LG_ERR_CUDA;
   }
-  int h[2] = {0, 0};
+  int h[kCoreStatus] = {};
   for (const bool left : {false, true}) {
     enqueue_core(nanals, 1, (const int*)(df + p), (const int64_t*)d, dh, df, dd, dr,
                  inflation_factor, LG_PREC_FP64, C, C + k * k, status, dt, dt + k * k, left, st);
@@ -2535,11 +2547,13 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
       return LG_ERR_CUDA;
     }
     memcpy(h, host.data() + sizeof(double) * (k * k + k), sizeof h);
-    if (h[0] < 0 || h[1] == 0) break;
+    if (h[0] < 0 || h[2] == 0) break;
   }
+  const int r = core_status(h);
+  if (r == LG_ERR_TIMEOUT) return r;  // nothing was computed
   memcpy(trans, host.data(), sizeof(double) * k * k);
   memcpy(overline_w, host.data() + sizeof(double) * k * k, sizeof(double) * k);
-  return core_status(h[0]);
+  return r;
 }
 
 void letkf_core_(const int* nanals, const int* nobsl, const double* hxens, const float* rdiaginv,

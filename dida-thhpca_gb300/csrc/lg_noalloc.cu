@@ -78,7 +78,7 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
   if (r != LG_OK) return r;
   double* C = scratch;
   double* t = C + (size_t)nbatch * ens * ens;
-  int* status = reinterpret_cast<int*>(t + (size_t)nbatch * ens);  // two words
+  int* status = reinterpret_cast<int*>(t + (size_t)nbatch * ens);  // as lg_core_batch's
   cudaStream_t st = (cudaStream_t)stream_v;
 
   lg::Geometry geo{};
@@ -97,34 +97,34 @@ extern "C" int lg_core_batch_noalloc(int ens, int nbatch, const int* d_nobsl,
   b.b_rloc = d_rloc;
   lg::HxDev hx{};
   lg::ListDev l{};
-  if (cudaMemsetAsync(status, 0, 2 * sizeof(int), st) != cudaSuccess) return LG_ERR_CUDA;
+  if (cudaMemsetAsync(status, 0, 3 * sizeof(int), st) != cudaSuccess) return LG_ERR_CUDA;
   if (precision == LG_PREC_MIXED && lg::gram_tc_supported(ens))
     lg::launch_gram_tc(geo, hx, l, b, nullptr, C, t, status, st);
   else
     lg::launch_gram64(geo, hx, l, b, nullptr, lg::ft_supported(geo), C, t, status, st);
   auto eigenvalues = [&]() {
-    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar, status,
-                         st);
+    lg::launch_eig_apply(geo, b, C, t, nullptr, nullptr, nullptr, nullptr, d_trans, d_wbar,
+                         status + 1, st);
   };
   if (lg::ft_supported(geo)) {
-    lg::launch_tridiag_in_place(geo, nbatch, C, nullptr, status + 1, st);
-    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar, status,
-                  st);
+    lg::launch_tridiag_in_place(geo, nbatch, C, nullptr, status + 2, st);
+    lg::launch_ft(geo, b, true, t, C, d_trans, nullptr, nullptr, nullptr, nullptr, d_wbar,
+                  status + 1, st);
   } else {
     eigenvalues();
   }
-  int h[2] = {0, 0};
+  int h[3] = {};
   auto read_status = [&]() {
     return cudaGetLastError() == cudaSuccess &&
            cudaMemcpyAsync(h, status, sizeof h, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
            cudaStreamSynchronize(st) == cudaSuccess;
   };
   if (!read_status()) return LG_ERR_CUDA;
-  if (h[0] >= 0 && h[1] > 0) {  // solves that the reduction left to the eigenvalue route
+  if (h[0] >= 0 && h[2] > 0) {  // solves that the reduction left to the eigenvalue route
     b.left = 1;
     eigenvalues();
     if (!read_status()) return LG_ERR_CUDA;
   }
   if (h[0] < 0) return h[0];  // a bounded tensor-core wait expired (LG_ERR_TIMEOUT)
-  return h[0] ? LG_ERR_EIG : LG_OK;
+  return h[1] ? LG_ERR_EIG : LG_OK;
 }

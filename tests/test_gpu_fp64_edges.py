@@ -228,3 +228,31 @@ def test_wait_limit_reports_timeout_and_context_recovers(name, ens):
     ctx.letkf_run(0, w.xb, w.axb, xa, axa)
     ctx.letkf_final()
     assert np.array_equal(xa, want[0]) and np.array_equal(axa, want[1])
+
+
+def test_core_reports_an_expired_wait(monkeypatch):
+    """An expired wait of the Gram is LG_ERR_TIMEOUT however many of the matrices that it left
+    unwritten the transform then finds not to be finite, and lg_letkf_core leaves its
+    outputs alone."""
+    import torch
+    import letkf_gb300 as lg
+    L = lg.load_library()
+    rng = np.random.default_rng(11)
+    cases = [_case(rng, 40, 200) for _ in range(60)]
+    nan = [(np.full_like(c[0], np.nan), *c[1:]) for c in cases]
+    want = _batch(cases, 1.05)
+    st, *_ = _batch(nan, 1.05)  # leaves NaN matrices behind in the core's memory
+    assert st == LG_ERR_EIG
+    monkeypatch.setenv("LETKF_GB300_WAIT_NS", "1")
+    st, *_ = _batch(cases, 1.05)
+    assert st == -11
+    trans, wbar = np.full((40, 40), 7.0), np.full(40, 7.0)
+    hx, rd, dep, rloc = cases[0]
+    P = lambda a, t=C.c_double: a.ctypes.data_as(C.POINTER(t))  # noqa: E731
+    assert L.lg_letkf_core(40, 200, P(hx), P(rd, C.c_float), P(dep), P(rloc), P(trans), P(wbar),
+                           1.05) == -11
+    assert (trans == 7.0).all() and (wbar == 7.0).all()
+    monkeypatch.delenv("LETKF_GB300_WAIT_NS")
+    got = _batch(cases, 1.05)
+    assert got[0] == 0 and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])
+    torch.cuda.synchronize()
