@@ -125,8 +125,11 @@ int prepare_ft_nodes() {
     for (int j = 0; j < ft::kMaxNodes; ++j) nodes[0][j] = nodes[1][j];
     count[0] = count[1];
   }
+  // (a copy from pageable memory may return before its transfer is complete, and a caller's
+  // stream need not wait for the legacy one)
   if (cudaMemcpyToSymbol(ft::g_nodes, nodes, sizeof nodes) != cudaSuccess ||
-      cudaMemcpyToSymbol(ft::g_count, count, sizeof count) != cudaSuccess) {
+      cudaMemcpyToSymbol(ft::g_count, count, sizeof count) != cudaSuccess ||
+      cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
     cudaGetLastError();
     return LG_ERR_CUDA;
   }

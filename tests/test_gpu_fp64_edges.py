@@ -256,3 +256,30 @@ def test_core_reports_an_expired_wait(monkeypatch):
     got = _batch(cases, 1.05)
     assert got[0] == 0 and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])
     torch.cuda.synchronize()
+
+
+def test_first_call_of_a_process_on_a_stream_of_its_own():
+    """The node table is on the device before the first launch that reads it, also where that
+    is on a non-blocking stream, which is not ordered after the upload's: a process's first
+    core call equals its second."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = (
+        "import sys, ctypes as C; sys.path[:0] = [%r, %r]\n"
+        "import torch, letkf_gb300 as lg\n"
+        "L = lg.load_library(); k, nb = 16, 2000\n"
+        "s = torch.cuda.Stream()\n"
+        "n = torch.zeros(nb, dtype=torch.int32).cuda(); off = n.long()\n"
+        "tr = [torch.zeros((nb, k, k), dtype=torch.float64).cuda() for _ in range(2)]\n"
+        "wb = torch.zeros((nb, k), dtype=torch.float64).cuda(); torch.cuda.synchronize()\n"
+        "P = lambda x: C.c_void_p(x.data_ptr())\n"
+        "for t in tr:\n"
+        "    assert L.lg_core_batch(k, nb, P(n), P(off), None, None, None, None, 1.05, 0, P(t), P(wb),\n"
+        "                           C.c_void_p(s.cuda_stream)) == 0\n"
+        "torch.cuda.synchronize()\n"
+        "assert torch.equal(*tr) and abs(float(tr[0][0, 0, 0]) - 1.05 ** 0.5) < 1e-14\n"
+        % (os.path.dirname(here), os.path.join(os.path.dirname(here), "dida-thhpca_gb300")))
+    for _ in range(3):
+        subprocess.run([sys.executable, "-c", code], check=True, timeout=120)
