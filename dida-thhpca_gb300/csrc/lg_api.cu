@@ -155,6 +155,28 @@ struct lg_ctx {
   bool graph_failed = false;
 };
 
+namespace lg {
+void raise_smem_limit(const void* kernel, size_t bytes) {
+  struct Limit {
+    int dev;
+    const void* kernel;
+    size_t bytes;
+  };
+  constexpr int kLimits = 512;  // kernels times devices; beyond, the plain request
+  static Limit limits[kLimits];
+  static int n = 0;
+  static std::mutex mu;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int i = 0;
+  while (i < n && (limits[i].kernel != kernel || limits[i].dev != dev)) ++i;
+  if (i == n && n < kLimits) limits[n++] = Limit{dev, kernel, 0};
+  if (i < n) bytes = limits[i].bytes = std::max(limits[i].bytes, bytes);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+}  // namespace lg
+
 namespace {
 
 #define CK(call)                                                                     \

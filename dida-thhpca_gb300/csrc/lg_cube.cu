@@ -324,7 +324,7 @@ void launch_cube_apply(const Geometry& g, const CubeDev& cd, int nsolves, const 
   auto run = [&](auto kernel, int threads) {
     const size_t batch = 2 * (threads / k);
     const size_t smem = 8 * ((size_t)k * (k + 1) + batch * (((k + 1) & ~1) + k + 3));
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kernel, smem);
     kernel<<<grid, threads, smem, stream>>>(g, cd, trans, xb, axb, xa, axa);
   };
   // Smaller blocks hide the steps between barriers better; above 64 members 128 threads

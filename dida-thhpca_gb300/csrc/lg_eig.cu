@@ -366,13 +366,11 @@ void launch_eig_apply(const Geometry& g, const SolveBatch& b, const double* C, c
   const int grid = b.solve_list || b.left ? std::min(b.nsolves, 152 * 6) : b.nsolves;
   if (n <= 64) {
     // one warp per matrix: the QL rotations are broadcast by shuffles, no block barriers
-    cudaFuncSetAttribute(eig_apply_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    allow_smem(eig_apply_kernel<32>, smem);
     eig_apply_kernel<32><<<grid, 32, smem, stream>>>(g, b, C, t, xb, axb, xa, axa, trans,
                                                           wbar, eig_fail);
   } else {
-    cudaFuncSetAttribute(eig_apply_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    allow_smem(eig_apply_kernel<128>, smem);
     eig_apply_kernel<128><<<grid, 128, smem, stream>>>(g, b, C, t, xb, axb, xa, axa,
                                                             trans, wbar, eig_fail);
   }

@@ -1129,7 +1129,7 @@ void launch_trans(const Geometry& g, const SolveBatch& b, const double* t, const
   if (b.nsolves == 0) return;
   const int nt = ((n + 1 + 31) / 32) * 32;
   const size_t smem = sizeof(float) * (size_t)n * nt;
-  cudaFuncSetAttribute(trans_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(trans_kernel, smem);
   trans_kernel<<<b.nsolves, nt, smem, stream>>>(n, b, t, tri, lam,
                                                 static_cast<const float2*>(rot_cs), rot_i, rot_n,
                                                 rot_cap, sqrt(g.inflation), trans);
@@ -1163,12 +1163,10 @@ void launch_eig2_t(const Geometry& g, const SolveBatch& b, const double* C, cons
     // CTA); LETKF_GB300_TRI_MW=1 takes them for every size (a diagnostic)
     static const bool mw_all = getenv("LETKF_GB300_TRI_MW") != nullptr;
     if (n > 64 || mw_all) {
-      cudaFuncSetAttribute(tridiag_mw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem_t);
+      allow_smem(tridiag_mw_kernel, smem_t);
       tridiag_mw_kernel<<<ns, 32 * kTriWarps, smem_t, stream>>>(n, ns, C, tri, u32);
     } else {
-      cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem_t);
+      allow_smem(tridiag_kernel, smem_t);
       tridiag_kernel<<<ns, 32, smem_t, stream>>>(n, ns, C, tri, u32);
     }
     if (ev_tri) record_event(ev_tri, stream);
@@ -1179,7 +1177,7 @@ void launch_eig2_t(const Geometry& g, const SolveBatch& b, const double* C, cons
     // three QL blocks, or QL blocks and those of the other streams, share an SM
     ql_warps = std::max(1, std::min(ql_warps, (int)(kSmemMax / (3 * sizeof(double) * 64 * n))));
     const size_t smem_q = sizeof(double) * (size_t)ql_warps * 64 * n;
-    cudaFuncSetAttribute(ql_kernel<LT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q);
+    allow_smem(ql_kernel<LT>, smem_q);
     const int ql_blocks = (ns + 32 * ql_warps - 1) / (32 * ql_warps);
     ql_kernel<LT><<<ql_blocks, 32 * ql_warps, smem_q, stream>>>(
         n, ns, (double)(n - 1) / g.inflation, sqrt(g.inflation), tri, lam, rot_cs, rot_i, rot_n,
@@ -1194,8 +1192,7 @@ void launch_eig2_t(const Geometry& g, const SolveBatch& b, const double* C, cons
     const size_t vper = sizeof(VT) * ((size_t)32 * n + (size_t)slots * n);
     const int vwarps = std::max(1, std::min(vec_warps, (int)(kSmemMax / vper)));
     const size_t smem_v = sizeof(VT) * ((size_t)vwarps * 32 * n + (size_t)vwarps * slots * n);
-    cudaFuncSetAttribute(vec_kernel<VT, LT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem_v);
+    allow_smem(vec_kernel<VT, LT>, smem_v);
     const int vblocks = (ns + slots * vwarps - 1) / (slots * vwarps);
     vec_kernel<VT, LT><<<vblocks, 32 * vwarps, smem_v, stream>>>(g, b, t, tri, lam, rot_cs, rot_i,
                                                                  rot_n, rot_cap, xb, axb, xa, axa);

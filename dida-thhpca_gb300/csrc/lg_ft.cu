@@ -815,7 +815,7 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
   };
   auto smem_of = [&](auto kernel, size_t doubles) {
     const size_t smem = sizeof(double) * doubles;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kernel, smem);
     return smem;
   };
   // solves that the vectors of a warp can touch, p to a solve, and warps

@@ -258,7 +258,7 @@ void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const S
     const int G = std::max(1, kGramThreads / NB);
     const size_t red = sizeof(double) * (size_t)(G - 1) * NB * 16;
     const size_t smem = std::max(tile, red);
-    cudaFuncSetAttribute(gram64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(gram64_kernel<1>, smem);
     gram64_kernel<1><<<grid, kGramThreads, smem, stream>>>(g, hx, l, b, axb, C, t, marked);
   } else {
     gram64_kernel<3><<<grid, kGramThreads, tile, stream>>>(g, hx, l, b, axb, C, t, marked);

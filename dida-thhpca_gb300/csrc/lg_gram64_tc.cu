@@ -968,7 +968,7 @@ void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, cons
   if (b.mode == 0 && g.vert_dist > 0.0)
     level_lnp_kernel<<<(b.nsolves + 127) / 128, 128, 0, stream>>>(g, b, axb, t);
   auto run = [&](auto kernel, int smem) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(kernel, smem);
     kernel<<<grid, g64::kThreads, smem, stream>>>(g, hx, l, b, lower ? 1 : 0,
                                                   (long long)g.tc_wait_ns, C, t, err);
   };

@@ -586,11 +586,11 @@ void launch_gram_col(const Geometry& g, const HxDev& hx, const ListDev& l, const
   const int grid = std::min(nitems, ctas > 0 ? ctas : sms);
   if (lean) {
     constexpr int bytes = colk::Layout<2, 2>::kBytes;
-    cudaFuncSetAttribute(gram_col_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    allow_smem(gram_col_kernel<2, 2>, bytes);
     gram_col_kernel<2, 2><<<grid, colk::kThreads, bytes, stream>>>(g, hx, l, b, axb, C, t, err, rec);
   } else {
     constexpr int bytes = colk::Layout<6, 4>::kBytes;
-    cudaFuncSetAttribute(gram_col_kernel<6, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    allow_smem(gram_col_kernel<6, 4>, bytes);
     gram_col_kernel<6, 4><<<grid, colk::kThreads, bytes, stream>>>(g, hx, l, b, axb, C, t, err, rec);
   }
 }

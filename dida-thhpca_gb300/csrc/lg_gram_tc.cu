@@ -309,7 +309,7 @@ void launch_gram_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const 
     launch_gram_tc128(g, hx, l, b, axb, C, t, err, r, stream);
     return;
   }
-  cudaFuncSetAttribute(gram_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(gram_tc_kernel, smem);
   gram_tc_kernel<<<b.nsolves, tc::kThreads, smem, stream>>>(g, hx, l, b, axb, C, t, err, r);
 }
 
@@ -550,8 +550,7 @@ void launch_gram_tc_stream(const Geometry& g, const HxDev& hx, const ListDev& l,
     return;
   }
   const size_t smem = 2 * tc::kStageBytes + 1024;
-  cudaFuncSetAttribute(gram_tc_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+  allow_smem(gram_tc_stream_kernel, smem);
   gram_tc_stream_kernel<<<b.nsolves, tc::kThreads, smem, stream>>>(g, hx, l, b, axb, C, t, err,
                                                                    rec);
 }

@@ -299,7 +299,7 @@ void launch_gram_tc128(const Geometry& g, const HxDev& hx, const ListDev& l, con
                        cudaStream_t stream) {
   if (b.nsolves == 0) return;
   constexpr int smem = t128::kSmem + 1024;
-  cudaFuncSetAttribute(gram_tc128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  allow_smem(gram_tc128_kernel, smem);
   gram_tc128_kernel<<<b.nsolves, t128::kThreads, smem, stream>>>(g, hx, l, b, axb, C, t, err,
                                                                  rec);
 }

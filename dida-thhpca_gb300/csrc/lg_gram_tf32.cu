@@ -289,7 +289,7 @@ void launch_gram_tf32(const Geometry& g, const HxDev& hx, const ListDev& l, cons
                       cudaStream_t stream) {
   if (b.nsolves == 0) return;
   constexpr int smem = tf32k::kSmem + 1024;
-  cudaFuncSetAttribute(gram_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  allow_smem(gram_tf32_kernel, smem);
   gram_tf32_kernel<<<b.nsolves, tf32k::kThreads, smem, stream>>>(g, hx, l, b, axb, C, t, err,
                                                                  rec);
 }

@@ -181,6 +181,15 @@ __host__ __device__ inline void solve_col_level(const SolveBatch& b, int s, int&
 // BF16 hi/lo (LG_PREC_MIXED) or TF32 hi/lo (LG_PREC_MIXED_TF32) contractions
 inline bool mixed_precision(int p) { return p == LG_PREC_MIXED || p == LG_PREC_MIXED_TF32; }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory on the current device.
+// The limit is the process's and is only ever raised: a thread that asked for less
+// between another's request and its launch would make that launch fail.
+void raise_smem_limit(const void* kernel, size_t bytes);
+template <typename K>
+inline void allow_smem(K* kernel, size_t bytes) {
+  raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // kernels (host launchers), all asynchronous on `stream`
 // cand[slot] of every copy slot (slot_obs[slot] = observation of the slot)
 void launch_cell_cands(const ObsDev& o, double obs_polar, const int* slot_obs, int nslots,

@@ -556,8 +556,7 @@ void launch_search_cells(const Geometry& g, const ObsDev& o, const CellIndex& ci
   }
   const int warps = 4;
   const size_t smem = sizeof(unsigned int) * (size_t)warps * ci.bitmap_words;
-  cudaFuncSetAttribute(search_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+  allow_smem(search_cells_kernel, smem);
   const int nc = l.col_list ? l.n_list : ncol;
   if (nc == 0) return;
   search_cells_kernel<<<(nc + warps - 1) / warps, 32 * warps, smem, stream>>>(g, o, ci, l, fill,

@@ -388,7 +388,7 @@ void launch_tridiag_in_place(const Geometry& g, int nsolves, double* C, int* lis
   // element, may be beyond 2^kFtLog (k - 1) / rho, or is not representable
   const int e_max = std::min(1023 + ilogb((double)(n - 1) / g.inflation) + kFtLog - 6, 2047 - 8);
   const size_t smem = sizeof(int4) * n + sizeof(int2) * ((size_t)n * (n + 1) / 2);
-  cudaFuncSetAttribute(tridiag_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(tridiag_fixed_kernel, smem);
   tridiag_fixed_kernel<<<nsolves, 32, smem, stream>>>(n, nsolves, e_max, C, list, count);
 }
 

@@ -283,3 +283,48 @@ def test_first_call_of_a_process_on_a_stream_of_its_own():
         % (os.path.dirname(here), os.path.join(os.path.dirname(here), "dida-thhpca_gb300")))
     for _ in range(3):
         subprocess.run([sys.executable, "-c", code], check=True, timeout=120)
+
+
+def test_core_calls_from_several_threads_and_streams():
+    """Calls of different sizes on four threads, each with its own stream, share the kernels'
+    shared-memory limits and the memory pool and
+    give the results of calls one after another."""
+    import threading
+    import torch
+    import letkf_gb300 as lg
+    L = lg.load_library()
+    rng = np.random.default_rng(77)
+    jobs = []
+    for k, nb in ((40, 300), (64, 40), (9, 900), (96, 60)):
+        base = [_case(rng, k, p) for p in (0, 5, 3 * k)]
+        cases = [base[i % 3] for i in range(nb)]
+        want = _batch(cases, 1.05)
+        n = np.array([c[0].shape[0] for c in cases], np.int32)
+        off = np.concatenate([[0], np.cumsum(n)[:-1]]).astype(np.int64)
+        dev = [torch.from_numpy(a).cuda() for a in (n, off)]
+        dev += [torch.from_numpy(np.concatenate([c[i] for c in cases])).cuda() for i in range(4)]
+        outs = [torch.zeros((nb, k, k), dtype=torch.float64, device="cuda"),
+                torch.zeros((nb, k), dtype=torch.float64, device="cuda")]
+        jobs.append((k, nb, dev, outs, want, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    P = lambda x: C.c_void_p(x.data_ptr())  # noqa: E731
+    bad = []
+
+    def work(k, nb, dev, outs, want, s):
+        torch.cuda.set_device(0)
+        for _ in range(20):
+            st = L.lg_core_batch(k, nb, *[P(d) for d in dev], 1.05, 0, P(outs[0]), P(outs[1]),
+                                 C.c_void_p(s.cuda_stream))
+            if st != 0:
+                bad.append((k, st))
+                return
+            with torch.cuda.stream(s):
+                got = [o.cpu().numpy() for o in outs]
+            if not all(np.array_equal(a, b) for a, b in zip(got, want[1:])):
+                bad.append(k)
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
