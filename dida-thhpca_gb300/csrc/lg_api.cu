@@ -2379,8 +2379,8 @@ void lg_destroy(lg_ctx* c) {
 namespace {
 // Device memory of the core entry points (one call's Gram matrices, projections
 // and, for lg_letkf_core, its arrays): a stream-ordered pool per device that
-// keeps up to kPoolKeep bytes between calls and returns the rest to the device
-// when a stream is synchronised.  The runtime makes it safe for several threads
+// keeps up to kPoolKeep bytes between calls; a call after which it holds more returns
+// the rest to the device (PoolCall).  The runtime makes it safe for several threads
 // and streams.  (A cudaMalloc and cudaFree pair per array cost 0.3 ms of a 0.57 ms
 // single-column call.)
 constexpr uint64_t kPoolKeep = (uint64_t)64 << 20;
@@ -2425,6 +2425,24 @@ struct PoolBuf {
   }
   ~PoolBuf() {
     if (p && cudaFreeAsync(p, st) != cudaSuccess) cudaGetLastError();
+  }
+};
+// Declared before a call's buffers, so that it ends after them: what the pool holds beyond
+// kPoolKeep goes back once the buffers' frees are through (a call that was synchronised
+// before it freed them would leave its whole workspace reserved).
+struct PoolCall {
+  cudaStream_t st;
+  explicit PoolCall(cudaStream_t s) : st(s) {}
+  PoolCall(const PoolCall&) = delete;
+  ~PoolCall() {
+    const cudaMemPool_t pool = core_pool();
+    uint64_t held = 0;
+    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) ==
+                    cudaSuccess && held <= kPoolKeep)
+      return;
+    if (!pool || cudaStreamSynchronize(st) != cudaSuccess ||
+        cudaMemPoolTrimTo(pool, kPoolKeep) != cudaSuccess)
+      cudaGetLastError();
   }
 };
 
@@ -2496,6 +2514,7 @@ int lg_core_batch(int ens, int nbatch, const int* d_nobsl, const int64_t* d_off,
   if (!d_nobsl || !d_off || !d_trans || !d_wbar) return LG_ERR_ARG;
   if (lg::prepare_ft_nodes() != LG_OK) return LG_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream_v;
+  PoolCall call(st);
   PoolBuf C(st), t(st), status(st);
   if (C.alloc(sizeof(double) * nbatch * ens * ens) != LG_OK ||
       t.alloc(sizeof(double) * nbatch * ens) != LG_OK || 
@@ -2530,6 +2549,7 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
   const size_t in = (n_in + 15) & ~(size_t)15, work = sizeof(double) * (k * k + k);
   const size_t out = sizeof(double) * (k * k + k) + sizeof(int) * kCoreStatus;
   const cudaStream_t st = nullptr;
+  PoolCall call(st);
   PoolBuf dev(st);
   if (dev.alloc(in + work + out) != LG_OK) return LG_ERR_NOMEM;
   std::vector<unsigned char> host(std::max(n_in, out));

@@ -328,3 +328,25 @@ def test_core_calls_from_several_threads_and_streams():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_core_workspace_is_given_back():
+    """A call that needed more than the pool keeps (64 MiB) returns the rest to the device
+    before it returns itself."""
+    import torch
+    import letkf_gb300 as lg
+    L = lg.load_library()
+    k, nb = 64, 8192  # 276 MB of workspace
+    n = torch.zeros(nb, dtype=torch.int32, device="cuda")
+    off = torch.zeros(nb, dtype=torch.int64, device="cuda")
+    tr = torch.zeros((nb, k, k), dtype=torch.float64, device="cuda")
+    wb = torch.zeros((nb, k), dtype=torch.float64, device="cuda")
+    P = lambda x: C.c_void_p(x.data_ptr())  # noqa: E731
+    s = torch.cuda.Stream()
+    for stream in (None, C.c_void_p(s.cuda_stream)):
+        for count in (64, nb):  # the small call first: kernels loaded, pool begun
+            before = torch.cuda.mem_get_info()[0]
+            assert L.lg_core_batch(k, count, P(n), P(off), None, None, None, None, 1.05, 0, P(tr),
+                                   P(wb), stream) == 0
+            held = before - torch.cuda.mem_get_info()[0]
+        assert held <= 72 << 20
