@@ -29,6 +29,9 @@
 
 using lg::Geometry;
 
+// default Gram workspace per chunk of solves [MiB] (more above 104 members, lg_create)
+constexpr int kChunkMb = 1024;
+
 struct lg_ctx {
   lg_config cfg;
   int dev = 0;
@@ -102,7 +105,8 @@ struct lg_ctx {
   double lnp_span = 1.0;
   int boff_nb = 0;  // bucket count d_boff was sized for
   // launch shapes and bucket boundaries (lg_set_tuning / lg_autotune)
-  lg_tuning tune{1024, LG_GRAM_AUTO, 512, 2, 4, 4, 0, 0.0};
+  lg_tuning tune{kChunkMb, LG_GRAM_AUTO, 512, 2, 4, 4, 0, 0.0};
+  bool chunk_default = true;  // tune.chunk_mb is not the caller's
   // status words: [0] err, [1] eig_fail, [2] nobsl_max, [3] n_capped
   int* d_status = nullptr;
   unsigned long long* d_band = nullptr;
@@ -558,8 +562,10 @@ int lg_create(lg_ctx** out, const lg_config* cfg) {
   // than 384 warps takes as long as a full one.  1 GiB of Gram matrices holds that many
   // solves up to 104 members; above, the workspace grows to hold them.  128 members,
   // 36 864 solves, on the default streams: 206 .. 214 ms at 1024 MiB (8192 solves), 188
-  // at 1536 (12 288), 187 .. 202 at 2048 and 3072.
-  c->tune.chunk_mb = std::max(1024, (int)((12288 * 8 * (size_t)g.ens * g.ens + (1 << 20) - 1) >> 20));
+  // at 1536 (12 288), 187 .. 202 at 2048 and 3072.  The four buffer sets then hold 35
+  // instead of 23 GB in mixed precision, 54 instead of 36 in FP64; prepare_capacity goes
+  // back to 1 GiB where they do not fit.
+  c->tune.chunk_mb = std::max(kChunkMb, (int)((12288 * 8 * (size_t)g.ens * g.ens + (1 << 20) - 1) >> 20));
   c->vec64 = getenv("LETKF_GB300_VEC64") != nullptr;
   if (lg::prepare_ft_nodes() != LG_OK) {
     delete c;
@@ -1034,6 +1040,13 @@ float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
 // groups (cube_nz levels on the vertical path, :431-436): the centre column
 // ((sj + ej) / 2, (si + ei) / 2) and centre level ((sk + ek) / 2) of every solve.
 // Fixed by the grid and configuration, so built once per context.
+void free_lane(lg_ctx::SolveLane& L) {
+  dfree(L.C); dfree(L.t); dfree(L.tri); dfree(L.lam); dfree(L.rot_cs); dfree(L.rot_i);
+  dfree(L.rot_n); dfree(L.ovf_list); dfree(L.ovf_n);
+  L.cap = 0;
+  L.rot_n_cap = 0;
+}
+
 // mixed precision cube solves form their trans in FP32 from the tridiagonal
 // form and the QL rotation log (trans_kernel); FP64 ones with eig_apply
 bool cube_trans_fp32(const lg_ctx* c) {
@@ -1089,7 +1102,7 @@ int build_cube_plan(lg_ctx* c) {
   return LG_OK;
 }
 
-int prepare_capacity(lg_ctx* c) {
+int prepare_capacity_once(lg_ctx* c) {
   if (c->capacity_ready) return LG_OK;
   const lg_config& g = c->cfg;
   const Geometry& geo = c->geo;
@@ -1197,10 +1210,7 @@ int prepare_capacity(lg_ctx* c) {
     for (int li = 0; li < 2; ++li) {
     lg_ctx::SolveLane& L = c->lane[li];
     if (L.cap < (size_t)c->cube_cs || L.rot_n_cap != (eig2 ? (size_t)c->rot_cap : 0)) {
-      dfree(L.C); dfree(L.t); dfree(L.tri); dfree(L.lam); dfree(L.rot_cs); dfree(L.rot_i);
-      dfree(L.rot_n); dfree(L.ovf_list); dfree(L.ovf_n);
-      L.cap = 0;
-      L.rot_n_cap = 0;
+      free_lane(L);
       const size_t cap = (size_t)c->cube_cs;
       r |= dalloc(&L.C, cap * k * k);
       r |= dalloc(&L.t, cap * k);
@@ -1241,10 +1251,7 @@ int prepare_capacity(lg_ctx* c) {
     lg_ctx::SolveLane& L = c->lane[li];
     const size_t cap = li < nl ? (size_t)c->chunk * levels : 0;
     if (L.cap >= cap && (cap > 0 || L.cap == 0) && L.rot_n_cap == (size_t)c->rot_cap) continue;
-    dfree(L.C); dfree(L.t); dfree(L.tri); dfree(L.lam); dfree(L.rot_cs); dfree(L.rot_i);
-    dfree(L.rot_n); dfree(L.ovf_list); dfree(L.ovf_n);
-    L.cap = 0;
-    L.rot_n_cap = 0;
+    free_lane(L);
     if (cap == 0) continue;
     int r = LG_OK;
     r |= dalloc(&L.C, cap * k * k);
@@ -1272,6 +1279,20 @@ int prepare_capacity(lg_ctx* c) {
   }
   c->capacity_ready = true;
   return LG_OK;
+}
+
+// The default chunk above 104 members asks for more workspace than 1 GiB of Gram matrices
+// does; where that cannot be had, the context goes on with 1 GiB.  A chunk size that the
+// caller chose is not changed.
+int prepare_capacity(lg_ctx* c) {
+  int r = prepare_capacity_once(c);
+  if (r == LG_ERR_NOMEM && c->chunk_default && c->tune.chunk_mb > kChunkMb &&
+      !getenv("LETKF_GB300_CHUNK_MB")) {
+    for (lg_ctx::SolveLane& L : c->lane) free_lane(L);
+    c->tune.chunk_mb = kChunkMb;
+    r = prepare_capacity_once(c);
+  }
+  return r;
 }
 
 // Host arrays of lg_run whose copies are part of the captured analysis (all
@@ -2138,6 +2159,7 @@ int lg_set_tuning(lg_ctx* c, const lg_tuning* t) {
       t->ql_warps < 1 || t->ql_warps > 6 || t->vec_warps < 1 || t->vec_warps > 8 ||
       t->solve_streams < 1 || t->solve_streams > 4 || t->gram_ctas < 0 || t->gram_ctas > 4096)
     return LG_ERR_ARG;
+  if (t->chunk_mb != c->tune.chunk_mb) c->chunk_default = false;
   c->tune = *t;
   c->capacity_ready = false;  // chunk size and bucket count size buffers
   drop_graph(c);
@@ -2157,7 +2179,7 @@ int lg_autotune(lg_ctx* c, const double* xb, const double* axb, double* xa, doub
                       : cur.solve_streams >= 3          ? LG_GRAM_COLUMN_LEAN
                                                         : LG_GRAM_COLUMN;
   // one untimed analysis (buffer sizing, graph capture), then the faster of two
-  auto measure = [&](const lg_tuning& t, double* ms) -> int {
+  auto measure = [&](lg_tuning& t, double* ms) -> int {
     int r = lg_set_tuning(c, &t);
     if (r != LG_OK) return r;
     if ((r = lg_run_device(c, 0, xb, axb, xa, axa, stream)) != LG_OK) return r;
@@ -2166,12 +2188,15 @@ int lg_autotune(lg_ctx* c, const double* xb, const double* axb, double* xa, doub
       if ((r = lg_run_device(c, 0, xb, axb, xa, axa, stream)) != LG_OK) return r;
       m = std::min(m, c->stats.ms_total);
     }
+    t.chunk_mb = c->tune.chunk_mb;  // 1 GiB where the default did not fit
     *ms = m;
     return LG_OK;
   };
   double best_ms = 0.0;
   int r = measure(cur, &best_ms);
   if (r != LG_OK) return r;
+  const bool chunk_default = c->chunk_default;
+  const int chunk_mb = cur.chunk_mb;
   auto try_param = [&](int lg_tuning::*field, std::initializer_list<int> cands) -> int {
     for (int v : cands) {
       if (cur.*field == v) continue;
@@ -2212,6 +2237,7 @@ int lg_autotune(lg_ctx* c, const double* xb, const double* axb, double* xa, doub
 
   cur.ms = best_ms;
   if ((r = lg_set_tuning(c, &cur)) != LG_OK) return r;
+  c->chunk_default = chunk_default && cur.chunk_mb == chunk_mb;
   // leave the context sized and captured for the chosen settings
   if ((r = lg_run_device(c, 0, xb, axb, xa, axa, stream)) != LG_OK) return r;
   *best = cur;
@@ -2357,8 +2383,7 @@ void lg_destroy(lg_ctx* c) {
   dfree(c->lists.capped);
   if (c->d_scan_tmp) cudaFree(c->d_scan_tmp);
   for (auto& L : c->lane) {
-    dfree(L.C); dfree(L.t); dfree(L.tri); dfree(L.lam); dfree(L.rot_cs); dfree(L.rot_i);
-    dfree(L.rot_n); dfree(L.ovf_list); dfree(L.ovf_n);
+    free_lane(L);
   }
   dfree(c->d_status); dfree(c->d_band);
   dfree(c->d_rec); dfree(c->d_boff);

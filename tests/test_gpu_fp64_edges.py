@@ -350,3 +350,34 @@ def test_core_workspace_is_given_back():
                                    P(wb), stream) == 0
             held = before - torch.cuda.mem_get_info()[0]
         assert held <= 72 << 20
+
+
+def test_default_chunk_falls_back_to_one_gib(monkeypatch):
+    """Above 104 members the default chunk is larger than 1 GiB of Gram matrices; where its
+    workspace cannot be had, the analysis runs in chunks of 1 GiB as before.  At 128 members
+    12 288 solves need 4.8 GB of rotation log per stream, 8192 need 3.2: 4000 MiB lies between."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset("tiny3d").replace(ens=128, num_lat=24, num_lon=48, nz=12,
+                                      precision=lg.LG_PREC_MIXED)  # 13 824 solves
+    w = synth.make_workload(cfg)
+    out = []
+    for limited in (False, True):
+        ctx = lg.Letkf(cfg)
+        assert ctx.tuning()["chunk_mb"] > 1024
+        ctx.set_obs(w.obs)
+        if limited:
+            monkeypatch.setenv("LETKF_GB300_ALLOC_LIMIT_MB", "4000")
+        else:
+            ctx.set_tuning(chunk_mb=1024)
+        xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+        ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+        out.append((xa, axa, ctx.stats()["n_chunks"]))
+        assert ctx.tuning()["chunk_mb"] == 1024
+        if limited:  # a chunk size that the caller asked for is not changed
+            ctx.set_tuning(chunk_mb=1536)
+            with pytest.raises(RuntimeError, match="LG_ERR_NOMEM"):
+                ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+        ctx.letkf_final()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert out[0][2] == out[1][2] == 2
