@@ -21,7 +21,9 @@
 #include <initializer_list>
 
 #include <algorithm>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -2577,9 +2579,12 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
   PoolCall call(st);
   PoolBuf dev(st);
   if (dev.alloc(in + work + out) != LG_OK) return LG_ERR_NOMEM;
-  std::vector<unsigned char> host(std::max(n_in, out));
+  // (no exception may leave a C entry point)
+  const std::unique_ptr<unsigned char[]> host(new (std::nothrow)
+                                                  unsigned char[std::max(n_in, out)]);
+  if (!host) return LG_ERR_NOMEM;
   {
-    unsigned char* h = host.data();
+    unsigned char* h = host.get();
     const int64_t zero = 0;
     auto put = [&](const void* src, size_t bytes) {
       if (bytes) memcpy(h, src, bytes);
@@ -2599,7 +2604,7 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
   double* const C = (double*)(d + in);
   double* const dt = (double*)(d + in + work);
   int* const status = (int*)(dt + k * k + k);
-  if (cudaMemcpyAsync(d, host.data(), n_in, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+  if (cudaMemcpyAsync(d, host.get(), n_in, cudaMemcpyHostToDevice, st) != cudaSuccess) {
     cudaGetLastError();
     return LG_ERR_CUDA;
   }
@@ -2608,18 +2613,18 @@ int lg_letkf_core(int nanals, int nobsl, const double* hxens, const float* rdiag
     enqueue_core(nanals, 1, (const int*)(df + p), (const int64_t*)d, dh, df, dd, dr,
                  inflation_factor, LG_PREC_FP64, C, C + k * k, status, dt, dt + k * k, left, st);
     if (cudaGetLastError() != cudaSuccess ||
-        cudaMemcpyAsync(host.data(), dt, out, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaMemcpyAsync(host.get(), dt, out, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
       cudaGetLastError();
       return LG_ERR_CUDA;
     }
-    memcpy(h, host.data() + sizeof(double) * (k * k + k), sizeof h);
+    memcpy(h, host.get() + sizeof(double) * (k * k + k), sizeof h);
     if (h[0] < 0 || h[2] == 0) break;
   }
   const int r = core_status(h);
   if (r == LG_ERR_TIMEOUT) return r;  // nothing was computed
-  memcpy(trans, host.data(), sizeof(double) * k * k);
-  memcpy(overline_w, host.data() + sizeof(double) * k * k, sizeof(double) * k);
+  memcpy(trans, host.get(), sizeof(double) * k * k);
+  memcpy(overline_w, host.get() + sizeof(double) * k * k, sizeof(double) * k);
   return r;
 }
 

@@ -381,3 +381,36 @@ def test_default_chunk_falls_back_to_one_gib(monkeypatch):
         ctx.letkf_final()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2] == 2
+
+
+def test_letkf_core_without_host_memory():
+    """lg_letkf_core's host staging block cannot be had (a data limit of the process below
+    its 200 MB): LG_ERR_NOMEM, the process goes on, and with the limit lifted the same call
+    works."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = (
+        "import sys, resource; sys.path[:0] = [%r, %r]\n"
+        "import numpy as np, torch, letkf_gb300 as lg\n"
+        "rng = np.random.default_rng(0)\n"
+        "def case(p, k=64):\n"
+        "    return rng.standard_normal((p, k)), np.ones(p, np.float32), np.ones(p), np.ones(p)\n"
+        "small, big = case(100), case(400_000)\n"
+        "lg.letkf_core(*small, 1.05)\n"
+        "data = [int(l.split()[1]) for l in open('/proc/self/status') if l.startswith('VmData')][0]\n"
+        "lim = resource.getrlimit(resource.RLIMIT_DATA)\n"
+        "resource.setrlimit(resource.RLIMIT_DATA, ((data << 10) + (64 << 20), lim[1]))\n"
+        "try:\n"
+        "    lg.letkf_core(*big, 1.05); st = 'no error'\n"
+        "except RuntimeError as e:\n"
+        "    st = str(e)\n"
+        "resource.setrlimit(resource.RLIMIT_DATA, lim)\n"
+        "t, w = lg.letkf_core(*big, 1.05)\n"
+        "assert np.isfinite(t).all() and np.isfinite(w).all()\n"
+        "print(st)\n"
+        % (os.path.dirname(here), os.path.join(os.path.dirname(here), "dida-thhpca_gb300")))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-500:]
+    assert "LG_ERR_NOMEM" in r.stdout
