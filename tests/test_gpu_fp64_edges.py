@@ -414,3 +414,24 @@ def test_letkf_core_without_host_memory():
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr[-500:]
     assert "LG_ERR_NOMEM" in r.stdout
+
+
+def test_entries_of_solves_redone_in_fp64_count_once():
+    """Ensemble rows below 2^-400 send every solve to the FP64 kernel; lg_stats counts its
+    entries once."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset("tiny2d").replace(ens=16)
+    w = synth.make_workload(cfg)
+    n = []
+    for scale in (1.0, 2.0 ** -450):
+        ctx = lg.Letkf(cfg)
+        ctx.set_obs(w.obs)
+        xb, axb = w.xb * scale, w.axb * 0.0  # (a mean would round the spread away in H(x))
+        xa, axa = np.zeros_like(xb), np.zeros_like(axb)
+        ctx.letkf_run(0, xb, axb, xa, axa)
+        yb, _ = ctx.hx(ctx.stats()["n_entries"])
+        n.append(ctx.stats()["n_gram_entries"])
+        ctx.letkf_final()
+        assert 0.0 < np.abs(yb).max() < 100.0 * scale
+    assert n[0] > 0 and n[0] == n[1]
