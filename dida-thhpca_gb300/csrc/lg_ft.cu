@@ -46,7 +46,6 @@
 // (lg_eig.cu), with the reduction: 32 768 cubes of 40 members 133 -> 8.3 ms.  Faster at
 // every size from 7 to 64 members; above, five arrays leave an SM one warp.
 #include <float.h>
-#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
@@ -523,27 +522,23 @@ __device__ inline void factor_twisted(int n, const double* D, const double* E, d
 }  // namespace ft
 
 // f(T) y per lane, one warp per block: t gives sqrt(k-1) T^(-1/2) y, the rows
-// (f(T) - sqrt(rho)) y and overline_w . x.  A warp takes `slots` solves with `rows`
-// rows and t each; a solve of more than 31 rows is spread over `parts` warps, each
-// with a t of its own.
+// (f(T) - sqrt(rho)) y and overline_w . x.  A warp takes `slots` solves, each with t and
+// its rows (at most 15: solves of more rows take the eigenvalue route, eig2_supported).
 // Shared memory, [element][lane] so that lanes never conflict: Y (the vector),
 // F (the forward solve), A (the sum over nodes), and for kPW (slot, node) pairs
 // the reciprocal pivots R and multipliers L of T + s; T's diagonals per slot.
 template <int kL, int kPW>
 __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Vecs z, int slots,
-                                                int rows, int parts, const double* tri,
-                                                int* eig_fail) {
+                                                const double* tri, int* eig_fail) {
   const int n = g.ens;
   const int lane = threadIdx.x;
-  const int lanes = (rows + 1) * kL;  // of a solve
-  const int s_first = parts > 1 ? (int)blockIdx.x / parts : (int)blockIdx.x * slots;
+  const int lanes = z.per * kL;  // of a solve
+  const int s_first = (int)blockIdx.x * slots;
   const int nsl = min(slots, b.nsolves - s_first);
-  const int first_row = parts > 1 ? ((int)blockIdx.x - s_first * parts) * rows : 0;
   const int sl = lane / lanes < nsl ? lane / lanes : 0, s = s_first + sl;
-  const int vl = (lane - sl * lanes) / kL;  // 0: t
-  const int part = lane % kL;               // this lane's nodes: part, part + kL, ..
-  const bool mine = lane / lanes < nsl && (vl == 0 || first_row + vl < z.per);
-  const int v = mine && vl > 0 ? first_row + vl : 0;
+  const int part = lane % kL;  // this lane's nodes: part, part + kL, ..
+  const bool mine = lane / lanes < nsl;
+  const int v = mine ? (lane - sl * lanes) / kL : 0;  // 0: t
   extern __shared__ double sm[];
   const int cap = n * 32;
   double *const Y = sm + lane, *const F = Y + cap;
@@ -559,7 +554,7 @@ __global__ void __launch_bounds__(32) ft_kernel(Geometry g, SolveBatch b, ft::Ve
   if (mine)
 #pragma unroll 4
     for (int i = 0; i < n; ++i) Y[32 * i] = io[(size_t)i * vs];
-  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, s_nan, 1, first_row == 0 ? 0 : LLONG_MAX, eig_fail);
+  ft::load_t(n, tri, s_first, nsl, shift, Dg, Eg, s_row, s_nan, 1, 0, eig_fail);
   const int nb = kPW / slots;  // nodes per batch: pair (slot, node) = slot + slots * node
   int nmax = 0;
   for (int q = 0; q < nsl; ++q) nmax = max(nmax, ft::g_count[s_row[q]]);
@@ -835,7 +830,7 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
       };
       if (core)
         run(reflect_kernel<kFirst, true, kL>);
-      else
+      else if constexpr (kL > 1)  // (at least two lanes: below)
         run(reflect_kernel<kFirst, false, kL>);
     });
   };
@@ -852,7 +847,7 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
   // 324 warps 122 / 123 / 143 / 188, 1296 warps 210 / 205 / 190 / 204, 2500 warps 321 /
   // 293 / 289 / 283; lr: 324 warps 73 / 92 / 122 / 198, 2500 warps 289 / 281 / 293 /
   // 365; of 40 members, 144 000 warps in eleven launches, lr 70.9 / 62.9 / 59.2 / 63.0 ms.
-  const long long warps = ((long long)b.nsolves * per + 31) / 32;  // (never INT_MAX)
+  const long long warps = ((long long)b.nsolves * per + 31) / 32;
   auto lanes_for = [&](int w8, int w4, int w2) {
     return warps < w8 ? 8 : warps < w4 ? 4 : warps < w2 ? 2 : 1;
   };
@@ -872,19 +867,17 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
     return;
   }
   int lf = lanes_for(400, 700, 2000);
-  const int lr = lanes_for(700, 2000, INT_MAX);
+  const int lr = warps < 700 ? 8 : warps < 2000 ? 4 : 2;
   // a solve's vectors have to fit a warp, nearly filling it
   while (lf > 1 && (per * lf > 32 || 32 % (per * lf) > 4)) lf /= 2;
-  const int parts = (per + 29) / 31, rows = (per - 1 + parts - 1) / parts;
   reflect(First(), per, lr);
   with(lf, [&](auto l) {
     constexpr int kL = decltype(l)::value;
-    const int sl = 32 / ((rows + 1) * kL);
-    const unsigned grid =
-        parts > 1 ? (unsigned)b.nsolves * parts : (unsigned)((b.nsolves + sl - 1) / sl);
+    const int sl = 32 / (per * kL);
+    const unsigned grid = (unsigned)((b.nsolves + sl - 1) / sl);
     auto run = [&](auto kernel, int pairs) {
       const size_t doubles = (3 * 32 + 2 * (size_t)pairs) * n + 2 * (size_t)sl * n;
-      kernel<<<grid, 32, smem_of(kernel, doubles), stream>>>(g, b, z, sl, rows, parts, tri, eig_fail);
+      kernel<<<grid, 32, smem_of(kernel, doubles), stream>>>(g, b, z, sl, tri, eig_fail);
     };
     // factors of 32 (solve, node) pairs at a time; from 57 members on that leaves an SM
     // two warps where 16 pairs leave three: 129 600 solves of 64 members 23.4 / 22.4 ms
