@@ -8,6 +8,7 @@ import pytest
 
 from test_gpu_ft import _check
 from test_gpu_gram64 import LG_ERR_EIG, _batch, _case, _reference
+from test_gpu_parity import RTOL_ANALYSIS, _rel_err, _run_both
 
 pytestmark = pytest.mark.gpu
 
@@ -435,3 +436,131 @@ def test_entries_of_solves_redone_in_fp64_count_once():
         ctx.letkf_final()
         assert 0.0 < np.abs(yb).max() < 100.0 * scale
     assert n[0] > 0 and n[0] == n[1]
+
+
+@pytest.mark.parametrize("k", [24, 40, 41, 64])
+def test_a_later_chunk_left_to_the_fp64_kernel(k):
+    """A list whose second chunk (896 kept entries make one) has values below 2^-400 after
+    the first has been written: the whole solve is redone.  With a NaN there, the solve
+    fails and its neighbours do not."""
+    rng = np.random.default_rng(60 + k)
+    good, late, nan = _case(rng, k, 1500), list(_case(rng, k, 1500)), list(_case(rng, k, 1500))
+    late[0] = late[0].copy()
+    late[0][896:] *= 2.0 ** -450
+    nan[0] = nan[0].copy()
+    nan[0][1300, 2] = np.nan
+    st, tr, wb = _batch([good, tuple(late), good], 1.05)
+    assert st == 0
+    for c, t, w in zip((good, late, good), tr, wb):
+        t0, w0 = _reference(*c, 1.05)
+        assert np.allclose(t, t0, rtol=1e-11, atol=1e-11)
+        assert np.allclose(w, w0, rtol=1e-11, atol=1e-11)
+    st, tr2, wb2 = _batch([good, tuple(nan), good], 1.05)
+    assert st == LG_ERR_EIG and np.isnan(tr2[1]).all()
+    for i in (0, 2):
+        assert np.array_equal(tr2[i], tr[i]) and np.array_equal(wb2[i], wb[i])
+
+
+@pytest.mark.parametrize("k", [9, 33, 40])
+def test_core_lanes_by_launch_size(k):
+    """Launches of 30, 100, 225, 900 and 6500 warps of vectors: 8, 4, 2, 1 and 1 lanes per
+    vector in the matrix kernel, 8, 8, 4, 2 and 1 in the reflections.  A solve's result does
+    not depend on the launch it is in."""
+    rng = np.random.default_rng(k)
+    base = [_case(rng, k, p) for p in (0, 5, 3 * k, 2)]
+    first = None
+    for warps in (30, 100, 225, 900, 6500):
+        nb = warps * 32 // k
+        st, tr, wb = _batch([base[i % 4] for i in range(nb)], 1.05)
+        assert st == 0
+        if first is None:
+            first = tr[:4], wb[:4]
+            for c, t, w in zip(base, tr, wb):
+                _check(c, 1.05, t, w)
+        for i in range(4):
+            assert (tr[i::4] == first[0][i]).all() and (wb[i::4] == first[1][i]).all()
+
+
+@pytest.mark.parametrize("nz,vcoord", [(7, 0), (8, 0), (32, 0), (8, 1), (300, 0)])
+def test_observations_at_and_around_half_levels(nz, vcoord):
+    """Observations exactly on a half level, one and a few roundings (FP64 and FP32) beside
+    it, above the top and below the ground: nz = 7 and 8 around the line from which the
+    levels are passed in FP32, 300 beyond the 256 levels that are.  H(x) against the
+    oracle's with the tolerance of the other H(x) tests, and every profile's levels both
+    ascending and descending (the search index persists)."""
+    import letkf_gb300 as lg
+    import synth
+    from oracle import oracle as orc
+    cfg = lg.preset("tiny3d").replace(nz=nz, vcoord=vcoord, ens=33, n_obs=10)
+    w = synth.make_workload(cfg)
+    w.xb[:, :, 0] = 0.0
+    w.axb[:, :, 0] = 98765.0
+    # temperatures that jump between levels, so that a wrong level shows
+    rng = np.random.default_rng(nz)
+    w.axb[:, :, 1:] += 50.0 * rng.standard_normal(w.axb[:, :, 1:].shape)
+    a, b, p0, ptop = lg.vertical_coord(cfg)
+    if vcoord == lg.LG_VCOORD_SIGMA:
+        lev = a * (98765.0 - ptop) + ptop
+    else:
+        lev = a * (p0 - ptop) + b * (98765.0 - ptop) + ptop
+    half = 0.5 * (lev[1:] + lev[:-1])
+    ph = [half, half * (1 + 2.0 ** -52), half * (1 - 2.0 ** -52), half * (1 + 2.0 ** -24),
+          half * (1 - 2.0 ** -24), half * (1 + 1e-6), half * (1 - 1e-6), [1.0, 2e5]]
+    ph = np.concatenate(ph)
+    n, onz = 400, 4
+    ph = rng.choice(ph, (n, onz))
+    ph[::2].sort(axis=1)
+    lat, lon = synth.obs_locations(cfg, rng, n)
+    obs = lg.ObsSet([(onz, 2, [1, 3])], np.zeros(n, np.int32), lat, lon, ph.ravel(),
+                    rng.standard_normal(n * onz * 2), np.ones(n * onz * 2))
+    ctx = lg.Letkf(cfg)
+    ctx.set_obs(obs)
+    xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+    ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+    o = orc.Oracle(cfg, obs)
+    yb_o, dis_o, _ = o.hx(w.xb, w.axb)
+    yb, dis = ctx.hx(o.n_entries)
+    ctx.letkf_final()
+    assert np.allclose(yb, yb_o, rtol=1e-12, atol=1e-12 * np.abs(yb_o).max())
+    assert np.allclose(dis, dis_o, rtol=1e-12, atol=1e-12 * np.abs(dis_o).max())
+
+
+@pytest.mark.parametrize("nz,ens", [(5, 16), (5, 33), (8, 33), (24, 16), (24, 33)])
+def test_analysis_lanes_by_launch_size(nz, ens, monkeypatch):
+    """Analyses of 500, 800 and 2400 warps of vectors: 4, 2 and 1 lanes per vector in the
+    solves, 8, 4 and 2 in the reflections (2-D analyses of this grid: 8 and 8), against the
+    QL route (a sweep limit below the default selects it) with the path's tolerance."""
+    import letkf_gb300 as lg
+    import synth
+    cfg = lg.preset("tiny3d").replace(nz=nz, ens=ens)
+    w = synth.make_workload(cfg)
+    out = []
+    for limit in (None, "59"):
+        if limit:
+            monkeypatch.setenv("LETKF_GB300_QL_ITERS", limit)
+        ctx = lg.Letkf(cfg)
+        ctx.set_obs(w.obs)
+        xa, axa = np.zeros_like(w.xb), np.zeros_like(w.axb)
+        ctx.letkf_run(0, w.xb, w.axb, xa, axa)
+        assert (ctx.stats()["ms_ql"] > 0.1) == bool(limit)  # the two routes
+        ctx.letkf_final()
+        out.append(xa + axa[..., None])
+    i = slice(cfg.halo, -cfg.halo)
+    inc = np.abs(out[1] - (w.xb + w.axb[..., None]))[i, i].max()
+    assert np.abs(out[0] - out[1])[i, i].max() <= 1e-10 * inc
+
+
+def test_rotation_log_overflow_above_64_members(monkeypatch):
+    """96 members take the QL route: with a log of one octet every solve overflows and is
+    redone by the accumulating solver, whose rounding differs from the replay's."""
+    out = []
+    for cap in (None, "5"):
+        if cap:
+            monkeypatch.setenv("LETKF_GB300_ROT_CAP", cap)
+        cfg, w, ctx, o, got, ref = _run_both("tiny3d", ens=96)
+        assert _rel_err(cfg, w, got, ref[:2]) < RTOL_ANALYSIS
+        assert ctx.stats()["n_eig_fail"] == 0
+        ctx.letkf_final()
+        out.append(got[0][cfg.halo:-cfg.halo, cfg.halo:-cfg.halo])
+    differ = (out[0] != out[1]).any(axis=(2, 3))
+    assert differ.all()  # in every column
