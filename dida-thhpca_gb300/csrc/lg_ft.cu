@@ -785,8 +785,11 @@ __global__ void __launch_bounds__(128) add_wbar_kernel(int n, SolveBatch b, cons
 
 bool ft_supported(const Geometry& g) {
   // below 7 members the tridiagonal form does not fit the Gram matrix's place;
-  // a lowered sweep limit asks for the QL iteration
-  return g.ens >= 7 && g.ens <= 64 && (g.ql_max_iter == 0 || g.ql_max_iter >= 60);
+  // a lowered sweep limit asks for the QL iteration; a shift (k - 1) / rho far from any
+  // inflation in use would leave FP32's range in load_t and the nodes' in factor
+  const double shift = (double)(g.ens - 1) / g.inflation;
+  return g.ens >= 7 && g.ens <= 64 && (g.ql_max_iter == 0 || g.ql_max_iter >= 60) &&
+         shift > 0x1p-100 && shift < 0x1p100;
 }
 
 size_t ft_vec_doubles(const Geometry& g) {

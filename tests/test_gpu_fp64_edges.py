@@ -564,3 +564,16 @@ def test_rotation_log_overflow_above_64_members(monkeypatch):
         out.append(got[0][cfg.halo:-cfg.halo, cfg.halo:-cfg.halo])
     differ = (out[0] != out[1]).any(axis=(2, 3))
     assert differ.all()  # in every column
+
+
+@pytest.mark.parametrize("rho", [1e-300, 1e-12, 1e12, 1e200])
+def test_any_inflation(rho):
+    """(k - 1) / rho far below or above a full-rank C: W is (C / (k - 1) + I / rho)^(-1/2)."""
+    rng = np.random.default_rng(8)
+    k, p = 12, 90
+    case = (rng.standard_normal((p, k)), np.ones(p, np.float32), rng.standard_normal(p), np.ones(p))
+    st, tr, wb = _batch([case], rho)
+    assert st == 0
+    t0, w0 = _reference(*case, rho)
+    assert np.allclose(wb[0], w0, rtol=1e-9, atol=1e-9 * np.abs(w0).max())
+    assert np.allclose(tr[0], t0, rtol=1e-9, atol=1e-9 * np.abs(t0).max())
