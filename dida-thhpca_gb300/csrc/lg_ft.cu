@@ -846,7 +846,9 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
   // 4 / 2 / 1: 20 warps 312 / 315 / 324 / 346, 160 warps 349 / 322 / 326 / 344, 320
   // warps 411 / 374 / 354 / 371, 640 warps 520 / 446 / 423 / 408; with lr: 160 warps
   // 285 / 291 / 320 / 369, 640 warps 456 / 410 / 423 / 463, 2880 warps 1479 / 1277 /
-  // 1204 / 1252, 41 000 warps 18.9 / 15.8 / 14.5 / 14.1 ms.  Analysis of 16 members, lf:
+  // 1204 / 1252, 41 000 warps 18.9 / 15.8 / 14.5 / 14.1 ms.  At 16, 28, 52 and 64 members
+  // and 10 to 12 000 warps the same lines stay within 5 % of the best of the four (9 % at
+  // 16 members and 450 warps).  Analysis of 16 members, lf:
   // 324 warps 122 / 123 / 143 / 188, 1296 warps 210 / 205 / 190 / 204, 2500 warps 321 /
   // 293 / 289 / 283; lr: 324 warps 73 / 92 / 122 / 198, 2500 warps 289 / 281 / 293 /
   // 365; of 40 members, 144 000 warps in eleven launches, lr 70.9 / 62.9 / 59.2 / 63.0 ms.
@@ -878,14 +880,21 @@ void launch_ft(const Geometry& g, const SolveBatch& b, bool core, double* t, con
     constexpr int kL = decltype(l)::value;
     const int sl = 32 / (per * kL);
     const unsigned grid = (unsigned)((b.nsolves + sl - 1) / sl);
-    auto run = [&](auto kernel, int pairs) {
-      const size_t doubles = (3 * 32 + 2 * (size_t)pairs) * n + 2 * (size_t)sl * n;
-      kernel<<<grid, 32, smem_of(kernel, doubles), stream>>>(g, b, z, sl, tri, eig_fail);
+    auto doubles = [&](int pairs) {
+      return (3 * 32 + 2 * (size_t)pairs) * n + 2 * (size_t)sl * n;
     };
-    // factors of 32 (solve, node) pairs at a time; from 57 members on that leaves an SM
-    // two warps where 16 pairs leave three: 129 600 solves of 64 members 23.4 / 22.4 ms
-    // at 32 / 16, 921 600 of 40 members 55.0 / 61.2
-    if (n > 56)
+    auto run = [&](auto kernel, int pairs) {
+      kernel<<<grid, 32, smem_of(kernel, doubles(pairs)), stream>>>(g, b, z, sl, tri, eig_fail);
+    };
+    // Factors of 32 (solve, node) pairs at a time, or 16 where 32 leave an SM two warps and
+    // 16 leave three (228 KB, a KB and the kernel's 160 bytes a block; with four state
+    // rows from 55 members on).  Transform of 129 600 solves, ms at 32 / 16: 40 members
+    // 6.70 / 7.31, 48 10.1 / 10.4 (three warps / four), 52 11.0 / 13.5, 56 15.9 / 15.0,
+    // 64 18.9 / 18.0.
+    auto warps_per_sm = [&](int pairs) {
+      return (int)((228 << 10) / (sizeof(double) * doubles(pairs) + 1024 + 160));
+    };
+    if (warps_per_sm(32) <= 2 && warps_per_sm(16) > warps_per_sm(32))
       run(ft_kernel<kL, 16>, 16);
     else
       run(ft_kernel<kL, 32>, 32);

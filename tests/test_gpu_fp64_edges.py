@@ -577,3 +577,11 @@ def test_any_inflation(rho):
     t0, w0 = _reference(*case, rho)
     assert np.allclose(wb[0], w0, rtol=1e-9, atol=1e-9 * np.abs(w0).max())
     assert np.allclose(tr[0], t0, rtol=1e-9, atol=1e-9 * np.abs(t0).max())
+
+
+@pytest.mark.parametrize("name,ens", [("tiny3d", 54), ("tiny3d", 55), ("tiny3d", 56), ("tiny2d", 55)])
+def test_pairs_factored_at_a_time(name, ens, monkeypatch):
+    """With four state rows 32 (solve, node) pairs are factored at a time up to 54 members and
+    16 from 55 on: both sides against the QL route, tolerance of the path."""
+    from test_gpu_ft import test_analysis_against_the_ql_route as against_ql
+    against_ql(name, ens, monkeypatch)
