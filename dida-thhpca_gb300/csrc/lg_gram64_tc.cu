@@ -12,7 +12,9 @@
 // |z| of the chunk (below a power of two 2^S), and Z is cut into six signed
 // 9-bit digits,
 //   z = 2^(S-53) Z,   Z = sum_a d_a 2^(45-9a),   -256 <= d_a <= 256,
-// which are exact in FP16.  A product of digits has at most 16 bits and a
+// which are exact in FP16 (the error-free splitting of K. Ozaki, T. Ogita, S. Oishi and S. M.
+// Rump, "Error-free transformations of matrix multiplication by using fast routines of matrix
+// multiplication and its applications", Numerical Algorithms 59, 2012).  A product of digits has at most 16 bits and a
 // tcgen05.mma accumulator holds 24 exactly, so the FP32 sums of up to 256
 // entries are exact integers; they are combined in 64-bit integers.  Pairs of
 // slices (a, b) with a + b >= 7 (below 2^-63 of the largest product) are left
@@ -58,7 +60,7 @@
 // operand and one buffer at 40 members left the MMAs waiting for the sums to be
 // taken out, and each sum's conversion to integers (16 lanes a cycle and SM) is
 // kept to four or five per element.  Measured alone against gram64_kernel: 921 600
-// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 93 ms (126 with
+// solves of 40 members and 379 entries (of 1562 candidates) 727 -> 92 ms (126 with
 // two slices per operand); 82 944 of 40 members, 24 entries 5.6 -> 2.7 ms; 2592 of
 // 16 members, 51 entries 0.18 -> 0.08 ms; 129 600 of 64 members, 954 entries 595 ->
 // 48 ms.  It wins at every size, so up to 64 members there is no other path.

@@ -297,7 +297,7 @@ void launch_eig_apply(const Geometry& g, const SolveBatch& b, const double* C, c
                       double* trans, double* wbar, int* eig_fail, cudaStream_t stream);
 size_t eig2_tri_doubles(int n);
 // FP64 transform without eigenvalues (lg_ft.cu), 7 to 64 members: tridiagonal
-// form in the Gram matrices' place (lg_tri.cu: D | E | H | reflectors), then the state
+// form in the Gram matrices' place (lg_tri.cu: D | E | G | reflectors), then the state
 // rows' update (core false, as launch_eig2's vectors; vec: ft_vec_doubles per
 // solve of scratch) or explicit trans and overline_w (core true, as
 // launch_eig_apply's modes 1 and cubes; vec: trans).  t is overwritten.
