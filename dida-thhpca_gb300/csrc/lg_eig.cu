@@ -363,7 +363,9 @@ void launch_eig_apply(const Geometry& g, const SolveBatch& b, const double* C, c
   const int n = g.ens;
   const int LD = n | 1;
   const size_t smem = sizeof(double) * ((size_t)n * LD + 6 * n + 8);
-  const int grid = b.solve_list || b.left ? std::min(b.nsolves, 152 * 6) : b.nsolves;
+  const int grid = b.left ? std::min(b.nsolves, 152)
+                   : b.solve_list ? std::min(b.nsolves, 152 * 6)
+                                  : b.nsolves;
   if (n <= 64) {
     // one warp per matrix: the QL rotations are broadcast by shuffles, no block barriers
     allow_smem(eig_apply_kernel<32>, smem);

@@ -297,9 +297,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
   __shared__ int s_wcnt[2][kPWarps];
   __shared__ longlong2 s_t[kThree ? 3 : 2][64];
   __shared__ int s_kmax, s_dmax, s_nf;
-  // entries with weight: of the finished solves, of the present one (gram64_kernel counts
-  // those of a solve left to it)
-  __shared__ int s_work, s_solve;
+  __shared__ int s_before[kPThreads];  // a weighing thread's count before the present solve
   __shared__ volatile int s_abort;
   __shared__ int s_stop[2];  // s_abort as the weighing and the adding warps agree on it
   __shared__ QueueHead s_head[kDepth];
@@ -319,7 +317,6 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       tc::mbar_init(&m_empty[i], kXWarps + 1 + kDWarps);
     }
     s_abort = 0;
-    s_work = s_solve = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // the operand buffers' rows that stay zero: zero slices, members above k, the
@@ -363,6 +360,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     const long long one_bits = __double_as_longlong(g.vert_dist);
     // (a product differs by less than two roundings from the quotient)
     const double inv_vd = 1.0 / g.vert_dist;
+    int work = 0;     // entries with weight
     unsigned nq = 0;  // queues filled so far
     // 1: a queue is filled; 0: the solve is left to gram64_kernel; -1: stop
     auto fill = [&](int s, int64_t base, int p, double al, int& scan, bool& first) -> int {
@@ -375,10 +373,6 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         s_kmax = 0;
         s_dmax = 0;
         s_nf = 0;
-        if (first) {
-          s_work += s_solve;
-          s_solve = 0;
-        }
         s_stop[0] = s_abort;
       }
       bar_sync(kBarP, kPThreads);
@@ -506,14 +500,13 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
           qd[q] = __double_as_longlong(d);
         }
       }
-      cnt = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+      work += cnt;
       kmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)kmax);
       dmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)dmax);
       nf = __any_sync(0xffffffffu, nf);
       if (lane == 0) {
         atomicMax(&s_kmax, kmax);
         atomicMax(&s_dmax, dmax);
-        atomicAdd(&s_solve, cnt);
         if (nf) s_nf = 1;
       }
       bar_sync(kBarP, kPThreads);
@@ -550,10 +543,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
         // 32 (|D| + bias) and the sign in the top bit, as digits_of leaves Z
         qd[q] = ((dq & 0x7fffffffffffffffll) + bias()) * 32 | (dq & (1ll << 63));
       }
-      if (tid == 0) {
-        s_head[qb] = QueueHead{s, qr / kStage, S, Sd, first ? 1 : 0, bad ? 1 : 0};
-        if (bad) s_solve = 0;
-      }
+      if (tid == 0) s_head[qb] = QueueHead{s, qr / kStage, S, Sd, first ? 1 : 0, bad ? 1 : 0};
+      if (bad) work = s_before[tid];  // gram64_kernel counts this solve's entries
       mbar_arrive(&m_full[qb]);
       ++nq;
       first = false;
@@ -574,6 +565,7 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
       int scan = 0;
       bool first = true;
       int r = 1;
+      s_before[tid] = work;
       do {
         r = fill(s, base, p, al, scan, first);
       } while (r > 0 && scan < p);
@@ -583,7 +575,8 @@ __global__ void __launch_bounds__(g64::kThreads, 1)
     if (nq >= kDepth) wait(&m_empty[qb], (nq / kDepth - 1) & 1);
     if (tid == 0) s_head[qb] = QueueHead{-1, 0, 0, 0, 0, 0};
     mbar_arrive(&m_full[qb]);
-    if (b.work && tid == 0) atomicAdd(b.work, (unsigned long long)(s_work + s_solve));
+    work = (int)__reduce_add_sync(0xffffffffu, (unsigned)work);
+    if (b.work && lane == 0 && work) atomicAdd(b.work, (unsigned long long)work);
   } else {
     // ================= the issuing warp
     const uint64_t desc0 = tc::make_desc(tc::smem_u32(smem_raw), 128, 256);
