@@ -1535,7 +1535,7 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
         lg::launch_gram_tc_stream(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, rec, st);
       else
         lg::launch_gram64(geo, c->hx, c->lists, b, axb, !cube_trans_fp32(c) && lg::ft_supported(geo),
-                          L.C, L.t, c->d_status, st);
+                          L.C, L.t, c->d_status, st, L.ovf_n);
       CK(record_event(kv[1], st));
       CK(record_event(kv[2], st));
       if (cube_trans_fp32(c)) {
@@ -1556,7 +1556,6 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
         CK(record_event(kv[6], st));
         launches += 5;
       } else if (lg::ft_supported(geo)) {
-        CK(cudaMemsetAsync(L.ovf_n, 0, sizeof(int), st));
         lg::launch_tridiag_in_place(geo, b.nsolves, L.C, L.ovf_list, L.ovf_n, st);
         CK(record_event(kv[3], st));
         for (int e = 4; e < 6; ++e) CK(record_event(kv[e], st));
@@ -1665,8 +1664,9 @@ int enqueue_analysis(lg_ctx* c, const double* xb, const double* axb, double* xa,
     else if (mixed_tc)
       lg::launch_gram_tc(geo, c->hx, c->lists, b, axb, L.C, L.t, c->d_status, s_g, &rec);
     else
-      lg::launch_gram64(geo, c->hx, c->lists, b, axb, c->use_ft, L.C, L.t, c->d_status, s_g);
-    CK(cudaMemsetAsync(L.ovf_n, 0, sizeof(int), s_g));
+      lg::launch_gram64(geo, c->hx, c->lists, b, axb, c->use_ft, L.C, L.t, c->d_status, s_g,
+                        L.ovf_n);
+    if (!c->use_ft) CK(cudaMemsetAsync(L.ovf_n, 0, sizeof(int), s_g));
     CK(record_event(kv[1], s_g));
     if (nl >= 3) {
       CK(cudaEventRecord(c->ev_phase[0][set], s_g));

@@ -30,7 +30,7 @@ constexpr int kGramThreads = 256;
 template <int kMaxBlk>
 __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
     gram64_kernel(Geometry g, HxDev hx, ListDev l, SolveBatch b, const double* axb,
-                  double* Cout, double* tout, int marked) {
+                  double* Cout, double* tout, int marked, int* clear) {
   constexpr int kQueueCap = kTE + kGramThreads;
   const int k = g.ens;
   const int kp = (k + 3) & ~3;
@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
   __shared__ int q_n;
   __shared__ double s_al;
 
+  if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
   // marked = 0: block s does solve s.  marked = 1 (after gram64_tc_kernel):
   // block i looks at solves 256 i .. 256 i + 255 and does those that kernel
   // left to this one.
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kGramThreads, kMaxBlk == 1 ? 3 : 1)
 
 void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
                    const double* axb, bool lower, double* C, double* t, int* err,
-                   cudaStream_t stream) {
+                   cudaStream_t stream, int* clear) {
   if (b.nsolves == 0) return;
   // up to 64 members: exact slices on the tensor cores, then the solves they
   // cannot hold (non-finite or extreme values) here
@@ -259,9 +260,9 @@ void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const S
     const size_t red = sizeof(double) * (size_t)(G - 1) * NB * 16;
     const size_t smem = std::max(tile, red);
     allow_smem(gram64_kernel<1>, smem);
-    gram64_kernel<1><<<grid, kGramThreads, smem, stream>>>(g, hx, l, b, axb, C, t, marked);
+    gram64_kernel<1><<<grid, kGramThreads, smem, stream>>>(g, hx, l, b, axb, C, t, marked, clear);
   } else {
-    gram64_kernel<3><<<grid, kGramThreads, tile, stream>>>(g, hx, l, b, axb, C, t, marked);
+    gram64_kernel<3><<<grid, kGramThreads, tile, stream>>>(g, hx, l, b, axb, C, t, marked, clear);
   }
 }
 

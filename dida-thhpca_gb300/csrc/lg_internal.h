@@ -223,10 +223,11 @@ void launch_scan_counts(const int* cnt, int64_t* off, int n, void* tmp, size_t t
                         cudaStream_t stream);
 size_t scan_tmp_bytes(int n);
 // FP64 Gram matrices and projections: exact slices on the tensor cores up to 64
-// members (lg_gram64_tc.cu; mode 0 needs hx.yexp), the FP64 pipe otherwise
+// members (lg_gram64_tc.cu; mode 0 needs hx.yexp), the FP64 pipe otherwise.  *clear, where
+// given, is set to zero on the way (a launch less).
 void launch_gram64(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
                    const double* axb, bool lower, double* C, double* t, int* err,
-                   cudaStream_t stream);
+                   cudaStream_t stream, int* clear = nullptr);
 bool gram64_tc_supported(int ens);
 void launch_gram64_tc(const Geometry& g, const HxDev& hx, const ListDev& l, const SolveBatch& b,
                       const double* axb, bool lower, double* C, double* t, int* err,
